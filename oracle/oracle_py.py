@@ -23,7 +23,7 @@ REFERENCE_TREE = "/root/reference"
 def build():
     subprocess.run(["make", "-s", "-C", _DIR], check=True)
     # the reference's own FCM and barrier sources, where the FilSim tree is present
-    if os.path.isdir(REFERENCE_TREE):
+    if os.path.isfile(os.path.join(REFERENCE_TREE, "FCMfunctions.cpp")):
         subprocess.run(["make", "-s", "-C", os.path.join(_DIR, "refshim"), "REF=" + REFERENCE_TREE], check=True)
 
 

@@ -9,8 +9,10 @@
 //      stencil reaches the tile (mono_and_dipole_force_distribution, :596-646);
 //      each lane owns grid points and sums in registers (FP32: Kahan-compensated,
 //      on packed f32x2 pairs): no atomics, bit-reproducible.
-//   3. cuFFT R2C (batched x3), 4. k_project / k_project_planes: the Stokes
-//      projection of flow_solve (:648-736), 5. cuFFT C2R (batched x3).
+//   3.-5. the forward transforms, the Stokes projection of flow_solve (:648-736) and
+//      the inverse transforms: the line transforms (fs_lines.cuh) on grids whose
+//      lengths they take, the warp transform (fs_fft.cu) on the largest FP32 ones,
+//      otherwise cuFFT with k_project / k_project_planes between.
 //   6. k_interp: one warp per bead (in spread-bin order for L2 locality)
 //      reduces U and Omega over the stencil (particle_velocities :740-770,
 //      particle_rotations :774-808) with warp shuffles.
@@ -979,10 +981,18 @@ fs_status ensure_plans(fs_ctx *c, int prec) {
   return FS_OK;
 }
 
+// the grid runs this library's transforms (fs_lines.cuh) at this precision; else cuFFT
+bool own_transform(const fs_ctx *c, int prec) {
+  return c->line_tw[prec][0] && (prec == FS_PREC_FP64 || c->tune_fft32 == 0);
+}
+
 template <typename R>
 fs_status flow_solve_t(fs_ctx *c) {
   const int prec = sizeof(R) == 8 ? FS_PREC_FP64 : FS_PREC_FP32;
-  if (prec == FS_PREC_FP32 && c->fft_tw && c->tune_fft32 == 0) return fft32_flow_solve(c);
+  if (own_transform(c, prec)) {
+    if (prec == FS_PREC_FP64) return lines_flow_solve64(c);
+    return fft32_preferred(c) ? fft32_flow_solve(c) : lines_flow_solve32(c);
+  }
   FS_TRY(ensure_plans(c, prec));
   cufftResult r;
   {
@@ -1119,8 +1129,10 @@ fs_status fcm_init(fs_ctx *c) {
   c->nbins = c->nbin[0] * c->nbin[1] * c->nbin[2];
   c->last_grid_prec = -1;
   FS_CUDA(cudaMalloc(&c->grid_real, sizeof(double) * 3 * c->N));
-  FS_CUDA(cudaMalloc(&c->grid_cplx, sizeof(double2) * 3 * c->NH));
-  c->bytes += sizeof(double) * 3 * c->N + sizeof(double2) * 3 * c->NH;
+  // the line transforms round their rows of nz / 2 + 1 values up to even
+  const size_t ncplx = 3 * (size_t)c->nx * c->ny * ((c->nzh + 1) & ~1);
+  FS_CUDA(cudaMalloc(&c->grid_cplx, sizeof(double2) * ncplx));
+  c->bytes += sizeof(double) * 3 * c->N + sizeof(double2) * ncplx;
   FS_TRY(fs_sort_alloc(&c->bins, c->nbins, c->max_beads, &c->bytes));
   FS_CUDA(cudaMalloc(&c->bead_sw, sizeof(int) * 3 * (size_t)(c->max_beads > 0 ? c->max_beads : 1)));
   c->bytes += sizeof(int) * 3 * (size_t)c->max_beads;
@@ -1170,7 +1182,21 @@ fs_status fcm_init(fs_ctx *c) {
   c->tune_spread_cols = 2;  // 2 x 16 x 8 blocks: fs_autotune's choice at 384^3 and 512^3
   c->tune_interp_wpb = 8;
   c->tune_fft32 = 0;
+  if (lines_supported(c)) {
+    FS_TRY(lines_init64(c));
+    FS_TRY(lines_init32(c));
+  }
   return fft32_init(c);
+}
+
+bool lines_supported(const fs_ctx *c) {
+  auto len = [](int n) {
+    static const int ok[] = {32, 48, 64, 80, 96, 112, 128, 144, 160, 192, 224, 256, 320, 384, 448, 512};
+    for (int v : ok)
+      if (n == v) return true;
+    return false;
+  };
+  return len(c->nx) && len(c->ny) && len(c->nz);
 }
 
 void fcm_free(fs_ctx *c) {
@@ -1184,6 +1210,10 @@ void fcm_free(fs_ctx *c) {
   cudaFree(c->grid_cplx);
   c->grid_real = c->grid_cplx = nullptr;
   fft32_free(c);
+  for (int p = 0; p < 2; ++p) {
+    cudaFree(c->line_tw[p][0]);  // the three axes' tables are one allocation
+    for (int a = 0; a < 3; ++a) c->line_tw[p][a] = nullptr;
+  }
   fs_sort_free(&c->bins);
   cudaFree(c->bead_sw);
   c->bead_sw = nullptr;
@@ -1193,7 +1223,7 @@ void fcm_free(fs_ctx *c) {
 
 fs_status fcm_set_stream(fs_ctx *c, cudaStream_t st) {
   const int prec = c->precision;
-  if (prec == FS_PREC_FP32 && c->fft_tw && c->tune_fft32 == 0) return FS_OK;  // the warp FFT uses no cuFFT plan
+  if (own_transform(c, prec)) return FS_OK;  // no cuFFT plan
   FS_TRY(ensure_plans(c, prec));
   if (cufftSetStream(c->plan_fwd[prec], st) != CUFFT_SUCCESS) return FS_ERR_CUFFT;
   if (cufftSetStream(c->plan_inv[prec], st) != CUFFT_SUCCESS) return FS_ERR_CUFFT;

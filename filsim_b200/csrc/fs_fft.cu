@@ -740,6 +740,16 @@ fs_status x_project(fs_ctx *c, float2 *B, const float2 *tw) {
 // line lengths of the warp transforms: 2^p in [lo, 512], or 96, 192, 384
 static bool fft_len(int n, int lo) { return n >= lo && (pow2_in(n, lo, 512) || n == 96 || n == 192 || n == 384); }
 
+// Where the warp transform is the faster one: 512-point x lines of the largest boxes,
+// whose contiguous x pass it does in 0.73 ms at 512^3 against 1.05 ms for the strided
+// one of the line transforms, more than its z passes lose (3.50 against 3.77 ms in all).
+// At 512 x 512 x 256 and 512 x 256 x 512 the two are equal (1.87, 1.89 and 1.82, 1.82 ms),
+// below them the line transforms lead (512 x 512 x 128: 0.99 against 1.08 ms, 384^3: 1.69
+// against 1.97 ms, 256^3: 0.50 against 0.57 ms, 384 x 96 x 96: 0.15 against 0.24 ms).
+bool fft32_preferred(const fs_ctx *c) {
+  return c->fft_tw && c->nx == 512 && (size_t)c->ny * c->nz > 512 * 256;
+}
+
 bool fft32_supported(const fs_ctx *c) { return fft_len(c->nx, 32) && fft_len(c->ny, 32) && fft_len(c->nz, 64); }
 
 fs_status fft32_init(fs_ctx *c) {

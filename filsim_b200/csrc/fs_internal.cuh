@@ -73,6 +73,7 @@ struct fs_ctx {
   int tune_spread_cols;   // FP32 spread: x width of a warp's column block (2, 4 or 8)
   int tune_interp_wpb;    // beads (warps) per interpolation CTA: 4, 8 or 16
   int tune_fft32;         // FP32 power-of-two grids: 0 warp FFT (fs_fft.cu), 1 cuFFT
+  void *line_tw[2][3];  // [precision][axis]: tables of the line transforms (fs_lines.cuh; null: not a supported grid)
   void *fft_tw;        // FP32 transform twiddle tables (null: grid not handled by fs_fft.cu, cuFFT is used)
 
   // collision cells
@@ -199,7 +200,7 @@ void prof_flush(fs_ctx *c);
 struct ProfScope {
   fs_ctx *c;
   int slot;
-  ProfScope(fs_ctx *ctx, int stage) : c(ctx), slot(prof_begin(ctx, stage)) {}
+  ProfScope(fs_ctx *ctx, int stage, bool on = true) : c(ctx), slot(on ? prof_begin(ctx, stage) : -1) {}
   ~ProfScope() { prof_end(c, slot); }
 };
 
@@ -217,7 +218,14 @@ fs_status fcm_spread_only(fs_ctx *c, const double *Y, const double *F, const dou
 fs_status fcm_interpolate_only(fs_ctx *c, const double *u, const double *Y, int np, double *V, double *W);
 void slab_free(fs_ctx *c);
 
+bool lines_supported(const fs_ctx *c);  // every axis has a length of the line transforms (fs_lines.cuh)
+fs_status lines_init64(fs_ctx *c);
+fs_status lines_init32(fs_ctx *c);
+fs_status lines_flow_solve64(fs_ctx *c);
+fs_status lines_flow_solve32(fs_ctx *c);
+
 bool fft32_supported(const fs_ctx *c);
+bool fft32_preferred(const fs_ctx *c);  // FP32: the warp transform rather than the line transforms
 fs_status fft32_init(fs_ctx *c);
 void fft32_free(fs_ctx *c);
 fs_status fft32_flow_solve(fs_ctx *c);

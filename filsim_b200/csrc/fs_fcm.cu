@@ -4,17 +4,18 @@
 //   1. k_fcm_bin_keys + counting sort: beads binned by the 16-point tile that
 //      holds the start of their Gaussian stencil (gaussian_setup's index rule,
 //      FCMfunctions.cpp:565-589).
-//   2. k_spread (FP64) / k_spread_records32 + k_spread32 (FP32 chain): CTAs over
-//      16^3 grid tiles gather the monopole + rotlet Gaussians of every bead whose
-//      stencil reaches the tile (mono_and_dipole_force_distribution, :596-646);
-//      each lane owns grid points and sums in registers (FP32: Kahan-compensated,
-//      on packed f32x2 pairs): no atomics, bit-reproducible.
+//   2. k_records64 + k_spread64 (FP64) / k_spread_records32 + k_spread32 (FP32 chain):
+//      CTAs over 16^3 grid tiles (FP64: half tiles) gather the monopole + rotlet
+//      Gaussians of every bead whose stencil reaches them
+//      (mono_and_dipole_force_distribution, :596-646); each lane owns grid points and
+//      sums in registers (FP32: Kahan-compensated, on packed f32x2 pairs): no
+//      atomics, bit-reproducible.
 //   3.-5. the forward transforms, the Stokes projection of flow_solve (:648-736) and
 //      the inverse transforms: the line transforms (fs_lines.cuh) on grids whose
 //      lengths they take, the warp transform (fs_fft.cu) on the largest FP32 ones,
 //      otherwise cuFFT with k_project / k_project_planes between.
-//   6. k_interp: one warp per bead (in spread-bin order for L2 locality)
-//      reduces U and Omega over the stencil (particle_velocities :740-770,
+//   6. k_interp64 / k_interp_q: one warp (or more) per bead (in spread-bin order for L2
+//      locality) reduces U and Omega over the stencil (particle_velocities :740-770,
 //      particle_rotations :774-808) with warp shuffles.
 // FP64 mode follows the reference arithmetic; FP32 mode keeps grids, FFTs and
 // weights in float, with Kahan-compensated spread sums and FP64 accumulation of
@@ -66,233 +67,268 @@ __global__ void k_fcm_bin_keys(const double *__restrict__ Y, int np, FcmConsts c
 }
 
 // ---- 2. spread ----------------------------------------------------------------
-// One CTA (16 warps) per 16^3 grid tile; the tile is cut into 2x2x8 blocks and
-// warp w owns the 8 blocks of column (bx, bz) = (w/2, w%2), one grid point per
-// lane. Candidate beads (stencil start in the tile's bin or the one before it,
-// per axis) are staged as per-axis weight tables indexed by tile coordinate
-// (zero outside the bead's stencil). Each warp builds, by ballots, the set of
-// staged beads that reach its column and, per block, those that reach the
-// block; every lane then sums those beads' contributions to its point in
-// registers, in sorted bead order, and writes the point once. No atomics and no
-// shared-memory read-modify-write; bit-reproducible. FP32 mode keeps Kahan
-// compensated register sums.
-#define FS_SPREAD_THREADS 512
+// Both precisions first write one record per bead in sorted (bin) order: its stencil
+// starts, F, T/2 and the Gaussian weights of its ngd stencil indices per axis
+// (gaussian_setup, FCMfunctions.cpp:565-589), read by the spread and the interpolation.
+//
+// FP64 record (double4 units): [0] stencil starts and bead id (four ints), F0, F1;
+// [1] F2, h0, h1, h2 (h = T / 2, GA_setup :536-547); then (g, d, r, r d) of axis a and
+// stencil index i at 2 + a ngd + i.
+__host__ __device__ inline int rec64_len(int ngd) { return 2 + 3 * ngd; }
 
-template <typename R>
-struct W4 {
-  R g, d, r, pad;
-};
-
-// CH beads are staged per pass (32 or 64, chosen per grid by fs_autotune)
-template <typename R, int CH>
-struct SpreadStage {
-  W4<R> w[CH][3][FS_TILE];  // weights by tile-local coordinate
-  R f[CH][4];                // force
-  R th[CH][4];               // half torque (GA_setup, :536-547)
-  unsigned mask[CH][3];      // per axis: tile-local coordinates covered
-};
-
-template <typename R>
-struct KAcc;
-template <>
-struct KAcc<double> {
-  double s;
-  __device__ void init() { s = 0.0; }
-  __device__ void add(double v) { s += v; }
-  __device__ double value() const { return s; }
-};
-template <>
-struct KAcc<float> {
-  float s, c;
-  __device__ void init() { s = 0.f; c = 0.f; }
-  __device__ void add(float v) {
-    float y = v - c;
-    float t = s + y;
-    c = (t - s) - y;
-    s = t;
+__global__ void k_records64(const double *__restrict__ Y, const double *__restrict__ F, const double *__restrict__ T,
+                            const int *__restrict__ sorted, const int *__restrict__ bead_sw, int np, FcmConsts c,
+                            double4 *__restrict__ rec) {
+  const int ngd = c.ngd, RL = rec64_len(ngd);
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (long long)np * RL) return;
+  const int q = (int)(t / RL), e = (int)(t - (long long)q * RL);
+  const int b = sorted[q];
+  double4 v;
+  if (e == 0) {
+    v.x = __hiloint2double(bead_sw[3 * b + 1], bead_sw[3 * b]);
+    v.y = __hiloint2double(b, bead_sw[3 * b + 2]);
+    v.z = F ? F[3 * b] : 0.0;
+    v.w = F ? F[3 * b + 1] : 0.0;
+  } else if (e == 1) {
+    v.x = F ? F[3 * b + 2] : 0.0;
+    v.y = T ? 0.5 * T[3 * b] : 0.0;
+    v.z = T ? 0.5 * T[3 * b + 1] : 0.0;
+    v.w = T ? 0.5 * T[3 * b + 2] : 0.0;
+  } else {
+    const int a = (e - 2) / ngd, i = (e - 2) - a * ngd;
+    const double Yv = Y[3 * b + a];
+    const int xg = (int)(Yv / c.dx) - c.ngdh + (i + 1);
+    const double xx = ((double)xg) * c.dx - Yv;
+    v.x = c.anorm * exp(-xx * xx / c.anorm2);
+    v.y = c.anormdip * exp(-xx * xx / c.anormdip2);
+    v.z = -xx / c.sigmadipsq;
+    v.w = v.z * v.y;
   }
-  __device__ float value() const { return s - c; }
+  rec[t] = v;
+}
+
+// The candidate bins of a tile per axis: its own and the ones before it that a stencil
+// reaches (fs_cand_bins: K per axis), in the order (x, y, z); combination r < K^3 names, by
+// its digit p of each axis, the bin K - 1 - p before the tile's own (empty when it would
+// repeat a bin on an axis with fewer than K bins).
+struct Cand {
+  int rs[27], len[27];
 };
-
-template <typename R>
-__device__ inline R fs_exp(R x);
-template <>
-__device__ inline double fs_exp<double>(double x) { return exp(x); }
-template <>
-__device__ inline float fs_exp<float>(float x) { return expf(x); }
-
-template <typename R, int CH>
-__global__ void __launch_bounds__(FS_SPREAD_THREADS)
-    k_spread(const double *__restrict__ Y, const double *__restrict__ F, const double *__restrict__ T,
-             const int *__restrict__ bin_start, const int *__restrict__ sorted, const int *__restrict__ bead_sw,
-             FcmConsts c, R *__restrict__ fgrid) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  SpreadStage<R, CH> &st = *reinterpret_cast<SpreadStage<R, CH> *>(smem_raw);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int tile = blockIdx.x;
-  const int tz = tile % c.nbin[2], ty = (tile / c.nbin[2]) % c.nbin[1], tx = tile / (c.nbin[2] * c.nbin[1]);
-  const int X0[3] = {tx * FS_TILE, ty * FS_TILE, tz * FS_TILE};
-  // candidate bins per axis: the tile's own bin and the ones before it that a
-  // stencil reaches (fs_cand_bins), each bin once on an axis with fewer bins
-  int cb[3][3], ncb[3];
-  const int tb[3] = {tx, ty, tz};
-  const int K = fs_cand_bins(c.ngd);
+__device__ __forceinline__ void cand_bins(Cand &cd, int tx, int ty, int tz, const int *__restrict__ bin_start,
+                                          const FcmConsts &c) {
+  const int K = fs_cand_bins(c.ngd), r = threadIdx.x;
+  if (r >= K * K * K) return;
+  const int tb[3] = {tx, ty, tz}, pick[3] = {r / (K * K), (r / K) % K, r % K};
+  int bin = 0;
+  bool valid = true;
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    ncb[d] = min(K, c.nbin[d]);
-    for (int j = 0; j < ncb[d]; ++j) cb[d][j] = wrap_int(tb[d] - (ncb[d] - 1 - j), c.nbin[d]);
+    const int back = K - 1 - pick[d];
+    valid = valid && back < c.nbin[d];
+    bin = bin * c.nbin[d] + wrap_int(tb[d] - back, c.nbin[d]);
   }
-  int rs[27], re[27], nr = 0, total = 0;
-  for (int a = 0; a < ncb[0]; ++a)
-    for (int b2 = 0; b2 < ncb[1]; ++b2)
-      for (int e = 0; e < ncb[2]; ++e) {
-        int bin = (cb[0][a] * c.nbin[1] + cb[1][b2]) * c.nbin[2] + cb[2][e];
-        rs[nr] = bin_start[bin];
-        re[nr] = bin_start[bin + 1];
-        total += re[nr] - rs[nr];
-        nr++;
-      }
-  // this lane's point in block (bx, by, bz): x = 2bx + (lane&1), y = 2by + ((lane>>1)&1), z = 8bz + (lane>>2)
-  const int bx = warp >> 1, bz = warp & 1;
-  const int px = 2 * bx + (lane & 1), pyo = (lane >> 1) & 1, pz = 8 * bz + (lane >> 2);
-  const size_t N = (size_t)c.N[0] * c.N[1] * c.N[2];
-  const int ngd = c.ngd;
-  for (int base = 0; base < total; base += CH) {
-    const int nb = min(CH, total - base);
-    __syncthreads();  // the previous chunk's tables are no longer read
-    // stage: one half-warp per (bead slot, axis), lane l -> tile-local coordinate l
-    const int nitems = nb * 3 * FS_TILE;
-    for (int it0 = warp * 32; it0 < nitems; it0 += FS_SPREAD_THREADS) {
-      const int it = it0 + lane;
-      const bool act = it < nitems;
-      const int s = act ? it / (3 * FS_TILE) : 0;
-      const int a = act ? (it / FS_TILE) % 3 : 0;
-      const int l = it % FS_TILE;
-      bool valid = false;
-      W4<R> wv = {(R)0, (R)0, (R)0, (R)0};
-      int bead = 0;
-      if (act) {
-        int rank = base + s, r = 0;
-        while (rank >= re[r] - rs[r]) {
-          rank -= re[r] - rs[r];
-          ++r;
-        }
-        bead = sorted[rs[r] + rank];
-        const int Nn = c.N[a];
-        // tile-local l holds stencil index i = (l + X0 - sw) mod N if i < ngd
-        const int i = wrap_near(l + wrap_near(X0[a] - bead_sw[3 * bead + a], Nn), Nn);
-        if (i < ngd) {
-          valid = true;
-          const double Yv = Y[3 * bead + a];
-          const int xc = (int)(Yv / c.dx);
-          const int xg = xc - c.ngdh + (i + 1);
-          const double xx = ((double)xg) * c.dx - Yv;
-          if (sizeof(R) == 8) {
-            wv.g = (R)(c.anorm * exp(-xx * xx / c.anorm2));
-            wv.d = (R)(c.anormdip * exp(-xx * xx / c.anormdip2));
-            wv.r = (R)(-xx / c.sigmadipsq);
-          } else {
-            const R xf = (R)xx;
-            wv.g = (R)c.anorm * fs_exp<R>(-xf * xf / (R)c.anorm2);
-            wv.d = (R)c.anormdip * fs_exp<R>(-xf * xf / (R)c.anormdip2);
-            wv.r = -xf / (R)c.sigmadipsq;
-          }
-        }
-        st.w[s][a][l] = wv;
-      }
-      const unsigned bal = __ballot_sync(0xffffffffu, valid);
-      if (act && l == 0) {
-        st.mask[s][a] = (bal >> (lane & 16)) & 0xffffu;
-        if (a == 0)
-          for (int d = 0; d < 3; ++d) {
-            st.f[s][d] = (R)F[3 * bead + d];
-            st.th[s][d] = (R)(0.5 * T[3 * bead + d]);
-          }
-      }
+  cd.rs[r] = valid ? bin_start[bin] : 0;
+  cd.len[r] = valid ? bin_start[bin + 1] - bin_start[bin] : 0;
+}
+// record of candidate q of the tile
+__device__ __forceinline__ int cand_slot(const Cand &cd, int q) {
+  int r = 0;
+  while (q >= cd.len[r]) {
+    q -= cd.len[r];
+    ++r;
+  }
+  return cd.rs[r] + q;
+}
+
+// FP64 spread: one CTA (8 warps) per half tile of 8 x 16 x 16 points (ZL = 8; a quarter of 8 x
+// 16 x 8 with ZL = 4). Warp w owns the 2 x 16 x ZL points x in {2 (w & 3), +1}, z in
+// [ZL (w >> 2), +ZL); a lane owns one x, one y and the ZL z, 3 ZL sums in registers. Per
+// staged bead that reaches the warp's points the lane forms the eight x-y factors of
+//   f0 = F0 gx gy . gz + h2 ry dx dy . dz - h1 dx dy . rz dz
+//   f1 = F1 gx gy . gz - h2 rx dx dy . dz + h0 dx dy . rz dz
+//   f2 = F2 gx gy . gz + (h1 rx - h0 ry) dx dy . dz
+// (mono_and_dipole_force_distribution, FCMfunctions.cpp:596-646, regrouped) and adds eight
+// FMAs per point of the covered z quads, the z weights broadcast from shared memory. The
+// candidates that reach the CTA are listed first, 256 at a time, then staged CH at a time in
+// that (sorted) order, the sums kept throughout: no atomics, each point written once,
+// bit-reproducible. Bound by issue at 24 warps per SM (80 registers): 1.63 ms at 512^3 /
+// 131,072 beads and 0.30 ms at 256^3 / 30,720, where one grid point per lane with the
+// Gaussians recomputed per tile took 2.38 and 0.52; without the list, every candidate
+// staged, 1.83 and 0.36; at 128 registers and 16 warps per SM 1.83, 0.32.
+#define FS_SPREAD64_THREADS 256
+constexpr int SPREAD64_CH = 32;  // beads staged at a time (64, at two CTAs per SM: 1.85 against 1.63 ms at 512^3)
+template <int ZL>
+struct SpreadStage64 {
+  static constexpr int CH = SPREAD64_CH;
+  double xg[CH][8], xd[CH][8], xr[CH][8];
+  double yg[CH][FS_TILE], yd[CH][FS_TILE], yr[CH][FS_TILE];
+  double2 zgd[CH][2 * ZL];  // (g, d)
+  double zrd[CH][2 * ZL];   // r d
+  double2 f[CH][3];         // (F0, F1), (F2, h0), (h1, h2)
+  // the beads of one batch of candidates that reach the CTA: record, covered x (8 bits) |
+  // covered z (2 ZL bits) << 16
+  int list[FS_SPREAD64_THREADS];
+  unsigned lmask[FS_SPREAD64_THREADS];
+  int count[FS_SPREAD64_THREADS / 32];
+};
+// points l < width from X0 on an axis of N points that a stencil of ngd from sw covers
+__device__ __forceinline__ unsigned cover_mask(int X0, int sw, int N, int ngd, int width) {
+  const int s0 = wrap_near(X0 - sw, N);  // stencil index of l = 0
+  unsigned m = s0 < ngd ? (1u << (ngd - s0)) - 1u : 0u;
+  if (N - s0 < width) m |= ((1u << ngd) - 1u) << (N - s0);
+  return m & ((1u << width) - 1u);
+}
+
+template <int ZL>
+__global__ void __launch_bounds__(FS_SPREAD64_THREADS, ZL == 4 ? 4 : 3)
+    k_spread64(const int *__restrict__ bin_start, const double4 *__restrict__ rec, FcmConsts c,
+               double *__restrict__ fgrid) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int CH = SPREAD64_CH;
+  typedef SpreadStage64<ZL> Stage;
+  Stage &st = *reinterpret_cast<Stage *>(smem_raw);
+  __shared__ Cand cd;
+  constexpr int ZP = FS_TILE / (2 * ZL), ZT = 2 * ZL / 8;  // CTAs along a tile's z; z entries per staging thread
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int part = blockIdx.x % (2 * ZP), tile = blockIdx.x / (2 * ZP);
+  const int tz = tile % c.nbin[2], ty = (tile / c.nbin[2]) % c.nbin[1], tx = tile / (c.nbin[2] * c.nbin[1]);
+  const int X0[3] = {tx * FS_TILE + 8 * (part & 1), ty * FS_TILE, tz * FS_TILE + 2 * ZL * (part >> 1)};
+  cand_bins(cd, tx, ty, tz, bin_start, c);
+  __syncthreads();
+  const int ngd = c.ngd, RL = rec64_len(ngd), K = fs_cand_bins(ngd), nr = K * K * K;
+  int total = 0;
+  for (int r = 0; r < nr; ++r) total += cd.len[r];
+  const int xp = warp & 3, zh = warp >> 2, yl = lane & 15, xl = 2 * xp + (lane >> 4);
+  double acc[ZL][3];
+#pragma unroll
+  for (int z = 0; z < ZL; ++z) acc[z][0] = acc[z][1] = acc[z][2] = 0.0;
+  // candidates 256 at a time: those whose stencil reaches the CTA's points, in order
+  for (int q0 = 0; q0 < total; q0 += FS_SPREAD64_THREADS) {
+    int slot = 0;
+    unsigned msk = 0;
+    if (q0 + tid < total) {
+      slot = cand_slot(cd, q0 + tid);
+      const double2 hd = *reinterpret_cast<const double2 *>(rec + (size_t)slot * RL);
+      const unsigned mx = cover_mask(X0[0], __double2loint(hd.x), c.N[0], ngd, 8);
+      const unsigned my = cover_mask(X0[1], __double2hiint(hd.x), c.N[1], ngd, FS_TILE);
+      const unsigned mz = cover_mask(X0[2], __double2loint(hd.y), c.N[2], ngd, 2 * ZL);
+      if (mx && my && mz) msk = mx | (mz << 16);
+    }
+    const unsigned hit = __ballot_sync(0xffffffffu, msk != 0);
+    if (lane == 0) st.count[warp] = __popc(hit);
+    __syncthreads();  // counts; and the previous list and tables are no longer read
+    int nhit = 0, at = 0;
+#pragma unroll
+    for (int w = 0; w < FS_SPREAD64_THREADS / 32; ++w) {
+      const int k = st.count[w];
+      if (w < warp) at += k;
+      nhit += k;
+    }
+    if (msk) {
+      at += __popc(hit & ((1u << lane) - 1u));
+      st.list[at] = slot;
+      st.lmask[at] = msk;
     }
     __syncthreads();
-    // beads reaching this warp's column (its x pair and z octet)
-    unsigned col[CH / 32];
+    for (int base = 0; base < nhit; base += CH) {
+      const int nb = min(CH, nhit - base);
+      if (base) __syncthreads();  // the previous tables are no longer read
+      // eight threads per slot: thread j takes x = j, y in {j, j + 8}, z likewise
+      for (int sl = tid >> 3; sl < nb; sl += FS_SPREAD64_THREADS / 8) {
+        const int j = tid & 7;
+        const double4 *rw = rec + (size_t)st.list[base + sl] * RL;
+        const double4 hd = rw[0];
+        const int swv[3] = {__double2loint(hd.x), __double2hiint(hd.x), __double2loint(hd.y)};
+        constexpr int NE = 3 + ZT;
+        double4 w[NE];
 #pragma unroll
-    for (int h = 0; h < CH / 32; ++h) {
-      const int s = 32 * h + lane;
-      unsigned mx = 0, mz = 0;
-      if (s < nb) {
-        mx = st.mask[s][0];
-        mz = st.mask[s][2];
+        for (int it = 0; it < NE; ++it) {
+          const int a = it == 0 ? 0 : it < 3 ? 1 : 2, l = j + 8 * (it == 2 || it == 4), Nn = c.N[a];
+          const int i = wrap_near(l + wrap_near(X0[a] - swv[a], Nn), Nn);
+          w[it] = i < ngd ? rw[2 + a * ngd + i] : make_double4(0.0, 0.0, 0.0, 0.0);
+        }
+        if (j < 3) {
+          const double4 h1 = rw[1];
+          st.f[sl][j] = j == 0 ? make_double2(hd.z, hd.w) : j == 1 ? make_double2(h1.x, h1.y) : make_double2(h1.z, h1.w);
+        }
+        st.xg[sl][j] = w[0].x;
+        st.xd[sl][j] = w[0].y;
+        st.xr[sl][j] = w[0].z;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          st.yg[sl][j + 8 * h] = w[1 + h].x;
+          st.yd[sl][j + 8 * h] = w[1 + h].y;
+          st.yr[sl][j + 8 * h] = w[1 + h].z;
+        }
+#pragma unroll
+        for (int h = 0; h < ZT; ++h) {
+          st.zgd[sl][j + 8 * h] = make_double2(w[3 + h].x, w[3 + h].y);
+          st.zrd[sl][j + 8 * h] = w[3 + h].w;
+        }
       }
-      col[h] = __ballot_sync(0xffffffffu, ((mx >> (2 * bx)) & 3u) && ((mz >> (8 * bz)) & 0xffu));
-    }
-    const W4<R> *wxp = &st.w[0][0][px];
-    const W4<R> *wzp = &st.w[0][2][pz];
-    // two passes of four y pairs; per bead the x and z factors and the rotlet cross
-    // terms are formed once per pass, each y row then needs one weight load:
-    //   f_a += F_a gx gy gz + (T/2 x grad)_a gdx gdy gdz, regrouped by y
-#pragma unroll 1
-    for (int half = 0; half < 2; ++half) {
-      KAcc<R> acc[4][3];
+      __syncthreads();
+      // staged beads reaching this warp's points
+      static_assert(CH == 32, "one ballot covers the staged beads");
+      const unsigned mm = lane < nb ? st.lmask[base + lane] : 0u;
+      unsigned m = __ballot_sync(0xffffffffu, ((mm >> (2 * xp)) & 3u) && ((mm >> (16 + ZL * zh)) & ((1u << ZL) - 1u)));
+      while (m) {
+        const int sl = __ffs(m) - 1;
+        m &= m - 1;
+        const unsigned zm = st.lmask[base + sl] >> (16 + ZL * zh);
+        const double gx = st.xg[sl][xl], dx = st.xd[sl][xl], rx = st.xr[sl][xl];
+        const double gy = st.yg[sl][yl], dy = st.yd[sl][yl], ry = st.yr[sl][yl];
+        const double2 f01 = st.f[sl][0], f2h0 = st.f[sl][1], h12 = st.f[sl][2];
+        const double p = gx * gy, q = dx * dy;
+        const double a0 = f01.x * p, a1 = f01.y * p, a2 = f2h0.x * p;
+        const double b0 = h12.y * ry * q, b1 = -h12.y * rx * q, b2 = (h12.x * rx - f2h0.y * ry) * q;
+        const double c0 = -h12.x * q, c1 = f2h0.y * q;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        acc[q][0].init();
-        acc[q][1].init();
-        acc[q][2].init();
-      }
+        for (int k = 0; k < ZL / 4; ++k) {
+          if (ZL == 4 || ((zm >> (4 * k)) & 0xfu)) {
 #pragma unroll
-      for (int h = 0; h < CH / 32; ++h) {
-        unsigned m = col[h];
-        while (m) {
-          const int s = 32 * h + __ffs(m) - 1;
-          m &= m - 1;
-          const unsigned my = (st.mask[s][1] >> (8 * half)) & 0xffu;  // y pairs 4 half .. 4 half + 3
-          if (my == 0) continue;
-          const W4<R> wx = wxp[s * 3 * FS_TILE], wz = wzp[s * 3 * FS_TILE];
-          const R F0 = st.f[s][0], F1 = st.f[s][1], F2 = st.f[s][2];
-          const R h0 = st.th[s][0], h1 = st.th[s][1], h2 = st.th[s][2];
-          const R gxz = wx.g * wz.g, dxz = wx.d * wz.d;
-          const R f0 = F0 * gxz, f1 = F1 * gxz, f2 = F2 * gxz;
-          const R h2d = h2 * dxz, h0d = h0 * dxz;
-          const R c0 = -h1 * wz.r * dxz, c1 = (-h2 * wx.r + h0 * wz.r) * dxz, c2 = h1 * wx.r * dxz;
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            if ((my >> (2 * q)) & 3u) {
-              const W4<R> wy = st.w[s][1][2 * (4 * half + q) + pyo];
-              acc[q][0].add(f0 * wy.g + (h2d * wy.r + c0) * wy.d);
-              acc[q][1].add(f1 * wy.g + c1 * wy.d);
-              acc[q][2].add(f2 * wy.g + (c2 - h0d * wy.r) * wy.d);
+            for (int z = 4 * k; z < 4 * k + 4; ++z) {
+              const double2 gd = st.zgd[sl][ZL * zh + z];
+              const double rd = st.zrd[sl][ZL * zh + z];
+              acc[z][0] += a0 * gd.x + (b0 * gd.y + c0 * rd);
+              acc[z][1] += a1 * gd.x + (b1 * gd.y + c1 * rd);
+              acc[z][2] += a2 * gd.x + b2 * gd.y;
             }
           }
         }
       }
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int py = 2 * (4 * half + q) + pyo;
-        const size_t m0 = ((size_t)(X0[0] + px) * c.N[1] + (X0[1] + py)) * c.N[2] + (X0[2] + pz);
-        if (base == 0) {
-          fgrid[m0] = acc[q][0].value();
-          fgrid[N + m0] = acc[q][1].value();
-          fgrid[2 * N + m0] = acc[q][2].value();
-        } else {  // more candidates than one chunk: add in chunk order
-          fgrid[m0] += acc[q][0].value();
-          fgrid[N + m0] += acc[q][1].value();
-          fgrid[2 * N + m0] += acc[q][2].value();
-        }
-      }
     }
   }
-  if (total == 0)
-    for (int by = 0; by < 8; ++by) {
-      const size_t m0 = ((size_t)(X0[0] + px) * c.N[1] + (X0[1] + 2 * by + pyo)) * c.N[2] + (X0[2] + pz);
-      fgrid[m0] = (R)0;
-      fgrid[N + m0] = (R)0;
-      fgrid[2 * N + m0] = (R)0;
-    }
+  // through shared memory, as many components at a time as the tables have room for, so
+  // that neighbouring lanes write whole rows of the CTA's z
+  constexpr int RP = ZL + 1;  // pairs per row: ZL and a pad
+  constexpr size_t ROWS = sizeof(double2) * 128 * RP;
+  static_assert(sizeof(Stage) >= ROWS, "the tables hold one component");
+  constexpr int NC = sizeof(Stage) >= 3 * ROWS ? 3 : 1;
+  const size_t N = (size_t)c.N[0] * c.N[1] * c.N[2];
+  double2 *T = reinterpret_cast<double2 *>(smem_raw);  // [component][128 (x, y)][RP]
+  double *out = fgrid + ((size_t)X0[0] * c.N[1] + X0[1]) * c.N[2] + X0[2] + 2 * (tid % ZL);
+#pragma unroll
+  for (int a0 = 0; a0 < 3; a0 += NC) {
+    __syncthreads();  // the tables, or the previous components, are no longer read
+#pragma unroll
+    for (int a = 0; a < NC; ++a)
+#pragma unroll
+      for (int z = 0; z < ZL; z += 2)
+        T[(128 * a + 16 * xl + yl) * RP + ZL / 2 * zh + z / 2] = make_double2(acc[z][a0 + a], acc[z + 1][a0 + a]);
+    __syncthreads();
+#pragma unroll
+    for (int a = 0; a < NC; ++a)
+#pragma unroll
+      for (int r = tid / ZL; r < 128; r += FS_SPREAD64_THREADS / ZL)
+        *reinterpret_cast<double2 *>(out + (a0 + a) * N + ((size_t)(r >> 4) * c.N[1] + (r & 15)) * c.N[2]) =
+            T[(128 * a + r) * RP + tid % ZL];
+  }
 }
 
 // ---- 2b. FP32 spread on packed pairs -------------------------------------------
-// The FP32 chain's spread. k_spread_records32 writes each bead's record once per
-// solve: stencil starts, F, T/2 and the weights (g, d, r, r d) per axis and
-// stencil index, with the FP32 arithmetic of k_spread<float> (gaussian_setup,
-// FCMfunctions.cpp:565-589: xx = xg dx - Y in double, then the float Gaussians).
+// The FP32 chain's spread. k_spread_records32 writes each bead's record with xx = xg dx - Y
+// in double and the Gaussians in float.
 // k_spread32 then runs one CTA (8 warps) per 16^3 tile, which stages tables of
 // the tile's candidate beads (by tile coordinate, from their records) and covers
 // its 16 column blocks in two passes; with the default 4 x 16 x 4 blocks, in
@@ -308,8 +344,8 @@ __global__ void __launch_bounds__(FS_SPREAD_THREADS)
 // per point (s + nc): no atomics, bit-reproducible.
 #define FS_SPREAD32_THREADS 256
 
-// Record of the bead in sorted slot q (float4 units): [0] stencil starts (int),
-// [1] F0, F1, F2, h0, [2] h1, h2, -, -, then (g, d, r, r d) for axis a and stencil
+// Record of the bead in sorted slot q (float4 units): [0] stencil starts and bead id
+// (int), [1] F0, F1, F2, h0, [2] h1, h2, -, -, then (g, d, r, r d) for axis a and stencil
 // index i at 3 + a ngd + i.
 __host__ __device__ inline int spread_rec_len(int ngd) { return 3 + 3 * ngd; }
 
@@ -324,7 +360,9 @@ __global__ void k_spread_records32(const double *__restrict__ Y, const double *_
   float4 v;
   if (e == 0) {
     v = make_float4(__int_as_float(bead_sw[3 * bead]), __int_as_float(bead_sw[3 * bead + 1]),
-                    __int_as_float(bead_sw[3 * bead + 2]), 0.f);
+                    __int_as_float(bead_sw[3 * bead + 2]), __int_as_float(bead));
+  } else if (e <= 2 && !F) {
+    v = make_float4(0.f, 0.f, 0.f, 0.f);
   } else if (e == 1) {
     v = make_float4((float)F[3 * bead], (float)F[3 * bead + 1], (float)F[3 * bead + 2], (float)(0.5 * T[3 * bead]));
   } else if (e == 2) {
@@ -377,30 +415,12 @@ __global__ void __launch_bounds__(FS_SPREAD32_THREADS, 3)
   const int tile = blockIdx.x;
   const int tz = tile % c.nbin[2], ty = (tile / c.nbin[2]) % c.nbin[1], tx = tile / (c.nbin[2] * c.nbin[1]);
   const int X0[3] = {tx * FS_TILE, ty * FS_TILE, tz * FS_TILE};
-  // candidate bins, the tile's own bin and the ones before it that a stencil
-  // reaches (fs_cand_bins: K per axis), in the order (x, y, z) of k_spread;
-  // thread r < K^3 reads combination r: per axis digit p in [0, K) names the bin
-  // K - 1 - p before the tile's own (empty when it would repeat a bin on an axis
-  // with fewer than K bins)
-  __shared__ int cand_rs[27], cand_len[27];
+  __shared__ Cand cd;
   const int K = fs_cand_bins(c.ngd), nr = K * K * K;
-  if (tid < nr) {
-    const int tb[3] = {tx, ty, tz};
-    const int pick[3] = {tid / (K * K), (tid / K) % K, tid % K};
-    int bin = 0;
-    bool valid = true;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      const int back = K - 1 - pick[d];
-      valid = valid && back < c.nbin[d];
-      bin = bin * c.nbin[d] + wrap_int(tb[d] - back, c.nbin[d]);
-    }
-    cand_rs[tid] = valid ? bin_start[bin] : 0;
-    cand_len[tid] = valid ? bin_start[bin + 1] - bin_start[bin] : 0;
-  }
+  cand_bins(cd, tx, ty, tz, bin_start, c);
   __syncthreads();
   int total = 0;
-  for (int r = 0; r < nr; ++r) total += cand_len[r];
+  for (int r = 0; r < nr; ++r) total += cd.len[r];
   const int ngd = c.ngd, RL = spread_rec_len(ngd);
   // staging of candidates [base, base + nb): tables by tile coordinate, eight
   // threads per bead slot (thread j takes x, y and z in {j, j + 8}), each reading
@@ -416,12 +436,7 @@ __global__ void __launch_bounds__(FS_SPREAD32_THREADS, 3)
       const bool act = sl < nb;
       bool cov[6] = {false, false, false, false, false, false};
       if (act) {
-        int q = base + sl, r = 0;
-        while (q >= cand_len[r]) {
-          q -= cand_len[r];
-          ++r;
-        }
-        const float4 *rw = rec + (size_t)(cand_rs[r] + q) * RL;
+        const float4 *rw = rec + (size_t)cand_slot(cd, base + sl) * RL;
         const float4 hd = __ldg(rw);
         if (j == 0) {
           st.fh[sl] = __ldg(rw + 1);
@@ -513,7 +528,7 @@ __global__ void __launch_bounds__(FS_SPREAD32_THREADS, 3)
           const float2 rz = *reinterpret_cast<const float2 *>(&st.zr[sl][zl]);
           const float4 fh = st.fh[sl];  // F0, F1, F2, h0 (h = T / 2, GA_setup :536-547)
           const float4 hh = st.hh[sl];  // h1, h2
-          // per z of the pair: f_a = F_a gx gz, the rotlet factors of k_spread (d = gdx gdz)
+          // per z of the pair: f_a = F_a gx gz, the rotlet factors (d = gdx gdz)
           const float gxz0 = wx.x * gz.x, gxz1 = wx.x * gz.y;
           const float dxz0 = wx.y * dz.x, dxz1 = wx.y * dz.y;
           const f2p f0 = f2_pack(fh.x * gxz0, fh.x * gxz1);
@@ -658,271 +673,258 @@ __global__ void k_project_planes(typename Cplx<R>::T *__restrict__ fh, size_t NH
 }
 
 // ---- 6. interpolation -------------------------------------------------------
-template <typename R>
-struct InterpWarp {
-  R g[3][FS_NGD_MAX], gd[3][FS_NGD_MAX], r[3][FS_NGD_MAX];
-  int ind[3][FS_NGD_MAX];
-};
-template <typename R>
-struct __align__(4 * sizeof(R)) XY4 {
-  R gg, dd, rx, ry;  // gx gy, gdx gdy, rx, ry of one (i, j) of the x-y stencil
-};
-// dynamic shared memory per warp: the per-axis tables, then per (i, j) the
-// products and the grid offset of (x_i, y_j, 0)
-template <typename R>
-__host__ __device__ constexpr size_t interp_xy_offset() {
-  return (sizeof(InterpWarp<R>) + 4 * sizeof(R) - 1) / (4 * sizeof(R)) * (4 * sizeof(R));
-}
-// rounded up to 32 bytes, so that every warp's tables and XY4 entries keep their
-// alignment also for odd ngd (ngd^2 (sizeof(XY4) + 8) is then an odd multiple of 8)
-template <typename R>
-__host__ __device__ constexpr size_t interp_warp_bytes(int ngd) {
-  return (interp_xy_offset<R>() + (size_t)ngd * ngd * (sizeof(XY4<R>) + sizeof(long long)) + 31) / 32 * 32;
-}
-
-// One warp per bead; lanes take the stencil points p = lane + 32 t (z fastest),
-// all 32 lanes busy. FP32 mode multiplies in FP32 and accumulates in FP64 per lane.
-template <typename R, int WPB>
-__global__ void __launch_bounds__(32 * WPB) k_interp(const R *__restrict__ u, const double *__restrict__ Y,
-                                                     const int *__restrict__ order, const int *__restrict__ bead_sw,
-                                                     int np, FcmConsts c, double *__restrict__ V,
-                                                     double *__restrict__ W) {
-  extern __shared__ __align__(32) unsigned char interp_smem[];
+// U and Omega of a bead from its stencil (particle_velocities :740-770,
+// particle_rotations :774-808): SPLIT warps per bead, in spread-bin order, weights from the
+// bead's record. interp_finish reduces the warps' lane sums (shuffles, then the bead's
+// warps in order) and writes; every thread of the CTA calls it.
+template <int WPB, int SPLIT>
+__device__ __forceinline__ void interp_finish(double (&v)[6], bool on, int b, double dx, double *__restrict__ V,
+                                              double *__restrict__ W) {
+  __shared__ double part[SPLIT > 1 ? WPB : 1][6];
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-  const int wid = blockIdx.x * WPB + wl;
-  if (wid >= np) return;
-  const int b = order[wid];
-  const int ngd = c.ngd, n2 = ngd * ngd, n3 = n2 * ngd;
-  unsigned char *base = interp_smem + (size_t)wl * interp_warp_bytes<R>(ngd);
-  InterpWarp<R> &s = *reinterpret_cast<InterpWarp<R> *>(base);
-  XY4<R> *xy = reinterpret_cast<XY4<R> *>(base + interp_xy_offset<R>());
-  long long *off = reinterpret_cast<long long *>(xy + n2);
-  for (int a = 0; a < 3; ++a) {  // lane i < ngd <= 20 takes stencil index i of each axis
-    const int i = lane;
-    if (i >= ngd) continue;
-    const double Yv = Y[3 * b + a];
-    const int xc = (int)(Yv / c.dx);
-    const int xg = xc - c.ngdh + (i + 1);
-    const int ix = bead_sw[3 * b + a] + i;  // (stencil start + i) mod N, as gaussian_setup's indx
-    s.ind[a][i] = ix >= c.N[a] ? ix - c.N[a] : ix;
-    const double xx = ((double)xg) * c.dx - Yv;
-    if (sizeof(R) == 8) {
-      s.g[a][i] = (R)(c.anorm * exp(-xx * xx / c.anorm2));
-      s.gd[a][i] = (R)(c.anormdip * exp(-xx * xx / c.anormdip2));
-      s.r[a][i] = (R)(-xx / c.sigmadipsq);
-    } else {
-      const R xf = (R)xx;
-      s.g[a][i] = (R)c.anorm * fs_exp<R>(-xf * xf / (R)c.anorm2);
-      s.gd[a][i] = (R)c.anormdip * fs_exp<R>(-xf * xf / (R)c.anormdip2);
-      s.r[a][i] = -xf / (R)c.sigmadipsq;
-    }
-  }
-  __syncwarp();
-  for (int ij = lane; ij < n2; ij += 32) {
-    const int i = ij / ngd, j = ij - i * ngd;
-    XY4<R> e;
-    e.gg = s.g[0][i] * s.g[1][j];
-    e.dd = s.gd[0][i] * s.gd[1][j];
-    e.rx = s.r[0][i];
-    e.ry = s.r[1][j];
-    xy[ij] = e;
-    off[ij] = ((long long)s.ind[0][i] * c.N[1] + s.ind[1][j]) * c.N[2];
-  }
-  __syncwarp();
-  const size_t N = (size_t)c.N[0] * c.N[1] * c.N[2];
-  const R *ux = u, *uy = u + N, *uz = u + 2 * N;
-  double v0 = 0, v1 = 0, v2 = 0, w0 = 0, w1 = 0, w2 = 0;
-  // point p = ij * ngd + k; a step of 32 points advances (ij, k) by (32 / ngd, 32 % ngd)
-  // (loads one point at a time: four points in flight per lane, at 64 registers,
-  // ran 0.97 ms at 512^3 against 0.72 ms for this loop; the gathers are bound by
-  // the load units, not by latency; the z tables packed into one float4 per index,
-  // three shared loads per point fewer, left it unchanged)
-  const int dij = 32 / ngd, dk = 32 - dij * ngd;
-  int ij = lane / ngd, k = lane - ij * ngd;
-  for (int p = lane; p < n3; p += 32) {
-    const XY4<R> e = xy[ij];
-    const long long m = off[ij] + s.ind[2][k];
-    const R temp = e.gg * s.g[2][k];    // (gx gy) gz, the reference's order
-    const R tempd = e.dd * s.gd[2][k];
-    const R zz = s.r[2][k];
-    const R a0 = ux[m], a1 = uy[m], a2 = uz[m];
-    v0 += (double)(a0 * temp);
-    v1 += (double)(a1 * temp);
-    v2 += (double)(a2 * temp);
-    w0 += (double)((a2 * e.ry - a1 * zz) * tempd);
-    w1 += (double)((a0 * zz - a2 * e.rx) * tempd);
-    w2 += (double)((a1 * e.rx - a0 * e.ry) * tempd);
-    k += dk;
-    ij += dij;
-    if (k >= ngd) {
-      k -= ngd;
-      ++ij;
-    }
-  }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    v0 += __shfl_xor_sync(0xffffffffu, v0, o);
-    v1 += __shfl_xor_sync(0xffffffffu, v1, o);
-    v2 += __shfl_xor_sync(0xffffffffu, v2, o);
-    w0 += __shfl_xor_sync(0xffffffffu, w0, o);
-    w1 += __shfl_xor_sync(0xffffffffu, w1, o);
-    w2 += __shfl_xor_sync(0xffffffffu, w2, o);
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int k = 0; k < 6; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+  if constexpr (SPLIT > 1) {
+    if (lane == 0)
+      for (int k = 0; k < 6; ++k) part[wl][k] = v[k];
+    __syncthreads();
+    if (wl % SPLIT == 0 && lane == 0)
+#pragma unroll
+      for (int w = 1; w < SPLIT; ++w)
+        for (int k = 0; k < 6; ++k) v[k] += part[wl + w][k];
   }
-  if (lane == 0) {
-    const double norm = c.dx * c.dx * c.dx;
-    V[3 * b + 0] = v0 * norm;
-    V[3 * b + 1] = v1 * norm;
-    V[3 * b + 2] = v2 * norm;
-    W[3 * b + 0] = -0.5 * w0 * norm;
-    W[3 * b + 1] = -0.5 * w1 * norm;
-    W[3 * b + 2] = -0.5 * w2 * norm;
+  if (on && wl % SPLIT == 0 && lane == 0) {
+    const double norm = dx * dx * dx;
+    for (int k = 0; k < 3; ++k) {
+      V[3 * b + k] = v[k] * norm;
+      W[3 * b + k] = -0.5 * v[3 + k] * norm;
+    }
   }
 }
 
+// FP64. A lane owns an aligned pair of z points and some of the stencil's y indices j, and
+// runs along x: per (j, pair) the eight sums over i
+//   Sg_c = sum gx u_c,  Sd_c = sum dx u_c (c = 0, 1, 2),  Sr_c = sum rx dx u_c (c = 1, 2)
+// need only the x weights, broadcast from shared memory, one FMA per point each; the y and
+// z weights are applied afterwards:
+//   V_c += gy gz Sg_c,  W0 += ry dy dz Sd_2 - dy rz dz Sd_1,
+//   W1 += dy rz dz Sd_0 - dy dz Sr_2,  W2 += dy dz Sr_1 - ry dy dz Sd_0.
+// The run of ngd points from zs touches P = (ngd + (zs & 1) + 1) / 2 pairs (a pair that a
+// short axis wraps onto twice has disjoint weights the two times); 32 / P rows j at once.
+// Bound by the latency of its gathers: 0.83 ms at 512^3 / 131,072 beads, 0.177 ms at 256^3 /
+// 30,720 (one point at a time with all weights from shared memory: 1.16, 0.26); with the
+// x-y products tabled per warp and the pairs walked across them 0.97, 0.21.
+struct InterpWarp64 {
+  double xg[FS_NGD_MAX], xd[FS_NGD_MAX], xr[FS_NGD_MAX];  // g, d, r d
+  double yg[FS_NGD_MAX], yd[FS_NGD_MAX], yr[FS_NGD_MAX];
+  long long xoff[FS_NGD_MAX];
+};
+template <int WPB, int SPLIT>
+__global__ void __launch_bounds__(32 * WPB) k_interp64(const double *__restrict__ u, const double4 *__restrict__ rec,
+                                                       int np, FcmConsts c, double *__restrict__ V,
+                                                       double *__restrict__ W) {
+  __shared__ InterpWarp64 sw[WPB];
+  const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+  const int slot = (blockIdx.x * WPB + wl) / SPLIT, ws = wl % SPLIT;
+  const bool on = slot < np;  // warp-uniform
+  InterpWarp64 &s = sw[wl];
+  double acc[6] = {0, 0, 0, 0, 0, 0};  // V, W
+  int b = 0;
+  if (on) {
+    const int ngd = c.ngd, Nz = c.N[2];
+    const double4 *rw = rec + (size_t)slot * rec64_len(ngd);
+    const double2 hd = *reinterpret_cast<const double2 *>(rw);
+    const int sx = __double2loint(hd.x), sy = __double2hiint(hd.x), zs = __double2loint(hd.y);
+    b = __double2hiint(hd.y);
+    rw += 2;
+    if (lane < ngd) {
+      const double4 x = rw[lane], y = rw[ngd + lane];
+      s.xg[lane] = x.x;
+      s.xd[lane] = x.y;
+      s.xr[lane] = x.w;
+      s.yg[lane] = y.x;
+      s.yd[lane] = y.y;
+      s.yr[lane] = y.w;
+      const int ix = sx + lane;
+      s.xoff[lane] = (long long)(ix >= c.N[0] ? ix - c.N[0] : ix) * c.N[1] * Nz;
+    }
+    const int odd = zs & 1, P = (ngd + odd + 1) >> 1, G = 32 / P;
+    const int pr = lane % P, g = lane / P;
+    double gz[2], dz[2], rz[2];
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      const int k = 2 * pr + t - odd;
+      const bool in = k >= 0 && k < ngd;
+      const double4 z = rw[2 * ngd + (in ? k : 0)];
+      gz[t] = in ? z.x : 0.0;
+      dz[t] = in ? z.y : 0.0;
+      rz[t] = in ? z.w : 0.0;
+    }
+    int z0 = zs - odd + 2 * pr;
+    if (z0 >= Nz) z0 -= Nz;
+    __syncwarp();
+    const size_t N = (size_t)c.N[0] * c.N[1] * Nz;
+    const int i0 = ws * ngd / SPLIT, i1 = (ws + 1) * ngd / SPLIT;
+    for (int j = g; j < ngd && g < G; j += G) {
+      const int iy = sy + j;
+      const double *base = u + (size_t)(iy >= c.N[1] ? iy - c.N[1] : iy) * Nz + z0;
+      double2 Sg[3], Sd[3], Sr[2];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) Sg[a] = Sd[a] = Sr[a < 2 ? a : 0] = make_double2(0.0, 0.0);
+      auto add = [](double2 &t, double w, const double2 &m) {
+        t.x += w * m.x;
+        t.y += w * m.y;
+      };
+#pragma unroll 4
+      for (int i = i0; i < i1; ++i) {
+        const double *q = base + s.xoff[i];
+        const double2 u0 = __ldg(reinterpret_cast<const double2 *>(q)),
+                      u1 = __ldg(reinterpret_cast<const double2 *>(q + N)),
+                      u2 = __ldg(reinterpret_cast<const double2 *>(q + 2 * N));
+        const double wg = s.xg[i], wd = s.xd[i], wr = s.xr[i];
+        add(Sg[0], wg, u0);
+        add(Sg[1], wg, u1);
+        add(Sg[2], wg, u2);
+        add(Sd[0], wd, u0);
+        add(Sd[1], wd, u1);
+        add(Sd[2], wd, u2);
+        add(Sr[0], wr, u1);
+        add(Sr[1], wr, u2);
+      }
+      const double yg = s.yg[j], yd = s.yd[j], yr = s.yr[j];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) acc[a] += yg * (gz[0] * Sg[a].x + gz[1] * Sg[a].y);
+      acc[3] += yr * (dz[0] * Sd[2].x + dz[1] * Sd[2].y) - yd * (rz[0] * Sd[1].x + rz[1] * Sd[1].y);
+      acc[4] += yd * ((rz[0] * Sd[0].x + rz[1] * Sd[0].y) - (dz[0] * Sr[1].x + dz[1] * Sr[1].y));
+      acc[5] += yd * (dz[0] * Sr[0].x + dz[1] * Sr[0].y) - yr * (dz[0] * Sd[0].x + dz[1] * Sd[0].y);
+    }
+  }
+  interp_finish<WPB, SPLIT>(acc, on, b, c.dx, V, W);
+}
 
-// FP32 interpolation with float4 gathers along z. The stencil's z run of ngd
-// points starting at zs lies in nq = ceil(((zs & 3) + ngd) / 4) aligned quads of
-// four points (a quad's first index is a multiple of 4; with Nz a multiple of 4 and
-// Nz >= ngd + 6 the quads of one run are distinct modulo Nz). A lane takes (ij,
-// quad) slots: one 16-byte load per component instead of four 4-byte ones, z weights
-// per quad position (zero off the run), the quad's four products summed in FP32
-// and the sum added in FP64. The products are k_interp<float>'s.
+// FP32, float4 gathers along z. The stencil's z run of ngd points starting at zs lies in
+// nq = ceil(((zs & 3) + ngd) / 4) aligned quads of four points (a quad that a short axis
+// wraps onto twice has disjoint weights the two times). A lane takes (ij, quad) slots: one
+// 16-byte load per component, z weights per quad position (zero off the run), the quad's
+// four products summed in FP32 and the sum added in FP64. 0.525 ms at 512^3 / 131,072
+// beads; the FP64 kernel's walk with packed FP32 pairs and FP64 flushes every four x
+// points: 0.62.
 constexpr int IQ_MAX = (FS_NGD_MAX + 6) / 4;  // quads a z run of ngd points can touch
 struct InterpQuad {
   float4 wg[IQ_MAX], wd[IQ_MAX], wr[IQ_MAX];  // g, gd, r of the quad's four points (0 off the run)
   int zq[IQ_MAX];                              // the quad's first z index
 };
-__host__ __device__ constexpr size_t interp_q_quad_offset() { return (sizeof(InterpWarp<float>) + 15) / 16 * 16; }
-__host__ __device__ constexpr size_t interp_q_xy_offset() {
-  return (interp_q_quad_offset() + sizeof(InterpQuad) + 15) / 16 * 16;
-}
+struct XY32 {
+  float gg, dd, rx, ry;  // gx gy, gdx gdy, rx, ry of one (i, j) of the x-y stencil
+};
+__host__ __device__ constexpr size_t interp_q_xy_offset() { return (sizeof(InterpQuad) + 15) / 16 * 16; }
 __host__ __device__ constexpr size_t interp_q_warp_bytes(int ngd) {
-  return (interp_q_xy_offset() + (size_t)ngd * ngd * (sizeof(XY4<float>) + sizeof(long long)) + 31) / 32 * 32;
+  return (interp_q_xy_offset() + (size_t)ngd * ngd * (sizeof(XY32) + sizeof(long long)) + 31) / 32 * 32;
 }
-inline bool interp_q_ok(const fs_ctx *c) { return c->nz % 4 == 0 && c->nz >= c->p.ngd + 6; }
 
-template <int WPB>
-__global__ void __launch_bounds__(32 * WPB) k_interp_q(const float *__restrict__ u, const double *__restrict__ Y,
-                                                       const int *__restrict__ order, const int *__restrict__ bead_sw,
+template <int WPB, int SPLIT>
+__global__ void __launch_bounds__(32 * WPB) k_interp_q(const float *__restrict__ u, const float4 *__restrict__ rec,
                                                        int np, FcmConsts c, double *__restrict__ V,
                                                        double *__restrict__ W) {
   extern __shared__ __align__(32) unsigned char interp_smem[];
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-  const int wid = blockIdx.x * WPB + wl;
-  if (wid >= np) return;
-  const int b = order[wid];
+  const int slot = (blockIdx.x * WPB + wl) / SPLIT, ws = wl % SPLIT;
+  const bool on = slot < np;  // warp-uniform
   const int ngd = c.ngd, n2 = ngd * ngd, Nz = c.N[2];
-  unsigned char *base = interp_smem + (size_t)wl * interp_q_warp_bytes(ngd);
-  InterpWarp<float> &s = *reinterpret_cast<InterpWarp<float> *>(base);
-  InterpQuad &q = *reinterpret_cast<InterpQuad *>(base + interp_q_quad_offset());
-  XY4<float> *xy = reinterpret_cast<XY4<float> *>(base + interp_q_xy_offset());
+  // the warps of one bead share its tables, each filling a part
+  unsigned char *base = interp_smem + (size_t)(wl / SPLIT) * interp_q_warp_bytes(ngd);
+  InterpQuad &q = *reinterpret_cast<InterpQuad *>(base);
+  XY32 *xy = reinterpret_cast<XY32 *>(base + interp_q_xy_offset());
   long long *off = reinterpret_cast<long long *>(xy + n2);
-  for (int a = 0; a < 3; ++a) {  // lane i < ngd takes stencil index i of each axis (as k_interp)
-    const int i = lane;
-    if (i >= ngd) continue;
-    const double Yv = Y[3 * b + a];
-    const int xc = (int)(Yv / c.dx);
-    const int xg = xc - c.ngdh + (i + 1);
-    const int ix = bead_sw[3 * b + a] + i;
-    s.ind[a][i] = ix >= c.N[a] ? ix - c.N[a] : ix;
-    const double xx = ((double)xg) * c.dx - Yv;
-    const float xf = (float)xx;
-    s.g[a][i] = (float)c.anorm * fs_exp<float>(-xf * xf / (float)c.anorm2);
-    s.gd[a][i] = (float)c.anormdip * fs_exp<float>(-xf * xf / (float)c.anormdip2);
-    s.r[a][i] = -xf / (float)c.sigmadipsq;
-  }
-  __syncwarp();
-  const int zs = s.ind[2][0];
-  const int nq = ((zs & 3) + ngd + 3) >> 2;
-  if (lane < nq) {
-    int z0 = (zs & ~3) + 4 * lane;
-    if (z0 >= Nz) z0 -= Nz;
-    float w[3][4];
+  double acc[6] = {0, 0, 0, 0, 0, 0};  // V, W
+  int b = 0, nq = 1;
+  if (on) {
+    const float4 *rw = rec + (size_t)slot * spread_rec_len(ngd);
+    const float4 hd = __ldg(rw);
+    const int sx = __float_as_int(hd.x), sy = __float_as_int(hd.y), zs = __float_as_int(hd.z);
+    b = __float_as_int(hd.w);
+    nq = ((zs & 3) + ngd + 3) >> 2;
+    if (lane < nq && ws == 0) {
+      int z0 = (zs & ~3) + 4 * lane;
+      if (z0 >= Nz) z0 -= Nz;
+      float w[3][4];
 #pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      int k = z0 + t - zs;
-      if (k < 0) k += Nz;
-      const bool on = k < ngd;
-      const int kk = on ? k : 0;  // the tables are read only inside the run
-      w[0][t] = on ? s.g[2][kk] : 0.f;
-      w[1][t] = on ? s.gd[2][kk] : 0.f;
-      w[2][t] = on ? s.r[2][kk] : 0.f;
+      for (int t = 0; t < 4; ++t) {
+        const int k = 4 * lane + t - (zs & 3);
+        const float4 wz = k >= 0 && k < ngd ? __ldg(rw + 3 + 2 * ngd + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        w[0][t] = wz.x;
+        w[1][t] = wz.y;
+        w[2][t] = wz.z;
+      }
+      q.wg[lane] = make_float4(w[0][0], w[0][1], w[0][2], w[0][3]);
+      q.wd[lane] = make_float4(w[1][0], w[1][1], w[1][2], w[1][3]);
+      q.wr[lane] = make_float4(w[2][0], w[2][1], w[2][2], w[2][3]);
+      q.zq[lane] = z0;
     }
-    q.wg[lane] = make_float4(w[0][0], w[0][1], w[0][2], w[0][3]);
-    q.wd[lane] = make_float4(w[1][0], w[1][1], w[1][2], w[1][3]);
-    q.wr[lane] = make_float4(w[2][0], w[2][1], w[2][2], w[2][3]);
-    q.zq[lane] = z0;
-  }
-  for (int ij = lane; ij < n2; ij += 32) {
-    const int i = ij / ngd, j = ij - i * ngd;
-    XY4<float> e;
-    e.gg = s.g[0][i] * s.g[1][j];
-    e.dd = s.gd[0][i] * s.gd[1][j];
-    e.rx = s.r[0][i];
-    e.ry = s.r[1][j];
-    xy[ij] = e;
-    off[ij] = ((long long)s.ind[0][i] * c.N[1] + s.ind[1][j]) * Nz;
-  }
-  __syncwarp();
-  const size_t N = (size_t)c.N[0] * c.N[1] * Nz;
-  const float *ux = u, *uy = u + N, *uz = u + 2 * N;
-  double v0 = 0, v1 = 0, v2 = 0, w0 = 0, w1 = 0, w2 = 0;
-  // slot sl = ij * nq + qi; a step of 32 slots advances (ij, qi) by (32 / nq, 32 % nq)
-  const int nslot = n2 * nq, dij = 32 / nq, dq = 32 - dij * nq;
-  int ij = lane / nq, qi = lane - ij * nq;
-  for (int sl = lane; sl < nslot; sl += 32) {
-    const XY4<float> e = xy[ij];
-    const long long m = off[ij] + q.zq[qi];
-    const float4 a0 = __ldg(reinterpret_cast<const float4 *>(ux + m));
-    const float4 a1 = __ldg(reinterpret_cast<const float4 *>(uy + m));
-    const float4 a2 = __ldg(reinterpret_cast<const float4 *>(uz + m));
-    const float4 g = q.wg[qi], gd = q.wd[qi], r = q.wr[qi];
-    float p0 = 0.f, p1 = 0.f, p2 = 0.f, p3 = 0.f, p4 = 0.f, p5 = 0.f;
-    auto acc = [&](float x0, float x1, float x2, float gz, float gdz, float zz) {
-      const float temp = e.gg * gz;  // (gx gy) gz, the reference's order
-      const float tempd = e.dd * gdz;
-      p0 += x0 * temp;
-      p1 += x1 * temp;
-      p2 += x2 * temp;
-      p3 += (x2 * e.ry - x1 * zz) * tempd;
-      p4 += (x0 * zz - x2 * e.rx) * tempd;
-      p5 += (x1 * e.rx - x0 * e.ry) * tempd;
-    };
-    acc(a0.x, a1.x, a2.x, g.x, gd.x, r.x);
-    acc(a0.y, a1.y, a2.y, g.y, gd.y, r.y);
-    acc(a0.z, a1.z, a2.z, g.z, gd.z, r.z);
-    acc(a0.w, a1.w, a2.w, g.w, gd.w, r.w);
-    v0 += (double)p0;
-    v1 += (double)p1;
-    v2 += (double)p2;
-    w0 += (double)p3;
-    w1 += (double)p4;
-    w2 += (double)p5;
-    qi += dq;
-    ij += dij;
-    if (qi >= nq) {
-      qi -= nq;
-      ++ij;
+    for (int ij = lane + 32 * ws; ij < n2; ij += 32 * SPLIT) {
+      const int i = ij / ngd, j = ij - i * ngd;
+      const float4 wx = __ldg(rw + 3 + i), wy = __ldg(rw + 3 + ngd + j);
+      XY32 e;
+      e.gg = wx.x * wy.x;
+      e.dd = wx.y * wy.y;
+      e.rx = wx.z;
+      e.ry = wy.z;
+      xy[ij] = e;
+      const int ix = sx + i, iy = sy + j;
+      off[ij] = ((long long)(ix >= c.N[0] ? ix - c.N[0] : ix) * c.N[1] + (iy >= c.N[1] ? iy - c.N[1] : iy)) * Nz;
     }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    v0 += __shfl_xor_sync(0xffffffffu, v0, o);
-    v1 += __shfl_xor_sync(0xffffffffu, v1, o);
-    v2 += __shfl_xor_sync(0xffffffffu, v2, o);
-    w0 += __shfl_xor_sync(0xffffffffu, w0, o);
-    w1 += __shfl_xor_sync(0xffffffffu, w1, o);
-    w2 += __shfl_xor_sync(0xffffffffu, w2, o);
+  if constexpr (SPLIT > 1)
+    __syncthreads();
+  else
+    __syncwarp();
+  if (on) {
+    const size_t N = (size_t)c.N[0] * c.N[1] * Nz;
+    const float *ux = u, *uy = u + N, *uz = u + 2 * N;
+    // slot sl = ij * nq + qi; a step advances (ij, qi) by (step / nq, step % nq)
+    constexpr int STEP = 32 * SPLIT;
+    const int nslot = n2 * nq, dij = STEP / nq, dq = STEP - dij * nq;
+    const int first = lane + 32 * ws;
+    int ij = first / nq, qi = first - ij * nq;
+    for (int sl = first; sl < nslot; sl += STEP) {
+      const XY32 e = xy[ij];
+      const long long m = off[ij] + q.zq[qi];
+      const float4 a0 = __ldg(reinterpret_cast<const float4 *>(ux + m));
+      const float4 a1 = __ldg(reinterpret_cast<const float4 *>(uy + m));
+      const float4 a2 = __ldg(reinterpret_cast<const float4 *>(uz + m));
+      const float4 g = q.wg[qi], gd = q.wd[qi], r = q.wr[qi];
+      float p0 = 0.f, p1 = 0.f, p2 = 0.f, p3 = 0.f, p4 = 0.f, p5 = 0.f;
+      auto add = [&](float x0, float x1, float x2, float gz, float gdz, float zz) {
+        const float temp = e.gg * gz;  // (gx gy) gz, the reference's order
+        const float tempd = e.dd * gdz;
+        p0 += x0 * temp;
+        p1 += x1 * temp;
+        p2 += x2 * temp;
+        p3 += (x2 * e.ry - x1 * zz) * tempd;
+        p4 += (x0 * zz - x2 * e.rx) * tempd;
+        p5 += (x1 * e.rx - x0 * e.ry) * tempd;
+      };
+      add(a0.x, a1.x, a2.x, g.x, gd.x, r.x);
+      add(a0.y, a1.y, a2.y, g.y, gd.y, r.y);
+      add(a0.z, a1.z, a2.z, g.z, gd.z, r.z);
+      add(a0.w, a1.w, a2.w, g.w, gd.w, r.w);
+      acc[0] += (double)p0;
+      acc[1] += (double)p1;
+      acc[2] += (double)p2;
+      acc[3] += (double)p3;
+      acc[4] += (double)p4;
+      acc[5] += (double)p5;
+      qi += dq;
+      ij += dij;
+      if (qi >= nq) {
+        qi -= nq;
+        ++ij;
+      }
+    }
   }
-  if (lane == 0) {
-    const double norm = c.dx * c.dx * c.dx;
-    V[3 * b + 0] = v0 * norm;
-    V[3 * b + 1] = v1 * norm;
-    V[3 * b + 2] = v2 * norm;
-    W[3 * b + 0] = -0.5 * w0 * norm;
-    W[3 * b + 1] = -0.5 * w1 * norm;
-    W[3 * b + 2] = -0.5 * w2 * norm;
-  }
+  interp_finish<WPB, SPLIT>(acc, on, b, c.dx, V, W);
 }
 
 template <typename A, typename B>
@@ -1029,23 +1031,34 @@ fs_status flow_solve_t(fs_ctx *c) {
   return FS_OK;
 }
 
-// binning, sort and the spread of the force grid into c->grid_real (R precision)
+// bins the beads of Y, sorts them and writes their records (F, T: null where only the
+// weights are read)
 template <typename R>
-fs_status spread_t(fs_ctx *c, const FcmConsts &k, const double *Y, const double *F, const double *T, int np) {
+fs_status bin_t(fs_ctx *c, const FcmConsts &k, const double *Y, const double *F, const double *T, int np) {
   if (np > 0) {
     k_fcm_bin_keys<<<fs_blocks(np, 256), 256, 0, c->stream>>>(Y, np, k, c->bins.key, c->bead_sw);
     FS_LAUNCH_CHECK();
   }
   FS_TRY(fs_sort_run(&c->bins, np, c->stream));
+  if (np <= 0) return FS_OK;
+  if (sizeof(R) == 4)
+    k_spread_records32<<<fs_blocks((long long)np * spread_rec_len(k.ngd), 256), 256, 0, c->stream>>>(
+        Y, F, T, c->bins.sorted, c->bead_sw, np, k, (float4 *)c->bead_rec);
+  else
+    k_records64<<<fs_blocks((long long)np * rec64_len(k.ngd), 256), 256, 0, c->stream>>>(
+        Y, F, T, c->bins.sorted, c->bead_sw, np, k, (double4 *)c->bead_rec);
+  FS_LAUNCH_CHECK();
+  return FS_OK;
+}
+
+// binning and the spread of the force grid into c->grid_real (R precision)
+template <typename R>
+fs_status spread_t(fs_ctx *c, const FcmConsts &k, const double *Y, const double *F, const double *T, int np) {
+  FS_TRY(bin_t<R>(c, k, Y, F, T, np));
+  ProfScope pk(c, FS_STAGE_K_SPREAD);
+  const int ch = c->tune_spread_chunk, cx = c->tune_spread_cols;
   if (sizeof(R) == 4) {
-    const float4 *rec = (const float4 *)c->spread_wb;
-    if (np > 0) {
-      k_spread_records32<<<fs_blocks((long long)np * spread_rec_len(k.ngd), 256), 256, 0, c->stream>>>(
-          Y, F, T, c->bins.sorted, c->bead_sw, np, k, c->spread_wb);
-      FS_LAUNCH_CHECK();
-    }
-    ProfScope pk(c, FS_STAGE_K_SPREAD);
-    const int ch = c->tune_spread_chunk, cx = c->tune_spread_cols;
+    const float4 *rec = (const float4 *)c->bead_rec;
 #define FS_SPREAD32_LAUNCH(CHV, CXV)                                                                             \
   k_spread32<CHV, CXV><<<c->nbins, FS_SPREAD32_THREADS, spread32_smem<CHV>(k.ngd), c->stream>>>(c->bins.start, rec, \
                                                                                                  k, (float *)c->grid_real)
@@ -1056,49 +1069,55 @@ fs_status spread_t(fs_ctx *c, const FcmConsts &k, const double *Y, const double 
     else if (cx == 8) FS_SPREAD32_LAUNCH(64, 8);
     else FS_SPREAD32_LAUNCH(64, 4);
 #undef FS_SPREAD32_LAUNCH
-  } else if (c->tune_spread_chunk == 32) {
-    ProfScope pk(c, FS_STAGE_K_SPREAD);
-    k_spread<R, 32><<<c->nbins, FS_SPREAD_THREADS, sizeof(SpreadStage<R, 32>), c->stream>>>(
-        Y, F, T, c->bins.start, c->bins.sorted, c->bead_sw, k, (R *)c->grid_real);
   } else {
-    ProfScope pk(c, FS_STAGE_K_SPREAD);
-    k_spread<R, 64><<<c->nbins, FS_SPREAD_THREADS, sizeof(SpreadStage<R, 64>), c->stream>>>(
-        Y, F, T, c->bins.start, c->bins.sorted, c->bead_sw, k, (R *)c->grid_real);
+    const double4 *rec = (const double4 *)c->bead_rec;
+    double *f = (double *)c->grid_real;
+    // half tiles, or quarter tiles where the half tiles would not fill the SMs three times
+    // (64^3: 28 -> 21 us; 256^3, 301 against 308, and 512^3, 1.63 against 1.77 ms, keep half)
+    if (2 * c->nbins < 3 * c->num_sms)
+      k_spread64<4><<<4 * c->nbins, FS_SPREAD64_THREADS, sizeof(SpreadStage64<4>), c->stream>>>(c->bins.start, rec, k,
+                                                                                                f);
+    else
+      k_spread64<8><<<2 * c->nbins, FS_SPREAD64_THREADS, sizeof(SpreadStage64<8>), c->stream>>>(c->bins.start, rec, k,
+                                                                                                f);
   }
   FS_LAUNCH_CHECK();
   return FS_OK;
 }
 
+// warps an SM is given before beads stop being split over several
+#define FS_INTERP_WARPS 20
+
 // interpolation of U, Omega from the velocity grid in c->grid_real (R precision); the
-// beads must have been binned (k_fcm_bin_keys + sort) for this Y
+// beads must have been binned (bin_t) at this precision
 template <typename R>
-fs_status interp_t(fs_ctx *c, const FcmConsts &k, const double *Y, double *V, double *W, int np) {
+fs_status interp_t(fs_ctx *c, const FcmConsts &k, double *V, double *W, int np) {
   if (np <= 0) return FS_OK;
   ProfScope ps(c, FS_STAGE_INTERP);
   ProfScope pk(c, FS_STAGE_K_INTERP);
-  const R *ug = (const R *)c->grid_real;
-  if constexpr (sizeof(R) == 4) {
-    if (interp_q_ok(c)) {  // float4 gathers along z
-      const size_t wq = interp_q_warp_bytes(c->p.ngd);
-      const int wpb = (c->tune_interp_wpb == 16 && 16 * wq > FS_SMEM_MAX) ? 8 : c->tune_interp_wpb;
-      if (wpb == 4)
-        k_interp_q<4><<<fs_blocks(np, 4), 128, 4 * wq, c->stream>>>(ug, Y, c->bins.sorted, c->bead_sw, np, k, V, W);
-      else if (wpb == 16)
-        k_interp_q<16><<<fs_blocks(np, 16), 512, 16 * wq, c->stream>>>(ug, Y, c->bins.sorted, c->bead_sw, np, k, V, W);
-      else
-        k_interp_q<8><<<fs_blocks(np, 8), 256, 8 * wq, c->stream>>>(ug, Y, c->bins.sorted, c->bead_sw, np, k, V, W);
-      FS_LAUNCH_CHECK();
-      return FS_OK;
-    }
+  const int sms = FS_INTERP_WARPS * c->num_sms;
+  const int split = 4 * np <= sms ? 4 : 2 * np <= sms ? 2 : 1;
+  const size_t wb = sizeof(R) == 4 ? interp_q_warp_bytes(k.ngd) : 0;  // dynamic shared memory per bead of a CTA
+  const int wpb = split > 1 ? 4 : (c->tune_interp_wpb == 16 && 16 * wb > FS_SMEM_MAX) ? 8 : c->tune_interp_wpb;
+#define FS_INTERP_LAUNCH(WPB, SPLIT)                                                                             \
+  if constexpr (sizeof(R) == 4)                                                                                  \
+    k_interp_q<WPB, SPLIT><<<fs_blocks(np, WPB / SPLIT), 32 * WPB, WPB / SPLIT * wb, c->stream>>>(                \
+        (const float *)c->grid_real, (const float4 *)c->bead_rec, np, k, V, W);                                  \
+  else                                                                                                           \
+    k_interp64<WPB, SPLIT><<<fs_blocks(np, WPB / SPLIT), 32 * WPB, 0, c->stream>>>(                               \
+        (const double *)c->grid_real, (const double4 *)c->bead_rec, np, k, V, W)
+  if (split == 4) {
+    FS_INTERP_LAUNCH(4, 4);
+  } else if (split == 2) {
+    FS_INTERP_LAUNCH(4, 2);
+  } else if (wpb == 4) {
+    FS_INTERP_LAUNCH(4, 1);
+  } else if (wpb == 16) {
+    FS_INTERP_LAUNCH(16, 1);
+  } else {
+    FS_INTERP_LAUNCH(8, 1);
   }
-  const size_t wb = interp_warp_bytes<R>(c->p.ngd);
-  const int wpb = (c->tune_interp_wpb == 16 && 16 * wb > FS_SMEM_MAX) ? 8 : c->tune_interp_wpb;
-  if (wpb == 4)
-    k_interp<R, 4><<<fs_blocks(np, 4), 128, 4 * wb, c->stream>>>(ug, Y, c->bins.sorted, c->bead_sw, np, k, V, W);
-  else if (wpb == 16)
-    k_interp<R, 16><<<fs_blocks(np, 16), 512, 16 * wb, c->stream>>>(ug, Y, c->bins.sorted, c->bead_sw, np, k, V, W);
-  else
-    k_interp<R, 8><<<fs_blocks(np, 8), 256, 8 * wb, c->stream>>>(ug, Y, c->bins.sorted, c->bead_sw, np, k, V, W);
+#undef FS_INTERP_LAUNCH
   FS_LAUNCH_CHECK();
   return FS_OK;
 }
@@ -1111,7 +1130,7 @@ fs_status mobility_t(fs_ctx *c, const double *Y, const double *F, const double *
     FS_TRY(spread_t<R>(c, k, Y, F, T, np));
   }
   FS_TRY(flow_solve_t<R>(c));
-  FS_TRY(interp_t<R>(c, k, Y, V, W, np));
+  FS_TRY(interp_t<R>(c, k, V, W, np));
   c->last_grid_prec = sizeof(R) == 8 ? FS_PREC_FP64 : FS_PREC_FP32;
   return FS_OK;
 }
@@ -1137,50 +1156,33 @@ fs_status fcm_init(fs_ctx *c) {
   FS_CUDA(cudaMalloc(&c->bead_sw, sizeof(int) * 3 * (size_t)(c->max_beads > 0 ? c->max_beads : 1)));
   c->bytes += sizeof(int) * 3 * (size_t)c->max_beads;
   {
-    const size_t nb = (size_t)(c->max_beads > 0 ? c->max_beads : 1);
-    const size_t nw = nb * spread_rec_len(c->p.ngd);
-    FS_CUDA(cudaMalloc(&c->spread_wb, sizeof(float4) * nw));
-    c->bytes += sizeof(float4) * nw;
+    // the beads' records of either precision (the FP64 ones are the larger)
+    const size_t bytes = sizeof(double4) * (size_t)(c->max_beads > 0 ? c->max_beads : 1) * rec64_len(c->p.ngd);
+    FS_CUDA(cudaMalloc(&c->bead_rec, bytes));
+    c->bytes += bytes;
   }
-  FS_CUDA(cudaFuncSetAttribute(k_spread32<64, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)spread32_smem<64>(FS_NGD_MAX)));
-  FS_CUDA(cudaFuncSetAttribute(k_spread32<64, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)spread32_smem<64>(FS_NGD_MAX)));
-  FS_CUDA(cudaFuncSetAttribute(k_spread32<64, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)spread32_smem<64>(FS_NGD_MAX)));
-  FS_CUDA(cudaFuncSetAttribute(k_spread32<32, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)spread32_smem<32>(FS_NGD_MAX)));
-  FS_CUDA(cudaFuncSetAttribute(k_spread32<32, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)spread32_smem<32>(FS_NGD_MAX)));
-  FS_CUDA(cudaFuncSetAttribute(k_spread32<32, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)spread32_smem<32>(FS_NGD_MAX)));
-  FS_CUDA(cudaFuncSetAttribute(k_spread<double, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)sizeof(SpreadStage<double, 64>)));
-  FS_CUDA(cudaFuncSetAttribute(k_spread<float, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)sizeof(SpreadStage<float, 64>)));
-  FS_CUDA(cudaFuncSetAttribute(k_spread<double, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)sizeof(SpreadStage<double, 32>)));
-  FS_CUDA(cudaFuncSetAttribute(k_spread<float, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)sizeof(SpreadStage<float, 32>)));
-  {
-    // the attribute is per kernel, shared by every context: set for the largest
-    // ngd (capped at what a CTA may ask for; larger launches take 8 warps per CTA)
-    const size_t wd = interp_warp_bytes<double>(FS_NGD_MAX), wf = interp_warp_bytes<float>(FS_NGD_MAX);
-    auto cap = [](size_t b) { return (int)(b < (size_t)FS_SMEM_MAX ? b : (size_t)FS_SMEM_MAX); };
-    FS_CUDA(cudaFuncSetAttribute(k_interp<double, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap(4 * wd)));
-    FS_CUDA(cudaFuncSetAttribute(k_interp<double, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap(8 * wd)));
-    FS_CUDA(cudaFuncSetAttribute(k_interp<double, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap(16 * wd)));
-    FS_CUDA(cudaFuncSetAttribute(k_interp<float, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap(4 * wf)));
-    FS_CUDA(cudaFuncSetAttribute(k_interp<float, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap(8 * wf)));
-    FS_CUDA(cudaFuncSetAttribute(k_interp<float, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap(16 * wf)));
-    const size_t wq = interp_q_warp_bytes(FS_NGD_MAX);
-    FS_CUDA(cudaFuncSetAttribute(k_interp_q<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap(4 * wq)));
-    FS_CUDA(cudaFuncSetAttribute(k_interp_q<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap(8 * wq)));
-    FS_CUDA(cudaFuncSetAttribute(k_interp_q<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap(16 * wq)));
-  }
+  // the attributes are per kernel, shared by every context: set for the largest ngd
+  // (capped at what a CTA may ask for; larger launches take 8 warps per CTA)
+  auto smem = [](const void *fn, size_t bytes) {
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)(bytes < (size_t)FS_SMEM_MAX ? bytes : (size_t)FS_SMEM_MAX));
+  };
+  const size_t s32 = spread32_smem<32>(FS_NGD_MAX), s64 = spread32_smem<64>(FS_NGD_MAX);
+  FS_CUDA(smem((const void *)k_spread32<64, 2>, s64));
+  FS_CUDA(smem((const void *)k_spread32<64, 4>, s64));
+  FS_CUDA(smem((const void *)k_spread32<64, 8>, s64));
+  FS_CUDA(smem((const void *)k_spread32<32, 2>, s32));
+  FS_CUDA(smem((const void *)k_spread32<32, 4>, s32));
+  FS_CUDA(smem((const void *)k_spread32<32, 8>, s32));
+  FS_CUDA(smem((const void *)k_spread64<4>, sizeof(SpreadStage64<4>)));
+  FS_CUDA(smem((const void *)k_spread64<8>, sizeof(SpreadStage64<8>)));
+  const size_t wq = interp_q_warp_bytes(FS_NGD_MAX);
+  FS_CUDA(smem((const void *)k_interp_q<4, 1>, 4 * wq));
+  FS_CUDA(smem((const void *)k_interp_q<8, 1>, 8 * wq));
+  FS_CUDA(smem((const void *)k_interp_q<16, 1>, 16 * wq));
   c->tune_spread_chunk = 64;
   c->tune_spread_cols = 2;  // 2 x 16 x 8 blocks: fs_autotune's choice at 384^3 and 512^3
-  c->tune_interp_wpb = 8;
+  c->tune_interp_wpb = 4;  // the fastest at 256^3 and 512^3 in both precisions (FP64 833, 873, 911 us for 4, 8, 16)
   c->tune_fft32 = 0;
   if (lines_supported(c)) {
     FS_TRY(lines_init64(c));
@@ -1217,8 +1219,8 @@ void fcm_free(fs_ctx *c) {
   fs_sort_free(&c->bins);
   cudaFree(c->bead_sw);
   c->bead_sw = nullptr;
-  cudaFree(c->spread_wb);
-  c->spread_wb = nullptr;
+  cudaFree(c->bead_rec);
+  c->bead_rec = nullptr;
 }
 
 fs_status fcm_set_stream(fs_ctx *c, cudaStream_t st) {
@@ -1250,18 +1252,15 @@ fs_status fcm_friction(fs_ctx *c, const double *F, const double *T, double *V, d
 fs_status fcm_interpolate_only(fs_ctx *c, const double *u, const double *Y, int np, double *V, double *W) {
   FcmConsts k = make_consts(c);
   const size_t n = 3 * c->N;
-  if (np > 0) {
-    k_fcm_bin_keys<<<fs_blocks(np, 256), 256, 0, c->stream>>>(Y, np, k, c->bins.key, c->bead_sw);
-    FS_LAUNCH_CHECK();
-  }
-  FS_TRY(fs_sort_run(&c->bins, np, c->stream));
+  FS_TRY(c->precision == FS_PREC_FP32 ? bin_t<float>(c, k, Y, nullptr, nullptr, np)
+                                      : bin_t<double>(c, k, Y, nullptr, nullptr, np));
   if (c->precision == FS_PREC_FP32) {
     k_convert<double, float><<<fs_blocks((long long)n, 256), 256, 0, c->stream>>>(u, (float *)c->grid_real, n);
     FS_LAUNCH_CHECK();
-    FS_TRY(interp_t<float>(c, k, Y, V, W, np));
+    FS_TRY(interp_t<float>(c, k, V, W, np));
   } else {
     FS_CUDA(cudaMemcpyAsync(c->grid_real, u, sizeof(double) * n, cudaMemcpyDeviceToDevice, c->stream));
-    FS_TRY(interp_t<double>(c, k, Y, V, W, np));
+    FS_TRY(interp_t<double>(c, k, V, W, np));
   }
   c->last_grid_prec = -1;
   return FS_OK;

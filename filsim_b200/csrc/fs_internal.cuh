@@ -67,7 +67,7 @@ struct fs_ctx {
   int nbin[3], nbins;  // spread bins (FS_TILE wide in stencil-start space)
   fs_sort bins;
   int *bead_sw;        // per bead, wrapped Gaussian stencil start per axis
-  float4 *spread_wb;   // FP32 chain: per sorted bead, stencil starts, F, T/2 and weights
+  void *bead_rec;      // per sorted bead: stencil starts, F, T/2 and Gaussian weights (FP64 or FP32 record)
   int last_grid_prec;  // precision of the grids from the last solve (-1: none)
   int tune_spread_chunk;  // beads staged per spread pass: 32 or 64 (fs_autotune)
   int tune_spread_cols;   // FP32 spread: x width of a warp's column block (2, 4 or 8)

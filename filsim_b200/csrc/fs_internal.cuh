@@ -32,7 +32,8 @@ struct fs_sort {
   int *key;      // per item
   int *count;    // nkeys
   int *start;    // nkeys + 1
-  int *cursor;   // nkeys
+  int *slot;     // per item, its place among its key's in arrival order
+  int *placed;   // items by (key, slot)
   int *sorted;   // items in (key, id) order
   int *block_sums;
 };

@@ -67,8 +67,6 @@ fs_status alloc_state(fs_ctx *c) {
   FS_CUDA(cudaMalloc(&c->fil_start, sizeof(int) * (nf + 1)));
   FS_CUDA(cudaMalloc(&c->fil_id, sizeof(int) * nb));
   FS_CUDA(cudaMalloc(&c->seg_id, sizeof(int) * nb));
-  FS_CUDA(cudaMalloc(&c->soff, sizeof(long long) * (nf + 1)));
-  FS_CUDA(cudaMalloc(&c->aoff, sizeof(long long) * (nf + 1)));
   const size_t hist = (size_t)c->p.broyden_maxiter * 6 * nb;
   FS_CUDA(cudaMalloc(&c->Cmat, sizeof(double) * hist));
   FS_CUDA(cudaMalloc(&c->Dmat, sizeof(double) * hist));
@@ -87,8 +85,8 @@ fs_status alloc_state(fs_ctx *c) {
 void free_state(fs_ctx *c) {
   void *ptrs[] = {c->X, c->Xs, c->Xt, c->U, c->Us, c->Ut, c->F, c->TAU, c->Y, c->V, c->W, c->lam, c->lam1,
                   c->lam2, c->q, c->qs, c->qt, c->err, c->newerr, c->upd, c->tmp, c->dE, c->kap, c->cc,
-                  c->fil_start, c->fil_id, c->seg_id, c->soff, c->aoff, c->Cmat, c->Dmat, c->dots, c->partials,
-                  c->scalars, c->flags, c->maxerr_bits, c->Sinv, c->aux, c->swim, c->spring_beads,
+                  c->fil_start, c->fil_id, c->seg_id, c->Cmat, c->Dmat, c->dots, c->partials,
+                  c->scalars, c->flags, c->maxerr_bits, c->jtri, c->swim, c->spring_beads,
                   c->spring_off, c->spring_ent};
   for (void *p : ptrs) cudaFree(p);
   if (c->flags_h) cudaFreeHost(c->flags_h);
@@ -484,7 +482,7 @@ static fs_status upload_layout(fs_ctx *c, const fs_host_state *s);
 static void spring_free(fs_ctx *c);
 static void swim_free(fs_ctx *c);
 
-// state arrays always; the filament layout (ids, offsets, Schur buffers) only
+// state arrays always; the filament layout (ids, offsets, Jacobian buffer) only
 // when it differs from the previous upload's
 fs_status fs_state_upload(fs_ctx *c, const fs_host_state *s) {
   if (!c || !s || !s->fil_start || s->nfil < 0 || s->np < 0) return FS_ERR_INVALID_ARG;
@@ -537,13 +535,11 @@ fs_status fs_state_upload(fs_ctx *c, const fs_host_state *s) {
   return FS_OK;
 }
 
-// the filament layout of an upload: ids, offsets, Schur buffers (fs_state_upload)
+// the filament layout of an upload: ids, offsets, Jacobian buffer (fs_state_upload)
 static fs_status upload_layout(fs_ctx *c, const fs_host_state *s) {
   const int nf = s->nfil, np = s->np;
   std::vector<int> fid(np > 0 ? np : 1), sid(np > 0 ? np : 1);
-  std::vector<long long> soff(nf + 1), aoff(nf + 1);
   int max_nw = 1, min_nw = nf > 0 ? 1 << 30 : 1;
-  soff[0] = aoff[0] = 0;
   for (int f = 0; f < nf; ++f) {
     const int nw = s->fil_start[f + 1] - s->fil_start[f];
     if (nw < 1) return FS_ERR_INVALID_ARG;
@@ -553,12 +549,10 @@ static fs_status upload_layout(fs_ctx *c, const fs_host_state *s) {
       fid[s->fil_start[f] + i] = f;
       sid[s->fil_start[f] + i] = i;
     }
-    soff[f + 1] = soff[f] + 9LL * nw * nw;
-    aoff[f + 1] = aoff[f] + fil_aux_size(nw);
   }
   const int prev_max_nw = c->max_nw;
   c->max_nw = max_nw;
-  if (fil_jacobian_prepare(c) != FS_OK) {  // the Schur complement of a filament lives in shared memory
+  if (fil_jacobian_prepare(c) != FS_OK) {  // a filament's blocks live in shared memory
     c->max_nw = prev_max_nw;
     return FS_ERR_INVALID_ARG;
   }
@@ -566,17 +560,13 @@ static fs_status upload_layout(fs_ctx *c, const fs_host_state *s) {
   c->nfil = nf;
   c->np = np;
   c->nlink = np - nf;
-  cudaFree(c->Sinv);
-  cudaFree(c->aux);
-  c->Sinv = c->aux = nullptr;
-  FS_CUDA(cudaMalloc(&c->Sinv, sizeof(double) * (size_t)(soff[nf] > 0 ? soff[nf] : 1)));
-  FS_CUDA(cudaMalloc(&c->aux, sizeof(double) * (size_t)(aoff[nf] > 0 ? aoff[nf] : 1)));
+  cudaFree(c->jtri);
+  c->jtri = nullptr;
+  FS_CUDA(cudaMalloc(&c->jtri, sizeof(double) * fil_jacobian_doubles(np > 0 ? np : 1)));
   cudaStream_t st = c->stream;
   FS_CUDA(cudaMemcpyAsync(c->fil_start, s->fil_start, sizeof(int) * (nf + 1), cudaMemcpyHostToDevice, st));
   FS_CUDA(cudaMemcpyAsync(c->fil_id, fid.data(), sizeof(int) * np, cudaMemcpyHostToDevice, st));
   FS_CUDA(cudaMemcpyAsync(c->seg_id, sid.data(), sizeof(int) * np, cudaMemcpyHostToDevice, st));
-  FS_CUDA(cudaMemcpyAsync(c->soff, soff.data(), sizeof(long long) * (nf + 1), cudaMemcpyHostToDevice, st));
-  FS_CUDA(cudaMemcpyAsync(c->aoff, aoff.data(), sizeof(long long) * (nf + 1), cudaMemcpyHostToDevice, st));
   FS_CUDA(cudaStreamSynchronize(st));  // the host vectors above go out of scope
   free(c->fil_start_h);
   c->fil_start_h = (int *)malloc(sizeof(int) * (nf + 1));

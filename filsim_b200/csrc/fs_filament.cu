@@ -8,12 +8,12 @@
 //   k_forces             setZeroForcesTorques, applyElasticTorques, applyConstraintForcesTorques,
 //                        applyExternalForcesTorques (Filament.hpp:271-402), one thread per bead
 //                        adding its links' terms in the reference's order
-//   k_jacobian_schur     buildApproximateJacobian with BlockC/D/E/F (Filament.hpp:803-1120) reduced
-//                        to the 3Nw x 3Nw Schur complement of its constraint block (one CTA per
-//                        filament); k_schur_gj inverts it in shared memory
+//   k_jacobian_rows, k_jacobian_factor
+//                        buildApproximateJacobian with BlockC/D/E/F (Filament.hpp:803-1120) as a
+//                        block tridiagonal matrix, factored (two warps per filament)
 //   k_error_check        ErrorCheckFCM + dexpinv (MobilityConstraints.cpp:109-143, 447-770)
-//   k_schur_apply        filamentJsolver::solve (FilamentJacobianSolver.hpp:49-73): J0^-1 b from
-//                        the Schur inverse, then the bad-Broyden history corrections
+//   k_tri_apply          filamentJsolver::solve (FilamentJacobianSolver.hpp:49-73): J0^-1 b from
+//                        the factors, then the bad-Broyden history corrections
 //   k_broyden_cols       history update of main.cpp:640-663
 //   k_update / k_step    Filament::update (Filament.hpp:425-452), Filament::step (:455-478); with
 //                        tension order 1 the tensions extrapolated linearly after lambda_extrap_step
@@ -420,21 +420,20 @@ __device__ __forceinline__ void frame(const double *qa, double *t, double *n, do
   q_normal(q, n);
   q_binormal(q, b);
 }
-// row-major store of a 3x3 block at (r0, c0) of an n-column matrix
-__device__ __forceinline__ void put3(double *J, int n, int r0, int c0, const M3 &a) {
+// store of a 3x3 block at column c0 of a 3 x 9 row (row-major)
+__device__ __forceinline__ void put3(double *J, int c0, const M3 &a) {
   for (int i = 0; i < 3; ++i)
-    for (int j = 0; j < 3; ++j) J[(size_t)(r0 + i) * n + c0 + j] = a.m[3 * i + j];
+    for (int j = 0; j < 3; ++j) J[9 * i + c0 + j] = a.m[3 * i + j];
 }
 
-// the three BlockE blocks of bead row k (Filament.hpp:958-1089), stored into
-// the 3nw x 3nw matrix J (row-major, leading dimension n = 3nw)
+// the three BlockE blocks of bead row k (Filament.hpp:958-1089), stored into the 3 x 9
+// row J: columns of bead k - 1 (not for the first bead), k, k + 1 (not for the last)
 __device__ void blockE_row(int k, int nw, const double *qs, const double *Us, const double *TAU, const double *lam,
                            double rad_k, double myC, double myKAP, const double *ST, double DL, double dt, double MU,
-                           double *J, int n) {
+                           double *J) {
   const double PI = FS_PI;
-  const int rE = 0, cE = 0;
   double t[3], nn[3], b[3], tp1[3], np1[3], bp1[3], tm1[3], nm1[3], bm1[3];
-  const double Tfac = 1 / (8 * PI * MU * pow(rad_k, 3));
+  const double Tfac = 1 / (8 * PI * MU * (rad_k * rad_k * rad_k));
   const M3 LieMat = mt(rcross(Us + 3 * k));
   const double tT[3] = {Tfac * TAU[3 * k], Tfac * TAU[3 * k + 1], Tfac * TAU[3 * k + 2]};
   const M3 OmegaMat = rcross(tT);
@@ -452,13 +451,13 @@ __device__ void blockE_row(int k, int nw, const double *qs, const double *Us, co
                            msc(madd(msc(rcross(nn), ST[0]), msc(rcross(b), ST[1])), 0.5)),
                       0.5 * myKAP));
     M3 dOmega = msc(madd(EP, ConstraintPart), Tfac);
-    put3(J, n, rE, cE, blockE_diag(dOmega, LieMat, OmegaMat, Us, dt));
+    put3(J, 3, blockE_diag(dOmega, LieMat, OmegaMat, Us, dt));
     EP = msc(msub(msc(rcross(tp1), beta), msc(outer(ttp, CP), 0.5 / DL)), 0.5 * myC);
     EP = madd(EP, msc(msub(msc(mmul(mt(rcross(t)), rcross(tp1)), 1. / DL),
                            msc(madd(msc(rcross(np1), ST[0]), msc(rcross(bp1), ST[1])), 0.5)),
                       0.5 * myKAP));
     dOmega = msc(EP, Tfac);
-    put3(J, n, rE, cE + 3, blockE_off(dOmega, LieMat, dt));
+    put3(J, 6, blockE_off(dOmega, LieMat, dt));
     return;
   }
   if (k == nw - 1) {
@@ -474,13 +473,13 @@ __device__ void blockE_row(int k, int nw, const double *qs, const double *Us, co
                            msc(madd(msc(rcross(nn), ST[0]), msc(rcross(b), ST[1])), 0.5)),
                       0.5 * myKAP));
     M3 dOmega = msc(madd(EP, ConstraintPart), Tfac);
-    put3(J, n, rE + 3 * k, cE + 3 * k, blockE_diag(dOmega, LieMat, OmegaMat, Us + 3 * k, dt));
+    put3(J, 3, blockE_diag(dOmega, LieMat, OmegaMat, Us + 3 * k, dt));
     EP = msc(msub(msc(rcross(tm1), beta), msc(outer(ttm, CPm), 0.5 / DL)), -0.5 * myC);
     EP = msub(EP, msc(msub(msc(mmul(rcross(t), rcross(tm1)), 1. / DL),
                            msc(madd(msc(rcross(nm1), ST[0]), msc(rcross(bm1), ST[1])), 0.5)),
                       0.5 * myKAP));
     dOmega = msc(EP, Tfac);
-    put3(J, n, rE + 3 * k, cE + 3 * k - 3, blockE_off(dOmega, LieMat, dt));
+    put3(J, 0, blockE_off(dOmega, LieMat, dt));
     return;
   }
   frame(qs + 4 * (k - 1), tm1, nm1, bm1);
@@ -504,529 +503,345 @@ __device__ void blockE_row(int k, int nw, const double *qs, const double *Us, co
                          msc(madd(msc(rcross(nn), ST[0]), msc(rcross(b), ST[1])), 0.5)),
                     0.5 * myKAP));
   M3 dOmega = msc(madd(ConstraintPart, EP), Tfac);
-  put3(J, n, rE + 3 * k, cE + 3 * k, blockE_diag(dOmega, LieMat, OmegaMat, Us + 3 * k, dt));
+  put3(J, 3, blockE_diag(dOmega, LieMat, OmegaMat, Us + 3 * k, dt));
   EP = msc(msub(msc(rcross(tm1), beta), msc(outer(tm, CPk), 0.5 / DL)), -0.5 * myC);
   EP = msub(EP, msc(msub(msc(mmul(rcross(t), rcross(tm1)), 1. / DL),
                          msc(madd(msc(rcross(nm1), ST[0]), msc(rcross(bm1), ST[1])), 0.5)),
                     0.5 * myKAP));
   dOmega = msc(EP, Tfac);
-  put3(J, n, rE + 3 * k, cE + 3 * k - 3, blockE_off(dOmega, LieMat, dt));
+  put3(J, 0, blockE_off(dOmega, LieMat, dt));
   // right block with the k-1 side beta (Filament.hpp:1083)
   EP = msc(msub(msc(rcross(tp1), beta), msc(outer(tp, CPk), 0.5 / DL)), 0.5 * myC);
   EP = madd(EP, msc(msub(msc(mmul(mt(rcross(t)), rcross(tp1)), 1. / DL),
                          msc(madd(msc(rcross(np1), ST[0]), msc(rcross(bp1), ST[1])), 0.5)),
                     0.5 * myKAP));
   dOmega = msc(EP, Tfac);
-  put3(J, n, rE + 3 * k, cE + 3 * k + 3, blockE_off(dOmega, LieMat, dt));
+  put3(J, 6, blockE_off(dOmega, LieMat, dt));
 }
 
-// ---- approximate Jacobian by the Schur complement of the constraint block --------
+// ---- approximate Jacobian as a block tridiagonal matrix ----------------------------
 //
 // With columns [X0 (3) | U (3nw) | lambda (3nw-3)] and rows [first-bead
 // position (3) | constraints (3nw-3) | Lie updates (3nw)], the reference's J
 // (Filament.hpp:803-867) is
 //     J = [ I  0  P  ]    P  = (temp/dt) [I 0 ... 0]
 //         [ 0  C  D' ]    C  = BlockC(DL/2), D' = 10 BlockD/dt (block bidiagonal, scalar blocks)
-//         [ 0  E  F' ]    E  = BlockE,       F' = BlockF/dt (block bidiagonal)
-// Eliminating lambda = D'^-1 (b1 - C u) leaves S u = b2 - F' D'^-1 b1 with
-// S = E - F' D'^-1 C (3nw x 3nw). k_jacobian_schur builds S in shared memory and
-// stores it; k_schur_gj inverts it (Gauss-Jordan, partial pivoting) in a lean
-// kernel with more CTAs per SM; k_schur_apply then applies J^-1 exactly, with the
-// reference's 1/dt scaling of the lambda rows (:864).
-//
-// Per-filament auxiliary data (aux, nw >= 2): d[nw-1], e[nw-1] (D' blocks),
-// Fd[nw-1][9] = F'(k,k), Fl[nw-1][9] = F'(k+1,k), t[nw][3] tangents, pcoef.
+//         [ 0  E  F' ]    E  = BlockE (block tridiagonal), F' = BlockF/dt (block bidiagonal)
+// C's rows are running sums along the filament (row r: fac c_0 + 2 fac sum_{1<=q<=r} c_q +
+// fac c_{r+1}, c_q = cross(u_q, t_q)), so the difference of two successive constraint rows
+// is fac (c_r + c_{r+1}) and D' becomes block tridiagonal: with the unknowns (u_k, lambda_k)
+// and the rows (Lie update k, constraint k - constraint k-1) of a bead taken together, J
+// is block tridiagonal with 6 x 6 blocks,
+//     A_k z_{k-1} + B_k z_k + G_k z_{k+1} = r_k
+// (the last bead has no lambda: its second half is the identity). It is factored once per
+// build, from both ends towards the bead in the middle (mid = nw / 2), two chains at a
+// time: with Dk = B_k - A_k W_{k-1} before the middle, B_k - G_k W_{k+1} after it and both
+// in it, each bead keeps 108 doubles: Dk^-1, W_k = Dk^-1 times the block towards the middle
+// (in the middle: G) and T_k = Dk^-1 times the block it came from (in the middle: A). An
+// application runs the chains y_k = Dk^-1 r_k - T_k y_before inwards and z_k = y_k - W_k
+// z_inner outwards. Linear in the filament's length, where the 3nw x 3nw inverse of the
+// Schur complement of D' is cubic to build and quadratic to apply; against J solved in 80
+// bits over filaments of 2 to 48 beads (dt 1e-3 to 0.3, moduli 0.1 to 100, ah 0.6 to 1.6)
+// it is within 2e-14, the Schur complement within 1e-13.
 #define FS_MAX_NW 48
+constexpr int TRI = 108;     // doubles of a bead's factors: D^-1, W, T (6 x 6 row-major each)
+constexpr int TRI_ROW = 39;  // doubles of a bead's row: E (3 x 9), F'(k,k) (9), tangent (3)
+constexpr int TRI_APPLY_WARPS = 2;  // filaments per CTA of k_tri_apply
 
-// column cc of rcross(t) (Av = cross(v, t))
-__device__ __forceinline__ void rcross_col(const double *t, int cc, double *col) {
-  if (cc == 0) { col[0] = 0.; col[1] = -t[2]; col[2] = t[1]; }
-  else if (cc == 1) { col[0] = t[2]; col[1] = 0.; col[2] = -t[0]; }
-  else { col[0] = -t[1]; col[1] = t[0]; col[2] = 0.; }
+// D' blocks of a row (BlockD(nt), Filament.hpp:912-949), of the radii of its bead and the next
+__device__ __forceinline__ double tri_dd(int nt, const FilConsts &k, double rad) {
+  double facn = -2. * k.dt / (18. * FS_PI * k.mu * rad);
+  if (nt <= k.impl_euler_steps) facn *= (3. / 2.);
+  return 10. * facn / k.dt;
+}
+__device__ __forceinline__ double tri_ee(int nt, const FilConsts &k, double rad_next) {
+  double facu = 2. * k.dt / (18. * FS_PI * k.mu * rad_next);
+  if (nt <= k.impl_euler_steps) facu *= (3. / 2.);
+  return 10. * facu / k.dt;
+}
+// entry (i, c) of the matrix u -> cross(u, t)
+__device__ __forceinline__ double cross_entry(const double *t, int i, int c) {
+  if (i == c) return 0.0;
+  const double v = t[3 - i - c];
+  return (i + 1) % 3 == c ? v : -v;
 }
 
-__global__ void __launch_bounds__(256) k_jacobian_schur(
-    const int *__restrict__ fil_start, const double *__restrict__ qs, const double *__restrict__ Us,
-    const double *__restrict__ TAU, const double *__restrict__ lam, const double *__restrict__ kap,
-    const double *__restrict__ cmod, const long long *__restrict__ soff, const long long *__restrict__ aoff,
-    double *__restrict__ Sinv_all, double *__restrict__ aux_all, int nt, FilConsts k, double a, double ah,
-    int *__restrict__ flags, const int *__restrict__ keep) {
-  extern __shared__ double S[];  // 3nw x 3nw, row-major
+// Bead rows of J, a thread per bead: the E row and F' block (that of bead k is F'(k,k) and,
+// a function of bead k alone, also F'(k,k-1)) and the tangent, as rows[entry][bead]. Bound by
+// the FP64 instructions of blockE_row, a few warps per SM at its registers.
+__global__ void __launch_bounds__(128) k_jacobian_rows(int np, const int *__restrict__ fil_id,
+                                                       const int *__restrict__ fil_start,
+                                                       const double *__restrict__ qs, const double *__restrict__ Us,
+                                                       const double *__restrict__ TAU, const double *__restrict__ lam,
+                                                       const double *__restrict__ kap, const double *__restrict__ cmod,
+                                                       double *__restrict__ rows, FilConsts k, double a, double ah,
+                                                       const int *__restrict__ keep) {
   if (keep && *keep) return;  // the previous step's J0 stays (fs_set_broyden_memory)
-  const int f = blockIdx.x;
-  const int b0 = fil_start[f], nw = fil_start[f + 1] - b0, l0 = b0 - f;
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= np) return;
+  const int f = fil_id[g], b0 = fil_start[f], nw = fil_start[f + 1] - b0, kk = g - b0;
   if (nw < 2) return;  // J0 is the identity
-  const int m = 3 * nw, nl = nw - 1;
-  const int tid = threadIdx.x, nthr = blockDim.x;
-  const double PI = FS_PI, dt = k.dt, DL = k.dl, MU = k.mu;
-  const double *q_f = qs + 4 * b0, *Us_f = Us + 3 * b0, *TAU_f = TAU + 3 * b0, *lam_f = lam + 3 * l0;
-  double *aux = aux_all + aoff[f];
-  double *dd = aux, *ee = aux + nl, *Fd = aux + 2 * nl, *Fl = Fd + 9 * nl, *tt = Fl + 9 * nl, *pcoef = tt + 3 * nw;
-#define RAD(kk) ((kk) == 0 ? ah : a)
-  for (int e = tid; e < m * m; e += nthr) S[e] = 0.0;
-  for (int kk = tid; kk < nw; kk += nthr) {
-    double tv[3];
-    q_tangent(qload(q_f + 4 * kk), tv);
-    for (int d = 0; d < 3; ++d) tt[3 * kk + d] = tv[d];
-  }
-  const double Jprefac = 10.;
-  for (int r = tid; r < nl; r += nthr) {
-    // Jprefac * BlockD(nt) / dt (Filament.hpp:912-949)
-    double facn = -2. * dt / (18. * PI * MU * RAD(r));
-    if (nt <= k.impl_euler_steps) facn *= (3. / 2.);
-    dd[r] = Jprefac * facn / dt;
-    double facu = 0.0;
-    if (r < nw - 2) {
-      facu = 2. * dt / (18. * PI * MU * RAD(r + 1));
-      if (nt <= k.impl_euler_steps) facu *= (3. / 2.);
-      facu = Jprefac * facu / dt;
-    }
-    ee[r] = facu;
-    // BlockF / dt (Filament.hpp:1099-1120)
-    double tv[3];
-    double fac2 = dt * DL / (24 * PI * MU * pow(RAD(r), 3.));
-    q_tangent(qload(q_f + 4 * r), tv);
-    M3 tmat = mt(rcross(tv));
-    M3 umat = rcross(Us_f + 3 * r);
-    M3 blk = msc(madd(msub(tmat, msc(mmul(umat, tmat), 0.5)), msc(mmul(mmul(umat, umat), tmat), 1. / 12.)), fac2 / dt);
-    for (int e = 0; e < 9; ++e) Fd[9 * r + e] = blk.m[e];
-    fac2 = dt * DL / (24. * PI * MU * pow(RAD(r + 1), 3));
-    q_tangent(qload(q_f + 4 * (r + 1)), tv);
-    tmat = mt(rcross(tv));
-    umat = rcross(Us_f + 3 * (r + 1));
-    blk = msc(madd(msub(tmat, msc(mmul(umat, tmat), 0.5)), msc(mmul(mmul(umat, umat), tmat), 1. / 12.)), fac2 / dt);
-    for (int e = 0; e < 9; ++e) Fl[9 * r + e] = blk.m[e];
-  }
-  if (tid == 0) *pcoef = (dt / (9 * PI * MU * RAD(0))) / dt;
-  __syncthreads();
+  const double *q_f = qs + 4 * b0, *Us_f = Us + 3 * b0;
+  const double rad = kk == 0 ? ah : a;
   // this->myStrainTwist as applyElasticTorques(nt) left it: its last link (nw >= 2 here)
-  double stj[3];
+  double stj[3], E[27], tv[3];
   link_strain_twist(k, f, nw, nw - 2, stj);
-  for (int kk = tid; kk < nw; kk += nthr)
-    blockE_row(kk, nw, q_f, Us_f, TAU_f, lam_f, RAD(kk), cmod[f], kap[f], stj, DL, dt, MU, S, m);
-#undef RAD
-  __syncthreads();
-  for (int e = tid; e < m; e += nthr) S[e * m + e] += 1.;  // BlockE's identity (Filament.hpp:1092-1094)
-  __syncthreads();
-  // S -= F' D'^-1 C, one column of C per thread
-  const double fac = 0.5 * DL;
-  for (int j = tid; j < m; j += nthr) {
-    const int mb = j / 3, cc = j % 3;
-    double col[3];
-    rcross_col(tt + 3 * mb, cc, col);
-    double y[3 * (FS_MAX_NW - 1)];
-    for (int r = nl - 1; r >= 0; --r) {  // y = D'^-1 C[:, j] (upper bidiagonal back substitution)
-      double cf = 0.0;
-      if (mb == 0 || mb == r + 1) cf = 1.0;
-      else if (mb >= 1 && mb <= r) cf = 2.0;
-      for (int d = 0; d < 3; ++d) {
-        double cv = (cf == 0.0) ? 0.0 : (cf == 1.0 ? fac * col[d] : fac * col[d] + fac * col[d]);
-        double nxt = (r + 1 < nl) ? ee[r] * y[3 * (r + 1) + d] : 0.0;
-        y[3 * r + d] = (cv - nxt) / dd[r];
-      }
-    }
-    for (int kb = 0; kb < nw; ++kb) {  // g = F' y, S[:, j] -= g
-      double g[3] = {0.0, 0.0, 0.0};
-      if (kb < nl)
-        for (int i2 = 0; i2 < 3; ++i2)
-          g[i2] += Fd[9 * kb + 3 * i2] * y[3 * kb] + Fd[9 * kb + 3 * i2 + 1] * y[3 * kb + 1] +
-                   Fd[9 * kb + 3 * i2 + 2] * y[3 * kb + 2];
-      if (kb >= 1)
-        for (int i2 = 0; i2 < 3; ++i2)
-          g[i2] += Fl[9 * (kb - 1) + 3 * i2] * y[3 * (kb - 1)] + Fl[9 * (kb - 1) + 3 * i2 + 1] * y[3 * (kb - 1) + 1] +
-                   Fl[9 * (kb - 1) + 3 * i2 + 2] * y[3 * (kb - 1) + 2];
-      for (int i2 = 0; i2 < 3; ++i2) S[(3 * kb + i2) * m + j] -= g[i2];
-    }
-  }
-  __syncthreads();
-  double *Sout = Sinv_all + soff[f];
-  for (int e = tid; e < m * m; e += nthr) Sout[e] = S[e];
+#pragma unroll
+  for (int e = 0; e < 27; ++e) E[e] = 0.0;
+  blockE_row(kk, nw, q_f, Us_f, TAU + 3 * b0, lam + 3 * (b0 - f), rad, cmod[f], kap[f], stj, k.dl, k.dt, k.mu, E);
+  for (int i = 0; i < 3; ++i) E[9 * i + 3 + i] += 1.;  // BlockE's identity (Filament.hpp:1092-1094)
+#pragma unroll
+  for (int e = 0; e < 27; ++e) rows[(size_t)e * np + g] = E[e];
+  // BlockF / dt (Filament.hpp:1099-1120)
+  const double fac2 = k.dt * k.dl / (24 * FS_PI * k.mu * (rad * rad * rad));
+  q_tangent(qload(q_f + 4 * kk), tv);
+  const M3 tmat = mt(rcross(tv)), umat = rcross(Us_f + 3 * kk);
+  const M3 F =
+      msc(madd(msub(tmat, msc(mmul(umat, tmat), 0.5)), msc(mmul(mmul(umat, umat), tmat), 1. / 12.)), fac2 / k.dt);
+#pragma unroll
+  for (int e = 0; e < 9; ++e) rows[(size_t)(27 + e) * np + g] = F.m[e];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) rows[(size_t)(36 + d) * np + g] = tv[d];
 }
 
-// Inverse of S (k_jacobian_schur's output, in place) by Gauss-Jordan with partial
-// pivoting (the first maximum wins); one CTA per filament with S in shared memory.
-__global__ void __launch_bounds__(384) k_schur_gj(const int *__restrict__ fil_start,
-                                                  const long long *__restrict__ soff, double *__restrict__ Sinv_all,
-                                                  int *__restrict__ flags, const int *__restrict__ keep) {
-  extern __shared__ double S[];
-  __shared__ int perm[3 * FS_MAX_NW];
-  __shared__ double fcol[3 * FS_MAX_NW];
-  __shared__ int colsrc[3 * FS_MAX_NW];
-  __shared__ int s_piv;
-  __shared__ double s_inv, s_diag;
+// Column c (0..5) of block A_k (which = -1), B_k (0) or G_k (+1); E: the bead's row, dd, ee
+// the D' entries of its constraint row, ddp, eep of the row before (0 where absent; dd = 1
+// and ee = 0 for the last bead, whose lambda is held at 0)
+__device__ __forceinline__ void tri_column(double v[6], int which, int c, const double *E, bool last, double fac,
+                                           double dd, double ee, double ddp, double eep) {
+  const int c3 = c % 3;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    double top, bot;  // rows i (Lie) and 3 + i (constraint)
+    if (c < 3) {
+      top = E[9 * i + 3 * which + 3 + c3];
+      bot = last || which < 0 ? 0.0 : fac * cross_entry(E + TRI_ROW * which + 36, i, c3);
+    } else {
+      top = which > 0 || (which == 0 && last) ? 0.0 : E[27 + 3 * i + c3];
+      bot = i != c3 ? 0.0 : which < 0 ? -ddp : which > 0 ? ee : dd - eep;
+    }
+    v[i] = top;
+    v[3 + i] = bot;
+  }
+}
+
+// The two chains of a filament, a warp each (then the middle bead by the first): 24 lanes
+// hold the columns of [Dk | I | towards | from] and run a Gauss-Jordan elimination of Dk on
+// them, pivot rows in place. Bound by the latency of that chain (search, reciprocal and
+// update of six pivots, each on the one before) and, with several filaments per SM, by its
+// instructions. 1,024 filaments of 32 beads, both kernels: 72 us, against 850 us for the Schur
+// complement's assembly and inverse (a warp per filament over all its beads, no second
+// chain: 110 us; 4,096 filaments 400 us, with two chains 208 us).
+__global__ void __launch_bounds__(64) k_jacobian_factor(int np, const int *__restrict__ fil_start,
+                                                        const double *__restrict__ rows, double *__restrict__ tri,
+                                                        int nt, FilConsts k, double a, double ah,
+                                                        int *__restrict__ flags, const int *__restrict__ keep) {
+  extern __shared__ __align__(16) double tri_smem[];
   if (keep && *keep) return;
-  const int f = blockIdx.x;
-  const int nw = fil_start[f + 1] - fil_start[f];
-  if (nw < 2) return;
-  const int m = 3 * nw;
-  const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5;
-  double *Sg = Sinv_all + soff[f];
-  for (int e = tid; e < m * m; e += nthr) S[e] = Sg[e];
-  __syncthreads();
-  // Gauss-Jordan inversion in place with partial pivoting (first maximum wins).
-  // Thread (g, c) owns column c for rows g, g + G, ...; per pivot: search (warp 0),
-  // swap + scale of the pivot row and a copy of column kc, elimination.
-  const int G = nthr / m;
-  const bool act = tid < G * m;
-  const int cj = tid % m, g0 = tid / m;
-  for (int kc = 0; kc < m; ++kc) {
-    if (warp == 0) {
-      double best = -1.0;
-      int bi = kc;
-      for (int r = kc + lane; r < m; r += 32) {
-        double v = fabs(S[r * m + kc]);
-        if (v > best) { best = v; bi = r; }
-      }
-      for (int o = 16; o > 0; o >>= 1) {
-        double ob = __shfl_xor_sync(0xffffffffu, best, o);
-        int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-      }
-      if (lane == 0) {
-        s_piv = bi;
-        s_inv = 1.0 / S[bi * m + kc];
-        s_diag = S[kc * m + kc];
-        perm[kc] = bi;
-        if (!(best > 0.0)) atomicOr(&flags[FLAG_PIVOT], 1);
-      }
-    }
-    __syncthreads();
-    const int p = s_piv;
-    const double inv = s_inv;
-    if (act && g0 == 0) {
-      const double a = S[kc * m + cj], b = S[p * m + cj];
-      if (p != kc) S[p * m + cj] = a;
-      S[kc * m + cj] = (cj == kc) ? inv : b * inv;  // in place: the pivot column turns into inv
-    }
-    for (int r = tid; r < m; r += nthr) fcol[r] = (r == p && p != kc) ? s_diag : (r == kc ? 0.0 : S[r * m + kc]);
-    __syncthreads();
-    if (act) {
-      const double prow = S[kc * m + cj];
-      for (int r = g0; r < m; r += G) {
-        if (r == kc) continue;
-        const double base = (cj == kc) ? 0.0 : S[r * m + cj];
-        S[r * m + cj] = base - fcol[r] * prow;
-      }
-    }
-    __syncthreads();
-  }
-  // undo the row interchanges on the columns: column c of the inverse is column colsrc[c]
-  if (tid == 0) {
-    for (int c = 0; c < m; ++c) colsrc[c] = c;
-    for (int kc = m - 1; kc >= 0; --kc) {
-      const int p = perm[kc];
-      if (p != kc) {
-        const int t = colsrc[kc];
-        colsrc[kc] = colsrc[p];
-        colsrc[p] = t;
-      }
-    }
+  const int f = blockIdx.x, tid = threadIdx.x, lane = tid & 31, side = tid >> 5;
+  const int b0 = fil_start[f], nw = fil_start[f + 1] - b0, nl = nw - 1, mid = nw / 2;
+  if (nw < 2) return;  // J0 is the identity
+  double *bead = tri_smem + 72;  // W of the two chains' last bead first
+  for (int e = tid; e < TRI_ROW * nw; e += 64) {
+    const int r = e / nw, kk = e - r * nw;
+    bead[TRI_ROW * kk + r] = rows[(size_t)r * np + b0 + kk];
   }
   __syncthreads();
-  for (int e = tid; e < m * m; e += nthr) {
-    const int r = e / m, c = e - r * m;
-    Sg[e] = S[r * m + colsrc[c]];
+  const double fac = 0.5 * k.dl, dd_a = tri_dd(nt, k, a), dd_h = tri_dd(nt, k, ah), ee_a = tri_ee(nt, k, a);
+  const int part = lane / 6, c = lane % 6;  // 0 D, 1 identity, 2 towards, 3 from (lanes 24.. idle)
+  double *out = tri + (size_t)TRI * b0;
+  bool singular = false;
+  const int steps = side == 0 ? mid + 1 : nl - mid;
+  for (int s = 0; s < steps; ++s) {
+    const int kk = side == 0 ? s : nl - s;
+    if (kk == mid) __syncthreads();  // the second chain is done; it waits below
+    const double *E = bead + TRI_ROW * kk;
+    const bool last = kk == nl;
+    const double dd = last ? 1.0 : kk == 0 ? dd_h : dd_a, ee = kk < nl - 1 ? ee_a : 0.0;
+    const double ddp = kk == 0 || last ? 0.0 : kk == 1 ? dd_h : dd_a, eep = kk > 0 && !last ? ee_a : 0.0;
+    const int dir = side == 0 ? 1 : -1;
+    double v[6];
+    if (part == 1 || part > 3) {
+#pragma unroll
+      for (int i = 0; i < 6; ++i) v[i] = part == 1 && i == c ? 1.0 : 0.0;
+    } else {
+      const int which = part == 0 ? 0 : part == 2 ? dir : -dir;
+      if ((which < 0 && kk == 0) || (which > 0 && last)) {
+#pragma unroll
+        for (int i = 0; i < 6; ++i) v[i] = 0.0;
+      } else {
+        tri_column(v, which, c, E, last, fac, dd, ee, ddp, eep);
+      }
+    }
+    if (part == 0) {
+      if (kk > 0 && kk <= mid) {  // D -= A W_{k-1}
+        double w[6];
+#pragma unroll
+        for (int l = 0; l < 6; ++l) w[l] = tri_smem[6 * l + c];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          v[i] -= (E[9 * i] * w[0] + E[9 * i + 1] * w[1] + E[9 * i + 2] * w[2]) +
+                  (E[27 + 3 * i] * w[3] + E[28 + 3 * i] * w[4] + E[29 + 3 * i] * w[5]);
+          v[3 + i] += ddp * w[3 + i];
+        }
+      }
+      if (kk < nl && kk >= mid) {  // D -= G W_{k+1}
+        double w[6];
+        const double *t = E + TRI_ROW + 36;
+#pragma unroll
+        for (int l = 0; l < 6; ++l) w[l] = tri_smem[36 + 6 * l + c];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          v[i] -= E[9 * i + 6] * w[0] + E[9 * i + 7] * w[1] + E[9 * i + 8] * w[2];
+          v[3 + i] -= fac * (w[(i + 1) % 3] * t[(i + 2) % 3] - w[(i + 2) % 3] * t[(i + 1) % 3]) + ee * w[3 + i];
+        }
+      }
+    }
+    unsigned used = 0, pos = 0;  // pivot rows taken; the column each register row served
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+      double col[6];
+#pragma unroll
+      for (int i = 0; i < 6; ++i) col[i] = __shfl_sync(0xffffffffu, v[i], j);
+      // the largest remaining entry, to the 17 leading bits of its significand
+      unsigned key[6];
+#pragma unroll
+      for (int i = 0; i < 6; ++i)
+        key[i] = (used >> i) & 1u ? 0u : (((unsigned)__double2hiint(col[i]) & 0x7ffffff8u) | (unsigned)i);
+      const int pr = max(max(max(key[0], key[1]), max(key[2], key[3])), max(key[4], key[5])) & 7u;
+      used |= 1u << pr;
+      pos |= (unsigned)j << (4 * pr);
+      const bool h0 = pr & 1, h1 = pr & 2, h2 = pr & 4;
+      const double piv = h2 ? (h0 ? col[5] : col[4]) : h1 ? (h0 ? col[3] : col[2]) : (h0 ? col[1] : col[0]);
+      double x = h2 ? (h0 ? v[5] : v[4]) : h1 ? (h0 ? v[3] : v[2]) : (h0 ? v[1] : v[0]);
+      singular |= !(fabs(piv) > 0.0);
+      x *= 1.0 / piv;
+#pragma unroll
+      for (int i = 0; i < 6; ++i) v[i] = pr == i ? x : v[i] - col[i] * x;
+    }
+    __syncwarp();  // the W before is no longer read
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+      const int j = (pos >> (4 * i)) & 7u;
+      if (part >= 1 && part <= 3) out[(size_t)TRI * kk + 36 * (part - 1) + 6 * j + c] = v[i];
+      if (part == 2) tri_smem[36 * side + 6 * j + c] = v[i];
+    }
+    __syncwarp();
   }
+  if (side == 1) __syncthreads();
+  if (singular && lane == 0) atomicOr(&flags[FLAG_PIVOT], 1);
 }
 
-// The same inversion with the matrix in registers, for m = 3 nw <= 96: warp
-// w = cb RB + rb (RB = ceil(m / 32) row blocks, CB = ceil(m / 24) column blocks)
-// holds rows 32 rb .. 32 rb + 31 (one per lane) of columns 24 cb .. 24 cb + 23:
-// 12 warps at m = 96, two matrices per SM.
-// Per pivot kc (row p and 1 / S[p][kc], found by the previous step):
-//   A: the lane holding row p publishes it scaled (prow = row p / v, with
-//      1 / v in column kc), the lane holding row kc publishes its old row, the
-//      warps holding column kc publish it (fcol);
-//   B: row r := r - fcol[r] prow for every r != kc (row p, the old row kc,
-//      takes the old (kc, kc) entry as its factor), row kc := prow, column kc
-//      of the other rows := -fcol[r] / v; then the warps holding column kc + 1
-//      search it over rows > kc (first maximum, by shuffles, per row block).
-// Each element sees the operations and roundings of k_schur_gj; two barriers per
-// pivot, one register-blocked outer product per thread.
-constexpr int GJ_CW = 24;        // columns per warp
-constexpr int GJ_MAX_M = 96;     // m handled by the register kernel
-__global__ void __launch_bounds__(384, 2) k_schur_gj_reg(const int *__restrict__ fil_start,
-                                                      const long long *__restrict__ soff,
-                                                      double *__restrict__ Sinv_all, int *__restrict__ flags,
-                                                      const int *__restrict__ keep) {
-  constexpr int CW = GJ_CW;
-  __shared__ double fcol[GJ_MAX_M], rowkc[GJ_MAX_M + CW];
-  __shared__ __align__(16) double prow_s[GJ_MAX_M + CW];
-  __shared__ double cand_v[3], cand_inv[3];
-  __shared__ int cand_r[3];
-  __shared__ int perm[GJ_MAX_M], colsrc[GJ_MAX_M], dstcol[GJ_MAX_M];
-  if (keep && *keep) return;
-  const int f = blockIdx.x;
-  const int nw = fil_start[f + 1] - fil_start[f], m = 3 * nw;
-  if (nw < 2 || m > GJ_MAX_M) return;  // block-uniform
-  const int RB = (m + 31) >> 5, CB = (m + CW - 1) / CW;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const bool wact = w < RB * CB;  // warp-uniform; spare warps only take the barriers
-  const int cb = w / RB, rb = w - cb * RB;
-  const int r = 32 * rb + lane, c0 = CW * cb;
-  double *Sg = Sinv_all + soff[f];
-  double a[CW];
-#pragma unroll
-  for (int k = 0; k < CW; ++k) a[k] = (wact && r < m && c0 + k < m) ? Sg[(size_t)r * m + c0 + k] : 0.0;
-  // first maximum of |a[k]| (k a compile-time slot after unrolling) over rows >
-  // after in this row block -> cand[rb]
-  auto search = [&](int k, int after) {
-    double v = 0.0;
-#pragma unroll
-    for (int kk = 0; kk < CW; ++kk)
-      if (kk == k) v = a[kk];
-    double best = (r > after && r < m) ? fabs(v) : -1.0, x = v;
-    int bi = r;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      const double ox = __shfl_xor_sync(0xffffffffu, x, o);
-      if (ob > best || (ob == best && oi < bi)) {
-        best = ob;
-        bi = oi;
-        x = ox;
-      }
-    }
-    if (lane == 0) {
-      cand_v[rb] = best;
-      cand_r[rb] = bi;
-      cand_inv[rb] = best >= 0.0 ? 1.0 / x : 0.0;
-    }
-  };
-  if (wact && cb == 0) search(0, -1);
-  __syncthreads();
-  // pivots kc = CW kb + kk: kk unrolled, so column kc is register slot kk of the
-  // warps with cb == kb
-  for (int kb = 0; kb < CB; ++kb) {
-#pragma unroll
-    for (int kk = 0; kk < CW; ++kk) {
-      const int kc = CW * kb + kk;
-      if (kc >= m) break;  // block-uniform
-      // phase A
-      double best = -1.0, inv = 0.0;
-      int p = kc;
-#pragma unroll
-      for (int q = 0; q < 3; ++q)
-        if (q < RB && cand_v[q] > best) {
-          best = cand_v[q];
-          p = cand_r[q];
-          inv = cand_inv[q];
-        }
-      if (wact) {
-        if (r == p) {
-#pragma unroll
-          for (int k = 0; k < CW; ++k) prow_s[c0 + k] = (cb == kb && k == kk) ? inv : a[k] * inv;
-        }
-        if (r == kc) {
-#pragma unroll
-          for (int k = 0; k < CW; ++k) rowkc[c0 + k] = a[k];
-        }
-        if (cb == kb && r < m) fcol[r] = a[kk];
-      }
-      if (threadIdx.x == 0) {
-        perm[kc] = p;
-        if (!(best > 0.0)) atomicOr(&flags[FLAG_PIVOT], 1);
-      }
-      __syncthreads();
-      // phase B
-      if (wact) {
-        if (r == kc) {
-#pragma unroll
-          for (int k = 0; k < CW; k += 2) {
-            const double2 q = *reinterpret_cast<const double2 *>(&prow_s[c0 + k]);
-            a[k] = q.x;
-            a[k + 1] = q.y;
-          }
-        } else {
-          const bool rp = (r == p);  // row p: the old row kc, factor = old (kc, kc)
-          const double fr = fcol[rp ? kc : (r < m ? r : 0)];
-          if (rp) {
-#pragma unroll
-            for (int k = 0; k < CW; ++k) a[k] = rowkc[c0 + k];
-          }
-          if (cb == kb) a[kk] = 0.0;
-#pragma unroll
-          for (int k = 0; k < CW; k += 2) {
-            const double2 q = *reinterpret_cast<const double2 *>(&prow_s[c0 + k]);
-            a[k] = a[k] - fr * q.x;
-            a[k + 1] = a[k + 1] - fr * q.y;
-          }
-        }
-        if (kc + 1 < m) {
-          if (kk + 1 < CW) {
-            if (cb == kb) search(kk + 1, kc);
-          } else if (cb == kb + 1) {
-            search(0, kc);
-          }
-        }
-      }
-      __syncthreads();
-    }
-  }
-  // undo the row interchanges on the columns: output column c is column colsrc[c]
-  if (threadIdx.x == 0) {
-    for (int c = 0; c < m; ++c) colsrc[c] = c;
-    for (int kc = m - 1; kc >= 0; --kc) {
-      const int p = perm[kc];
-      if (p != kc) {
-        const int t = colsrc[kc];
-        colsrc[kc] = colsrc[p];
-        colsrc[p] = t;
-      }
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x < m) dstcol[colsrc[threadIdx.x]] = threadIdx.x;
-  __syncthreads();
-  if (wact && r < m) {
-#pragma unroll
-    for (int k = 0; k < CW; ++k)
-      if (c0 + k < m) Sg[(size_t)r * m + dstcol[c0 + k]] = a[k];
-  }
+// v -= M (v of lanes src .. src + 5): one link of a chain, lane row i of M's six
+__device__ __forceinline__ double tri_link(double g, const double *row, double v, int src) {
+  const double2 t0 = *reinterpret_cast<const double2 *>(row), t1 = *reinterpret_cast<const double2 *>(row + 2),
+                t2 = *reinterpret_cast<const double2 *>(row + 4);
+  const double v0 = __shfl_sync(0xffffffffu, v, src), v1 = __shfl_sync(0xffffffffu, v, src + 1),
+               v2 = __shfl_sync(0xffffffffu, v, src + 2), v3 = __shfl_sync(0xffffffffu, v, src + 3),
+               v4 = __shfl_sync(0xffffffffu, v, src + 4), v5 = __shfl_sync(0xffffffffu, v, src + 5);
+  return (g - (t0.x * v0 + t0.y * v1 + t1.x * v2)) - (t1.y * v3 + t2.x * v4 + t2.y * v5);
 }
 
-// x = J0^-1 b for one filament (shared-memory vectors; 128 threads)
-// b: 6nw entries [first-bead position rows | constraint rows | Lie rows]
-// x: 6nw entries [X0 | U | lambda/dt]
-// aux_g: the filament's D', F', tangents and P coefficient in HBM; aux: shared
-// memory for their copy (the serial link recurrences then wait on shared, not
-// global, loads)
-__device__ void schur_apply_one(int nw, const double *__restrict__ Sinv, const double *__restrict__ aux_g,
-                                double *aux, const double *bb, double *x, double *y, double *w, double dt,
-                                double fac) {
-  const int m = 3 * nw, nl = nw - 1;
-  const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarp = nthr >> 5;
-  for (int i = tid; i < 20 * nl + 3 * nw + 1; i += nthr) aux[i] = aux_g[i];
-  __syncthreads();
-  const double *dd = aux, *ee = aux + nl, *Fd = aux + 2 * nl, *Fl = Fd + 9 * nl, *tt = Fl + 9 * nl;
-  const double pcoef = tt[3 * nw];
-  const double *b1 = bb + 3, *b2 = bb + m;
-  // y = D'^-1 b1
-  if (tid < 3) {
-    const int d = tid;
-    for (int r = nl - 1; r >= 0; --r) {
-      double nxt = (r + 1 < nl) ? ee[r] * y[3 * (r + 1) + d] : 0.0;
-      y[3 * r + d] = (b1[3 * r + d] - nxt) / dd[r];
-    }
+// J0^-1 b for one filament of nw >= 2 beads, by one warp and in place. b (shared): 6nw entries
+// [first-bead position rows | constraint rows | Lie rows], then [X0 | U | lambda/dt]. wt
+// (shared, 16-byte aligned): 72nw doubles; y (shared): 6nw.
+__device__ __forceinline__ void tri_apply(int nw, const double *__restrict__ tri, double *b, double *wt, double *y,
+                                          double dt, double pcoef) {
+  const int lane = threadIdx.x & 31, nl = nw - 1, m = 3 * nw, mid = nw / 2;
+  const unsigned dst = (unsigned)__cvta_generic_to_shared(wt);
+  for (int e = lane; e < 36 * nw; e += 32) {  // W and T arrive while the lanes form y_k = Dk^-1 r_k
+    const int kk = e / 36, j = e - 36 * kk;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * e),
+                 "l"(tri + (size_t)TRI * kk + 36 + 2 * j)
+                 : "memory");
   }
-  __syncthreads();
-  // w = b2 - F' y
-  for (int row = tid; row < m; row += nthr) {
-    const int kb = row / 3, i2 = row % 3;
-    double g = 0.0;
-    if (kb < nl) g += Fd[9 * kb + 3 * i2] * y[3 * kb] + Fd[9 * kb + 3 * i2 + 1] * y[3 * kb + 1] + Fd[9 * kb + 3 * i2 + 2] * y[3 * kb + 2];
-    if (kb >= 1)
-      g += Fl[9 * (kb - 1) + 3 * i2] * y[3 * (kb - 1)] + Fl[9 * (kb - 1) + 3 * i2 + 1] * y[3 * (kb - 1) + 1] +
-           Fl[9 * (kb - 1) + 3 * i2 + 2] * y[3 * (kb - 1) + 2];
-    w[row] = b2[row] - g;
-  }
-  __syncthreads();
-  // u = S^-1 w: each warp takes eight rows at a time (coalesced row reads, all
-  // of their loads in flight together); per row the lane-strided sum and the
-  // shuffle tree of a one-row-per-warp product
-  double *u = x + 3;
-  constexpr int RU = 8;
-  for (int row0 = warp * RU; row0 < m; row0 += nwarp * RU) {
-    double acc[RU];
-#pragma unroll
-    for (int q = 0; q < RU; ++q) acc[q] = 0.0;
+  const double *b1 = b + 3, *b2 = b + m;
 #pragma unroll 3
-    for (int c = lane; c < m; c += 32) {
-      const double wc = w[c];
-#pragma unroll
-      for (int q = 0; q < RU; ++q)
-        if (row0 + q < m) acc[q] += Sinv[(size_t)(row0 + q) * m + c] * wc;
-    }
-#pragma unroll
-    for (int q = 0; q < RU; ++q)
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
-    if (lane == 0)
-#pragma unroll
-      for (int q = 0; q < RU; ++q)
-        if (row0 + q < m) u[row0 + q] = acc[q];
+  for (int e = lane; e < 6 * nw; e += 32) {
+    const int kk = e / 6, i = e - 6 * kk;
+    const double2 *d = reinterpret_cast<const double2 *>(tri + (size_t)TRI * kk + 6 * i);
+    const double2 d0 = d[0], d1 = d[1], d2 = d[2];
+    double r[3] = {0.0, 0.0, 0.0};
+    if (kk < nl)
+      for (int c = 0; c < 3; ++c) r[c] = kk > 0 ? b1[3 * kk + c] - b1[3 * kk - 3 + c] : b1[c];
+    y[e] = (d0.x * b2[3 * kk] + d0.y * b2[3 * kk + 1] + d1.x * b2[3 * kk + 2]) + (d1.y * r[0] + d2.x * r[1] + d2.y * r[2]);
   }
-  __syncthreads();
-  // z = b1 - C u, (C u)_r = fac c_0 + 2 fac sum_{1<=q<=r} c_q + fac c_{r+1}, c_q = cross(u_q, t_q)
-  // (y is reused for z, then for lambda)
-  if (tid < 3) {
-    const int d = tid;
-    const int d1 = (d + 1) % 3, d2 = (d + 2) % 3;
-    double c0 = u[d1] * tt[d2] - u[d2] * tt[d1];
-    double run = 0.0;
-    for (int r = 0; r < nl; ++r) {
-      const int q = r + 1;
-      double cq = u[3 * q + d1] * tt[3 * q + d2] - u[3 * q + d2] * tt[3 * q + d1];
-      double cu = fac * c0 + 2.0 * fac * run + fac * cq;
-      y[3 * r + d] = b1[3 * r + d] - cu;
-      run += cq;
-    }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncwarp();
+  // lanes 0..5: the chain from the first bead; 8..13: from the last (other lanes follow along)
+  const bool down = lane & 8;
+  const int src = down ? 8 : 0, i = (lane & 7) < 6 ? lane & 7 : 0;
+  const bool mine = lane < 16 && (lane & 7) < 6;
+  double v = y[6 * (down ? nl : 0) + i];
+  for (int s = 1; s < mid; ++s) {  // inwards
+    const int kk = down ? nl - s : s;
+    const bool on = !down || kk > mid;
+    const double u = tri_link(y[6 * kk + i], wt + 72 * kk + 36 + 6 * i, v, src);
+    if (on) v = u;
+    if (on && mine) y[6 * kk + i] = v;
   }
-  __syncthreads();
-  // lambda = D'^-1 z (in place), then X0 = b0 - P lambda
-  if (tid < 3) {
-    const int d = tid;
-    for (int r = nl - 1; r >= 0; --r) {
-      double nxt = (r + 1 < nl) ? ee[r] * y[3 * (r + 1) + d] : 0.0;
-      y[3 * r + d] = (y[3 * r + d] - nxt) / dd[r];
-    }
-    x[d] = bb[d] - pcoef * y[d];
+  {  // the middle: T_m of the first chain, W_m of the second
+    double u = tri_link(0.0, wt + 72 * mid + (down ? 0 : 36) + 6 * i, v, src);
+    if (down && mid == nl) u = 0.0;
+    const double o = __shfl_xor_sync(0xffffffffu, u, 8);
+    v = y[6 * mid + i] + (down ? o + u : u + o);
+    __syncwarp();
+    if (mine && !down) y[6 * mid + i] = v;
   }
-  __syncthreads();
-  for (int i = tid; i < 3 * nl; i += nthr) x[3 + m + i] = y[i] / dt;
-  __syncthreads();
+  for (int s = 1; s <= mid; ++s) {  // outwards
+    const int kk = down ? (mid + s < nl ? mid + s : nl) : mid - s;
+    const bool on = !down || mid + s <= nl;
+    const double u = tri_link(y[6 * kk + i], wt + 72 * kk + 6 * i, v, src);
+    if (on) v = u;
+    if (on && mine) y[6 * kk + i] = v;
+  }
+  __syncwarp();
+  for (int e = lane; e < m; e += 32) {
+    const int kk = e / 3, d = e - 3 * kk;
+    b[3 + e] = y[6 * kk + d];
+    if (kk < nl) b[3 + m + e] = y[6 * kk + 3 + d] / dt;  // the reference's 1/dt rows (Filament.hpp:863-865)
+  }
+  if (lane < 3) b[lane] -= pcoef * y[3 + lane];
+  __syncwarp();
 }
+__host__ __device__ constexpr int tri_apply_doubles(int nw) { return (72 + 6 + 6) * nw; }
 
-// x_f = J0_f^-1 b_f, then x += sum_i C_i dots_i (FilamentJacobianSolver.hpp:49-73)
-__global__ void __launch_bounds__(128) k_schur_apply(const int *__restrict__ fil_start,
-                                                     const long long *__restrict__ soff,
-                                                     const long long *__restrict__ aoff,
-                                                     const double *__restrict__ Sinv_all,
-                                                     const double *__restrict__ aux_all, const double *__restrict__ b,
-                                                     double *__restrict__ x, const double *__restrict__ C,
-                                                     const double *__restrict__ dots, int iter,
-                                                     const int *__restrict__ iter_d,
-                                                     const int *__restrict__ off_d, size_t n6, double dt,
-                                                     double fac) {
-  __shared__ double bb[6 * FS_MAX_NW], xs[6 * FS_MAX_NW], y[3 * FS_MAX_NW], w[3 * FS_MAX_NW];
-  __shared__ double auxs[20 * (FS_MAX_NW - 1) + 3 * FS_MAX_NW + 1];
-  const int f = blockIdx.x;
+// x_f = J0_f^-1 b_f (one bead: the identity), then x += sum_i C_i dots_i
+// (FilamentJacobianSolver.hpp:49-73); a warp per filament. Bound by the latency of the two
+// chains (a shuffle and two dependent products per bead) and the factors' load before them.
+// 1,024 filaments of 32 beads, 6 columns: 34 us.
+__global__ void __launch_bounds__(32 * TRI_APPLY_WARPS) k_tri_apply(
+    int nfil, const int *__restrict__ fil_start, const double *__restrict__ tri, const double *__restrict__ b,
+    double *__restrict__ x, const double *__restrict__ C, const double *__restrict__ dots, int iter,
+    const int *__restrict__ iter_d, const int *__restrict__ off_d, size_t n6, double dt, double pcoef, int max_nw) {
+  extern __shared__ __align__(16) double tri_smem[];
+  const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+  const int f = blockIdx.x * TRI_APPLY_WARPS + wl;
+  if (f >= nfil) return;  // warp-uniform; no block barrier below
   const int b0 = fil_start[f], nw = fil_start[f + 1] - b0, s0 = 6 * b0, n = 6 * nw;
-  const int tid = threadIdx.x, nthr = blockDim.x;
-  for (int r = tid; r < n; r += nthr) bb[r] = b[s0 + r];
-  __syncthreads();
-  if (nw < 2) {
-    for (int r = tid; r < n; r += nthr) xs[r] = bb[r];
-    __syncthreads();
-  } else {
-    schur_apply_one(nw, Sinv_all + soff[f], aux_all + aoff[f], auxs, bb, xs, y, w, dt, fac);
-  }
+  double *wt = tri_smem + (size_t)wl * tri_apply_doubles(max_nw), *bb = wt + 72 * max_nw, *y = bb + 6 * max_nw;
+  for (int r = lane; r < n; r += 32) bb[r] = b[s0 + r];
+  __syncwarp();
+  if (nw >= 2) tri_apply(nw, tri + (size_t)TRI * b0, bb, wt, y, dt, pcoef);
   const int ncol = (iter_d ? *iter_d : iter) + (off_d ? *off_d : 0);
-  for (int r = tid; r < n; r += nthr) {
-    double v = xs[r];
-#pragma unroll 4
+  for (int r = lane; r < n; r += 32) {
+    double v = bb[r];
+#pragma unroll 8
     for (int i = 0; i < ncol; ++i) v += C[(size_t)i * n6 + s0 + r] * dots[i];
     x[s0 + r] = v;
   }
 }
 
 // explicit inverse of filament f's J0 (with the 1/dt rows), one column per CTA (test access)
-__global__ void __launch_bounds__(128) k_schur_inverse(int nw, const double *__restrict__ Sinv,
-                                                       const double *__restrict__ aux, double dt, double fac,
-                                                       double *__restrict__ out) {
-  __shared__ double bb[6 * FS_MAX_NW], xs[6 * FS_MAX_NW], y[3 * FS_MAX_NW], w[3 * FS_MAX_NW];
-  __shared__ double auxs[20 * (FS_MAX_NW - 1) + 3 * FS_MAX_NW + 1];
-  const int n = 6 * nw, e = blockIdx.x, tid = threadIdx.x;
-  for (int r = tid; r < n; r += blockDim.x) bb[r] = (r == e) ? 1.0 : 0.0;
-  __syncthreads();
-  if (nw < 2) {
-    for (int r = tid; r < n; r += blockDim.x) xs[r] = bb[r];
-    __syncthreads();
-  } else {
-    schur_apply_one(nw, Sinv, aux, auxs, bb, xs, y, w, dt, fac);
-  }
-  for (int r = tid; r < n; r += blockDim.x) out[(size_t)r * n + e] = xs[r];
+__global__ void __launch_bounds__(32) k_tri_inverse(int nw, const double *__restrict__ tri, double dt, double pcoef,
+                                                    double *__restrict__ out) {
+  extern __shared__ __align__(16) double tri_smem[];
+  double *bb = tri_smem + 72 * nw, *y = bb + 6 * nw;
+  const int n = 6 * nw, e = blockIdx.x, lane = threadIdx.x;
+  for (int r = lane; r < n; r += 32) bb[r] = (r == e) ? 1.0 : 0.0;
+  __syncwarp();
+  if (nw >= 2) tri_apply(nw, tri, bb, tri_smem, y, dt, pcoef);
+  for (int r = lane; r < n; r += 32) out[(size_t)r * n + e] = bb[r];
 }
 
 // ---- error check ---------------------------------------------------------------
@@ -1287,44 +1102,33 @@ fs_status fil_jacobian_build(fs_ctx *c, int nt, const int *keep) {
   ProfScope ps(c, FS_STAGE_JACOBIAN);
   FilConsts k = make_fconsts(c);
   k.tt = nt * c->p.dt;
-  const size_t smem = sizeof(double) * 9 * (size_t)c->max_nw * c->max_nw;
-  // one thread per Schur column (3 Nw, rounded to warps): three filaments share an SM
-  const int jthreads = std::min(256, 32 * ((3 * c->max_nw + 31) / 32));
-  k_jacobian_schur<<<c->nfil, jthreads, smem, c->stream>>>(c->fil_start, c->qs, c->Us, c->TAU, c->lam, c->kap, c->cc,
-                                                      c->soff, c->aoff, c->Sinv, c->aux, nt, k, c->p.a, c->p.ah,
-                                                      c->flags, keep);
+  if (c->np == 0) return FS_OK;
+  double *rows = c->jtri + (size_t)TRI * c->np;
+  k_jacobian_rows<<<fs_blocks(c->np, 128), 128, 0, c->stream>>>(c->np, c->fil_id, c->fil_start, c->qs, c->Us, c->TAU,
+                                                                c->lam, c->kap, c->cc, rows, k, c->p.a, c->p.ah, keep);
   FS_LAUNCH_CHECK();
-  // all filaments of at most 32 beads: the register kernel; otherwise the
-  // shared-memory kernel for every filament
-  if (3 * c->max_nw <= GJ_MAX_M) {
-    const int m = 3 * c->max_nw, warps = ((m + 31) / 32) * ((m + GJ_CW - 1) / GJ_CW);
-    k_schur_gj_reg<<<c->nfil, 32 * warps, 0, c->stream>>>(c->fil_start, c->soff, c->Sinv, c->flags, keep);
-  } else {
-    k_schur_gj<<<c->nfil, 384, smem, c->stream>>>(c->fil_start, c->soff, c->Sinv, c->flags, keep);
-  }
+  k_jacobian_factor<<<c->nfil, 64, sizeof(double) * (72 + TRI_ROW * c->max_nw), c->stream>>>(
+      c->np, c->fil_start, rows, c->jtri, nt, k, c->p.a, c->p.ah, c->flags, keep);
   FS_LAUNCH_CHECK();
   return FS_OK;
 }
 
 fs_status fil_jacobian_prepare(fs_ctx *c) {
   if (c->max_nw > FS_MAX_NW) return FS_ERR_INVALID_ARG;
-  const size_t smem = sizeof(double) * 9 * (size_t)c->max_nw * c->max_nw;
-  FS_CUDA(cudaFuncSetAttribute(k_jacobian_schur, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  FS_CUDA(cudaFuncSetAttribute(k_schur_gj, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  FS_CUDA(cudaFuncSetAttribute(k_tri_apply, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)(sizeof(double) * TRI_APPLY_WARPS * tri_apply_doubles(FS_MAX_NW))));
   return FS_OK;
 }
 
-int fil_aux_size(int nw) { return nw < 2 ? 1 : 20 * (nw - 1) + 3 * nw + 1; }
+size_t fil_jacobian_doubles(int np) { return (size_t)(TRI + TRI_ROW) * np; }
+
+// P's coefficient (temp / dt, Filament.hpp:820-830)
+static double tri_pcoef(const fs_ctx *c) { return (c->p.dt / (9 * FS_PI * c->p.mu * c->p.ah)) / c->p.dt; }
 
 fs_status fil_jacobian_inverse(fs_ctx *c, int f, double *out_d) {
-  int fs_h[2];
-  long long so, ao;
-  FS_CUDA(cudaMemcpyAsync(fs_h, c->fil_start + f, 2 * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-  FS_CUDA(cudaMemcpyAsync(&so, c->soff + f, sizeof(long long), cudaMemcpyDeviceToHost, c->stream));
-  FS_CUDA(cudaMemcpyAsync(&ao, c->aoff + f, sizeof(long long), cudaMemcpyDeviceToHost, c->stream));
-  FS_CUDA(cudaStreamSynchronize(c->stream));
-  const int nw = fs_h[1] - fs_h[0], n = 6 * nw;
-  k_schur_inverse<<<n, 128, 0, c->stream>>>(nw, c->Sinv + so, c->aux + ao, c->p.dt, 0.5 * c->p.dl, out_d);
+  const int b0 = c->fil_start_h[f], nw = c->fil_start_h[f + 1] - b0, n = 6 * nw;
+  k_tri_inverse<<<n, 32, sizeof(double) * tri_apply_doubles(nw), c->stream>>>(nw, c->jtri + (size_t)TRI * b0, c->p.dt,
+                                                                              tri_pcoef(c), out_d);
   FS_LAUNCH_CHECK();
   return FS_OK;
 }
@@ -1359,8 +1163,9 @@ fs_status fil_broyden_apply(fs_ctx *c, const double *b, double *x, int iter, con
                                                              off_d);
     FS_LAUNCH_CHECK();
   }
-  k_schur_apply<<<c->nfil, 128, 0, c->stream>>>(c->fil_start, c->soff, c->aoff, c->Sinv, c->aux, b, x, c->Cmat,
-                                                 c->dots, iter, iter_d, off_d, n6, c->p.dt, 0.5 * c->p.dl);
+  k_tri_apply<<<fs_blocks(c->nfil, TRI_APPLY_WARPS), 32 * TRI_APPLY_WARPS,
+                sizeof(double) * TRI_APPLY_WARPS * tri_apply_doubles(c->max_nw), c->stream>>>(
+      c->nfil, c->fil_start, c->jtri, b, x, c->Cmat, c->dots, iter, iter_d, off_d, n6, c->p.dt, tri_pcoef(c), c->max_nw);
   FS_LAUNCH_CHECK();
   return learn_diag_apply(c, b, x);  // learned initial inverse-Jacobian diagonal, when on
 }

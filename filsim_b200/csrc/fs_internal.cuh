@@ -100,9 +100,7 @@ struct fs_ctx {
   double *Y, *V, *W;
   double *err, *newerr, *upd, *tmp, *dE;
   double *Cmat, *Dmat;   // broyden_maxiter x 6Np
-  double *Sinv;          // per-filament inverse Schur complement (3Nw x 3Nw row-major) at soff[f]
-  double *aux;           // per-filament D', F' blocks, tangents, P coefficient at aoff[f]
-  long long *soff, *aoff;
+  double *jtri;          // factors of the filaments' J0 (fil_jacobian_doubles, fs_filament.cu)
   int max_nw, min_nw;  // longest and shortest filament
   // swimming drive (fs_set_swimming): per filament (alpha, beta, phase, wavenumber,
   // angular frequency); null when off. Spring links (fs_set_spring_links): bead
@@ -241,7 +239,7 @@ fs_status fil_initial_guess(fs_ctx *c);
 fs_status fil_forces(fs_ctx *c, int nt);
 fs_status fil_jacobian_build(fs_ctx *c, int nt, const int *keep = nullptr);
 fs_status fil_jacobian_prepare(fs_ctx *c);  // after an upload: kernel attributes for the filament lengths
-int fil_aux_size(int nw);
+size_t fil_jacobian_doubles(int np);  // doubles of c->jtri for np beads
 fs_status fil_jacobian_inverse(fs_ctx *c, int f, double *out_d);
 fs_status fil_error_check(fs_ctx *c, const double *V, const double *W, double *err, int nt);
 fs_status fil_broyden_apply(fs_ctx *c, const double *b, double *x, int iter, const int *iter_d = nullptr,

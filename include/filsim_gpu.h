@@ -398,7 +398,7 @@ enum {
   FS_STAGE_LINK = 5,        /* cell binning (ColBarri, link) */
   FS_STAGE_BARRIER = 6,     /* pair forces (ColBarri) */
   FS_STAGE_FORCES = 7,      /* unRobotArmify + filament forces + assign (Assign F) */
-  FS_STAGE_JACOBIAN = 8,    /* J build + Schur-complement inverse (Bld Jinv) */
+  FS_STAGE_JACOBIAN = 8,    /* J build and factorisation (Bld Jinv) */
   FS_STAGE_ERROR_CHECK = 9, /* ErrorChk */
   FS_STAGE_BROYDEN = 10,    /* J0^-1 applications + history (Slv Jinv) */
   FS_STAGE_UPDATE = 11,     /* state update + step */

@@ -9,10 +9,9 @@
 // LinkedList::apply_collision_barrier (:24-271) walks cells in order, and for
 // each bead i the rest of its own cell and the 13 half-shell neighbour cells,
 // adding the pair force to i and subtracting it from j. k_barrier gives each
-// bead one thread that collects every interaction it takes part in (as i and
-// as j), sorts them by the reference's visiting order
-// (cell of i, list position of i, neighbour slot, list position of j) and
-// folds them in that order, so each bead's total is bit-identical to the
+// bead a group of lanes that collects every interaction it takes part in (as i
+// and as j), orders them as the reference visits them (cell of i, list
+// position of i, neighbour slot, list position of j) and folds them in that order, so each bead's total is bit-identical to the
 // reference's sequential accumulation. Pair arithmetic uses explicit
 // round-to-nearest intrinsics (no FMA contraction) to match the reference's
 // x86-64 doubles.
@@ -30,10 +29,24 @@ struct BarrierConsts {
   int mode, np;  // pair filter (FS_BARRIER_*) and bead count
 };
 
-// bulkmap neighbour offsets (CollisionBarrierFilament.cpp:326-338)
-__constant__ int c_nb_off[13][3] = {{1, 0, 0},  {1, 1, 0},  {0, 1, 0},  {-1, 1, 0}, {1, 0, -1},
-                                    {1, 1, -1}, {0, 1, -1}, {-1, 1, -1}, {1, 0, 1}, {1, 1, 1},
-                                    {0, 1, 1},  {-1, 1, 1}, {0, 0, 1}};
+// bulkmap neighbour offsets (CollisionBarrierFilament.cpp:326-338) of slots 1..13, after slot
+// 0 (the cell itself); two bits per slot and dimension hold the offset plus one
+struct NbPack {
+  unsigned d[3];
+};
+__host__ __device__ constexpr NbPack nb_pack() {
+  const int off[14][3] = {{0, 0, 0},  {1, 0, 0},  {1, 1, 0},  {0, 1, 0}, {-1, 1, 0}, {1, 0, -1}, {1, 1, -1},
+                          {0, 1, -1}, {-1, 1, -1}, {1, 0, 1}, {1, 1, 1}, {0, 1, 1},  {-1, 1, 1}, {0, 0, 1}};
+  NbPack p = {{0, 0, 0}};
+  for (int s = 0; s < 14; ++s)
+    for (int d = 0; d < 3; ++d) p.d[d] |= (unsigned)(off[s][d] + 1) << (2 * s);
+  return p;
+}
+__device__ __forceinline__ int nb_off(int slot, int d) {
+  constexpr NbPack p = nb_pack();
+  const unsigned w = d == 0 ? p.d[0] : d == 1 ? p.d[1] : p.d[2];
+  return (int)((w >> (2 * slot)) & 3u) - 1;
+}
 
 __device__ __forceinline__ int icell(const int *M, int x, int y, int z) {
   int xx = (x + M[0]) % M[0], yy = (y + M[1]) % M[1], zz = (z + M[2]) % M[2];
@@ -45,7 +58,7 @@ __global__ void k_bulkmap(int Mx, int My, int Mz, int *__restrict__ map) {
   int M[3] = {Mx, My, Mz};
   if (c >= Mx * My * Mz) return;
   int x = c % Mx, y = (c / Mx) % My, z = c / (Mx * My);
-  for (int nb = 0; nb < 13; ++nb) map[13 * c + nb] = icell(M, x + c_nb_off[nb][0], y + c_nb_off[nb][1], z + c_nb_off[nb][2]);
+  for (int nb = 0; nb < 13; ++nb) map[13 * c + nb] = icell(M, x + nb_off(nb + 1, 0), y + nb_off(nb + 1, 1), z + nb_off(nb + 1, 2));
 }
 
 // cell of an unwrapped position (CollisionBarrierFilament.cpp:387-409)
@@ -82,20 +95,24 @@ __global__ void k_cell_lists(const int *__restrict__ start, const int *__restric
   }
 }
 
-// one pair as the reference computes it (CollisionBarrierFilament.cpp:80-149);
-// returns 1 inside the barrier range
-__device__ __noinline__ int pair_force(const BarrierConsts &k, const double *__restrict__ Yi,
-                                       const double *__restrict__ Yj, double *rsq_out, double *f) {
-  double d[3];
+// minimum-image separation of a pair and its square as the reference computes them
+// (CollisionBarrierFilament.cpp:80-100). Below 0.49 L the quotient plus one half lies within
+// (0, 1), so its floor is 0 and the separation is x itself: the division is left out.
+__device__ __forceinline__ double pair_dist(const BarrierConsts &k, const double *Yi, const double *Yj, double *d) {
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    double x = __dsub_rn(Yi[a], Yj[a]);
-    double s = floor(__dadd_rn(__ddiv_rn(x, k.L[a]), 0.5));
-    d[a] = __dsub_rn(x, __dmul_rn(k.L[a], s));
+    const double x = __dsub_rn(Yi[a], Yj[a]);
+    d[a] = x;
+    if (!(fabs(x) < 0.49 * k.L[a])) {
+      const double s = floor(__dadd_rn(__ddiv_rn(x, k.L[a]), 0.5));
+      d[a] = __dsub_rn(x, __dmul_rn(k.L[a], s));
+    }
   }
-  double rijsq = __dadd_rn(__dadd_rn(__dmul_rn(d[0], d[0]), __dmul_rn(d[1], d[1])), __dmul_rn(d[2], d[2]));
-  *rsq_out = rijsq;
-  if (!(rijsq < k.chiRnm2)) return 0;
+  return __dadd_rn(__dadd_rn(__dmul_rn(d[0], d[0]), __dmul_rn(d[1], d[1])), __dmul_rn(d[2], d[2]));
+}
+
+// force of a pair inside the barrier range (CollisionBarrierFilament.cpp:101-149)
+__device__ __forceinline__ void pair_force(const BarrierConsts &k, double *d, double rijsq, double *f) {
   if (rijsq < k.cap2) {
     double rij = __dsqrt_rn(rijsq);
 #pragma unroll
@@ -109,7 +126,6 @@ __device__ __noinline__ int pair_force(const BarrierConsts &k, const double *__r
   prefac = __dmul_rn(prefac, k.fs);
 #pragma unroll
   for (int a = 0; a < 3; ++a) f[a] = __dmul_rn(prefac, d[a]);
-  return 1;
 }
 
 __device__ __forceinline__ unsigned long long ev_key(int cell, int pos_i, int slot, int pos_j) {
@@ -126,159 +142,147 @@ __device__ __forceinline__ bool excluded(const BarrierConsts &k, const int *fil_
   return (fil_id[j] == fil_id[i] && abs(seg_id[j] - seg_id[i]) == 1) && !(k.nt < k.initial_friction_steps);
 }
 
-// mode 0: add barrier forces to F; mode 1: count i-role pairs; mode 2: write pairs
-__global__ void __launch_bounds__(128) k_barrier(const double *__restrict__ Y, double *__restrict__ F, int np,
-                                                 BarrierConsts k, const int *__restrict__ cell_of,
-                                                 const int *__restrict__ start, const int *__restrict__ sorted,
-                                                 const int *__restrict__ rank_desc, const int *__restrict__ map,
-                                                 const int *__restrict__ fil_id, const int *__restrict__ seg_id,
-                                                 unsigned long long *__restrict__ min_bits, int *__restrict__ flags,
-                                                 int mode, int *__restrict__ pair_count,
-                                                 const int *__restrict__ pair_off, int *__restrict__ pairs,
-                                                 int max_pairs) {
+// Pairs inside the range, b as i, in the reference's order: pairs == nullptr counts them per
+// bead, else writes them from pair_off[b]
+__global__ void __launch_bounds__(128) k_pairs(const double *__restrict__ Y, int np, BarrierConsts k,
+                                               const int *__restrict__ cell_of, const int *__restrict__ start,
+                                               const int *__restrict__ sorted, const int *__restrict__ rank_desc,
+                                               const int *__restrict__ map, const int *__restrict__ fil_id,
+                                               const int *__restrict__ seg_id, int *__restrict__ pair_count,
+                                               const int *__restrict__ pair_off, int *__restrict__ pairs,
+                                               int max_pairs) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= np) return;
-  const int cb = cell_of[b];
-  const int pb = rank_desc[b];
-  const int e0 = start[cb + 1];
-  const int p_asc = e0 - 1 - pb;
+  const int cb = cell_of[b], p_asc = start[cb + 1] - 1 - rank_desc[b];
   const double Yb[3] = {Y[3 * b], Y[3 * b + 1], Y[3 * b + 2]};
-  unsigned long long keys[FS_MAX_EVENTS];
-  double fx[FS_MAX_EVENTS], fy[FS_MAX_EVENTS], fz[FS_MAX_EVENTS];
-  int nev = 0, overflow = 0;
-  double local_min = 100000.0;
-  int npairs_here = 0;
-  int out_base = (mode == 2) ? pair_off[b] : 0;
-  double f[3], rsq;
-  // cell ranges of both halves loaded up front (independent loads in flight together)
-  int rs_i[14], re_i[14];
-#pragma unroll
+  int n = 0;
+  double d[3];
   for (int slot = 0; slot < 14; ++slot) {
-    const int cj = slot == 0 ? cb : map[13 * cb + slot - 1];
-    rs_i[slot] = start[cj];
-    re_i[slot] = start[cj + 1];
-  }
-  // ---- b as i: the rest of its own cell, then the 13 neighbour cells ----
-#pragma unroll 1
-  for (int slot = 0; slot < 14; ++slot) {
-    const int qs = rs_i[slot];
-    const int qe = slot == 0 ? p_asc : re_i[slot];  // own cell: ascending positions below b's
-    const int ej = re_i[slot];
+    const int cj = slot == 0 ? cb : map[13 * cb + slot - 1], qs = start[cj];
+    const int qe = slot == 0 ? p_asc : start[cj + 1];  // own cell: ascending positions below b's
     for (int q = qe - 1; q >= qs; --q) {
       const int j = sorted[q];
       if (excluded(k, fil_id, seg_id, b, j)) continue;
       const double Yj[3] = {Y[3 * j], Y[3 * j + 1], Y[3 * j + 2]};
-      if (pair_force(k, Yb, Yj, &rsq, f)) {
-        if (mode == 0) {
-          if (nev < FS_MAX_EVENTS) {
-            keys[nev] = ev_key(cb, pb, slot, ej - 1 - q);
-            fx[nev] = f[0];
-            fy[nev] = f[1];
-            fz[nev] = f[2];
-            nev++;
-          } else {
-            overflow = 1;
-          }
-        } else if (mode == 2) {
-          int o = out_base + npairs_here;
-          if (o < max_pairs) {
-            pairs[2 * o] = b;
-            pairs[2 * o + 1] = j;
-          }
-        }
-        npairs_here++;
+      if (!(pair_dist(k, Yb, Yj, d) < k.chiRnm2)) continue;
+      if (pairs && pair_off[b] + n < max_pairs) {
+        pairs[2 * (pair_off[b] + n)] = b;
+        pairs[2 * (pair_off[b] + n) + 1] = j;
       }
-      if (rsq < local_min) local_min = rsq;
+      ++n;
     }
   }
-  if (mode == 1) {
-    pair_count[b] = npairs_here;
-    return;
-  }
-  if (mode == 2) return;
-  // ---- b as j: beads before it in its own cell, and the cells whose slot maps to b's cell ----
-  const int Mx = k.M[0], My = k.M[1];
-  const int cx = cb % Mx, cy = (cb / Mx) % My, cz = cb / (Mx * My);
-  int rs_j[14], re_j[14], ci_j[14];
+  if (!pairs && pair_count) pair_count[b] = n;
+}
+
+// Barrier forces: G lanes per bead. Each lane walks some of the 28 cell ranges in which the
+// bead takes part (as i: slots 0..13; as j: the cells whose slot is its own cell), the pairs
+// in range are ordered by their keys, and the forces, a lane each, are folded in that order.
+// Bound by the latency of cell -> range -> bead -> position, so by how many of a bead's cells
+// are looked at together. With a lane for every range (G = 32) while the beads' warps fit the
+// chip in about one wave, 8 lanes beyond: with the launch before it, 480 beads 15.5 us (8
+// lanes 19.3), 3,840 beads 16.5 (20.8), 16,384 beads 24.0 (20.3), 131,072 beads 98 (62). A
+// thread per bead over all ranges took 53 us for 480 beads and 89 us for 131,072.
+constexpr int BARRIER_WIDE_PER_SM = 48;  // beads per SM
+template <int G>
+__global__ void __launch_bounds__(128) k_barrier(const double *__restrict__ Y, double *__restrict__ F, int np,
+                                                 BarrierConsts k, const int *__restrict__ cell_of,
+                                                 const int *__restrict__ start, const int *__restrict__ sorted,
+                                                 const int *__restrict__ rank_desc, const int *__restrict__ fil_id,
+                                                 const int *__restrict__ seg_id,
+                                                 unsigned long long *__restrict__ min_bits, int *__restrict__ flags) {
+  constexpr int BEADS = 128 / G;
+  __shared__ unsigned long long s_key[BEADS][FS_MAX_EVENTS];
+  __shared__ int s_other[BEADS][FS_MAX_EVENTS];  // the other bead; complemented where b is j
+  __shared__ unsigned char s_ord[BEADS][FS_MAX_EVENTS];
+  __shared__ int s_n[BEADS];
+  const int l = threadIdx.x % G, w = threadIdx.x / G;
+  const int b = blockIdx.x * BEADS + w;
+  const bool live = b < np;
+  if (l == 0) s_n[w] = 0;
+  __syncwarp();
+  double Yb[3] = {0.0, 0.0, 0.0}, d[3], local_min = 100000.0;
+  if (live) {
+    const int cb = cell_of[b], pb = rank_desc[b];
 #pragma unroll
-  for (int slot = 0; slot < 14; ++slot) {
-    const int ci = slot == 0 ? cb
-                             : icell(k.M, cx - c_nb_off[slot - 1][0], cy - c_nb_off[slot - 1][1],
-                                     cz - c_nb_off[slot - 1][2]);
-    ci_j[slot] = ci;
-    rs_j[slot] = start[ci];
-    re_j[slot] = start[ci + 1];
-  }
-#pragma unroll 1
-  for (int slot = 0; slot < 14; ++slot) {
-    int qs, qe;
-    if (slot == 0) {
-      qs = p_asc + 1;
-      qe = e0;
-    } else {
-      qs = rs_j[slot];
-      qe = re_j[slot];
-    }
-    const int ci = ci_j[slot], ei = re_j[slot];
-    for (int q = qs; q < qe; ++q) {
-      const int i = sorted[q];
-      if (excluded(k, fil_id, seg_id, i, b)) continue;
-      const double Yi[3] = {Y[3 * i], Y[3 * i + 1], Y[3 * i + 2]};
-      if (pair_force(k, Yi, Yb, &rsq, f)) {
-        if (nev < FS_MAX_EVENTS) {
-          keys[nev] = ev_key(ci, ei - 1 - q, slot, pb);
-          fx[nev] = -f[0];  // marks subtraction; folded as acc - f
-          fy[nev] = -f[1];
-          fz[nev] = -f[2];
-          nev++;
-        } else {
-          overflow = 1;
+    for (int a = 0; a < 3; ++a) Yb[a] = Y[3 * b + a];
+    const int cx = cb % k.M[0], cyz = cb / k.M[0], cy = cyz % k.M[1], cz = cyz / k.M[1];
+    for (int s = l; s < 28; s += G) {
+      const bool as_i = s < 14;
+      const int slot = as_i ? s : s - 14, sg = as_i ? 1 : -1;
+      int x = cx + sg * nb_off(slot, 0), y = cy + sg * nb_off(slot, 1), z = cz + sg * nb_off(slot, 2);
+      x = x < 0 ? x + k.M[0] : x >= k.M[0] ? x - k.M[0] : x;
+      y = y < 0 ? y + k.M[1] : y >= k.M[1] ? y - k.M[1] : y;
+      z = z < 0 ? z + k.M[2] : z >= k.M[2] ? z - k.M[2] : z;
+      const int cell = x + (y + z * k.M[1]) * k.M[0];
+      int qs = start[cell], qe = start[cell + 1];
+      const int e = qe;
+      if (slot == 0) {  // own cell: b is i to the ascending positions below its own, j to those above
+        if (as_i) qe = e - 1 - pb;
+        else qs = e - pb;
+      }
+      for (int q = qs; q < qe; ++q) {
+        const int j = sorted[q];
+        if (excluded(k, fil_id, seg_id, b, j)) continue;
+        const double Yj[3] = {Y[3 * j], Y[3 * j + 1], Y[3 * j + 2]};
+        const double rsq = as_i ? pair_dist(k, Yb, Yj, d) : pair_dist(k, Yj, Yb, d);
+        if (rsq < k.chiRnm2) {
+          const int n = atomicAdd(&s_n[w], 1);
+          if (n < FS_MAX_EVENTS) {
+            s_key[w][n] = as_i ? ev_key(cb, pb, slot, e - 1 - q) : ev_key(cell, e - 1 - q, slot, pb);
+            s_other[w][n] = as_i ? j : ~j;
+          }
         }
+        if (as_i && rsq < local_min) local_min = rsq;
       }
     }
   }
-  if (overflow) atomicOr(&flags[FLAG_CAPACITY], 1);
-  // insertion sort by visiting order
-  for (int a = 1; a < nev; ++a) {
-    unsigned long long kk = keys[a];
-    double x = fx[a], y = fy[a], z = fz[a];
-    int j = a - 1;
-    while (j >= 0 && keys[j] > kk) {
-      keys[j + 1] = keys[j];
-      fx[j + 1] = fx[j];
-      fy[j + 1] = fy[j];
-      fz[j + 1] = fz[j];
-      --j;
+  __syncwarp();
+  int n = s_n[w];
+  if (n > FS_MAX_EVENTS) {
+    if (l == 0) atomicOr(&flags[FLAG_CAPACITY], 1);
+    n = FS_MAX_EVENTS;
+  }
+  for (int e = l; e < n; e += G) {
+    const unsigned long long mine = s_key[w][e];
+    int r = 0;
+    for (int o = 0; o < n; ++o) r += s_key[w][o] < mine;
+    s_ord[w][r] = (unsigned char)e;
+  }
+  __syncwarp();
+  // fold in order: adding -f equals subtracting f exactly
+  double acc[3] = {0.0, 0.0, 0.0};
+  for (int c0 = 0; __any_sync(0xffffffffu, c0 < n); c0 += G) {
+    double f[3] = {0.0, 0.0, 0.0};
+    if (c0 + l < n) {
+      const int o = s_other[w][s_ord[w][c0 + l]], j = o < 0 ? ~o : o;
+      const double Yj[3] = {Y[3 * j], Y[3 * j + 1], Y[3 * j + 2]};
+      const double rsq = o >= 0 ? pair_dist(k, Yb, Yj, d) : pair_dist(k, Yj, Yb, d);
+      pair_force(k, d, rsq, f);
+      if (o < 0)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) f[a] = -f[a];
     }
-    keys[j + 1] = kk;
-    fx[j + 1] = x;
-    fy[j + 1] = y;
-    fz[j + 1] = z;
+    for (int e = 0; __any_sync(0xffffffffu, c0 + e < n) && e < G; ++e) {
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        const double v = __shfl_sync(0xffffffffu, f[a], e, G);
+        if (c0 + e < n) acc[a] = __dadd_rn(acc[a], v);
+      }
+    }
   }
-  // fold: adding -f equals subtracting f exactly
-  double ax = 0.0, ay = 0.0, az = 0.0;
-  for (int a = 0; a < nev; ++a) {
-    ax = __dadd_rn(ax, fx[a]);
-    ay = __dadd_rn(ay, fy[a]);
-    az = __dadd_rn(az, fz[a]);
+  if (live && l < 3) {
+    const double v = l == 0 ? acc[0] : l == 1 ? acc[1] : acc[2];
+    F[3 * b + l] = __dadd_rn(F[3 * b + l], v);
   }
-  F[3 * b] = __dadd_rn(F[3 * b], ax);
-  F[3 * b + 1] = __dadd_rn(F[3 * b + 1], ay);
-  F[3 * b + 2] = __dadd_rn(F[3 * b + 2], az);
-  // the minimum squared distance: one atomic per full warp after a shuffle
-  // reduction (per bead, all beads would contend for one address); the last,
-  // partial warp of the grid keeps per-thread atomics
+  // the minimum squared distance: an atomic per warp, and only below what is there already
   unsigned long long mb = fs_dbits(local_min);
-  if (__activemask() == 0xffffffffu) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long other = __shfl_xor_sync(0xffffffffu, mb, o);
-      mb = other < mb ? other : mb;
-    }
-    if ((threadIdx.x & 31) == 0) atomicMin(min_bits, mb);
-  } else {
-    atomicMin(min_bits, mb);
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long other = __shfl_xor_sync(0xffffffffu, mb, o);
+    mb = other < mb ? other : mb;
   }
+  if ((threadIdx.x & 31) == 0 && mb < *(volatile unsigned long long *)min_bits) atomicMin(min_bits, mb);
 }
 
 __global__ void k_pair_pos(const int *__restrict__ cell_of, const int *__restrict__ start,
@@ -384,9 +388,9 @@ fs_status cells_barrier(fs_ctx *c, const double *Y, double *F, int np, int nt, c
   if (np == 0) return FS_OK;
   const int T = 128;
   if (npairs_h) {
-    k_barrier<<<fs_blocks(np, T), T, 0, c->stream>>>(Y, F, np, k, c->cells.key, c->cells.start, c->cells.sorted,
-                                                     c->cell_rank, c->map, fil_id, seg_id, c->min_dist2_bits,
-                                                     c->flags, 1, c->pair_count, nullptr, nullptr, 0);
+    k_pairs<<<fs_blocks(np, T), T, 0, c->stream>>>(Y, np, k, c->cells.key, c->cells.start, c->cells.sorted,
+                                                   c->cell_rank, c->map, fil_id, seg_id, c->pair_count, nullptr,
+                                                   nullptr, 0);
     FS_LAUNCH_CHECK();
     // offsets in the reference's visiting order of the i beads
     k_pair_pos<<<fs_blocks(np, 256), 256, 0, c->stream>>>(c->cells.key, c->cells.start, c->cell_rank, c->pair_count,
@@ -398,16 +402,21 @@ fs_status cells_barrier(fs_ctx *c, const double *Y, double *F, int np, int nt, c
     k_pair_off<<<fs_blocks(np, 256), 256, 0, c->stream>>>(c->cells.key, c->cells.start, c->cell_rank, c->pair_count,
                                                            np, c->pair_off);
     FS_LAUNCH_CHECK();
-    k_barrier<<<fs_blocks(np, T), T, 0, c->stream>>>(Y, F, np, k, c->cells.key, c->cells.start, c->cells.sorted,
-                                                     c->cell_rank, c->map, fil_id, seg_id, c->min_dist2_bits,
-                                                     c->flags, 2, nullptr, c->pair_off, pairs_d, max_pairs);
+    k_pairs<<<fs_blocks(np, T), T, 0, c->stream>>>(Y, np, k, c->cells.key, c->cells.start, c->cells.sorted,
+                                                   c->cell_rank, c->map, fil_id, seg_id, nullptr, c->pair_off,
+                                                   pairs_d, max_pairs);
     FS_LAUNCH_CHECK();
     FS_CUDA(cudaStreamSynchronize(c->stream));
     return FS_OK;
   }
-  k_barrier<<<fs_blocks(np, T), T, 0, c->stream>>>(Y, F, np, k, c->cells.key, c->cells.start, c->cells.sorted,
-                                                   c->cell_rank, c->map, fil_id, seg_id, c->min_dist2_bits, c->flags,
-                                                   0, nullptr, nullptr, nullptr, 0);
+  if (np <= BARRIER_WIDE_PER_SM * c->num_sms)
+    k_barrier<32><<<fs_blocks(np, T / 32), T, 0, c->stream>>>(Y, F, np, k, c->cells.key, c->cells.start,
+                                                              c->cells.sorted, c->cell_rank, fil_id, seg_id,
+                                                              c->min_dist2_bits, c->flags);
+  else
+    k_barrier<8><<<fs_blocks(np, T / 8), T, 0, c->stream>>>(Y, F, np, k, c->cells.key, c->cells.start,
+                                                            c->cells.sorted, c->cell_rank, fil_id, seg_id,
+                                                            c->min_dist2_bits, c->flags);
   FS_LAUNCH_CHECK();
   return FS_OK;
 }

@@ -809,7 +809,8 @@ __host__ __device__ constexpr int tri_apply_doubles(int nw) { return (72 + 6 + 6
 // x_f = J0_f^-1 b_f (one bead: the identity), then x += sum_i C_i dots_i
 // (FilamentJacobianSolver.hpp:49-73); a warp per filament. Bound by the latency of the two
 // chains (a shuffle and two dependent products per bead) and the factors' load before them.
-// 1,024 filaments of 32 beads, 6 columns: 34 us.
+// With the dots before it, 1,024 filaments of 32 beads and 6 columns: 33 us (the columns one
+// load after another: 42); 4,096 filaments 97 us (132).
 __global__ void __launch_bounds__(32 * TRI_APPLY_WARPS) k_tri_apply(
     int nfil, const int *__restrict__ fil_start, const double *__restrict__ tri, const double *__restrict__ b,
     double *__restrict__ x, const double *__restrict__ C, const double *__restrict__ dots, int iter,
@@ -824,11 +825,29 @@ __global__ void __launch_bounds__(32 * TRI_APPLY_WARPS) k_tri_apply(
   __syncwarp();
   if (nw >= 2) tri_apply(nw, tri + (size_t)TRI * b0, bb, wt, y, dt, pcoef);
   const int ncol = (iter_d ? *iter_d : iter) + (off_d ? *off_d : 0);
-  for (int r = lane; r < n; r += 32) {
-    double v = bb[r];
-#pragma unroll 8
-    for (int i = 0; i < ncol; ++i) v += C[(size_t)i * n6 + s0 + r] * dots[i];
-    x[s0 + r] = v;
+  // three entries a lane and four columns at a time: twelve loads in flight
+  for (int r0 = lane; r0 < n; r0 += 96) {
+    double v[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) v[j] = r0 + 32 * j < n ? bb[r0 + 32 * j] : 0.0;
+    for (int i0 = 0; i0 < ncol; i0 += 4) {
+      double w[4][3], d[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        d[u] = i0 + u < ncol ? dots[i0 + u] : 0.0;
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+          w[u][j] = i0 + u < ncol && r0 + 32 * j < n ? C[(size_t)(i0 + u) * n6 + s0 + r0 + 32 * j] : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (i0 + u < ncol)
+#pragma unroll
+          for (int j = 0; j < 3; ++j) v[j] += w[u][j] * d[u];
+    }
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+      if (r0 + 32 * j < n) x[s0 + r0 + 32 * j] = v[j];
   }
 }
 

@@ -21,6 +21,7 @@
 // weights in float, with Kahan-compensated spread sums and FP64 accumulation of
 // the interpolation products.
 #include "fs_internal.cuh"
+#include <type_traits>
 #include "fs_f32x2.cuh"
 
 namespace {
@@ -329,20 +330,21 @@ __global__ void __launch_bounds__(FS_SPREAD64_THREADS, ZL == 4 ? 4 : 3)
 // ---- 2b. FP32 spread on packed pairs -------------------------------------------
 // The FP32 chain's spread. k_spread_records32 writes each bead's record with xx = xg dx - Y
 // in double and the Gaussians in float.
-// k_spread32 then runs one CTA (8 warps) per 16^3 tile, which stages tables of
-// the tile's candidate beads (by tile coordinate, from their records) and covers
-// its 16 column blocks in two passes; with the default 4 x 16 x 4 blocks, in
-// pass p warp w owns x in [4(w&3), +4), z in [4cz, +4) with cz = (w>>2) + 2p;
-// lane l owns x = 4(w&3) + (l&3), the z pair 4cz + 2((l>>2)&1) + {0, 1} and
-// y = (l>>3) + 4k, k < 4: eight points held as four packed pairs per component
-// (two blocks per warp even out the warps' bead counts; the block shape is a
-// template knob). Per staged bead reaching the warp's column the lane forms the
-// x-z factors of its pair once, then each covered y row costs three packed
-// FMA chains and three packed Kahan updates:
+// In k_spread32 a 16^3 tile is 16 column blocks, a warp each, shared out over 1, 2 or 4 CTAs. A
+// CTA lists the beads whose stencil reaches its points, stages tables of them (by tile
+// coordinate, from their records) and sums its columns; with the default 2 x 16 x 8 blocks,
+// column q has x in [2 (q % 8), +2), z in [8 (q / 8), +8) and lane l owns x = 2 (q % 8) +
+// (l & 1), the z pair 8 (q / 8) + 2 ((l >> 1) & 3) + {0, 1} and y = (l >> 3) + 4k, k < 4:
+// eight points held as four packed pairs per component. Per staged bead reaching the warp's
+// column the lane forms the x-z factors of its pair once, then each covered y row costs
+// three packed FMA chains and three packed Kahan updates:
 //   y = term + nc, t = s + y, nc = y - (t - s), s = t      (nc = -c of Kahan)
 // The sums run over the candidates in sorted bead order and are written once
 // per point (s + nc): no atomics, bit-reproducible.
-#define FS_SPREAD32_THREADS 256
+// Bound by a CTA's chain (bins -> headers -> records -> tables) on small grids and by the
+// packed updates (half of the lanes' points lie in a stencil) with that chain on large ones;
+// staging only the beads of the list (20 to 25% of the candidates) is what helps both.
+constexpr int SPREAD32_BATCH = 256;
 
 // Record of the bead in sorted slot q (float4 units): [0] stencil starts and bead id
 // (int), [1] F0, F1, F2, h0, [2] h1, h2, -, -, then (g, d, r, r d) for axis a and stencil
@@ -392,136 +394,154 @@ struct SpreadStage32 {
   float4 yw[CH][FS_TILE];                    // (g, g, d, d) by tile-local y
   float2 yrd[CH][FS_TILE];                   // (r d, r d)
   float4 fh[CH], hh[CH];                     // (F0, F1, F2, h0), (h1, h2, -, -): h = T / 2
-  unsigned xzm[CH];                          // x coverage (16 bits) | z coverage (16 bits) << 16
-  unsigned rows[CH];                         // y rows k with a covered y in [4k, 4k + 4)
+  // the beads of one batch of candidates that reach the CTA: record, covered x (16 bits) |
+  // covered z (16 bits) << 16, y rows k with a covered y in [4k, 4k + 4)
+  int list[SPREAD32_BATCH];
+  unsigned lmask[SPREAD32_BATCH];
+  unsigned char lrows[SPREAD32_BATCH];
+  int count[SPREAD32_BATCH / 32];
 };
 
-template <int CH>
-__host__ __device__ constexpr size_t spread32_smem(int) {
-  return (sizeof(SpreadStage32<CH>) + 15) / 16 * 16;
-}
-
-// CX: the shape of a warp's column block, CX x 16 x (16 / CX) points (x, y, z),
-// an autotuner knob (2, 4 or 8); a lane owns one x, one z pair and four y rows
-template <int CH, int CX>
-__global__ void __launch_bounds__(FS_SPREAD32_THREADS, 3)
+// CX: the shape of a warp's column block, CX x 16 x (16 / CX) points (x, y, z), an autotuner
+// knob (2, 4 or 8); a lane owns one x, one z pair and four y rows. NW: warps (column blocks)
+// per CTA, PASSES: columns a warp does in turn on the same tables. Measured (us, 12-point
+// stencils, 4 to 8 beads per tile), against a whole tile in two passes over all candidates:
+//   tiles               27    64   216   512   864 (20-point)   4,096   32,768
+//   before              31    39    22    35       109            234      927
+//   4 warps, 1 pass     15    21    21    34        86            270     1487
+//   8 warps, 1 pass     18    22    20    33        78            237     1308
+//   8 warps, 2 passes   27    35    27    36        86            226      992
+//   4 warps, 4 passes   53    68    47    57       121            254      909
+// so quarter tiles below one tile per SM, then half tiles; the list is made once for a whole
+// tile where there are many CTAs and few beads in each, and by four warps only if it also
+// fits one stage (4,096 tiles with twice the beads: half 306, whole 313).
+template <int CH, int CX, int NW, int PASSES>
+__global__ void __launch_bounds__(32 * NW, NW == 4 && PASSES == 4 ? 6 : 3)
     k_spread32(const int *__restrict__ bin_start, const float4 *__restrict__ rec, FcmConsts c,
                float *__restrict__ fgrid) {
   static_assert(CX == 2 || CX == 4 || CX == 8, "column widths");
   constexpr int CZ = FS_TILE / CX, NCX = FS_TILE / CX;  // z width; columns across x
+  constexpr int NT = 32 * NW, PARTS = 16 / (NW * PASSES), COLS = NW * PASSES;  // columns per CTA
+  constexpr int XW = NCX > COLS ? CX * COLS : FS_TILE, ZW = NCX > COLS ? CZ : CZ * (COLS / NCX);  // the CTA's points
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SpreadStage32<CH> &st = *reinterpret_cast<SpreadStage32<CH> *>(smem_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int tile = blockIdx.x;
+  const int part = blockIdx.x % PARTS, tile = blockIdx.x / PARTS;
   const int tz = tile % c.nbin[2], ty = (tile / c.nbin[2]) % c.nbin[1], tx = tile / (c.nbin[2] * c.nbin[1]);
   const int X0[3] = {tx * FS_TILE, ty * FS_TILE, tz * FS_TILE};
+  const int xlo = NCX > COLS ? CX * ((part * COLS) % NCX) : 0, zlo = CZ * ((part * COLS) / NCX);
+  const unsigned ctam = ((((1u << XW) - 1u) << xlo) & 0xffffu) | (((1u << ZW) - 1u) << (16 + zlo));
   __shared__ Cand cd;
-  const int K = fs_cand_bins(c.ngd), nr = K * K * K;
   cand_bins(cd, tx, ty, tz, bin_start, c);
   __syncthreads();
+  const int ngd = c.ngd, RL = spread_rec_len(ngd), K = fs_cand_bins(ngd), nr = K * K * K;
   int total = 0;
   for (int r = 0; r < nr; ++r) total += cd.len[r];
-  const int ngd = c.ngd, RL = spread_rec_len(ngd);
-  // staging of candidates [base, base + nb): tables by tile coordinate, eight
-  // threads per bead slot (thread j takes x, y and z in {j, j + 8}), each reading
-  // its slot's record (candidate base + sl: bin range r, rank q in it) from global
-  // memory; not copying the records in first keeps a CTA at 55 KB of shared memory
-  // with 64 beads per pass (92.5 KB with the copies), so three CTAs fit on an SM
-  auto stage = [&](int base, int nb) {
-    __syncthreads();  // the previous tables are no longer read
-    const int j = tid & 7;
+  const int ly = lane >> 3;
+  int nhit = 0;
 #pragma unroll 1
-    for (int s0 = 0; s0 < CH; s0 += FS_SPREAD32_THREADS / 8) {
-      const int sl = s0 + (tid >> 3);
-      const bool act = sl < nb;
-      bool cov[6] = {false, false, false, false, false, false};
-      if (act) {
-        const float4 *rw = rec + (size_t)cand_slot(cd, base + sl) * RL;
-        const float4 hd = __ldg(rw);
-        if (j == 0) {
-          st.fh[sl] = __ldg(rw + 1);
-          st.hh[sl] = __ldg(rw + 2);
-        }
-        const int swv[3] = {__float_as_int(hd.x), __float_as_int(hd.y), __float_as_int(hd.z)};
-        float4 w[6];
-#pragma unroll
-        for (int it = 0; it < 6; ++it) {
-          const int a = it >> 1, l = j + 8 * (it & 1), Nn = c.N[a];
-          const int i = wrap_near(l + wrap_near(X0[a] - swv[a], Nn), Nn);
-          cov[it] = i < ngd;
-          w[it] = cov[it] ? __ldg(rw + 3 + a * ngd + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-        st.xw[sl][j] = w[0];
-        st.xw[sl][j + 8] = w[1];
-        st.yw[sl][j] = make_float4(w[2].x, w[2].x, w[2].y, w[2].y);
-        st.yrd[sl][j] = make_float2(w[2].w, w[2].w);
-        st.yw[sl][j + 8] = make_float4(w[3].x, w[3].x, w[3].y, w[3].y);
-        st.yrd[sl][j + 8] = make_float2(w[3].w, w[3].w);
-        st.zg[sl][j] = w[4].x;
-        st.zd[sl][j] = w[4].y;
-        st.zr[sl][j] = w[4].z;
-        st.zg[sl][j + 8] = w[5].x;
-        st.zd[sl][j + 8] = w[5].y;
-        st.zr[sl][j + 8] = w[5].z;
-      }
-      // coverage masks by ballot: lanes 8q .. 8q+7 of this warp hold slot s0 + 4 warp + q
-      unsigned bal[6];
-#pragma unroll
-      for (int it = 0; it < 6; ++it) bal[it] = __ballot_sync(0xffffffffu, cov[it]);
-      if (act && j == 0) {
-        const int sh = lane & 24;
-        unsigned m3[3];
-#pragma unroll
-        for (int a = 0; a < 3; ++a) m3[a] = ((bal[2 * a] >> sh) & 0xffu) | (((bal[2 * a + 1] >> sh) & 0xffu) << 8);
-        st.xzm[sl] = m3[0] | (m3[2] << 16);
-        unsigned rows = 0;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) rows |= ((m3[1] >> (4 * k)) & 0xfu) ? (1u << k) : 0u;
-        st.rows[sl] = rows;
-      }
-    }
-    __syncthreads();
-  };
-  const bool one_chunk = total <= CH;
-  if (one_chunk && total > 0) stage(0, total);  // both column passes read these tables
-  // two column passes over the tile's 16 column blocks: in pass p warp w owns block
-  // w + 8 p, x in [CX cx, +CX) and z in [CZ cz, +CZ) (CX = 4: the lane roles of the
-  // header); a lane owns x = CX cx + lane % CX, the z pair (lane / CX) % (CZ / 2)
-  // and the four y rows ly + 4 k, ly = lane / 8
-  // (8 is a multiple of NCX, so a warp keeps its x columns in both passes)
-  const int ly = lane >> 3, cx = warp % NCX;
-  const int xl = CX * cx + (lane % CX);
-#pragma unroll 1
-  for (int pass = 0; pass < 2; ++pass) {
-    const int cz = warp / NCX + (8 / NCX) * pass;
-    const int zl = CZ * cz + 2 * ((lane / CX) % (CZ / 2));
+  for (int pass = 0; pass < PASSES; ++pass) {
+    const int cx = (part * COLS + pass * NW + warp) % NCX, cz = (part * COLS + pass * NW + warp) / NCX;
+    const unsigned warpm = (((1u << CX) - 1u) << (CX * cx)) | (((1u << CZ) - 1u) << (16 + CZ * cz));
+    const int xl = CX * cx + (lane % CX), zl = CZ * cz + 2 * ((lane / CX) % (CZ / 2));
     f2p s[4][3], nc[4][3];
 #pragma unroll
     for (int k = 0; k < 4; ++k)
 #pragma unroll
       for (int a = 0; a < 3; ++a) s[k][a] = nc[k][a] = 0ull;
-    for (int base = 0; base < total; base += CH) {
-      const int nb = min(CH, total - base);
-      if (!one_chunk) stage(base, nb);  // block-uniform
-      // staged beads reaching this warp's column
-      unsigned col[CH / 32];
+    // candidates SPREAD32_BATCH at a time: those whose stencil reaches the CTA's points, in order
+    for (int q0 = 0; q0 < total; q0 += SPREAD32_BATCH) {
+      if (pass == 0 || total > SPREAD32_BATCH) {  // else the first pass's list stands
+        constexpr int H = SPREAD32_BATCH / NT;
+        int slot[H];
+        unsigned msk[H], rows[H], hit[H];
 #pragma unroll
-      for (int h = 0; h < CH / 32; ++h) {
-        const int sl = 32 * h + lane;
-        bool hit = false;
-        if (sl < nb) {
-          const unsigned m = st.xzm[sl];
-          hit = ((m >> (CX * cx)) & ((1u << CX) - 1u)) && ((m >> (16 + CZ * cz)) & ((1u << CZ) - 1u)) && st.rows[sl];
+        for (int h = 0; h < H; ++h) {
+          const int q = q0 + h * NT + tid;
+          slot[h] = 0;
+          msk[h] = rows[h] = 0;
+          if (q < total) {
+            slot[h] = cand_slot(cd, q);
+            const float4 hd = __ldg(rec + (size_t)slot[h] * RL);
+            const unsigned m = cover_mask(X0[0], __float_as_int(hd.x), c.N[0], ngd, FS_TILE) |
+                               (cover_mask(X0[2], __float_as_int(hd.z), c.N[2], ngd, FS_TILE) << 16);
+            const unsigned my = cover_mask(X0[1], __float_as_int(hd.y), c.N[1], ngd, FS_TILE);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) rows[h] |= ((my >> (4 * k)) & 0xfu) ? (1u << k) : 0u;
+            if ((m & ctam & 0xffffu) && (m & ctam) >> 16 && my) msk[h] = m;
+          }
+          hit[h] = __ballot_sync(0xffffffffu, msk[h] != 0);
+          if (lane == 0) st.count[NW * h + warp] = __popc(hit[h]);
         }
-        col[h] = __ballot_sync(0xffffffffu, hit);
-      }
+        __syncthreads();  // counts; and the previous list and tables are no longer read
+        int at[H];
+        nhit = 0;
 #pragma unroll
-      for (int h = 0; h < CH / 32; ++h) {
-        unsigned m = col[h];
+        for (int w = 0; w < SPREAD32_BATCH / 32; ++w) {
+#pragma unroll
+          for (int h = 0; h < H; ++h)
+            if (w == NW * h + warp) at[h] = nhit;
+          nhit += st.count[w];
+        }
+#pragma unroll
+        for (int h = 0; h < H; ++h)
+          if (msk[h]) {
+            const int i = at[h] + __popc(hit[h] & ((1u << lane) - 1u));
+            st.list[i] = slot[h];
+            st.lmask[i] = msk[h];
+            st.lrows[i] = (unsigned char)rows[h];
+          }
+        __syncthreads();
+      }
+      for (int base = 0; base < nhit; base += CH) {
+        const int nb = min(CH, nhit - base);
+        if (pass == 0 || total > SPREAD32_BATCH || nhit > CH) {  // else the first pass's tables stand
+          if (base || pass) __syncthreads();  // the previous tables are no longer read
+          // tables by tile coordinate, eight threads per slot (thread j takes x, y and z in
+          // {j, j + 8}), each reading its slot's record from global memory; not copying the
+          // records in first keeps a CTA at 57 KB of shared memory with 64 beads a stage
+          for (int sl = tid >> 3; sl < nb; sl += NT / 8) {
+            const int j = tid & 7;
+            const float4 *rw = rec + (size_t)st.list[base + sl] * RL;
+            const float4 hd = __ldg(rw);
+            if (j == 0) st.fh[sl] = __ldg(rw + 1);
+            if (j == 1) st.hh[sl] = __ldg(rw + 2);
+            const int swv[3] = {__float_as_int(hd.x), __float_as_int(hd.y), __float_as_int(hd.z)};
+            float4 w[6];
+#pragma unroll
+            for (int it = 0; it < 6; ++it) {
+              const int a = it >> 1, l = j + 8 * (it & 1), Nn = c.N[a];
+              const int i = wrap_near(l + wrap_near(X0[a] - swv[a], Nn), Nn);
+              w[it] = i < ngd ? __ldg(rw + 3 + a * ngd + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+            st.xw[sl][j] = w[0];
+            st.xw[sl][j + 8] = w[1];
+            st.yw[sl][j] = make_float4(w[2].x, w[2].x, w[2].y, w[2].y);
+            st.yrd[sl][j] = make_float2(w[2].w, w[2].w);
+            st.yw[sl][j + 8] = make_float4(w[3].x, w[3].x, w[3].y, w[3].y);
+            st.yrd[sl][j + 8] = make_float2(w[3].w, w[3].w);
+            st.zg[sl][j] = w[4].x;
+            st.zd[sl][j] = w[4].y;
+            st.zr[sl][j] = w[4].z;
+            st.zg[sl][j + 8] = w[5].x;
+            st.zd[sl][j + 8] = w[5].y;
+            st.zr[sl][j + 8] = w[5].z;
+          }
+          __syncthreads();
+        }
+        // staged beads reaching this warp's column
+        typedef typename std::conditional<CH == 64, unsigned long long, unsigned>::type mask_t;
+        mask_t m = 0;
+#pragma unroll
+        for (int h = 0; h < CH / 32; ++h) {
+          const int sl = 32 * h + lane;
+          const unsigned mm = sl < nb ? st.lmask[base + sl] & warpm : 0u;
+          m |= (mask_t)__ballot_sync(0xffffffffu, (mm & 0xffffu) && (mm >> 16)) << (32 * h % (8 * sizeof(mask_t)));
+        }
         while (m) {
-          const int sl = 32 * h + __ffs(m) - 1;
+          const int sl = (CH == 64 ? __ffsll((long long)m) : __ffs((int)m)) - 1;
           m &= m - 1;
-          const unsigned rows = st.rows[sl];
+          const unsigned rows = st.lrows[base + sl];
           const float4 wx = st.xw[sl][xl];
           const float2 gz = *reinterpret_cast<const float2 *>(&st.zg[sl][zl]);
           const float2 dz = *reinterpret_cast<const float2 *>(&st.zd[sl][zl]);
@@ -565,15 +585,35 @@ __global__ void __launch_bounds__(FS_SPREAD32_THREADS, 3)
         }
       }
     }
-    // one write per point: s - c
     const size_t N = (size_t)c.N[0] * c.N[1] * c.N[2];
-    const int gx = X0[0] + xl, gz0 = X0[2] + zl;
+    if constexpr (PASSES > 1) {  // one write per point, s - c (the tables are read again)
+      float *out = fgrid + ((size_t)(X0[0] + xl) * c.N[1] + X0[1] + ly) * c.N[2] + X0[2] + zl;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const size_t m0 = ((size_t)gx * c.N[1] + (X0[1] + ly + 4 * k)) * c.N[2] + gz0;
+      for (int k = 0; k < 4; ++k)
 #pragma unroll
-      for (int a = 0; a < 3; ++a)
-        *reinterpret_cast<float2 *>(fgrid + a * N + m0) = f2_unpack(f2_add(s[k][a], nc[k][a]));
+        for (int a = 0; a < 3; ++a)
+          *reinterpret_cast<float2 *>(out + a * N + (size_t)(4 * k) * c.N[2]) = f2_unpack(f2_add(s[k][a], nc[k][a]));
+    } else {
+      // one write per point, s - c: through shared memory, so that neighbouring lanes write whole
+      // rows of the CTA's z (a warp's own columns are parts of sectors)
+      constexpr int XP = FS_TILE * ZW + 4;  // floats per x plane and component
+      static_assert(PASSES > 1 || sizeof(SpreadStage32<CH>) >= sizeof(float) * 3 * XW * XP, "the tables hold the points");
+      __syncthreads();
+      float *T = reinterpret_cast<float *>(smem_raw);
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+          *reinterpret_cast<float2 *>(T + (a * XW + xl - xlo) * XP + (ly + 4 * k) * ZW + zl - zlo) =
+              f2_unpack(f2_add(s[k][a], nc[k][a]));
+      __syncthreads();
+      constexpr int Q = ZW / 4;  // float4 per row
+      for (int i = tid; i < 3 * XW * FS_TILE * Q; i += NT) {
+        const int z4 = i % Q, y = (i / Q) % FS_TILE, ax = i / (Q * FS_TILE), a = ax / XW, x = ax - a * XW;
+        const float4 v = *reinterpret_cast<const float4 *>(T + ax * XP + y * ZW + 4 * z4);
+        *reinterpret_cast<float4 *>(fgrid + a * N + ((size_t)(X0[0] + xlo + x) * c.N[1] + X0[1] + y) * c.N[2] + X0[2] +
+                                    zlo + 4 * z4) = v;
+      }
     }
   }
 }
@@ -1059,16 +1099,34 @@ fs_status spread_t(fs_ctx *c, const FcmConsts &k, const double *Y, const double 
   const int ch = c->tune_spread_chunk, cx = c->tune_spread_cols;
   if (sizeof(R) == 4) {
     const float4 *rec = (const float4 *)c->bead_rec;
-#define FS_SPREAD32_LAUNCH(CHV, CXV)                                                                             \
-  k_spread32<CHV, CXV><<<c->nbins, FS_SPREAD32_THREADS, spread32_smem<CHV>(k.ngd), c->stream>>>(c->bins.start, rec, \
-                                                                                                 k, (float *)c->grid_real)
-    if (ch == 32 && cx == 2) FS_SPREAD32_LAUNCH(32, 2);
-    else if (ch == 32 && cx == 8) FS_SPREAD32_LAUNCH(32, 8);
-    else if (ch == 32) FS_SPREAD32_LAUNCH(32, 4);
-    else if (cx == 2) FS_SPREAD32_LAUNCH(64, 2);
-    else if (cx == 8) FS_SPREAD32_LAUNCH(64, 8);
-    else FS_SPREAD32_LAUNCH(64, 4);
+    // beads whose stencil reaches a tile, if they lie evenly
+    const double e = (k.ngd + FS_TILE - 1) / (double)FS_TILE, reach = (double)np / c->nbins * (e * e * e);
+    const bool quarter = c->nbins < c->num_sms, sparse = c->nbins >= 8192 && reach <= 28,
+               whole = c->nbins >= 10 * c->num_sms && reach <= 48;
+#define FS_SPREAD32_LAUNCH1(CHV, CXV, NWV, PV)                                                                    \
+  {                                                                                                               \
+    constexpr size_t bytes = sizeof(SpreadStage32<CHV>);                                                          \
+    if (bytes > 48 * 1024)                                                                                        \
+      FS_CUDA(cudaFuncSetAttribute((const void *)k_spread32<CHV, CXV, NWV, PV>,                                   \
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));                     \
+    k_spread32<CHV, CXV, NWV, PV>                                                                                 \
+        <<<16 / (NWV * PV) * c->nbins, 32 * NWV, bytes, c->stream>>>(c->bins.start, rec, k, (float *)c->grid_real); \
+  }
+#define FS_SPREAD32_LAUNCH(CHV, CXV)                      \
+  {                                                       \
+    if (quarter) FS_SPREAD32_LAUNCH1(CHV, CXV, 4, 1)      \
+    else if (sparse) FS_SPREAD32_LAUNCH1(CHV, CXV, 4, 4)  \
+    else if (whole) FS_SPREAD32_LAUNCH1(CHV, CXV, 8, 2)   \
+    else FS_SPREAD32_LAUNCH1(CHV, CXV, 8, 1)              \
+  }
+    if (ch == 32 && cx == 2) FS_SPREAD32_LAUNCH(32, 2)
+    else if (ch == 32 && cx == 8) FS_SPREAD32_LAUNCH(32, 8)
+    else if (ch == 32) FS_SPREAD32_LAUNCH(32, 4)
+    else if (cx == 2) FS_SPREAD32_LAUNCH(64, 2)
+    else if (cx == 8) FS_SPREAD32_LAUNCH(64, 8)
+    else FS_SPREAD32_LAUNCH(64, 4)
 #undef FS_SPREAD32_LAUNCH
+#undef FS_SPREAD32_LAUNCH1
   } else {
     const double4 *rec = (const double4 *)c->bead_rec;
     double *f = (double *)c->grid_real;
@@ -1167,20 +1225,13 @@ fs_status fcm_init(fs_ctx *c) {
     return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)(bytes < (size_t)FS_SMEM_MAX ? bytes : (size_t)FS_SMEM_MAX));
   };
-  const size_t s32 = spread32_smem<32>(FS_NGD_MAX), s64 = spread32_smem<64>(FS_NGD_MAX);
-  FS_CUDA(smem((const void *)k_spread32<64, 2>, s64));
-  FS_CUDA(smem((const void *)k_spread32<64, 4>, s64));
-  FS_CUDA(smem((const void *)k_spread32<64, 8>, s64));
-  FS_CUDA(smem((const void *)k_spread32<32, 2>, s32));
-  FS_CUDA(smem((const void *)k_spread32<32, 4>, s32));
-  FS_CUDA(smem((const void *)k_spread32<32, 8>, s32));
   FS_CUDA(smem((const void *)k_spread64<4>, sizeof(SpreadStage64<4>)));
   FS_CUDA(smem((const void *)k_spread64<8>, sizeof(SpreadStage64<8>)));
   const size_t wq = interp_q_warp_bytes(FS_NGD_MAX);
   FS_CUDA(smem((const void *)k_interp_q<4, 1>, 4 * wq));
   FS_CUDA(smem((const void *)k_interp_q<8, 1>, 8 * wq));
   FS_CUDA(smem((const void *)k_interp_q<16, 1>, 16 * wq));
-  c->tune_spread_chunk = 64;
+  c->tune_spread_chunk = 32;
   c->tune_spread_cols = 2;  // 2 x 16 x 8 blocks: fs_autotune's choice at 384^3 and 512^3
   c->tune_interp_wpb = 4;  // the fastest at 256^3 and 512^3 in both precisions (FP64 833, 873, 911 us for 4, 8, 16)
   c->tune_fft32 = 0;

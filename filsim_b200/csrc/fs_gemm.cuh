@@ -3,8 +3,9 @@
 //
 //   D[m][n] = sum_k A[m][k] B[n][k]      A: M x K, B: N x K, both K contiguous (bf16)
 //
-// One CTA (4 warps) computes a 128 x BN tile. K advances in 64-element blocks
-// through a three-stage shared-memory ring filled by TMA (cp.async.bulk.tensor,
+// One CTA (4 warps) computes a 128 x BN tile, over all of K or one of gridDim.z ranges of it
+// (partial sums, added up in a fixed order by the caller). K advances in 64-element blocks
+// through a shared-memory ring filled by TMA (cp.async.bulk.tensor,
 // 128-byte swizzle: row r, 16-byte chunk j at r*128 + (j ^ (r & 7))*16, the
 // canonical K-major layout the MMA descriptors name). Thread 0 is the producer:
 // per block it waits until the stage's previous MMAs have drained ("empty"
@@ -12,7 +13,10 @@
 // tile loads, which complete that barrier. Thread 32 issues the MMAs: it waits on
 // "full", issues four K=16 MMAs and commits them to "empty"; after the last block
 // it commits to "done". Then each warp reads its 32 accumulator lanes with
-// tcgen05.ld and applies the epilogue. Every wait is bounded: on timeout the
+// tcgen05.ld, 32 columns at a time, and applies the epilogue; row-major results go through
+// shared memory (the drained ring) so that a warp writes whole 128-byte (FP32) or 64-byte (BF16)
+// row segments, where a lane per row wrote 4 bytes to each of 32 rows (a 4096 x 256 x 256 SiLU
+// layer of 128-column tiles: 29 to 18 us). Every wait is bounded: on timeout the
 // kernel records an error, skips the epilogue, frees its tensor memory and returns.
 #pragma once
 #include <cuda.h>
@@ -22,9 +26,10 @@
 typedef __nv_bfloat16 fs_bf16;
 
 enum {
-  GEMM_EPI_F32 = 0,    // outF = acc (+ bias)
-  GEMM_EPI_SILU = 1,   // z = acc + bias -> aux = z, outH = silu(z), outT = silu(z)^T
+  GEMM_EPI_F32 = 0,    // outF = acc (+ bias); K range z of gridDim.z to outF + z M ldo
+  GEMM_EPI_SILU = 1,   // z = acc + bias -> aux = z, outH = silu(z), outT = silu(z)^T (aux, outT if given)
   GEMM_EPI_DSILU = 2,  // dz = acc * silu'(aux) -> outH = dz, outT = dz^T
+  GEMM_EPI_DENORM = 3, // outF = (acc + bias) sd + mu on the first `rows` rows and `cols` columns
 };
 
 struct GemmArgs {
@@ -37,13 +42,16 @@ struct GemmArgs {
   fs_bf16 *outH;      // [M x N], ldh
   fs_bf16 *outT;      // [N x M], ldt
   float *aux;         // [M x N], ldx: pre-activation (stored by SILU, read by DSILU)
+  const float *mu, *sd;  // [N] (DENORM)
+  int rows, cols;
   int ldo, ldh, ldt, ldx;
   int *err;           // set to 1 on a timed-out wait
 };
 
 namespace fsg {
 
-constexpr int BM = 128, BK = 64, STAGES = 3, THREADS = 128;
+constexpr int BM = 128, BK = 64, THREADS = 128;
+__host__ __device__ constexpr int stages(int bn) { return bn == 64 ? 4 : 3; }  // 96 KB: two CTAs per SM
 constexpr int GEMM_GROUP_M = 32;  // rows of tiles per group of the tile order
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -129,11 +137,12 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
 __device__ __forceinline__ float silu_sig(float z) { return 1.0f / (1.0f + expf(-z)); }
 
 template <int BN>
-constexpr int smem_bytes() { return STAGES * (BM * 128 + BN * 128) + 1024; }
+constexpr int smem_bytes() { return stages(BN) * (BM * 128 + BN * 128) + 1024; }
 
 template <int BN, int EPI>
 __global__ void __launch_bounds__(THREADS)
     k_gemm_bf16(GemmArgs g, const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB) {
+  constexpr int STAGES = stages(BN);
   constexpr uint32_t A_BYTES = BM * 128, B_BYTES = BN * 128, STAGE_BYTES = A_BYTES + B_BYTES;
   constexpr uint32_t IDESC = idesc_bf16(BN);
   extern __shared__ uint8_t gemm_smem_raw[];
@@ -167,7 +176,8 @@ __global__ void __launch_bounds__(THREADS)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
-  const int nk = g.K / BK;
+  const int nkb = g.K / BK, kb0 = (int)((long long)nkb * blockIdx.z / gridDim.z),
+            nk = (int)((long long)nkb * (blockIdx.z + 1) / gridDim.z) - kb0;  // this CTA's K blocks
   if (tid == 0) {  // producer
     for (int kb = 0; kb < nk; ++kb) {
       const int s = kb % STAGES;
@@ -177,8 +187,8 @@ __global__ void __launch_bounds__(THREADS)
       }
       const uint32_t sA = base + s * STAGE_BYTES, sB = sA + A_BYTES;
       mbar_expect_tx(smem_u32(&full[s]), STAGE_BYTES);
-      tma_load_2d(sA, &tmA, kb * BK, m0, smem_u32(&full[s]));
-      tma_load_2d(sB, &tmB, kb * BK, n0, smem_u32(&full[s]));
+      tma_load_2d(sA, &tmA, (kb0 + kb) * BK, m0, smem_u32(&full[s]));
+      tma_load_2d(sB, &tmB, (kb0 + kb) * BK, n0, smem_u32(&full[s]));
       s_issued = kb + 1;
     }
   } else if (tid == 32) {  // MMA issuer
@@ -206,45 +216,86 @@ __global__ void __launch_bounds__(THREADS)
       mbar_wait(smem_u32(&full[kb % STAGES]), (kb / STAGES) & 1);
   tc_fence_after();
   if (ok) {
-    const int row = m0 + warp * 32 + lane;
+    const int row0 = m0 + warp * 32, row = row0 + lane;
+    // the warp's staging: 32 rows of 32 floats (or BF16), padded so that both a lane's row and
+    // eight lanes' columns are conflict-free 16-byte accesses
+    constexpr int SF = 36, SH = 20;  // row strides in 4-byte words
+    uint32_t *sw = reinterpret_cast<uint32_t *>(gemm_smem_raw + (base - smem_u32(gemm_smem_raw))) + warp * 32 * SF;
 #pragma unroll 1
-    for (int c0 = 0; c0 < BN; c0 += 16) {
-      float v[16];
-      tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + c0, v);
+    for (int c0 = 0; c0 < BN; c0 += 32) {
+      float v[32];
+      tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + c0, *reinterpret_cast<float(*)[16]>(v));
+      tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + c0 + 16, *reinterpret_cast<float(*)[16]>(v + 16));
       const int col = n0 + c0;
-      if (EPI == GEMM_EPI_F32) {
-        if (g.bias)
+      if (EPI != GEMM_EPI_DSILU && g.bias)
 #pragma unroll
-          for (int i = 0; i < 16; ++i) v[i] += g.bias[col + i];
-        float4 *o = reinterpret_cast<float4 *>(g.outF + (size_t)row * g.ldo + col);
+        for (int i = 0; i < 32; ++i) v[i] += __ldg(g.bias + col + i);
+      if (EPI == GEMM_EPI_DENORM)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) o[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-      } else {
-        float h[16];
-        if (EPI == GEMM_EPI_SILU) {
-          float *zx = g.aux + (size_t)row * g.ldx + col;
+        for (int i = 0; i < 32; ++i) v[i] = v[i] * __ldg(g.sd + col + i) + __ldg(g.mu + col + i);
+      if (EPI == GEMM_EPI_DSILU) {  // z to the lanes' rows
+        const float *zx = g.aux + (size_t)row0 * g.ldx + col;
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const float z = v[i] + g.bias[col + i];
-            zx[i] = z;
-            h[i] = z * silu_sig(z);
+        for (int r = 0; r < 8; ++r)
+          *reinterpret_cast<uint4 *>(sw + (4 * r + lane / 8) * SF + 4 * (lane % 8)) =
+              *reinterpret_cast<const uint4 *>(zx + (size_t)(4 * r + lane / 8) * g.ldx + 4 * (lane % 8));
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float4 z4 = *reinterpret_cast<const float4 *>(sw + lane * SF + 4 * i);
+          const float z[4] = {z4.x, z4.y, z4.z, z4.w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float s = silu_sig(z[j]);
+            v[4 * i + j] = v[4 * i + j] * s * (1.0f + z[j] * (1.0f - s));
           }
+        }
+        __syncwarp();
+      } else if (EPI != GEMM_EPI_SILU || g.aux) {  // rows of FP32 results
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          *reinterpret_cast<float4 *>(sw + lane * SF + 4 * i) =
+              make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+        __syncwarp();
+        if (EPI == GEMM_EPI_DENORM) {  // rows of any alignment
+          if (col + lane < g.cols)
+#pragma unroll 8
+            for (int r = 0; r < 32; ++r)
+              if (row0 + r < g.rows) g.outF[(size_t)(row0 + r) * g.ldo + col + lane] = __uint_as_float(sw[r * SF + lane]);
         } else {
-          const float *zx = g.aux + (size_t)row * g.ldx + col;
+          float *o = EPI == GEMM_EPI_SILU ? g.aux + (size_t)row0 * g.ldx
+                                          : g.outF + ((size_t)blockIdx.z * g.M + row0) * g.ldo;
+          const int ld = EPI == GEMM_EPI_SILU ? g.ldx : g.ldo;
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const float z = zx[i], s = silu_sig(z);
-            h[i] = v[i] * s * (1.0f + z * (1.0f - s));
+          for (int r = 0; r < 8; ++r)
+            *reinterpret_cast<uint4 *>(o + (size_t)(4 * r + lane / 8) * ld + col + 4 * (lane % 8)) =
+                *reinterpret_cast<const uint4 *>(sw + (4 * r + lane / 8) * SF + 4 * (lane % 8));
+        }
+        __syncwarp();
+      }
+      if (EPI == GEMM_EPI_SILU)
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] *= silu_sig(v[i]);
+      if (EPI == GEMM_EPI_SILU || EPI == GEMM_EPI_DSILU) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          uint32_t w[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const __nv_bfloat162 h = __floats2bfloat162_rn(v[8 * i + 2 * j], v[8 * i + 2 * j + 1]);
+            w[j] = *reinterpret_cast<const uint32_t *>(&h);
           }
+          *reinterpret_cast<uint4 *>(sw + lane * SH + 4 * i) = make_uint4(w[0], w[1], w[2], w[3]);
         }
-        if (g.outH) {
-          __nv_bfloat162 *o = reinterpret_cast<__nv_bfloat162 *>(g.outH + (size_t)row * g.ldh + col);
+        __syncwarp();
 #pragma unroll
-          for (int i = 0; i < 8; ++i) o[i] = __floats2bfloat162_rn(h[2 * i], h[2 * i + 1]);
-        }
-        if (g.outT)
+        for (int r = 0; r < 4; ++r)
+          *reinterpret_cast<uint4 *>(g.outH + (size_t)(row0 + 8 * r + lane / 4) * g.ldh + col + 8 * (lane % 4)) =
+              *reinterpret_cast<const uint4 *>(sw + (8 * r + lane / 4) * SH + 4 * (lane % 4));
+        if (g.outT)  // a lane per row: 64 bytes of each transposed row
 #pragma unroll
-          for (int i = 0; i < 16; ++i) g.outT[(size_t)(col + i) * g.ldt + row] = __float2bfloat16_rn(h[i]);
+          for (int i = 0; i < 32; ++i) g.outT[(size_t)(col + i) * g.ldt + row] = __float2bfloat16_rn(v[i]);
+        __syncwarp();
       }
     }
   } else if (tid == 0) {

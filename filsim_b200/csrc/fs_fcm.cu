@@ -51,6 +51,7 @@ __device__ __forceinline__ int wrap_near(int x, int n) {
 // for the spread and interpolation kernels so they need no integer division.
 __global__ void k_fcm_bin_keys(const double *__restrict__ Y, int np, FcmConsts c, int *__restrict__ key,
                                int *__restrict__ sw_out) {
+  FS_AFTER_PREVIOUS();
   int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= np) return;
   int bi[3];
@@ -80,6 +81,7 @@ __host__ __device__ inline int rec64_len(int ngd) { return 2 + 3 * ngd; }
 __global__ void k_records64(const double *__restrict__ Y, const double *__restrict__ F, const double *__restrict__ T,
                             const int *__restrict__ sorted, const int *__restrict__ bead_sw, int np, FcmConsts c,
                             double4 *__restrict__ rec) {
+  FS_AFTER_PREVIOUS();
   const int ngd = c.ngd, RL = rec64_len(ngd);
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long long)np * RL) return;
@@ -185,6 +187,7 @@ template <int ZL>
 __global__ void __launch_bounds__(FS_SPREAD64_THREADS, ZL == 4 ? 4 : 3)
     k_spread64(const int *__restrict__ bin_start, const double4 *__restrict__ rec, FcmConsts c,
                double *__restrict__ fgrid) {
+  FS_AFTER_PREVIOUS();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int CH = SPREAD64_CH;
   typedef SpreadStage64<ZL> Stage;
@@ -354,6 +357,7 @@ __host__ __device__ inline int spread_rec_len(int ngd) { return 3 + 3 * ngd; }
 __global__ void k_spread_records32(const double *__restrict__ Y, const double *__restrict__ F,
                                    const double *__restrict__ T, const int *__restrict__ sorted,
                                    const int *__restrict__ bead_sw, int np, FcmConsts c, float4 *__restrict__ rec) {
+  FS_AFTER_PREVIOUS();
   const int ngd = c.ngd, RL = spread_rec_len(ngd);
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long long)np * RL) return;
@@ -419,6 +423,7 @@ template <int CH, int CX, int NW, int PASSES>
 __global__ void __launch_bounds__(32 * NW, NW == 4 && PASSES == 4 ? 6 : 3)
     k_spread32(const int *__restrict__ bin_start, const float4 *__restrict__ rec, FcmConsts c,
                float *__restrict__ fgrid) {
+  FS_AFTER_PREVIOUS();
   static_assert(CX == 2 || CX == 4 || CX == 8, "column widths");
   constexpr int CZ = FS_TILE / CX, NCX = FS_TILE / CX;  // z width; columns across x
   constexpr int NT = 32 * NW, PARTS = 16 / (NW * PASSES), COLS = NW * PASSES;  // columns per CTA
@@ -645,6 +650,7 @@ __device__ inline R wavenumber(int i, int n, R ff) {
 template <typename R>
 __global__ void k_project(typename Cplx<R>::T *__restrict__ fh, size_t NH, int nx, int ny, int nz, int nzh, R ffx,
                           R ffy, R ffz, R total) {
+  FS_AFTER_PREVIOUS();
   typedef typename Cplx<R>::T C;
   size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= NH) return;
@@ -670,6 +676,7 @@ __global__ void k_project(typename Cplx<R>::T *__restrict__ fh, size_t NH, int n
 template <typename R>
 __global__ void k_project_planes(typename Cplx<R>::T *__restrict__ fh, size_t NH, int nx, int ny, int nz, int nzh,
                                  R ffx, R ffy, R ffz, R total) {
+  FS_AFTER_PREVIOUS();
   typedef typename Cplx<R>::T C;
   const int ij = blockIdx.x * blockDim.x + threadIdx.x;
   if (ij >= nx * ny) return;
@@ -765,6 +772,7 @@ template <int WPB, int SPLIT>
 __global__ void __launch_bounds__(32 * WPB) k_interp64(const double *__restrict__ u, const double4 *__restrict__ rec,
                                                        int np, FcmConsts c, double *__restrict__ V,
                                                        double *__restrict__ W) {
+  FS_AFTER_PREVIOUS();
   __shared__ InterpWarp64 sw[WPB];
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
   const int slot = (blockIdx.x * WPB + wl) / SPLIT, ws = wl % SPLIT;
@@ -868,6 +876,7 @@ template <int WPB, int SPLIT>
 __global__ void __launch_bounds__(32 * WPB) k_interp_q(const float *__restrict__ u, const float4 *__restrict__ rec,
                                                        int np, FcmConsts c, double *__restrict__ V,
                                                        double *__restrict__ W) {
+  FS_AFTER_PREVIOUS();
   extern __shared__ __align__(32) unsigned char interp_smem[];
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
   const int slot = (blockIdx.x * WPB + wl) / SPLIT, ws = wl % SPLIT;
@@ -969,12 +978,14 @@ __global__ void __launch_bounds__(32 * WPB) k_interp_q(const float *__restrict__
 
 template <typename A, typename B>
 __global__ void k_convert(const A *__restrict__ in, B *__restrict__ out, size_t n) {
+  FS_AFTER_PREVIOUS();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) out[i] = (B)in[i];
 }
 
 __global__ void k_friction(const double *__restrict__ F, const double *__restrict__ T, double *__restrict__ V,
                            double *__restrict__ W, int n3, double a1, double a2) {
+  FS_AFTER_PREVIOUS();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n3) {
     V[i] = a1 * F[i];
@@ -1053,11 +1064,12 @@ fs_status flow_solve_t(fs_ctx *c) {
   C *fh = (C *)c->grid_cplx;
   {
     ProfScope ps(c, FS_STAGE_PROJECT);
-    k_project<R><<<fs_blocks((long long)c->NH, 256), 256, 0, c->stream>>>(fh, c->NH, c->nx, c->ny, c->nz, c->nzh,
-                                                                            ffx, ffy, ffz, total);
+    fs_launch(k_project<R>, fs_blocks((long long)c->NH, 256), 256, 0, c->stream, fh, c->NH, c->nx, c->ny, c->nz,
+              c->nzh, ffx, ffy, ffz, total);
     FS_LAUNCH_CHECK();
     dim3 gp(fs_blocks((long long)c->nx * c->ny, 256), 2);
-    k_project_planes<R><<<gp, 256, 0, c->stream>>>(fh, c->NH, c->nx, c->ny, c->nz, c->nzh, ffx, ffy, ffz, total);
+    fs_launch(k_project_planes<R>, gp, 256, 0, c->stream, fh, c->NH, c->nx, c->ny, c->nz, c->nzh, ffx, ffy, ffz,
+              total);
     FS_LAUNCH_CHECK();
   }
   {
@@ -1076,17 +1088,17 @@ fs_status flow_solve_t(fs_ctx *c) {
 template <typename R>
 fs_status bin_t(fs_ctx *c, const FcmConsts &k, const double *Y, const double *F, const double *T, int np) {
   if (np > 0) {
-    k_fcm_bin_keys<<<fs_blocks(np, 256), 256, 0, c->stream>>>(Y, np, k, c->bins.key, c->bead_sw);
+    fs_launch(k_fcm_bin_keys, fs_blocks(np, 256), 256, 0, c->stream, Y, np, k, c->bins.key, c->bead_sw);
     FS_LAUNCH_CHECK();
   }
   FS_TRY(fs_sort_run(&c->bins, np, c->stream));
   if (np <= 0) return FS_OK;
   if (sizeof(R) == 4)
-    k_spread_records32<<<fs_blocks((long long)np * spread_rec_len(k.ngd), 256), 256, 0, c->stream>>>(
-        Y, F, T, c->bins.sorted, c->bead_sw, np, k, (float4 *)c->bead_rec);
+    fs_launch(k_spread_records32, fs_blocks((long long)np * spread_rec_len(k.ngd), 256), 256, 0, c->stream, Y, F, T,
+              c->bins.sorted, c->bead_sw, np, k, (float4 *)c->bead_rec);
   else
-    k_records64<<<fs_blocks((long long)np * rec64_len(k.ngd), 256), 256, 0, c->stream>>>(
-        Y, F, T, c->bins.sorted, c->bead_sw, np, k, (double4 *)c->bead_rec);
+    fs_launch(k_records64, fs_blocks((long long)np * rec64_len(k.ngd), 256), 256, 0, c->stream, Y, F, T,
+              c->bins.sorted, c->bead_sw, np, k, (double4 *)c->bead_rec);
   FS_LAUNCH_CHECK();
   return FS_OK;
 }
@@ -1109,8 +1121,8 @@ fs_status spread_t(fs_ctx *c, const FcmConsts &k, const double *Y, const double 
     if (bytes > 48 * 1024)                                                                                        \
       FS_CUDA(cudaFuncSetAttribute((const void *)k_spread32<CHV, CXV, NWV, PV>,                                   \
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));                     \
-    k_spread32<CHV, CXV, NWV, PV>                                                                                 \
-        <<<16 / (NWV * PV) * c->nbins, 32 * NWV, bytes, c->stream>>>(c->bins.start, rec, k, (float *)c->grid_real); \
+    fs_launch(k_spread32<CHV, CXV, NWV, PV>, 16 / (NWV * PV) * c->nbins, 32 * NWV, bytes, c->stream, \
+              c->bins.start, rec, k, (float *)c->grid_real); \
   }
 #define FS_SPREAD32_LAUNCH(CHV, CXV)                      \
   {                                                       \
@@ -1133,11 +1145,11 @@ fs_status spread_t(fs_ctx *c, const FcmConsts &k, const double *Y, const double 
     // half tiles, or quarter tiles where the half tiles would not fill the SMs three times
     // (64^3: 28 -> 21 us; 256^3, 301 against 308, and 512^3, 1.63 against 1.77 ms, keep half)
     if (2 * c->nbins < 3 * c->num_sms)
-      k_spread64<4><<<4 * c->nbins, FS_SPREAD64_THREADS, sizeof(SpreadStage64<4>), c->stream>>>(c->bins.start, rec, k,
-                                                                                                f);
+      fs_launch(k_spread64<4>, 4 * c->nbins, FS_SPREAD64_THREADS, sizeof(SpreadStage64<4>), c->stream, c->bins.start,
+                rec, k, f);
     else
-      k_spread64<8><<<2 * c->nbins, FS_SPREAD64_THREADS, sizeof(SpreadStage64<8>), c->stream>>>(c->bins.start, rec, k,
-                                                                                                f);
+      fs_launch(k_spread64<8>, 2 * c->nbins, FS_SPREAD64_THREADS, sizeof(SpreadStage64<8>), c->stream, c->bins.start,
+                rec, k, f);
   }
   FS_LAUNCH_CHECK();
   return FS_OK;
@@ -1159,11 +1171,11 @@ fs_status interp_t(fs_ctx *c, const FcmConsts &k, double *V, double *W, int np) 
   const int wpb = split > 1 ? 4 : (c->tune_interp_wpb == 16 && 16 * wb > FS_SMEM_MAX) ? 8 : c->tune_interp_wpb;
 #define FS_INTERP_LAUNCH(WPB, SPLIT)                                                                             \
   if constexpr (sizeof(R) == 4)                                                                                  \
-    k_interp_q<WPB, SPLIT><<<fs_blocks(np, WPB / SPLIT), 32 * WPB, WPB / SPLIT * wb, c->stream>>>(                \
-        (const float *)c->grid_real, (const float4 *)c->bead_rec, np, k, V, W);                                  \
+    fs_launch(k_interp_q<WPB, SPLIT>, fs_blocks(np, WPB / SPLIT), 32 * WPB, WPB / SPLIT * wb, c->stream, \
+              (const float *)c->grid_real, (const float4 *)c->bead_rec, np, k, V, W); \
   else                                                                                                           \
-    k_interp64<WPB, SPLIT><<<fs_blocks(np, WPB / SPLIT), 32 * WPB, 0, c->stream>>>(                               \
-        (const double *)c->grid_real, (const double4 *)c->bead_rec, np, k, V, W)
+    fs_launch(k_interp64<WPB, SPLIT>, fs_blocks(np, WPB / SPLIT), 32 * WPB, 0, c->stream, \
+              (const double *)c->grid_real, (const double4 *)c->bead_rec, np, k, V, W)
   if (split == 4) {
     FS_INTERP_LAUNCH(4, 4);
   } else if (split == 2) {
@@ -1294,7 +1306,7 @@ fs_status fcm_friction(fs_ctx *c, const double *F, const double *T, double *V, d
   const double a2 = 1. / (8 * PI * a * a * a * mu);
   if (np > 0) {
     ProfScope ps(c, FS_STAGE_FRICTION);
-    k_friction<<<fs_blocks(3 * np, 256), 256, 0, c->stream>>>(F, T, V, W, 3 * np, a1, a2);
+    fs_launch(k_friction, fs_blocks(3 * np, 256), 256, 0, c->stream, F, T, V, W, 3 * np, a1, a2);
     FS_LAUNCH_CHECK();
   }
   return FS_OK;
@@ -1306,7 +1318,7 @@ fs_status fcm_interpolate_only(fs_ctx *c, const double *u, const double *Y, int 
   FS_TRY(c->precision == FS_PREC_FP32 ? bin_t<float>(c, k, Y, nullptr, nullptr, np)
                                       : bin_t<double>(c, k, Y, nullptr, nullptr, np));
   if (c->precision == FS_PREC_FP32) {
-    k_convert<double, float><<<fs_blocks((long long)n, 256), 256, 0, c->stream>>>(u, (float *)c->grid_real, n);
+    fs_launch(k_convert<double, float>, fs_blocks((long long)n, 256), 256, 0, c->stream, u, (float *)c->grid_real, n);
     FS_LAUNCH_CHECK();
     FS_TRY(interp_t<float>(c, k, V, W, np));
   } else {
@@ -1322,7 +1334,8 @@ fs_status fcm_spread_only(fs_ctx *c, const double *Y, const double *F, const dou
   const size_t n = 3 * c->N;
   if (c->precision == FS_PREC_FP32) {
     FS_TRY(spread_t<float>(c, k, Y, F, T, np));
-    k_convert<float, double><<<fs_blocks((long long)n, 256), 256, 0, c->stream>>>((const float *)c->grid_real, f, n);
+    fs_launch(k_convert<float, double>, fs_blocks((long long)n, 256), 256, 0, c->stream, (const float *)c->grid_real,
+              f, n);
     FS_LAUNCH_CHECK();
   } else {
     FS_TRY(spread_t<double>(c, k, Y, F, T, np));
@@ -1336,10 +1349,11 @@ fs_status fcm_flow_solve_only(fs_ctx *c, const double *f, double *u) {
   const size_t n = 3 * c->N;
   if (c->precision == FS_PREC_FP32) {
     // FP32 chain: f rounded to float, solved, widened back
-    k_convert<double, float><<<fs_blocks((long long)n, 256), 256, 0, c->stream>>>(f, (float *)c->grid_real, n);
+    fs_launch(k_convert<double, float>, fs_blocks((long long)n, 256), 256, 0, c->stream, f, (float *)c->grid_real, n);
     FS_LAUNCH_CHECK();
     FS_TRY(flow_solve_t<float>(c));
-    k_convert<float, double><<<fs_blocks((long long)n, 256), 256, 0, c->stream>>>((const float *)c->grid_real, u, n);
+    fs_launch(k_convert<float, double>, fs_blocks((long long)n, 256), 256, 0, c->stream, (const float *)c->grid_real,
+              u, n);
     FS_LAUNCH_CHECK();
     c->last_grid_prec = FS_PREC_FP32;
     return FS_OK;

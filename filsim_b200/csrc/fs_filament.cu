@@ -200,6 +200,7 @@ __global__ void k_initial_guess(int np, const int *__restrict__ seg_id, const do
                                 const double *__restrict__ Ut, const double *__restrict__ q, double *__restrict__ Xs,
                                 double *__restrict__ Us, double *__restrict__ qs, int order,
                                 const double *__restrict__ Xtt, const int *__restrict__ hist_ok) {
+  FS_AFTER_PREVIOUS();
   int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= np) return;
   if (seg_id[b] == 0) {
@@ -224,6 +225,7 @@ __global__ void k_initial_guess(int np, const int *__restrict__ seg_id, const do
 // fmod(X, L) of assign_filament_data runs per lane.
 __global__ void k_unrobot_assign(int nfil, const int *__restrict__ fil_start, const double *__restrict__ qs,
                                  double *__restrict__ Xs, double *__restrict__ Y, FilConsts k) {
+  FS_AFTER_PREVIOUS();
   const int f = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (f >= nfil) return;  // warp-uniform
   const int b0 = fil_start[f], b1 = fil_start[f + 1];
@@ -278,6 +280,7 @@ __global__ void k_forces(int np, const int *__restrict__ fil_id, const int *__re
                          const double *__restrict__ lam, const double *__restrict__ kap,
                          const double *__restrict__ cmod, double *__restrict__ F, double *__restrict__ TAU,
                          FilConsts k) {
+  FS_AFTER_PREVIOUS();
   int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= np) return;
   const int f = fil_id[b], i = seg_id[b];
@@ -326,6 +329,7 @@ __global__ void k_forces(int np, const int *__restrict__ fil_id, const int *__re
 __global__ void k_spring_forces(int np, const int *__restrict__ off, const int *__restrict__ ent,
                                 const int *__restrict__ beads, const double *__restrict__ Xs, double ks, double l0,
                                 FilConsts k, double *__restrict__ F) {
+  FS_AFTER_PREVIOUS();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= np) return;
   double f[3] = {F[3 * b], F[3 * b + 1], F[3 * b + 2]};
@@ -576,6 +580,7 @@ __global__ void __launch_bounds__(128) k_jacobian_rows(int np, const int *__rest
                                                        const double *__restrict__ kap, const double *__restrict__ cmod,
                                                        double *__restrict__ rows, FilConsts k, double a, double ah,
                                                        const int *__restrict__ keep) {
+  FS_AFTER_PREVIOUS();
   if (keep && *keep) return;  // the previous step's J0 stays (fs_set_broyden_memory)
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= np) return;
@@ -636,6 +641,7 @@ __global__ void __launch_bounds__(64) k_jacobian_factor(int np, const int *__res
                                                         const double *__restrict__ rows, double *__restrict__ tri,
                                                         int nt, FilConsts k, double a, double ah,
                                                         int *__restrict__ flags, const int *__restrict__ keep) {
+  FS_AFTER_PREVIOUS();
   extern __shared__ __align__(16) double tri_smem[];
   if (keep && *keep) return;
   const int f = blockIdx.x, tid = threadIdx.x, lane = tid & 31, side = tid >> 5;
@@ -815,6 +821,7 @@ __global__ void __launch_bounds__(32 * TRI_APPLY_WARPS) k_tri_apply(
     int nfil, const int *__restrict__ fil_start, const double *__restrict__ tri, const double *__restrict__ b,
     double *__restrict__ x, const double *__restrict__ C, const double *__restrict__ dots, int iter,
     const int *__restrict__ iter_d, const int *__restrict__ off_d, size_t n6, double dt, double pcoef, int max_nw) {
+  FS_AFTER_PREVIOUS();
   extern __shared__ __align__(16) double tri_smem[];
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
   const int f = blockIdx.x * TRI_APPLY_WARPS + wl;
@@ -854,6 +861,7 @@ __global__ void __launch_bounds__(32 * TRI_APPLY_WARPS) k_tri_apply(
 // explicit inverse of filament f's J0 (with the 1/dt rows), one column per CTA (test access)
 __global__ void __launch_bounds__(32) k_tri_inverse(int nw, const double *__restrict__ tri, double dt, double pcoef,
                                                     double *__restrict__ out) {
+  FS_AFTER_PREVIOUS();
   extern __shared__ __align__(16) double tri_smem[];
   double *bb = tri_smem + 72 * nw, *y = bb + 6 * nw;
   const int n = 6 * nw, e = blockIdx.x, lane = threadIdx.x;
@@ -870,6 +878,7 @@ __global__ void k_error_check(int np, const int *__restrict__ fil_id, const int 
                               const double *__restrict__ Us, const double *__restrict__ U,
                               const double *__restrict__ V, const double *__restrict__ W, double *__restrict__ err,
                               int nt, FilConsts k, int *__restrict__ flags, unsigned long long *__restrict__ maxbits) {
+  FS_AFTER_PREVIOUS();
   int b = blockIdx.x * blockDim.x + threadIdx.x;
   bool over = false, nonfin = false, expl = false;
   double mx = 0.0;
@@ -916,6 +925,7 @@ __global__ void k_error_check(int np, const int *__restrict__ fil_id, const int 
 __global__ void __launch_bounds__(RED_THREADS) k_dots(const double *__restrict__ D, const double *__restrict__ b,
                                                        size_t n6, int iter, const int *__restrict__ iter_d,
                                                        const int *__restrict__ off_d, double *__restrict__ partial) {
+  FS_AFTER_PREVIOUS();
   // columns in groups of DOT_COLS: a thread reads b[k] once per group and keeps
   // the group's loads in flight together; each column's sum runs in the same
   // order as one column at a time (k ascending per thread, then the shuffle
@@ -953,6 +963,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_dots(const double *__restrict__
 // fixed-order final sums: one warp per output
 __global__ void k_reduce_rows(const double *__restrict__ partial, int nparts, int nrows, double *__restrict__ out,
                               int do_sqrt, const int *__restrict__ nrows_d, const int *__restrict__ off_d) {
+  FS_AFTER_PREVIOUS();
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= (nrows_d ? *nrows_d : nrows) + (off_d ? *off_d : 0)) return;
@@ -966,6 +977,7 @@ __global__ void k_reduce_rows(const double *__restrict__ partial, int nparts, in
 __global__ void __launch_bounds__(RED_THREADS) k_diff_sq(const double *__restrict__ ne, const double *__restrict__ e,
                                                           double *__restrict__ dE, size_t n6,
                                                           double *__restrict__ partial) {
+  FS_AFTER_PREVIOUS();
   __shared__ double sh[RED_THREADS / 32];
   double acc = 0.0;
   for (size_t k = (size_t)blockIdx.x * RED_THREADS + threadIdx.x; k < n6; k += (size_t)gridDim.x * RED_THREADS) {
@@ -990,6 +1002,7 @@ __global__ void k_broyden_cols(const double *__restrict__ tmp, const double *__r
                                const double *__restrict__ dE, const double *__restrict__ nrm, size_t n6,
                                double *__restrict__ Cmat, double *__restrict__ Dmat, int iter,
                                const int *__restrict__ iter_d, const int *__restrict__ off_d) {
+  FS_AFTER_PREVIOUS();
   size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n6) return;
   const size_t col = (size_t)((iter_d ? *iter_d : iter) + (off_d ? *off_d : 0)) * n6;
@@ -1007,6 +1020,7 @@ __global__ void k_update(int np, const int *__restrict__ fil_id, const int *__re
                          const int *__restrict__ fil_start, const double *__restrict__ u, double *__restrict__ Xs,
                          double *__restrict__ Us, const double *__restrict__ q, double *__restrict__ qs,
                          double *__restrict__ lam) {
+  FS_AFTER_PREVIOUS();
   int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= np) return;
   const int f = fil_id[b], i = seg_id[b];
@@ -1031,6 +1045,7 @@ __global__ void k_step(int np, int nlink, double *__restrict__ X, double *__rest
                        double *__restrict__ U, double *__restrict__ Us, double *__restrict__ Ut,
                        double *__restrict__ q, double *__restrict__ qt, double *__restrict__ lam,
                        double *__restrict__ lam1, double *__restrict__ lam2, int nt, int ex, int tension_order) {
+  FS_AFTER_PREVIOUS();
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < np) {
     const int b = t;
@@ -1090,8 +1105,8 @@ fs_status fil_initial_guess(fs_ctx *c) {
   if (!c->have_state) return FS_ERR_STATE;
   ProfScope ps(c, FS_STAGE_UPDATE);
   const int order = (c->start_order == 2 && c->hist_Xtt) ? 2 : 1;
-  k_initial_guess<<<fs_blocks(c->np, 256), 256, 0, c->stream>>>(c->np, c->seg_id, c->X, c->Xt, c->U, c->Ut, c->q,
-                                                                 c->Xs, c->Us, c->qs, order, c->hist_Xtt, c->hist_ok);
+  fs_launch(k_initial_guess, fs_blocks(c->np, 256), 256, 0, c->stream, c->np, c->seg_id, c->X, c->Xt, c->U, c->Ut,
+            c->q, c->Xs, c->Us, c->qs, order, c->hist_Xtt, c->hist_ok);
   FS_LAUNCH_CHECK();
   return FS_OK;
 }
@@ -1101,15 +1116,14 @@ fs_status fil_forces(fs_ctx *c, int nt) {
   ProfScope ps(c, FS_STAGE_FORCES);
   FilConsts k = make_fconsts(c);
   k.tt = nt * c->p.dt;  // double tt = nt*dt (Filament.hpp:295)
-  k_unrobot_assign<<<fs_blocks(c->nfil, 4), 128, 0, c->stream>>>(c->nfil, c->fil_start, c->qs, c->Xs, c->Y, k);
+  fs_launch(k_unrobot_assign, fs_blocks(c->nfil, 4), 128, 0, c->stream, c->nfil, c->fil_start, c->qs, c->Xs, c->Y, k);
   FS_LAUNCH_CHECK();
-  k_forces<<<fs_blocks(c->np, 256), 256, 0, c->stream>>>(c->np, c->fil_id, c->seg_id, c->fil_start, c->qs, c->lam,
-                                                          c->kap, c->cc, c->F, c->TAU, k);
+  fs_launch(k_forces, fs_blocks(c->np, 256), 256, 0, c->stream, c->np, c->fil_id, c->seg_id, c->fil_start, c->qs,
+            c->lam, c->kap, c->cc, c->F, c->TAU, k);
   FS_LAUNCH_CHECK();
   if (c->nspring > 0) {
-    k_spring_forces<<<fs_blocks(c->np, 256), 256, 0, c->stream>>>(c->np, c->spring_off, c->spring_ent,
-                                                                   c->spring_beads, c->Xs, c->spring_k,
-                                                                   c->spring_l0, k, c->F);
+    fs_launch(k_spring_forces, fs_blocks(c->np, 256), 256, 0, c->stream, c->np, c->spring_off, c->spring_ent,
+              c->spring_beads, c->Xs, c->spring_k, c->spring_l0, k, c->F);
     FS_LAUNCH_CHECK();
   }
   return FS_OK;
@@ -1123,9 +1137,11 @@ fs_status fil_jacobian_build(fs_ctx *c, int nt, const int *keep) {
   k.tt = nt * c->p.dt;
   if (c->np == 0) return FS_OK;
   double *rows = c->jtri + (size_t)TRI * c->np;
-  k_jacobian_rows<<<fs_blocks(c->np, 128), 128, 0, c->stream>>>(c->np, c->fil_id, c->fil_start, c->qs, c->Us, c->TAU,
-                                                                c->lam, c->kap, c->cc, rows, k, c->p.a, c->p.ah, keep);
+  fs_launch(k_jacobian_rows, fs_blocks(c->np, 128), 128, 0, c->stream, c->np, c->fil_id, c->fil_start, c->qs, c->Us,
+            c->TAU, c->lam, c->kap, c->cc, rows, k, c->p.a, c->p.ah, keep);
   FS_LAUNCH_CHECK();
+  // a plain launch: its CTAs all fit at once, and placed while the rows' kernel still fills some
+  // of the SMs they crowd the others (1,024 filaments of 32 beads: 104 us for both, 72 so)
   k_jacobian_factor<<<c->nfil, 64, sizeof(double) * (72 + TRI_ROW * c->max_nw), c->stream>>>(
       c->np, c->fil_start, rows, c->jtri, nt, k, c->p.a, c->p.ah, c->flags, keep);
   FS_LAUNCH_CHECK();
@@ -1146,8 +1162,8 @@ static double tri_pcoef(const fs_ctx *c) { return (c->p.dt / (9 * FS_PI * c->p.m
 
 fs_status fil_jacobian_inverse(fs_ctx *c, int f, double *out_d) {
   const int b0 = c->fil_start_h[f], nw = c->fil_start_h[f + 1] - b0, n = 6 * nw;
-  k_tri_inverse<<<n, 32, sizeof(double) * tri_apply_doubles(nw), c->stream>>>(nw, c->jtri + (size_t)TRI * b0, c->p.dt,
-                                                                              tri_pcoef(c), out_d);
+  fs_launch(k_tri_inverse, n, 32, sizeof(double) * tri_apply_doubles(nw), c->stream, nw, c->jtri + (size_t)TRI * b0,
+            c->p.dt, tri_pcoef(c), out_d);
   FS_LAUNCH_CHECK();
   return FS_OK;
 }
@@ -1158,9 +1174,8 @@ fs_status fil_error_check(fs_ctx *c, const double *V, const double *W, double *e
   FilConsts k = make_fconsts(c);
   FS_CUDA(cudaMemsetAsync(c->flags, 0, sizeof(int) * 3, c->stream));  // check, nonfinite, explode
   FS_CUDA(cudaMemsetAsync(c->maxerr_bits, 0, sizeof(unsigned long long), c->stream));
-  k_error_check<<<fs_blocks(c->np, 256), 256, 0, c->stream>>>(c->np, c->fil_id, c->seg_id, c->fil_start, c->Xs, c->X,
-                                                               c->Xt, c->Us, c->U, V, W, err, nt, k, c->flags,
-                                                               c->maxerr_bits);
+  fs_launch(k_error_check, fs_blocks(c->np, 256), 256, 0, c->stream, c->np, c->fil_id, c->seg_id, c->fil_start, c->Xs,
+            c->X, c->Xt, c->Us, c->U, V, W, err, nt, k, c->flags, c->maxerr_bits);
   FS_LAUNCH_CHECK();
   return FS_OK;
 }
@@ -1176,15 +1191,15 @@ fs_status fil_broyden_apply(fs_ctx *c, const double *b, double *x, int iter, con
     // iter 0 and no iter_d: the count is the carried and current columns, off_d)
     const int base = iter_d ? c->p.broyden_maxiter : iter;
     const int rows = off_d ? c->p.broyden_maxiter + c->bmem_cols + base : base;
-    k_dots<<<RED_BLOCKS, RED_THREADS, 0, c->stream>>>(c->Dmat, b, n6, iter, iter_d, off_d, c->partials);
+    fs_launch(k_dots, RED_BLOCKS, RED_THREADS, 0, c->stream, c->Dmat, b, n6, iter, iter_d, off_d, c->partials);
     FS_LAUNCH_CHECK();
-    k_reduce_rows<<<fs_blocks(rows, 8), 256, 0, c->stream>>>(c->partials, RED_BLOCKS, iter, c->dots, 0, iter_d,
-                                                             off_d);
+    fs_launch(k_reduce_rows, fs_blocks(rows, 8), 256, 0, c->stream, c->partials, RED_BLOCKS, iter, c->dots, 0, iter_d,
+              off_d);
     FS_LAUNCH_CHECK();
   }
-  k_tri_apply<<<fs_blocks(c->nfil, TRI_APPLY_WARPS), 32 * TRI_APPLY_WARPS,
-                sizeof(double) * TRI_APPLY_WARPS * tri_apply_doubles(c->max_nw), c->stream>>>(
-      c->nfil, c->fil_start, c->jtri, b, x, c->Cmat, c->dots, iter, iter_d, off_d, n6, c->p.dt, tri_pcoef(c), c->max_nw);
+  fs_launch(k_tri_apply, fs_blocks(c->nfil, TRI_APPLY_WARPS), 32 * TRI_APPLY_WARPS,
+            sizeof(double) * TRI_APPLY_WARPS * tri_apply_doubles(c->max_nw), c->stream, c->nfil, c->fil_start,
+            c->jtri, b, x, c->Cmat, c->dots, iter, iter_d, off_d, n6, c->p.dt, tri_pcoef(c), c->max_nw);
   FS_LAUNCH_CHECK();
   return learn_diag_apply(c, b, x);  // learned initial inverse-Jacobian diagonal, when on
 }
@@ -1194,15 +1209,15 @@ fs_status fil_broyden_update(fs_ctx *c, int iter, const int *iter_d, const int *
   const size_t n6 = (size_t)6 * c->np;
   {
     ProfScope ps(c, FS_STAGE_BROYDEN);
-    k_diff_sq<<<RED_BLOCKS, RED_THREADS, 0, c->stream>>>(c->newerr, c->err, c->dE, n6, c->partials);
+    fs_launch(k_diff_sq, RED_BLOCKS, RED_THREADS, 0, c->stream, c->newerr, c->err, c->dE, n6, c->partials);
     FS_LAUNCH_CHECK();
-    k_reduce_rows<<<1, 32, 0, c->stream>>>(c->partials, RED_BLOCKS, 1, c->scalars, 1, nullptr, nullptr);
+    fs_launch(k_reduce_rows, 1, 32, 0, c->stream, c->partials, RED_BLOCKS, 1, c->scalars, 1, nullptr, nullptr);
     FS_LAUNCH_CHECK();
   }
   FS_TRY(fil_broyden_apply(c, c->dE, c->tmp, iter, iter_d, off_d));
   ProfScope ps(c, FS_STAGE_BROYDEN);
-  k_broyden_cols<<<fs_blocks((long long)n6, 256), 256, 0, c->stream>>>(c->tmp, c->upd, c->dE, c->scalars, n6,
-                                                                       c->Cmat, c->Dmat, iter, iter_d, off_d);
+  fs_launch(k_broyden_cols, fs_blocks((long long)n6, 256), 256, 0, c->stream, c->tmp, c->upd, c->dE, c->scalars, n6,
+            c->Cmat, c->Dmat, iter, iter_d, off_d);
   FS_LAUNCH_CHECK();
   return FS_OK;
 }
@@ -1210,8 +1225,8 @@ fs_status fil_broyden_update(fs_ctx *c, int iter, const int *iter_d, const int *
 fs_status fil_state_update(fs_ctx *c, const double *upd) {
   if (!c->have_state) return FS_ERR_STATE;
   ProfScope ps(c, FS_STAGE_UPDATE);
-  k_update<<<fs_blocks(c->np, 256), 256, 0, c->stream>>>(c->np, c->fil_id, c->seg_id, c->fil_start, upd, c->Xs,
-                                                          c->Us, c->q, c->qs, c->lam);
+  fs_launch(k_update, fs_blocks(c->np, 256), 256, 0, c->stream, c->np, c->fil_id, c->seg_id, c->fil_start, upd, c->Xs,
+            c->Us, c->q, c->qs, c->lam);
   FS_LAUNCH_CHECK();
   return FS_OK;
 }
@@ -1220,9 +1235,8 @@ fs_status fil_step(fs_ctx *c, int nt) {
   if (!c->have_state) return FS_ERR_STATE;
   ProfScope ps(c, FS_STAGE_UPDATE);
   int n = c->np > 3 * c->nlink ? c->np : 3 * c->nlink;
-  k_step<<<fs_blocks(n, 256), 256, 0, c->stream>>>(c->np, c->nlink, c->X, c->Xs, c->Xt, c->U, c->Us, c->Ut, c->q,
-                                                    c->qt, c->lam, c->lam1, c->lam2, nt, c->p.lambda_extrap_step,
-                                                    c->tension_order == 1 ? 1 : 2);
+  fs_launch(k_step, fs_blocks(n, 256), 256, 0, c->stream, c->np, c->nlink, c->X, c->Xs, c->Xt, c->U, c->Us, c->Ut,
+            c->q, c->qt, c->lam, c->lam1, c->lam2, nt, c->p.lambda_extrap_step, c->tension_order == 1 ? 1 : 2);
   FS_LAUNCH_CHECK();
   return FS_OK;
 }

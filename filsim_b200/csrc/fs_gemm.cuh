@@ -142,6 +142,7 @@ constexpr int smem_bytes() { return stages(BN) * (BM * 128 + BN * 128) + 1024; }
 template <int BN, int EPI>
 __global__ void __launch_bounds__(THREADS)
     k_gemm_bf16(GemmArgs g, const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB) {
+  FS_AFTER_PREVIOUS();
   constexpr int STAGES = stages(BN);
   constexpr uint32_t A_BYTES = BM * 128, B_BYTES = BN * 128, STAGE_BYTES = A_BYTES + B_BYTES;
   constexpr uint32_t IDESC = idesc_bf16(BN);

@@ -212,6 +212,7 @@ struct YShape {
 template <int N, typename T, bool INV>
 __global__ void __launch_bounds__(YShape<N, T>::THREADS, YShape<N, T>::CTAS)
     k_lines_y(V16 *__restrict__ A, int ncol, int nv, int nvp, const V16 *__restrict__ tw) {
+  FS_AFTER_PREVIOUS();
   typedef Line<N> L;
   constexpr int COLS = YShape<N, T>::COLS, MS = YShape<N, T>::MS;
   extern __shared__ V16 line_smem[];
@@ -302,6 +303,7 @@ struct XArgs {
 template <int N, typename T>
 __global__ void __launch_bounds__(XShape<N>::THREADS, XShape<N>::CTAS)
     k_lines_x_project(V16 *__restrict__ A, XArgs g, const V16 *__restrict__ tw) {
+  FS_AFTER_PREVIOUS();
   typedef LineX<N> L;
   constexpr int COLS = XShape<N>::COLS, MS = XShape<N>::MS, NS = XShape<N>::NS;
   extern __shared__ V16 line_smem[];
@@ -457,6 +459,7 @@ __device__ __forceinline__ void untangle(const V16 *S, int k, const V16 *__restr
 template <int M, typename T>
 __global__ void __launch_bounds__(ZShape<M>::THREADS) k_lines_z_fwd(const void *__restrict__ f_, V16 *__restrict__ A,
                                                                     int nunit, int nvp, const V16 *__restrict__ tw) {
+  FS_AFTER_PREVIOUS();
   typedef Line<M> L;
   typedef ZShape<M> Z;
   constexpr bool F64 = Num<T>::IS_DOUBLE;
@@ -528,6 +531,7 @@ __global__ void __launch_bounds__(ZShape<M>::THREADS) k_lines_z_fwd(const void *
 template <int M, typename T>
 __global__ void __launch_bounds__(ZShape<M>::THREADS) k_lines_z_inv(const V16 *__restrict__ A, void *__restrict__ u_,
                                                                     int nunit, int nvp, const V16 *__restrict__ tw) {
+  FS_AFTER_PREVIOUS();
   typedef Line<M> L;
   typedef ZShape<M> Z;
   constexpr bool F64 = Num<T>::IS_DOUBLE;
@@ -690,8 +694,8 @@ template <int N, typename T>
 fs_status z_fwd(fs_ctx *c, V16 *A, const V16 *tw) {
   const int nunit = 3 * c->nx * c->ny / (Num<T>::IS_DOUBLE ? 1 : 2);
   typedef ZShape<N / 2> Z;
-  k_lines_z_fwd<N / 2, T><<<fs_blocks(nunit, Z::LU), Z::THREADS, Z::SMEM, c->stream>>>(c->grid_real, A, nunit,
-                                                                                        lines_nvp<T>(N), tw);
+  fs_launch(k_lines_z_fwd<N / 2, T>, fs_blocks(nunit, Z::LU), Z::THREADS, Z::SMEM, c->stream, c->grid_real, A, nunit,
+            lines_nvp<T>(N), tw);
   FS_LAUNCH_CHECK();
   return FS_OK;
 }
@@ -699,8 +703,8 @@ template <int N, typename T>
 fs_status z_inv(fs_ctx *c, const V16 *A, const V16 *tw) {
   const int nunit = 3 * c->nx * c->ny / (Num<T>::IS_DOUBLE ? 1 : 2);
   typedef ZShape<N / 2> Z;
-  k_lines_z_inv<N / 2, T><<<fs_blocks(nunit, Z::LU), Z::THREADS, Z::SMEM, c->stream>>>(A, c->grid_real, nunit,
-                                                                                        lines_nvp<T>(N), tw);
+  fs_launch(k_lines_z_inv<N / 2, T>, fs_blocks(nunit, Z::LU), Z::THREADS, Z::SMEM, c->stream, A, c->grid_real, nunit,
+            lines_nvp<T>(N), tw);
   FS_LAUNCH_CHECK();
   return FS_OK;
 }
@@ -710,9 +714,9 @@ fs_status y_lines(fs_ctx *c, V16 *A, const V16 *tw, bool inv) {
   typedef YShape<N, T> Y;
   const size_t smem = Y::SMEM;
   if (inv)
-    k_lines_y<N, T, true><<<fs_blocks(ncol, Y::COLS), Y::THREADS, smem, c->stream>>>(A, ncol, nv, nvp, tw);
+    fs_launch(k_lines_y<N, T, true>, fs_blocks(ncol, Y::COLS), Y::THREADS, smem, c->stream, A, ncol, nv, nvp, tw);
   else
-    k_lines_y<N, T, false><<<fs_blocks(ncol, Y::COLS), Y::THREADS, smem, c->stream>>>(A, ncol, nv, nvp, tw);
+    fs_launch(k_lines_y<N, T, false>, fs_blocks(ncol, Y::COLS), Y::THREADS, smem, c->stream, A, ncol, nv, nvp, tw);
   FS_LAUNCH_CHECK();
   return FS_OK;
 }
@@ -731,8 +735,7 @@ fs_status x_lines(fs_ctx *c, V16 *A, const V16 *tw) {
   g.ffz = TwoPI / (c->nz * c->p.dx);
   g.inv_total = 1.0 / ((double)c->nx * (double)c->ny * (double)c->nz);
   typedef XShape<N> X;
-  k_lines_x_project<N, T><<<fs_blocks(g.ncol, X::COLS), X::THREADS, X::SMEM, c->stream>>>(A, g,
-                                                                                                             tw);
+  fs_launch(k_lines_x_project<N, T>, fs_blocks(g.ncol, X::COLS), X::THREADS, X::SMEM, c->stream, A, g, tw);
   FS_LAUNCH_CHECK();
   return FS_OK;
 }

@@ -104,6 +104,7 @@ __global__ void k_features(int nfil, const int *__restrict__ fil_start, int nw_m
                            const double *__restrict__ Ut, const double *__restrict__ lam,
                            const double *__restrict__ lam1, const double *__restrict__ lam2,
                            const double *__restrict__ kap, double inv_dt, int nfeat, float *__restrict__ out) {
+  FS_AFTER_PREVIOUS();
   const int f = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (f >= nfil) return;
   const int b0 = fil_start[f], nw = fil_start[f + 1] - b0;
@@ -173,6 +174,7 @@ __device__ __forceinline__ void write_tile(const TransposeTile &t, int r0, int c
 __global__ void __launch_bounds__(256) k_prep_input(const float *__restrict__ raw, int n, int cap, int nfeat, int k_in,
                                                     const float *__restrict__ mu, const float *__restrict__ sd,
                                                     fs_bf16 *__restrict__ X, fs_bf16 *__restrict__ XT) {
+  FS_AFTER_PREVIOUS();
   __shared__ TransposeTile t;
   const int c0 = blockIdx.x * TT, r0 = blockIdx.y * TT, c = threadIdx.x % TT;
   const bool used = c0 + c < nfeat;
@@ -192,6 +194,7 @@ __global__ void __launch_bounds__(256) k_loss_grad(const float *__restrict__ Y, 
                                                    const float *__restrict__ sd, float scale,
                                                    fs_bf16 *__restrict__ dY, fs_bf16 *__restrict__ dYT,
                                                    double *__restrict__ loss) {
+  FS_AFTER_PREVIOUS();
   __shared__ TransposeTile t;
   const int c0 = blockIdx.x * TT, r0 = blockIdx.y * TT, c = threadIdx.x % TT;
   const bool used = c0 + c < ntgt;
@@ -223,6 +226,7 @@ __global__ void __launch_bounds__(256) k_loss_grad(const float *__restrict__ Y, 
 __global__ void __launch_bounds__(256) k_grad_reduce(const float *__restrict__ part, int splits, int nW, int wblocks,
                                                      float *__restrict__ dW, const fs_bf16 *__restrict__ MT, int rows,
                                                      int cap, float *__restrict__ db) {
+  FS_AFTER_PREVIOUS();
   if ((int)blockIdx.x < wblocks) {
     const int i = 4 * (blockIdx.x * 256 + threadIdx.x);
     if (i >= nW) return;
@@ -260,6 +264,7 @@ __global__ void __launch_bounds__(256) k_grad_reduce(const float *__restrict__ p
 __global__ void k_adam(float *__restrict__ P, const float *__restrict__ G, float *__restrict__ m, float *__restrict__ v,
                        int n, float lr, float b1, float b2, float eps, float bc1, float bc2, int rows, int cols,
                        fs_bf16 *__restrict__ Pb, fs_bf16 *__restrict__ PTb) {
+  FS_AFTER_PREVIOUS();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float g = isfinite(G[i]) ? G[i] : 0.f;
@@ -277,6 +282,7 @@ __global__ void k_adam(float *__restrict__ P, const float *__restrict__ G, float
 
 __global__ void k_bf16_copies(const float *__restrict__ P, int rows, int cols, fs_bf16 *__restrict__ Pb,
                               fs_bf16 *__restrict__ PTb) {
+  FS_AFTER_PREVIOUS();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= rows * cols) return;
   const fs_bf16 h = __float2bfloat16_rn(P[i]);
@@ -289,6 +295,7 @@ __global__ void k_bf16_copies(const float *__restrict__ P, int rows, int cols, f
 __global__ void k_learn_apply(int nfil, const int *__restrict__ fil_start, int nw_model, int ntgt,
                               const float *__restrict__ pred, const int *__restrict__ plain,
                               double *__restrict__ upd, double *__restrict__ jdiag) {
+  FS_AFTER_PREVIOUS();
   const int f = blockIdx.x;
   const int b0 = fil_start[f], nw = fil_start[f + 1] - b0;
   const bool model = nw == nw_model && !(plain && plain[f]);
@@ -305,6 +312,7 @@ __global__ void k_learn_apply(int nfil, const int *__restrict__ fil_start, int n
 // per-filament max |E| (non-finite counts as infinite)
 __global__ void k_fil_maxabs(int nfil, const int *__restrict__ fil_start, const double *__restrict__ err,
                              float *__restrict__ r) {
+  FS_AFTER_PREVIOUS();
   const int f = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (f >= nfil) return;
   const int b0 = fil_start[f], nw = fil_start[f + 1] - b0;
@@ -322,6 +330,7 @@ __global__ void k_fil_maxabs(int nfil, const int *__restrict__ fil_start, const 
 // started plain this step
 __global__ void k_flag_worse(int nfil, const int *__restrict__ fil_start, int nw_model, const float *__restrict__ rP,
                              const float *__restrict__ rL, int *__restrict__ plain, int *__restrict__ count) {
+  FS_AFTER_PREVIOUS();
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= nfil || fil_start[f + 1] - fil_start[f] != nw_model) return;
   if (plain[f]) atomicAdd(count, 1);
@@ -334,6 +343,7 @@ __global__ void k_fallback(int nfil, const int *__restrict__ fil_start, int nw_m
                            const double *__restrict__ gqs, const double *__restrict__ glam, double *__restrict__ Xs,
                            double *__restrict__ Us, double *__restrict__ qs, double *__restrict__ lam,
                            int *__restrict__ count) {
+  FS_AFTER_PREVIOUS();
   const int f = blockIdx.x;
   const int b0 = fil_start[f], nw = fil_start[f + 1] - b0, l0 = b0 - f;
   if (nw != nw_model || !(rL[f] > rP[f])) return;
@@ -353,6 +363,7 @@ __global__ void k_targets(int nfil, const int *__restrict__ fil_start, int nw_mo
                           const double *__restrict__ gXs, const double *__restrict__ gUs,
                           const double *__restrict__ glam, const double *__restrict__ C, const double *__restrict__ D,
                           int iters, const int *__restrict__ off, size_t n6, float *__restrict__ tgt) {
+  FS_AFTER_PREVIOUS();
   const int f = blockIdx.x;
   const int b0 = fil_start[f], nw = fil_start[f + 1] - b0, l0 = b0 - f;
   for (int t = threadIdx.x; t < ntgt; t += blockDim.x) {
@@ -378,6 +389,7 @@ __global__ void k_targets(int nfil, const int *__restrict__ fil_start, int nw_mo
 }
 
 __global__ void k_diag_axpy(size_t n, const double *__restrict__ d, const double *__restrict__ b, double *__restrict__ x) {
+  FS_AFTER_PREVIOUS();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) x[i] += d[i] * b[i];
 }
@@ -449,7 +461,7 @@ fs_status gemm_bn(cudaStream_t st, const GemmArgs &g, int splits) {
   FS_TRY(tma_map_bf16(&ta, g.A, g.M, g.K, g.lda, fsg::BM));
   FS_TRY(tma_map_bf16(&tb, g.B, g.N, g.K, g.ldb, BN));
   dim3 grid(g.M / fsg::BM, g.N / BN, splits);
-  fsg::k_gemm_bf16<BN, EPI><<<grid, fsg::THREADS, fsg::smem_bytes<BN>(), st>>>(g, ta, tb);
+  fs_launch(fsg::k_gemm_bf16<BN, EPI>, grid, fsg::THREADS, fsg::smem_bytes<BN>(), st, g, ta, tb);
   FS_LAUNCH_CHECK();
   return FS_OK;
 }
@@ -558,7 +570,8 @@ fs_status layer_gradients(fs_ctx *c, const fs_bf16 *dT, const fs_bf16 *inT, int 
   g.outF = splits > 1 ? m->part : dW;
   g.ldo = N;
   FS_TRY(gemm<GEMM_EPI_F32>(c, g, splits));
-  k_grad_reduce<<<wblocks + fs_blocks(M, 8), 256, 0, c->stream>>>(m->part, splits, nW, wblocks, dW, dT, M, m->cap, db);
+  fs_launch(k_grad_reduce, wblocks + fs_blocks(M, 8), 256, 0, c->stream, m->part, splits, nW, wblocks, dW, dT, M,
+            m->cap, db);
   FS_LAUNCH_CHECK();
   return FS_OK;
 }
@@ -569,8 +582,8 @@ fs_status backward(fs_ctx *c, const float *tgt, int n) {
   const int cap = m->cap, h = m->hidden;
   FS_CUDA(cudaMemsetAsync(m->loss, 0, sizeof(double), c->stream));
   const float scale = 1.0f / ((float)n * (float)m->ntgt);
-  k_loss_grad<<<dim3(m->k_out / TT, cap / TT), 256, 0, c->stream>>>(m->Y, tgt, n, cap, m->ntgt, m->k_out, m->out_mu,
-                                                                    m->out_sd, scale, m->dY, m->dYT, m->loss);
+  fs_launch(k_loss_grad, dim3(m->k_out / TT, cap / TT), 256, 0, c->stream, m->Y, tgt, n, cap, m->ntgt, m->k_out,
+            m->out_mu, m->out_sd, scale, m->dY, m->dYT, m->loss);
   FS_LAUNCH_CHECK();
   FS_TRY(layer_gradients(c, m->dYT, m->HT[2], m->k_out, h, m->dW[3], m->db[3]));
   const fs_bf16 *gin = m->dY;
@@ -595,8 +608,8 @@ fs_status backward(fs_ctx *c, const float *tgt, int n) {
 
 fs_status prepare(fs_ctx *c, const float *feat, int n, bool train) {
   fs_mlp *m = c->mlp;
-  k_prep_input<<<dim3(m->k_in / TT, m->cap / TT), 256, 0, c->stream>>>(feat, n, m->cap, m->nfeat, m->k_in, m->in_mu,
-                                                                       m->in_sd, m->X, train ? m->XT : nullptr);
+  fs_launch(k_prep_input, dim3(m->k_in / TT, m->cap / TT), 256, 0, c->stream, feat, n, m->cap, m->nfeat, m->k_in,
+            m->in_mu, m->in_sd, m->X, train ? m->XT : nullptr);
   FS_LAUNCH_CHECK();
   return FS_OK;
 }
@@ -721,9 +734,9 @@ fs_status learn_save_guess(fs_ctx *c) {
 fs_status learn_features(fs_ctx *c, float *out) {
   fs_mlp *m = c->mlp;
   FS_TRY(ensure_step_buffers(c));
-  k_features<<<fs_blocks(c->nfil, 8), 256, 0, c->stream>>>(c->nfil, c->fil_start, m->nw, c->X, c->Xt, c->hist_Xtt, c->hist_ok,
-                                                           c->q, c->U, c->Ut, c->lam, c->lam1, c->lam2, c->kap,
-                                                           1.0 / c->p.dt, m->nfeat, out);
+  fs_launch(k_features, fs_blocks(c->nfil, 8), 256, 0, c->stream, c->nfil, c->fil_start, m->nw, c->X, c->Xt,
+            c->hist_Xtt, c->hist_ok, c->q, c->U, c->Ut, c->lam, c->lam1, c->lam2, c->kap, 1.0 / c->p.dt, m->nfeat,
+            out);
   FS_LAUNCH_CHECK();
   return FS_OK;
 }
@@ -744,9 +757,8 @@ fs_status learn_warm_start(fs_ctx *c, int nt, fs_status (*solve)(fs_ctx *, int))
   const bool carried = m->bound_refresh > 0 && m->bound_ok && m->bound_age < m->bound_refresh;
   {
     ProfScope ps(c, FS_STAGE_LEARN);
-    k_learn_apply<<<c->nfil, 128, 0, c->stream>>>(c->nfil, c->fil_start, m->nw, m->ntgt, m->pred,
-                                                  carried ? m->plain_next : nullptr, m->updl,
-                                                  m->mode == 2 ? m->jdiag : nullptr);
+    fs_launch(k_learn_apply, c->nfil, 128, 0, c->stream, c->nfil, c->fil_start, m->nw, m->ntgt, m->pred,
+              carried ? m->plain_next : nullptr, m->updl, m->mode == 2 ? m->jdiag : nullptr);
     FS_LAUNCH_CHECK();
     m->jdiag_on = m->mode == 2;
   }
@@ -760,11 +772,11 @@ fs_status learn_warm_start(fs_ctx *c, int nt, fs_status (*solve)(fs_ctx *, int))
     FS_TRY(fil_forces(c, nt));
     FS_TRY(solve(c, nt));
     FS_TRY(fil_error_check(c, c->V, c->W, c->err, nt));
-    k_fil_maxabs<<<fs_blocks(c->nfil, 8), 256, 0, c->stream>>>(c->nfil, c->fil_start, c->err, m->rL);
+    fs_launch(k_fil_maxabs, fs_blocks(c->nfil, 8), 256, 0, c->stream, c->nfil, c->fil_start, c->err, m->rL);
     FS_LAUNCH_CHECK();
     FS_CUDA(cudaMemsetAsync(m->count, 0, sizeof(int), c->stream));
-    k_flag_worse<<<fs_blocks(c->nfil, 128), 128, 0, c->stream>>>(c->nfil, c->fil_start, m->nw, m->rP, m->rL,
-                                                                 m->plain_next, m->count);
+    fs_launch(k_flag_worse, fs_blocks(c->nfil, 128), 128, 0, c->stream, c->nfil, c->fil_start, m->nw, m->rP, m->rL,
+              m->plain_next, m->count);
     FS_LAUNCH_CHECK();
     FS_CUDA(cudaMemcpyAsync(m->count_h, m->count, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     FS_CUDA(cudaStreamSynchronize(c->stream));
@@ -781,7 +793,7 @@ fs_status learn_warm_start(fs_ctx *c, int nt, fs_status (*solve)(fs_ctx *, int))
     // plain start, measured: the comparison of this step and the bound of the next ones
     FS_TRY(solve(c, nt));
     FS_TRY(fil_error_check(c, c->V, c->W, c->err, nt));
-    k_fil_maxabs<<<fs_blocks(c->nfil, 8), 256, 0, c->stream>>>(c->nfil, c->fil_start, c->err, m->rP);
+    fs_launch(k_fil_maxabs, fs_blocks(c->nfil, 8), 256, 0, c->stream, c->nfil, c->fil_start, c->err, m->rP);
     FS_LAUNCH_CHECK();
     if (m->bound_refresh > 0) {
       m->bound_ok = true;
@@ -794,11 +806,11 @@ fs_status learn_warm_start(fs_ctx *c, int nt, fs_status (*solve)(fs_ctx *, int))
   FS_TRY(fil_forces(c, nt));
   FS_TRY(solve(c, nt));
   FS_TRY(fil_error_check(c, c->V, c->W, c->newerr, nt));
-  k_fil_maxabs<<<fs_blocks(c->nfil, 8), 256, 0, c->stream>>>(c->nfil, c->fil_start, c->newerr, m->rL);
+  fs_launch(k_fil_maxabs, fs_blocks(c->nfil, 8), 256, 0, c->stream, c->nfil, c->fil_start, c->newerr, m->rL);
   FS_LAUNCH_CHECK();
   FS_CUDA(cudaMemsetAsync(m->count, 0, sizeof(int), c->stream));
-  k_fallback<<<c->nfil, 128, 0, c->stream>>>(c->nfil, c->fil_start, m->nw, m->rP, m->rL, m->gXs, m->gUs, m->gqs,
-                                             m->glam, c->Xs, c->Us, c->qs, c->lam, m->count);
+  fs_launch(k_fallback, c->nfil, 128, 0, c->stream, c->nfil, c->fil_start, m->nw, m->rP, m->rL, m->gXs, m->gUs,
+            m->gqs, m->glam, c->Xs, c->Us, c->qs, c->lam, m->count);
   FS_LAUNCH_CHECK();
   FS_CUDA(cudaMemcpyAsync(m->count_h, m->count, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   FS_CUDA(cudaStreamSynchronize(c->stream));
@@ -833,16 +845,16 @@ fs_status learn_diag_apply(fs_ctx *c, const double *b, double *x) {
   fs_mlp *m = c->mlp;
   if (!m || !m->jdiag_on) return FS_OK;
   const size_t n6 = (size_t)6 * c->np;
-  k_diag_axpy<<<fs_blocks((long long)n6, 256), 256, 0, c->stream>>>(n6, m->jdiag, b, x);
+  fs_launch(k_diag_axpy, fs_blocks((long long)n6, 256), 256, 0, c->stream, n6, m->jdiag, b, x);
   FS_LAUNCH_CHECK();
   return FS_OK;
 }
 
 fs_status learn_capture_targets(fs_ctx *c, int iters) {
   fs_mlp *m = c->mlp;
-  k_targets<<<c->nfil, 128, 0, c->stream>>>(c->nfil, c->fil_start, m->nw, m->ntgt, c->Xs, c->Us, c->lam, m->gXs,
-                                            m->gUs, m->glam, c->Cmat, c->Dmat, bmem_off(c) ? 0 : iters, bmem_off(c),
-                                            (size_t)6 * c->np, m->tgt);
+  fs_launch(k_targets, c->nfil, 128, 0, c->stream, c->nfil, c->fil_start, m->nw, m->ntgt, c->Xs, c->Us, c->lam,
+            m->gXs, m->gUs, m->glam, c->Cmat, c->Dmat, bmem_off(c) ? 0 : iters, bmem_off(c), (size_t)6 * c->np,
+            m->tgt);
   FS_LAUNCH_CHECK();
   m->have_targets = true;
   return FS_OK;
@@ -991,7 +1003,8 @@ fs_status fs_mlp_create(fs_ctx *c, int nw, int hidden, int batch_capacity, unsig
       hbuf[i] = (float)((2 * u - 1) * bound);
     }
     FS_CUDA(cudaMemcpy(m->b[l], hbuf.data(), sizeof(float) * d[l + 1], cudaMemcpyHostToDevice));
-    k_bf16_copies<<<fs_blocks((long long)nW, 256), 256, 0, c->stream>>>(m->W[l], d[l + 1], d[l], m->Wb[l], m->WTb[l]);
+    fs_launch(k_bf16_copies, fs_blocks((long long)nW, 256), 256, 0, c->stream, m->W[l], d[l + 1], d[l], m->Wb[l],
+              m->WTb[l]);
     FS_LAUNCH_CHECK();
   }
   FS_TRY(gemm_attrs());
@@ -1044,8 +1057,8 @@ fs_status fs_mlp_set_params(fs_ctx *c, const float *params_h, size_t count) {
     o += nW;
     FS_CUDA(cudaMemcpy(m->b[l], params_h + o, sizeof(float) * m->dims[l + 1], cudaMemcpyHostToDevice));
     o += m->dims[l + 1];
-    k_bf16_copies<<<fs_blocks((long long)nW, 256), 256, 0, c->stream>>>(m->W[l], m->dims[l + 1], m->dims[l], m->Wb[l],
-                                                                        m->WTb[l]);
+    fs_launch(k_bf16_copies, fs_blocks((long long)nW, 256), 256, 0, c->stream, m->W[l], m->dims[l + 1], m->dims[l],
+              m->Wb[l], m->WTb[l]);
     FS_LAUNCH_CHECK();
   }
   m->adam_t = 0;
@@ -1122,11 +1135,11 @@ fs_status fs_mlp_train_step(fs_ctx *c, const float *features_d, const float *tar
     const float bc1 = 1.f - powf(b1, (float)m->adam_t), bc2 = 1.f - powf(b2, (float)m->adam_t);
     for (int l = 0; l < 4; ++l) {
       const int rows = m->dims[l + 1], cols = m->dims[l];
-      k_adam<<<fs_blocks((long long)rows * cols, 256), 256, 0, c->stream>>>(
-          m->W[l], m->dW[l], m->mW[l], m->vW[l], rows * cols, lr, b1, b2, eps, bc1, bc2, rows, cols, m->Wb[l], m->WTb[l]);
+      fs_launch(k_adam, fs_blocks((long long)rows * cols, 256), 256, 0, c->stream, m->W[l], m->dW[l], m->mW[l],
+                m->vW[l], rows * cols, lr, b1, b2, eps, bc1, bc2, rows, cols, m->Wb[l], m->WTb[l]);
       FS_LAUNCH_CHECK();
-      k_adam<<<fs_blocks(rows, 256), 256, 0, c->stream>>>(m->b[l], m->db[l], m->mb[l], m->vb[l], rows, lr, b1, b2, eps,
-                                                          bc1, bc2, rows, 1, nullptr, nullptr);
+      fs_launch(k_adam, fs_blocks(rows, 256), 256, 0, c->stream, m->b[l], m->db[l], m->mb[l], m->vb[l], rows, lr, b1,
+                b2, eps, bc1, bc2, rows, 1, nullptr, nullptr);
       FS_LAUNCH_CHECK();
     }
   }

@@ -15,12 +15,14 @@ fs_status fs_exclusive_scan(const int *in, int *out, int n, int *block_sums, cud
 #define SCAN_SPAN (SCAN_THREADS * SCAN_ITEMS)
 
 __global__ void k_sort_count(const int *__restrict__ key, int n, int *__restrict__ count, int *__restrict__ slot) {
+  FS_AFTER_PREVIOUS();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) slot[i] = atomicAdd(&count[key[i]], 1);
 }
 
 // exclusive scan of in[0..n) into out, block totals into bsum
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_block(const int *in, int *out, int n, int *bsum) {
+  FS_AFTER_PREVIOUS();
   __shared__ int warp_tot[32];
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
   const long long base = (long long)blockIdx.x * SCAN_SPAN + (long long)t * SCAN_ITEMS;
@@ -62,12 +64,14 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_block(const int *in, int 
 }
 
 __global__ void k_scan_add(int *__restrict__ out, int n, const int *__restrict__ bsum) {
+  FS_AFTER_PREVIOUS();
   long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx < n) out[idx] += bsum[idx / SCAN_SPAN];
 }
 
 __global__ void k_sort_scatter(const int *__restrict__ key, const int *__restrict__ slot, int n,
                                const int *__restrict__ start, int *__restrict__ placed) {
+  FS_AFTER_PREVIOUS();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) placed[start[key[i]] + slot[i]] = i;
 }
@@ -76,6 +80,7 @@ __global__ void k_sort_scatter(const int *__restrict__ key, const int *__restric
 // thread per key took 15 to 27 us at 8 to 30 items a key, this 3 to 5)
 __global__ void k_sort_rank(const int *__restrict__ key, int n, const int *__restrict__ start,
                             const int *__restrict__ placed, int *__restrict__ sorted) {
+  FS_AFTER_PREVIOUS();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int k = key[i], s0 = start[k], s1 = start[k + 1];
@@ -91,6 +96,7 @@ __global__ void k_sort_rank(const int *__restrict__ key, int n, const int *__res
 constexpr int SORT1_THREADS = 1024, SORT1_ITEMS = 4096, SORT1_KEYS = 40960;
 __global__ void __launch_bounds__(SORT1_THREADS) k_sort_one(const int *__restrict__ key, int n, int nkeys,
                                                             int *__restrict__ start, int *__restrict__ sorted) {
+  FS_AFTER_PREVIOUS();
   extern __shared__ int sort_smem[];
   __shared__ int warp_tot[32];
   int *cnt = sort_smem, *placed = sort_smem + nkeys + 1;
@@ -184,20 +190,21 @@ fs_status fs_sort_run(fs_sort *s, int n, cudaStream_t st) {
   const int nk1 = s->nkeys + 1;
   // one CTA as far as its shared memory goes (see k_sort_one)
   if (n <= SORT1_ITEMS && s->nkeys <= SORT1_KEYS) {
-    k_sort_one<<<1, SORT1_THREADS, sizeof(int) * (nk1 + (n > 0 ? n : 1)), st>>>(s->key, n, s->nkeys, s->start, s->sorted);
+    fs_launch(k_sort_one, 1, SORT1_THREADS, sizeof(int) * (nk1 + (n > 0 ? n : 1)), st, s->key, n, s->nkeys, s->start,
+              s->sorted);
     FS_LAUNCH_CHECK();
     return FS_OK;
   }
   FS_CUDA(cudaMemsetAsync(s->count, 0, sizeof(int) * nk1, st));
   if (n > 0) {
-    k_sort_count<<<fs_blocks(n, 256), 256, 0, st>>>(s->key, n, s->count, s->slot);
+    fs_launch(k_sort_count, fs_blocks(n, 256), 256, 0, st, s->key, n, s->count, s->slot);
     FS_LAUNCH_CHECK();
   }
   FS_TRY(fs_exclusive_scan(s->count, s->start, nk1, s->block_sums, st));
   if (n > 0) {
-    k_sort_scatter<<<fs_blocks(n, 256), 256, 0, st>>>(s->key, s->slot, n, s->start, s->placed);
+    fs_launch(k_sort_scatter, fs_blocks(n, 256), 256, 0, st, s->key, s->slot, n, s->start, s->placed);
     FS_LAUNCH_CHECK();
-    k_sort_rank<<<fs_blocks(n, 256), 256, 0, st>>>(s->key, n, s->start, s->placed, s->sorted);
+    fs_launch(k_sort_rank, fs_blocks(n, 256), 256, 0, st, s->key, n, s->start, s->placed, s->sorted);
     FS_LAUNCH_CHECK();
   }
   return FS_OK;
@@ -208,12 +215,12 @@ fs_status fs_exclusive_scan(const int *in, int *out, int n, int *block_sums, cud
   if (n <= 0) return FS_OK;
   int nblk = (n + SCAN_SPAN - 1) / SCAN_SPAN;
   if (nblk > SCAN_SPAN) return FS_ERR_INVALID_ARG;
-  k_scan_block<<<nblk, SCAN_THREADS, 0, st>>>(in, out, n, block_sums);
+  fs_launch(k_scan_block, nblk, SCAN_THREADS, 0, st, in, out, n, block_sums);
   FS_LAUNCH_CHECK();
   if (nblk > 1) {
-    k_scan_block<<<1, SCAN_THREADS, 0, st>>>(block_sums, block_sums, nblk, nullptr);
+    fs_launch(k_scan_block, 1, SCAN_THREADS, 0, st, block_sums, block_sums, nblk, nullptr);
     FS_LAUNCH_CHECK();
-    k_scan_add<<<fs_blocks(n, 256), 256, 0, st>>>(out, n, block_sums);
+    fs_launch(k_scan_add, fs_blocks(n, 256), 256, 0, st, out, n, block_sums);
     FS_LAUNCH_CHECK();
   }
   return FS_OK;

@@ -32,6 +32,7 @@ namespace {
 
 // hist_ok counts the steps since the history was last reset, up to 2
 __global__ void k_hist_tick(int *ok) {
+  FS_AFTER_PREVIOUS();
   if (*ok < 2) ++*ok;
 }
 
@@ -40,6 +41,7 @@ __global__ void k_hist_tick(int *ok) {
 __global__ void k_hist_same(size_t n, const double *__restrict__ X, const double *__restrict__ Xt,
                             const double *__restrict__ pX, const double *__restrict__ pXt, int *__restrict__ ok,
                             int *__restrict__ carried, int *__restrict__ vp_ok) {
+  FS_AFTER_PREVIOUS();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n && (X[i] != pX[i] || Xt[i] != pXt[i])) {
     *ok = 0;
@@ -52,6 +54,7 @@ __global__ void k_hist_same(size_t n, const double *__restrict__ X, const double
 __global__ void k_vpred_extrap(size_t n, const double *__restrict__ V1, const double *__restrict__ V2,
                                const double *__restrict__ W1, const double *__restrict__ W2, double *__restrict__ Vs,
                                double *__restrict__ Ws) {
+  FS_AFTER_PREVIOUS();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   Vs[i] = __dsub_rn(__dmul_rn(2.0, V1[i]), V2[i]);
@@ -61,6 +64,7 @@ __global__ void k_vpred_extrap(size_t n, const double *__restrict__ V1, const do
 // the predicted residual times the weight; without two recorded states zero, so
 // that the update is zero and leaves the state bitwise as it was
 __global__ void k_vpred_gate(size_t n, const int *__restrict__ ok, double weight, double *__restrict__ err) {
+  FS_AFTER_PREVIOUS();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) err[i] = *ok < 2 ? 0.0 : weight * err[i];
 }
@@ -79,11 +83,11 @@ fs_status vpred_step(fs_ctx *c, int nt) {
   if (c->vpred_weight == 0.0) return FS_OK;
   const size_t n3 = (size_t)3 * c->np, n6 = 2 * n3;
   if (n3 == 0) return FS_OK;
-  k_vpred_extrap<<<fs_blocks((long long)n3, 256), 256, 0, c->stream>>>(n3, c->vp_V1, c->vp_V2, c->vp_W1, c->vp_W2,
-                                                                      c->vp_Vs, c->vp_Ws);
+  fs_launch(k_vpred_extrap, fs_blocks((long long)n3, 256), 256, 0, c->stream, n3, c->vp_V1, c->vp_V2, c->vp_W1,
+            c->vp_W2, c->vp_Vs, c->vp_Ws);
   FS_LAUNCH_CHECK();
   FS_TRY(fil_error_check(c, c->vp_Vs, c->vp_Ws, c->err, nt));
-  k_vpred_gate<<<fs_blocks((long long)n6, 256), 256, 0, c->stream>>>(n6, c->vp_ok, c->vpred_weight, c->err);
+  fs_launch(k_vpred_gate, fs_blocks((long long)n6, 256), 256, 0, c->stream, n6, c->vp_ok, c->vpred_weight, c->err);
   FS_LAUNCH_CHECK();
   FS_TRY(fil_broyden_apply(c, c->err, c->upd, 0, nullptr, bmem_off(c)));
   FS_TRY(fil_state_update(c, c->upd));
@@ -98,7 +102,7 @@ fs_status vpred_end_step(fs_ctx *c) {
   FS_CUDA(cudaMemcpyAsync(c->vp_W2, c->vp_W1, b, cudaMemcpyDeviceToDevice, c->stream));
   FS_CUDA(cudaMemcpyAsync(c->vp_V1, c->V, b, cudaMemcpyDeviceToDevice, c->stream));
   FS_CUDA(cudaMemcpyAsync(c->vp_W1, c->W, b, cudaMemcpyDeviceToDevice, c->stream));
-  k_hist_tick<<<1, 1, 0, c->stream>>>(c->vp_ok);
+  fs_launch(k_hist_tick, 1, 1, 0, c->stream, c->vp_ok);
   FS_LAUNCH_CHECK();
   return FS_OK;
 }
@@ -159,7 +163,7 @@ fs_status hist_end_step(fs_ctx *c) {
   if (c->np > 0)
     FS_CUDA(cudaMemcpyAsync(c->hist_Xtt, c->Xt, sizeof(double) * 3 * (size_t)c->np, cudaMemcpyDeviceToDevice,
                             c->stream));
-  k_hist_tick<<<1, 1, 0, c->stream>>>(c->hist_ok);
+  fs_launch(k_hist_tick, 1, 1, 0, c->stream, c->hist_ok);
   FS_LAUNCH_CHECK();
   return FS_OK;
 }
@@ -185,8 +189,8 @@ fs_status hist_after_upload(fs_ctx *c) {
   if (!c->hist_cmp_pending) return FS_OK;
   c->hist_cmp_pending = false;
   const size_t n = (size_t)3 * c->np;
-  k_hist_same<<<fs_blocks((long long)n, 256), 256, 0, c->stream>>>(n, c->X, c->Xt, c->hist_pX, c->hist_pXt,
-                                                                  c->hist_ok, c->bmem_d, c->vp_ok);
+  fs_launch(k_hist_same, fs_blocks((long long)n, 256), 256, 0, c->stream, n, c->X, c->Xt, c->hist_pX, c->hist_pXt,
+            c->hist_ok, c->bmem_d, c->vp_ok);
   FS_LAUNCH_CHECK();
   return FS_OK;
 }

@@ -3,9 +3,9 @@
 //
 //   k_initial_guess      Filament::initialGuess (Filament.hpp:227-237, Bead.hpp:202-217); with
 //                        start order 2 the first bead extrapolated to second order (fs_start.cu)
-//   k_unrobot_assign     Filament::unRobotArmify (Filament.hpp:489-505) +
+//   k_assign_forces      Filament::unRobotArmify (Filament.hpp:489-505) +
 //                        Fcm::assign_filament_data's Y = fmod(Xs, L) (FCMfunctions.cpp:882-918)
-//   k_forces             setZeroForcesTorques, applyElasticTorques, applyConstraintForcesTorques,
+//                        and, in CTAs of its own, setZeroForcesTorques, applyElasticTorques, applyConstraintForcesTorques,
 //                        applyExternalForcesTorques (Filament.hpp:271-402), one thread per bead
 //                        adding its links' terms in the reference's order
 //   k_jacobian_rows, k_jacobian_factor
@@ -14,7 +14,7 @@
 //   k_error_check        ErrorCheckFCM + dexpinv (MobilityConstraints.cpp:109-143, 447-770)
 //   k_tri_apply          filamentJsolver::solve (FilamentJacobianSolver.hpp:49-73): J0^-1 b from
 //                        the factors, then the bad-Broyden history corrections
-//   k_broyden_cols       history update of main.cpp:640-663
+//   k_broyden_cols       history update of main.cpp:640-663 (with a learned diagonal; else k_tri_apply)
 //   k_update / k_step    Filament::update (Filament.hpp:425-452), Filament::step (:455-478); with
 //                        tension order 1 the tensions extrapolated linearly after lambda_extrap_step
 #include <algorithm>
@@ -223,10 +223,10 @@ __global__ void k_initial_guess(int np, const int *__restrict__ seg_id, const do
 // (tangents broadcast by shuffles; the same additions in the same order as one
 // thread walking the filament) and keeps its own bead's position; the
 // fmod(X, L) of assign_filament_data runs per lane.
-__global__ void k_unrobot_assign(int nfil, const int *__restrict__ fil_start, const double *__restrict__ qs,
-                                 double *__restrict__ Xs, double *__restrict__ Y, FilConsts k) {
-  FS_AFTER_PREVIOUS();
-  const int f = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+__device__ __forceinline__ void unrobot_assign(int block, int nfil, const int *__restrict__ fil_start,
+                                               const double *__restrict__ qs, double *__restrict__ Xs,
+                                               double *__restrict__ Y, const FilConsts &k) {
+  const int f = block * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (f >= nfil) return;  // warp-uniform
   const int b0 = fil_start[f], b1 = fil_start[f + 1];
   const double half = 0.5 * k.dl;
@@ -275,13 +275,22 @@ __device__ void elastic_link(const double *qi_, const double *qj_, double oneOve
   q_rotate(qm, vtmp);
 }
 
-__global__ void k_forces(int np, const int *__restrict__ fil_id, const int *__restrict__ seg_id,
-                         const int *__restrict__ fil_start, const double *__restrict__ qs,
-                         const double *__restrict__ lam, const double *__restrict__ kap,
-                         const double *__restrict__ cmod, double *__restrict__ F, double *__restrict__ TAU,
-                         FilConsts k) {
+// Positions (CTAs below ublocks, a warp per filament) and forces (the others, a thread per
+// bead): neither reads what the other writes
+__global__ void __launch_bounds__(128) k_assign_forces(int ublocks, int nfil, int np, const int *__restrict__ fil_id,
+                                                       const int *__restrict__ seg_id,
+                                                       const int *__restrict__ fil_start,
+                                                       const double *__restrict__ qs, const double *__restrict__ lam,
+                                                       const double *__restrict__ kap,
+                                                       const double *__restrict__ cmod, double *__restrict__ Xs,
+                                                       double *__restrict__ Y, double *__restrict__ F,
+                                                       double *__restrict__ TAU, FilConsts k) {
   FS_AFTER_PREVIOUS();
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if ((int)blockIdx.x < ublocks) {
+    unrobot_assign(blockIdx.x, nfil, fil_start, qs, Xs, Y, k);
+    return;
+  }
+  const int b = (blockIdx.x - ublocks) * blockDim.x + threadIdx.x;
   if (b >= np) return;
   const int f = fil_id[b], i = seg_id[b];
   const int nw = fil_start[f + 1] - fil_start[f];
@@ -813,14 +822,16 @@ __device__ __forceinline__ void tri_apply(int nw, const double *__restrict__ tri
 __host__ __device__ constexpr int tri_apply_doubles(int nw) { return (72 + 6 + 6) * nw; }
 
 // x_f = J0_f^-1 b_f (one bead: the identity), then x += sum_i C_i dots_i
-// (FilamentJacobianSolver.hpp:49-73); a warp per filament. Bound by the latency of the two
+// (FilamentJacobianSolver.hpp:49-73); a warp per filament. With upd given x is not written: b is
+// dE, and columns ncol of Cnew and Dnew are (C's columns below ncol are what is read). Bound by the latency of the two
 // chains (a shuffle and two dependent products per bead) and the factors' load before them.
 // With the dots before it, 1,024 filaments of 32 beads and 6 columns: 33 us (the columns one
 // load after another: 42); 4,096 filaments 97 us (132).
 __global__ void __launch_bounds__(32 * TRI_APPLY_WARPS) k_tri_apply(
     int nfil, const int *__restrict__ fil_start, const double *__restrict__ tri, const double *__restrict__ b,
     double *__restrict__ x, const double *__restrict__ C, const double *__restrict__ dots, int iter,
-    const int *__restrict__ iter_d, const int *__restrict__ off_d, size_t n6, double dt, double pcoef, int max_nw) {
+    const int *__restrict__ iter_d, const int *__restrict__ off_d, size_t n6, double dt, double pcoef, int max_nw,
+    const double *__restrict__ upd, const double *__restrict__ nrm, double *Cnew, double *Dnew) {
   FS_AFTER_PREVIOUS();
   extern __shared__ __align__(16) double tri_smem[];
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
@@ -852,9 +863,22 @@ __global__ void __launch_bounds__(32 * TRI_APPLY_WARPS) k_tri_apply(
 #pragma unroll
           for (int j = 0; j < 3; ++j) v[j] += w[u][j] * d[u];
     }
+    if (upd) {  // the history's next column, as k_broyden_cols forms it
+      const double nn = nrm[0];
 #pragma unroll
-    for (int j = 0; j < 3; ++j)
-      if (r0 + 32 * j < n) x[s0 + r0 + 32 * j] = v[j];
+      for (int j = 0; j < 3; ++j)
+        if (r0 + 32 * j < n) {
+          const size_t r = s0 + r0 + 32 * j;
+          double t = v[j] * (-1. / nn);
+          t -= upd[r] / nn;
+          Cnew[(size_t)ncol * n6 + r] = t;
+          Dnew[(size_t)ncol * n6 + r] = b[r] / nn;
+        }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+        if (r0 + 32 * j < n) x[s0 + r0 + 32 * j] = v[j];
+    }
   }
 }
 
@@ -995,6 +1019,39 @@ __global__ void __launch_bounds__(RED_THREADS) k_diff_sq(const double *__restric
   }
 }
 
+// The same sums for short vectors, a CTA per column, in one launch: out[i] = D_i . b, or with
+// e given D_i . (b - e); then the last CTA also writes dE = b - e and *norm = |dE|.
+__global__ void __launch_bounds__(1024) k_dots_small(const double *__restrict__ D, const double *__restrict__ b,
+                                                     const double *__restrict__ e, double *__restrict__ dE, int n6,
+                                                     int iter, const int *__restrict__ iter_d,
+                                                     const int *__restrict__ off_d, double *__restrict__ out,
+                                                     double *__restrict__ norm) {
+  FS_AFTER_PREVIOUS();
+  __shared__ double sh[32];
+  const int ncol = (iter_d ? *iter_d : iter) + (off_d ? *off_d : 0), tid = threadIdx.x;
+  const bool diff = e && blockIdx.x == gridDim.x - 1;
+  if (!diff && (int)blockIdx.x >= ncol) return;
+  const double *col = D + (size_t)blockIdx.x * n6;
+  double acc = 0.0;
+#pragma unroll 4
+  for (int k = tid; k < n6; k += 1024) {
+    const double v = e ? b[k] - e[k] : b[k];
+    if (diff) dE[k] = v;
+    acc += (diff ? v : col[k]) * v;
+  }
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if ((tid & 31) == 0) sh[tid >> 5] = acc;
+  __syncthreads();
+  if (tid < 32) {
+    acc = sh[tid];
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (tid == 0) {
+      if (diff) *norm = sqrt(acc);
+      else out[blockIdx.x] = acc;
+    }
+  }
+}
+
 // C_iter = -tmp/|dE| - upd/|dE|, D_iter = dE/|dE| (main.cpp:657-661)
 // column iter (iter_d ? *iter_d : iter) of the history, after the columns carried
 // from earlier steps (off_d ? *off_d : 0)
@@ -1116,10 +1173,9 @@ fs_status fil_forces(fs_ctx *c, int nt) {
   ProfScope ps(c, FS_STAGE_FORCES);
   FilConsts k = make_fconsts(c);
   k.tt = nt * c->p.dt;  // double tt = nt*dt (Filament.hpp:295)
-  fs_launch(k_unrobot_assign, fs_blocks(c->nfil, 4), 128, 0, c->stream, c->nfil, c->fil_start, c->qs, c->Xs, c->Y, k);
-  FS_LAUNCH_CHECK();
-  fs_launch(k_forces, fs_blocks(c->np, 256), 256, 0, c->stream, c->np, c->fil_id, c->seg_id, c->fil_start, c->qs,
-            c->lam, c->kap, c->cc, c->F, c->TAU, k);
+  const int ublocks = fs_blocks(c->nfil, 4);
+  fs_launch(k_assign_forces, ublocks + fs_blocks(c->np, 128), 128, 0, c->stream, ublocks, c->nfil, c->np, c->fil_id,
+            c->seg_id, c->fil_start, c->qs, c->lam, c->kap, c->cc, c->Xs, c->Y, c->F, c->TAU, k);
   FS_LAUNCH_CHECK();
   if (c->nspring > 0) {
     fs_launch(k_spring_forces, fs_blocks(c->np, 256), 256, 0, c->stream, c->np, c->spring_off, c->spring_ent,
@@ -1182,40 +1238,69 @@ fs_status fil_error_check(fs_ctx *c, const double *V, const double *W, double *e
 
 // iter_d (graph capture): the history length is read on the device; off_d: the
 // columns carried from earlier steps before it (fs_set_broyden_memory), or none
+// Vectors up to this long: a CTA per column. With the application of 6 columns: 480 beads 17.3
+// us, against 21.0 for blocks of partial sums and their reduction; 4,096 beads 19.8 (21.4);
+// 8,192 beads 25.7 (22.4).
+constexpr size_t DOTS_SMALL = 24576;
+
+// dots[i] = D_i . b; with e given D_i . dE, dE = b - e and c->scalars[0] = |dE|
+static fs_status broyden_dots(fs_ctx *c, const double *b, const double *e, int iter, const int *iter_d,
+                              const int *off_d) {
+  const size_t n6 = (size_t)6 * c->np;
+  // rows launched: a bound on the device count (with the memory on, callers pass
+  // iter 0 and no iter_d: the count is the carried and current columns, off_d)
+  const int base = iter_d ? c->p.broyden_maxiter : iter;
+  const int rows = off_d ? c->p.broyden_maxiter + c->bmem_cols + base : base;
+  if (n6 <= DOTS_SMALL) {
+    if (rows == 0 && !e) return FS_OK;
+    fs_launch(k_dots_small, rows + (e ? 1 : 0), 1024, 0, c->stream, c->Dmat, b, e, c->dE, (int)n6, iter, iter_d, off_d,
+              c->dots, c->scalars);
+    FS_LAUNCH_CHECK();
+    return FS_OK;
+  }
+  if (e) {
+    fs_launch(k_diff_sq, RED_BLOCKS, RED_THREADS, 0, c->stream, b, e, c->dE, n6, c->partials);
+    FS_LAUNCH_CHECK();
+    fs_launch(k_reduce_rows, 1, 32, 0, c->stream, c->partials, RED_BLOCKS, 1, c->scalars, 1, nullptr, nullptr);
+    FS_LAUNCH_CHECK();
+  }
+  if (rows == 0) return FS_OK;
+  fs_launch(k_dots, RED_BLOCKS, RED_THREADS, 0, c->stream, c->Dmat, e ? c->dE : b, n6, iter, iter_d, off_d,
+            c->partials);
+  FS_LAUNCH_CHECK();
+  fs_launch(k_reduce_rows, fs_blocks(rows, 8), 256, 0, c->stream, c->partials, RED_BLOCKS, iter, c->dots, 0, iter_d,
+            off_d);
+  FS_LAUNCH_CHECK();
+  return FS_OK;
+}
+
+// x = J0^-1 b + C dots, or with upd given the history's next column
+static fs_status tri_apply_launch(fs_ctx *c, const double *b, double *x, const double *upd, int iter,
+                                  const int *iter_d, const int *off_d) {
+  fs_launch(k_tri_apply, fs_blocks(c->nfil, TRI_APPLY_WARPS), 32 * TRI_APPLY_WARPS,
+            sizeof(double) * TRI_APPLY_WARPS * tri_apply_doubles(c->max_nw), c->stream, c->nfil, c->fil_start,
+            c->jtri, b, x, c->Cmat, c->dots, iter, iter_d, off_d, (size_t)6 * c->np, c->p.dt, tri_pcoef(c), c->max_nw,
+            upd, c->scalars, c->Cmat, c->Dmat);
+  FS_LAUNCH_CHECK();
+  return FS_OK;
+}
+
 fs_status fil_broyden_apply(fs_ctx *c, const double *b, double *x, int iter, const int *iter_d, const int *off_d) {
   if (!c->have_state) return FS_ERR_STATE;
   ProfScope ps(c, FS_STAGE_BROYDEN);
-  const size_t n6 = (size_t)6 * c->np;
-  if (iter > 0 || iter_d || off_d) {
-    // rows launched: a bound on the device count (with the memory on, callers pass
-    // iter 0 and no iter_d: the count is the carried and current columns, off_d)
-    const int base = iter_d ? c->p.broyden_maxiter : iter;
-    const int rows = off_d ? c->p.broyden_maxiter + c->bmem_cols + base : base;
-    fs_launch(k_dots, RED_BLOCKS, RED_THREADS, 0, c->stream, c->Dmat, b, n6, iter, iter_d, off_d, c->partials);
-    FS_LAUNCH_CHECK();
-    fs_launch(k_reduce_rows, fs_blocks(rows, 8), 256, 0, c->stream, c->partials, RED_BLOCKS, iter, c->dots, 0, iter_d,
-              off_d);
-    FS_LAUNCH_CHECK();
-  }
-  fs_launch(k_tri_apply, fs_blocks(c->nfil, TRI_APPLY_WARPS), 32 * TRI_APPLY_WARPS,
-            sizeof(double) * TRI_APPLY_WARPS * tri_apply_doubles(c->max_nw), c->stream, c->nfil, c->fil_start,
-            c->jtri, b, x, c->Cmat, c->dots, iter, iter_d, off_d, n6, c->p.dt, tri_pcoef(c), c->max_nw);
-  FS_LAUNCH_CHECK();
+  FS_TRY(broyden_dots(c, b, nullptr, iter, iter_d, off_d));
+  FS_TRY(tri_apply_launch(c, b, x, nullptr, iter, iter_d, off_d));
   return learn_diag_apply(c, b, x);  // learned initial inverse-Jacobian diagonal, when on
 }
 
 // main.cpp:641-663 with the current err/newerr/upd: history column `iter`
 fs_status fil_broyden_update(fs_ctx *c, int iter, const int *iter_d, const int *off_d) {
-  const size_t n6 = (size_t)6 * c->np;
-  {
-    ProfScope ps(c, FS_STAGE_BROYDEN);
-    fs_launch(k_diff_sq, RED_BLOCKS, RED_THREADS, 0, c->stream, c->newerr, c->err, c->dE, n6, c->partials);
-    FS_LAUNCH_CHECK();
-    fs_launch(k_reduce_rows, 1, 32, 0, c->stream, c->partials, RED_BLOCKS, 1, c->scalars, 1, nullptr, nullptr);
-    FS_LAUNCH_CHECK();
-  }
-  FS_TRY(fil_broyden_apply(c, c->dE, c->tmp, iter, iter_d, off_d));
   ProfScope ps(c, FS_STAGE_BROYDEN);
+  FS_TRY(broyden_dots(c, c->newerr, c->err, iter, iter_d, off_d));
+  if (!learn_diag_on(c)) return tri_apply_launch(c, c->dE, c->tmp, c->upd, iter, iter_d, off_d);
+  FS_TRY(tri_apply_launch(c, c->dE, c->tmp, nullptr, iter, iter_d, off_d));
+  FS_TRY(learn_diag_apply(c, c->dE, c->tmp));
+  const size_t n6 = (size_t)6 * c->np;
   fs_launch(k_broyden_cols, fs_blocks((long long)n6, 256), 256, 0, c->stream, c->tmp, c->upd, c->dE, c->scalars, n6,
             c->Cmat, c->Dmat, iter, iter_d, off_d);
   FS_LAUNCH_CHECK();

@@ -304,6 +304,7 @@ void learn_gate_record(fs_ctx *c, bool learned, long long solves);
 bool learn_recording(const fs_ctx *c);
 fs_status learn_save_guess(fs_ctx *c);
 fs_status learn_warm_start(fs_ctx *c, int nt, fs_status (*solve)(fs_ctx *, int));
+bool learn_diag_on(const fs_ctx *c);  // this step applies a learned diagonal
 fs_status learn_diag_apply(fs_ctx *c, const double *b, double *x);
 fs_status learn_capture_targets(fs_ctx *c, int iters);
 fs_status learn_end_step(fs_ctx *c);

@@ -841,6 +841,8 @@ fs_status learn_prepare_capture(fs_ctx *c) {
   return ensure_step_buffers(c);
 }
 
+bool learn_diag_on(const fs_ctx *c) { return c->mlp && c->mlp->jdiag_on; }
+
 fs_status learn_diag_apply(fs_ctx *c, const double *b, double *x) {
   fs_mlp *m = c->mlp;
   if (!m || !m->jdiag_on) return FS_OK;

@@ -16,6 +16,7 @@
 // round-to-nearest intrinsics (no FMA contraction) to match the reference's
 // x86-64 doubles.
 #include "fs_internal.cuh"
+#include "fs_sort.cuh"
 
 fs_status fs_exclusive_scan(const int *in, int *out, int n, int *block_sums, cudaStream_t st);
 
@@ -63,24 +64,25 @@ __global__ void k_bulkmap(int Mx, int My, int Mz, int *__restrict__ map) {
 }
 
 // cell of an unwrapped position (CollisionBarrierFilament.cpp:387-409)
-__global__ void k_cell_keys(const double *__restrict__ Xs, int np, BarrierConsts k, int *__restrict__ key) {
-  FS_AFTER_PREVIOUS();
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= np) return;
-  const int large_number = 100000;
-  int ci[3];
+struct CellKey {
+  const double *Xs;
+  BarrierConsts k;
+  __device__ int operator()(int b) const {
+    const int large_number = 100000;
+    int ci[3];
 #pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    const double x = Xs[3 * b + d];
-    const int w = __double2int_rz(__dadd_rn(__ddiv_rn(x, k.L[d]), (double)large_number)) - large_number;
-    const double xr = __dsub_rn(x, __dmul_rn(k.L[d], (double)w));
-    int cc = __double2int_rz(__dmul_rn(__ddiv_rn(xr, k.L[d]), (double)k.M[d]));
-    cc = cc >= k.M[d] ? k.M[d] - 1 : cc;
-    cc = cc < 0 ? 0 : cc;
-    ci[d] = cc;
+    for (int d = 0; d < 3; ++d) {
+      const double x = Xs[3 * b + d];
+      const int w = __double2int_rz(__dadd_rn(__ddiv_rn(x, k.L[d]), (double)large_number)) - large_number;
+      const double xr = __dsub_rn(x, __dmul_rn(k.L[d], (double)w));
+      int cc = __double2int_rz(__dmul_rn(__ddiv_rn(xr, k.L[d]), (double)k.M[d]));
+      cc = cc >= k.M[d] ? k.M[d] - 1 : cc;
+      cc = cc < 0 ? 0 : cc;
+      ci[d] = cc;
+    }
+    return ci[0] + ci[1] * k.M[0] + ci[2] * k.M[0] * k.M[1];
   }
-  key[b] = ci[0] + ci[1] * k.M[0] + ci[2] * k.M[0] * k.M[1];
-}
+};
 
 __global__ void k_cell_lists(const int *__restrict__ start, const int *__restrict__ sorted, int ncell,
                              int *__restrict__ head, int *__restrict__ list, int *__restrict__ rank_desc,
@@ -340,6 +342,7 @@ fs_status cells_init(fs_ctx *c) {
   }
   c->ncell = c->M[0] * c->M[1] * c->M[2];
   FS_TRY(fs_sort_alloc(&c->cells, c->ncell, c->max_beads, &c->bytes));
+  FS_TRY(fs_sort_prepare<CellKey>());
   const int nb = c->max_beads > 0 ? c->max_beads : 1;
   FS_CUDA(cudaMalloc(&c->head, sizeof(int) * c->ncell));
   FS_CUDA(cudaMalloc(&c->list, sizeof(int) * nb));
@@ -371,11 +374,7 @@ void cells_free(fs_ctx *c) {
 fs_status cells_link(fs_ctx *c, const double *Xs, int np) {
   ProfScope ps(c, FS_STAGE_LINK);
   BarrierConsts k = make_bconsts(c, 0);
-  if (np > 0) {
-    fs_launch(k_cell_keys, fs_blocks(np, 256), 256, 0, c->stream, Xs, np, k, c->cells.key);
-    FS_LAUNCH_CHECK();
-  }
-  FS_TRY(fs_sort_run(&c->cells, np, c->stream));
+  FS_TRY(fs_sort_run(&c->cells, CellKey{Xs, k}, np, c->stream));
   fs_launch(k_cell_lists, fs_blocks(c->ncell, 256), 256, 0, c->stream, c->cells.start, c->cells.sorted, c->ncell,
             c->head, c->list, c->cell_rank, c->flags);
   FS_LAUNCH_CHECK();

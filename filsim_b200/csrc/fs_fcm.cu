@@ -1,7 +1,7 @@
 // fs_fcm.cu -- Force Coupling Method mobility solve on sm_100a.
 //
 // Replaces Fcm::mobility_solve (FCMfunctions.cpp:175-464):
-//   1. k_fcm_bin_keys + counting sort: beads binned by the 16-point tile that
+//   1. counting sort (BinKey): beads binned by the 16-point tile that
 //      holds the start of their Gaussian stencil (gaussian_setup's index rule,
 //      FCMfunctions.cpp:565-589).
 //   2. k_records64 + k_spread64 (FP64) / k_spread_records32 + k_spread32 (FP32 chain):
@@ -21,6 +21,7 @@
 // weights in float, with Kahan-compensated spread sums and FP64 accumulation of
 // the interpolation products.
 #include "fs_internal.cuh"
+#include "fs_sort.cuh"
 #include <type_traits>
 #include "fs_f32x2.cuh"
 
@@ -49,24 +50,25 @@ __device__ __forceinline__ int wrap_near(int x, int n) {
 // key: the tile bin of the wrapped stencil start; sw: the wrapped stencil
 // start per axis (gaussian_setup's index rule, FCMfunctions.cpp:565-585), kept
 // for the spread and interpolation kernels so they need no integer division.
-__global__ void k_fcm_bin_keys(const double *__restrict__ Y, int np, FcmConsts c, int *__restrict__ key,
-                               int *__restrict__ sw_out) {
-  FS_AFTER_PREVIOUS();
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= np) return;
-  int bi[3];
+struct BinKey {
+  const double *Y;
+  FcmConsts c;
+  int *sw_out;
+  __device__ int operator()(int b) const {
+    int bi[3];
 #pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    int xc = (int)(Y[3 * b + d] / c.dx);
-    // the stencil start in the whole box, then in this grid (a slab window holds the
-    // beads whose x start lies in its own planes; others are clamped, never out of range)
-    int sw = wrap_int(xc - c.ngdh + 1, d == 0 ? c.gnx : c.N[d]) - (d == 0 ? c.x0 : 0);
-    sw = sw < 0 ? 0 : (sw >= c.N[d] ? c.N[d] - 1 : sw);
-    sw_out[3 * b + d] = sw;
-    bi[d] = sw / FS_TILE;
+    for (int d = 0; d < 3; ++d) {
+      int xc = (int)(Y[3 * b + d] / c.dx);
+      // the stencil start in the whole box, then in this grid (a slab window holds the
+      // beads whose x start lies in its own planes; others are clamped, never out of range)
+      int sw = wrap_int(xc - c.ngdh + 1, d == 0 ? c.gnx : c.N[d]) - (d == 0 ? c.x0 : 0);
+      sw = sw < 0 ? 0 : (sw >= c.N[d] ? c.N[d] - 1 : sw);
+      sw_out[3 * b + d] = sw;
+      bi[d] = sw / FS_TILE;
+    }
+    return (bi[0] * c.nbin[1] + bi[1]) * c.nbin[2] + bi[2];
   }
-  key[b] = (bi[0] * c.nbin[1] + bi[1]) * c.nbin[2] + bi[2];
-}
+};
 
 // ---- 2. spread ----------------------------------------------------------------
 // Both precisions first write one record per bead in sorted (bin) order: its stencil
@@ -1087,11 +1089,7 @@ fs_status flow_solve_t(fs_ctx *c) {
 // weights are read)
 template <typename R>
 fs_status bin_t(fs_ctx *c, const FcmConsts &k, const double *Y, const double *F, const double *T, int np) {
-  if (np > 0) {
-    fs_launch(k_fcm_bin_keys, fs_blocks(np, 256), 256, 0, c->stream, Y, np, k, c->bins.key, c->bead_sw);
-    FS_LAUNCH_CHECK();
-  }
-  FS_TRY(fs_sort_run(&c->bins, np, c->stream));
+  FS_TRY(fs_sort_run(&c->bins, BinKey{Y, k, c->bead_sw}, np, c->stream));
   if (np <= 0) return FS_OK;
   if (sizeof(R) == 4)
     fs_launch(k_spread_records32, fs_blocks((long long)np * spread_rec_len(k.ngd), 256), 256, 0, c->stream, Y, F, T,
@@ -1223,6 +1221,7 @@ fs_status fcm_init(fs_ctx *c) {
   FS_CUDA(cudaMalloc(&c->grid_cplx, sizeof(double2) * ncplx));
   c->bytes += sizeof(double) * 3 * c->N + sizeof(double2) * ncplx;
   FS_TRY(fs_sort_alloc(&c->bins, c->nbins, c->max_beads, &c->bytes));
+  FS_TRY(fs_sort_prepare<BinKey>());
   FS_CUDA(cudaMalloc(&c->bead_sw, sizeof(int) * 3 * (size_t)(c->max_beads > 0 ? c->max_beads : 1)));
   c->bytes += sizeof(int) * 3 * (size_t)c->max_beads;
   {

@@ -242,7 +242,6 @@ struct ProfScope {
 // ---- entry points implemented across the .cu files (internal C++ linkage) ----
 fs_status fs_sort_alloc(fs_sort *s, int nkeys, int max_items, size_t *bytes);
 void fs_sort_free(fs_sort *s);
-fs_status fs_sort_run(fs_sort *s, int n, cudaStream_t st);  // keys in s->key must be set
 
 fs_status fcm_init(fs_ctx *c);
 void fcm_free(fs_ctx *c);

@@ -1,11 +1,11 @@
 // fs_sort.cu -- deterministic counting sort of items by integer key.
 //
-// count (an atomic per item, which also gives the item a slot of its key) -> exclusive
+// keys and count (an atomic per item, which also gives the item a slot of its key) -> exclusive
 // scan -> scatter to the slots -> rank of each item by id among its key's. The slots depend
 // on atomic timing; the ranks make the output a pure function of the keys: items ascend by
 // (key, id). This is the order the collision linked list of LinkedList::link
 // (CollisionBarrierFilament.cpp:370-433) encodes in reverse. Small sorts run all steps in
-// one CTA.
+// one CTA. The steps that form the keys are templates on them (fs_sort.cuh).
 #include "fs_internal.cuh"
 
 fs_status fs_exclusive_scan(const int *in, int *out, int n, int *block_sums, cudaStream_t st);
@@ -13,12 +13,6 @@ fs_status fs_exclusive_scan(const int *in, int *out, int n, int *block_sums, cud
 #define SCAN_THREADS 1024
 #define SCAN_ITEMS 4
 #define SCAN_SPAN (SCAN_THREADS * SCAN_ITEMS)
-
-__global__ void k_sort_count(const int *__restrict__ key, int n, int *__restrict__ count, int *__restrict__ slot) {
-  FS_AFTER_PREVIOUS();
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) slot[i] = atomicAdd(&count[key[i]], 1);
-}
 
 // exclusive scan of in[0..n) into out, block totals into bsum
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_block(const int *in, int *out, int n, int *bsum) {
@@ -89,75 +83,6 @@ __global__ void k_sort_rank(const int *__restrict__ key, int n, const int *__res
   sorted[s0 + r] = i;
 }
 
-// The whole sort in one CTA: counts, then starts, in shared memory (nkeys + 1 ints), then
-// the placed items (n ints). Bound by its chain of barriers: with the key kernel and the
-// lists of LinkedList::link 17 us at 480 beads / 2,197 cells, 27 at 4,000 / 39,304, where
-// the separate launches take 34 and 42; both limits are what shared memory holds.
-constexpr int SORT1_THREADS = 1024, SORT1_ITEMS = 4096, SORT1_KEYS = 40960;
-__global__ void __launch_bounds__(SORT1_THREADS) k_sort_one(const int *__restrict__ key, int n, int nkeys,
-                                                            int *__restrict__ start, int *__restrict__ sorted) {
-  FS_AFTER_PREVIOUS();
-  extern __shared__ int sort_smem[];
-  __shared__ int warp_tot[32];
-  int *cnt = sort_smem, *placed = sort_smem + nkeys + 1;
-  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-  constexpr int PER = SORT1_ITEMS / SORT1_THREADS;
-  for (int k = t; k <= nkeys; k += SORT1_THREADS) cnt[k] = 0;
-  __syncthreads();
-  int ks[PER], slot[PER];
-#pragma unroll
-  for (int q = 0; q < PER; ++q) {
-    const int i = t + q * SORT1_THREADS;
-    ks[q] = i < n ? key[i] : -1;
-    slot[q] = i < n ? atomicAdd(&cnt[ks[q]], 1) : 0;
-  }
-  __syncthreads();
-  // exclusive scan in place, thread t over keys [t c, (t + 1) c)
-  // (c odd: the threads' strided accesses fall on different banks)
-  const int c = ((nkeys + SORT1_THREADS) / SORT1_THREADS) | 1, k0 = min(t * c, nkeys + 1), k1 = min(k0 + c, nkeys + 1);
-  int sum = 0;
-  for (int k = k0; k < k1; ++k) sum += cnt[k];
-  int incl = sum;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += y;
-  }
-  if (lane == 31) warp_tot[w] = incl;
-  __syncthreads();
-  if (w == 0) {
-    const int x = warp_tot[lane];
-    int ix = x;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, ix, o);
-      if (lane >= o) ix += y;
-    }
-    warp_tot[lane] = ix - x;
-  }
-  __syncthreads();
-  int run = incl - sum + warp_tot[w];
-  for (int k = k0; k < k1; ++k) {
-    const int v = cnt[k];
-    cnt[k] = run;
-    run += v;
-  }
-  __syncthreads();
-  for (int k = t; k <= nkeys; k += SORT1_THREADS) start[k] = cnt[k];
-#pragma unroll
-  for (int q = 0; q < PER; ++q)
-    if (ks[q] >= 0) placed[cnt[ks[q]] + slot[q]] = t + q * SORT1_THREADS;
-  __syncthreads();
-#pragma unroll
-  for (int q = 0; q < PER; ++q) {
-    if (ks[q] < 0) continue;
-    const int i = t + q * SORT1_THREADS, s0 = cnt[ks[q]], s1 = cnt[ks[q] + 1];
-    int r = 0;
-    for (int p = s0; p < s1; ++p) r += placed[p] < i;
-    sorted[s0 + r] = i;
-  }
-}
-
 fs_status fs_sort_alloc(fs_sort *s, int nkeys, int max_items, size_t *bytes) {
   s->nkeys = nkeys;
   int nblk = (nkeys + 1 + SCAN_SPAN - 1) / SCAN_SPAN;
@@ -170,8 +95,6 @@ fs_status fs_sort_alloc(fs_sort *s, int nkeys, int max_items, size_t *bytes) {
   FS_CUDA(cudaMalloc(&s->sorted, sizeof(int) * (size_t)(max_items > 0 ? max_items : 1)));
   FS_CUDA(cudaMalloc(&s->block_sums, sizeof(int) * (size_t)(nblk + 1)));
   *bytes += sizeof(int) * ((size_t)4 * (max_items > 0 ? max_items : 1) + 2 * (size_t)(nkeys + 1) + nblk + 1);
-  FS_CUDA(cudaFuncSetAttribute(k_sort_one, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)(sizeof(int) * (SORT1_KEYS + 1 + SORT1_ITEMS))));
   return FS_OK;
 }
 
@@ -186,21 +109,8 @@ void fs_sort_free(fs_sort *s) {
   s->key = s->count = s->start = s->slot = s->placed = s->sorted = s->block_sums = nullptr;
 }
 
-fs_status fs_sort_run(fs_sort *s, int n, cudaStream_t st) {
-  const int nk1 = s->nkeys + 1;
-  // one CTA as far as its shared memory goes (see k_sort_one)
-  if (n <= SORT1_ITEMS && s->nkeys <= SORT1_KEYS) {
-    fs_launch(k_sort_one, 1, SORT1_THREADS, sizeof(int) * (nk1 + (n > 0 ? n : 1)), st, s->key, n, s->nkeys, s->start,
-              s->sorted);
-    FS_LAUNCH_CHECK();
-    return FS_OK;
-  }
-  FS_CUDA(cudaMemsetAsync(s->count, 0, sizeof(int) * nk1, st));
-  if (n > 0) {
-    fs_launch(k_sort_count, fs_blocks(n, 256), 256, 0, st, s->key, n, s->count, s->slot);
-    FS_LAUNCH_CHECK();
-  }
-  FS_TRY(fs_exclusive_scan(s->count, s->start, nk1, s->block_sums, st));
+fs_status fs_sort_finish(fs_sort *s, int n, cudaStream_t st) {
+  FS_TRY(fs_exclusive_scan(s->count, s->start, s->nkeys + 1, s->block_sums, st));
   if (n > 0) {
     fs_launch(k_sort_scatter, fs_blocks(n, 256), 256, 0, st, s->key, s->slot, n, s->start, s->placed);
     FS_LAUNCH_CHECK();

@@ -122,7 +122,7 @@ def memory_label(mem):
 
 def warp_fft_length(n):
     """Grid lengths the FP32 warp transform covers on every axis (fs_fft.cu): 2^p in
-    [64, 512] or 96, 192, 384; other grids run cuFFT."""
+    [64, 512] or 96, 192, 384, where fs_autotune compares the library's own transform with cuFFT."""
     return (64 <= n <= 512 and n & (n - 1) == 0) or n in (96, 192, 384)
 
 

@@ -1041,10 +1041,16 @@ bool own_transform(const fs_ctx *c, int prec) {
   return c->line_tw[prec][0] && (prec == FS_PREC_FP64 || c->tune_fft32 == 0);
 }
 
+fs_status prepare_transform(fs_ctx *c, int prec) {
+  if (prec == FS_PREC_FP64) return lines_prepare64(c);
+  return fft32_preferred(c) ? FS_OK : lines_prepare32(c);
+}
+
 template <typename R>
 fs_status flow_solve_t(fs_ctx *c) {
   const int prec = sizeof(R) == 8 ? FS_PREC_FP64 : FS_PREC_FP32;
   if (own_transform(c, prec)) {
+    FS_TRY(prepare_transform(c, prec));
     if (prec == FS_PREC_FP64) return lines_flow_solve64(c);
     return fft32_preferred(c) ? fft32_flow_solve(c) : lines_flow_solve32(c);
   }
@@ -1287,7 +1293,7 @@ void fcm_free(fs_ctx *c) {
 
 fs_status fcm_set_stream(fs_ctx *c, cudaStream_t st) {
   const int prec = c->precision;
-  if (own_transform(c, prec)) return FS_OK;  // no cuFFT plan
+  if (own_transform(c, prec)) return prepare_transform(c, prec);  // no cuFFT plan
   FS_TRY(ensure_plans(c, prec));
   if (cufftSetStream(c->plan_fwd[prec], st) != CUFFT_SUCCESS) return FS_ERR_CUFFT;
   if (cufftSetStream(c->plan_inv[prec], st) != CUFFT_SUCCESS) return FS_ERR_CUFFT;

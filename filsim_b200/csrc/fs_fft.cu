@@ -1,4 +1,4 @@
-// fs_fft.cu -- FP32 periodic Stokes solve on power-of-two grids for sm_100a:
+// fs_fft.cu -- FP32 periodic Stokes solve on the largest grids (fft32_preferred) for sm_100a:
 // the forward real 3-D transform, the projection of flow_solve
 // (FCMfunctions.cpp:648-736) and the inverse real transform in five passes
 // over HBM, replacing cuFFT R2C + projection + C2R in the mixed-precision path.

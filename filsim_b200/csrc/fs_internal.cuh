@@ -73,9 +73,10 @@ struct fs_ctx {
   int tune_spread_chunk;  // beads staged per spread pass: 32 or 64 (fs_autotune)
   int tune_spread_cols;   // FP32 spread: x width of a warp's column block (2, 4 or 8)
   int tune_interp_wpb;    // beads (warps) per interpolation CTA: 4, 8 or 16
-  int tune_fft32;         // FP32 power-of-two grids: 0 warp FFT (fs_fft.cu), 1 cuFFT
+  int tune_fft32;         // FP32 grids: 0 own transform where there is one (fs_lines.cuh, fs_fft.cu), 1 cuFFT
+  bool line_ready[2];   // [precision]: the line kernels' attributes are set
   void *line_tw[2][3];  // [precision][axis]: tables of the line transforms (fs_lines.cuh; null: not a supported grid)
-  void *fft_tw;        // FP32 transform twiddle tables (null: grid not handled by fs_fft.cu, cuFFT is used)
+  void *fft_tw;        // twiddle tables of the FP32 warp transform (null: grid not handled by fs_fft.cu)
 
   // collision cells
   int M[3], ncell;
@@ -255,6 +256,8 @@ void slab_free(fs_ctx *c);
 bool lines_supported(const fs_ctx *c);  // every axis has a length of the line transforms (fs_lines.cuh)
 fs_status lines_init64(fs_ctx *c);
 fs_status lines_init32(fs_ctx *c);
+fs_status lines_prepare64(fs_ctx *c);
+fs_status lines_prepare32(fs_ctx *c);
 fs_status lines_flow_solve64(fs_ctx *c);
 fs_status lines_flow_solve32(fs_ctx *c);
 

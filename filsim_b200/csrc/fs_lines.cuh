@@ -740,7 +740,7 @@ fs_status x_lines(fs_ctx *c, V16 *A, const V16 *tw) {
   return FS_OK;
 }
 
-// twiddle tables and kernel attributes of the context's grid; tables at c->line_tw[prec][axis]
+// twiddle tables of the context's grid, at c->line_tw[prec][axis]
 template <typename T>
 fs_status lines_init_t(fs_ctx *c) {
   std::vector<TwRoot> roots;
@@ -768,9 +768,19 @@ fs_status lines_init_t(fs_ctx *c) {
   for (int a = 0; a < 3; ++a) c->line_tw[prec][a] = d + off[a];
   c->bytes += sizeof(V16) * h.size();
   FS_CUDA(cudaMemcpy(d, h.data(), sizeof(V16) * h.size(), cudaMemcpyHostToDevice));
+  return FS_OK;
+}
+
+// the attributes of the grid's kernels, which loads them: before the context's first solve at
+// this precision (and before a capture), so that a context loads no kernel that it never runs
+template <typename T>
+fs_status lines_prepare_t(fs_ctx *c) {
+  bool &ready = c->line_ready[Num<T>::IS_DOUBLE ? FS_PREC_FP64 : FS_PREC_FP32];
+  if (ready) return FS_OK;
   FS_LINES_SWITCH(c->nx, x_attrs);
   FS_LINES_SWITCH(c->ny, y_attrs);
   FS_LINES_SWITCH(c->nz, z_attrs);
+  ready = true;
   return FS_OK;
 }
 

@@ -6,4 +6,5 @@
 #include "fs_lines.cuh"
 
 fs_status lines_init32(fs_ctx *c) { return lines_init_t<F2>(c); }
+fs_status lines_prepare32(fs_ctx *c) { return lines_prepare_t<F2>(c); }
 fs_status lines_flow_solve32(fs_ctx *c) { return lines_flow_solve_t<F2>(c); }

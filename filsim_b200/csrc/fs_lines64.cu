@@ -6,4 +6,5 @@
 #include "fs_lines.cuh"
 
 fs_status lines_init64(fs_ctx *c) { return lines_init_t<double>(c); }
+fs_status lines_prepare64(fs_ctx *c) { return lines_prepare_t<double>(c); }
 fs_status lines_flow_solve64(fs_ctx *c) { return lines_flow_solve_t<double>(c); }

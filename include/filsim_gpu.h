@@ -135,7 +135,7 @@ int fs_abi_version(void);
 const char *fs_status_string(fs_status s);
 void fs_params_default(fs_params *p, int npts_x, int npts_y, int npts_z);
 
-/* Allocates grids, cuFFT plans and bead buffers for up to max_beads beads and
+/* Allocates grids, transform tables and bead buffers for up to max_beads beads and
  * max_filaments filaments (the suspension itself is uploaded later).
  * Replaces Fcm::initialise (FCMfunctions.cpp:10-168) and
  * LinkedList::initialise (CollisionBarrierFilament.cpp:274-304).
@@ -361,7 +361,7 @@ fs_status fs_set_graph_mode(fs_ctx *ctx, int on);
 
 /* ---- autotuner (no reference counterpart) -----------------------------------
  * choice = {beads staged per spread pass (32 | 64), beads per interpolation CTA
- * (4 | 8 | 16), FP32 power-of-two grids: 0 warp FFT | 1 cuFFT, FP32 spread: x
+ * (4 | 8 | 16), FP32 grids of 2^p or 3 2^p points: 0 own transform | 1 cuFFT, FP32 spread: x
  * width of a warp's column block in the 16^3 tile (2 | 4 | 8; the block is
  * w x 16 x 16/w points)}: four ints. fs_autotune times every combination on the
  * uploaded suspension (reps mobility solves each, after one warm-up) and keeps

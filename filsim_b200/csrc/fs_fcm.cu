@@ -157,12 +157,14 @@ __device__ __forceinline__ int cand_slot(const Cand &cd, int q) {
 // FMAs per point of the covered z quads, the z weights broadcast from shared memory. The
 // candidates that reach the CTA are listed first, 256 at a time, then staged CH at a time in
 // that (sorted) order, the sums kept throughout: no atomics, each point written once,
-// bit-reproducible. Bound by issue at 24 warps per SM (80 registers): 1.63 ms at 512^3 /
-// 131,072 beads and 0.30 ms at 256^3 / 30,720, where one grid point per lane with the
-// Gaussians recomputed per tile took 2.38 and 0.52; without the list, every candidate
-// staged, 1.83 and 0.36; at 128 registers and 16 warps per SM 1.83, 0.32.
+// bit-reproducible. Bound by issue at 24 warps per SM (80 registers) and the staging chain: 1.58
+// ms at 512^3 / 131,072 beads and 0.288 ms at 256^3 / 30,720, where one grid point per lane with
+// the Gaussians recomputed per tile took 2.38 and 0.52. Before the sums were chains of FMAs (a
+// product, a sum and an addition each, eleven operations a point for eight) 1.63 and 0.301, and of
+// that form without the list, every candidate staged, 1.83 and 0.36; at 128 registers and 16
+// warps per SM 1.83, 0.32.
 #define FS_SPREAD64_THREADS 256
-constexpr int SPREAD64_CH = 32;  // beads staged at a time (64, at two CTAs per SM: 1.85 against 1.63 ms at 512^3)
+constexpr int SPREAD64_CH = 32;  // beads staged at a time (64, at two CTAs per SM: 1.13 times as long at 512^3)
 template <int ZL>
 struct SpreadStage64 {
   static constexpr int CH = SPREAD64_CH;
@@ -296,9 +298,9 @@ __global__ void __launch_bounds__(FS_SPREAD64_THREADS, ZL == 4 ? 4 : 3)
             for (int z = 4 * k; z < 4 * k + 4; ++z) {
               const double2 gd = st.zgd[sl][ZL * zh + z];
               const double rd = st.zrd[sl][ZL * zh + z];
-              acc[z][0] += a0 * gd.x + (b0 * gd.y + c0 * rd);
-              acc[z][1] += a1 * gd.x + (b1 * gd.y + c1 * rd);
-              acc[z][2] += a2 * gd.x + b2 * gd.y;
+              acc[z][0] = fma(a0, gd.x, fma(b0, gd.y, fma(c0, rd, acc[z][0])));
+              acc[z][1] = fma(a1, gd.x, fma(b1, gd.y, fma(c1, rd, acc[z][1])));
+              acc[z][2] = fma(a2, gd.x, fma(b2, gd.y, acc[z][2]));
             }
           }
         }
@@ -1147,7 +1149,8 @@ fs_status spread_t(fs_ctx *c, const FcmConsts &k, const double *Y, const double 
     const double4 *rec = (const double4 *)c->bead_rec;
     double *f = (double *)c->grid_real;
     // half tiles, or quarter tiles where the half tiles would not fill the SMs three times
-    // (64^3: 28 -> 21 us; 256^3, 301 against 308, and 512^3, 1.63 against 1.77 ms, keep half)
+    // (before the FMA chains 64^3 21 us against 28; half tiles 256^3 301 against 308, 512^3 1.63
+    // against 1.77 ms)
     if (2 * c->nbins < 3 * c->num_sms)
       fs_launch(k_spread64<4>, 4 * c->nbins, FS_SPREAD64_THREADS, sizeof(SpreadStage64<4>), c->stream, c->bins.start,
                 rec, k, f);

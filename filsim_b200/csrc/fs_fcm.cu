@@ -764,9 +764,10 @@ __device__ __forceinline__ void interp_finish(double (&v)[6], bool on, int b, do
 //   W1 += dy rz dz Sd_0 - dy dz Sr_2,  W2 += dy dz Sr_1 - ry dy dz Sd_0.
 // The run of ngd points from zs touches P = (ngd + (zs & 1) + 1) / 2 pairs (a pair that a
 // short axis wraps onto twice has disjoint weights the two times); 32 / P rows j at once.
-// Bound by the latency of its gathers: 0.83 ms at 512^3 / 131,072 beads, 0.177 ms at 256^3 /
-// 30,720 (one point at a time with all weights from shared memory: 1.16, 0.26); with the
-// x-y products tabled per warp and the pairs walked across them 0.97, 0.21.
+// Bound by the latency of its gathers, eighteen in flight a lane: 0.72 ms at 512^3 / 131,072
+// beads, 0.156 ms at 256^3 / 30,720 (one point at a time with all weights from shared memory:
+// 1.16, 0.26; steps of 2, 4, 12 along x in place of 6: 0.86, 0.81, 0.86 and 0.184, 0.171, 0.184);
+// with the x-y products tabled per warp and the pairs walked across them 0.97, 0.21.
 struct InterpWarp64 {
   double xg[FS_NGD_MAX], xd[FS_NGD_MAX], xr[FS_NGD_MAX];  // g, d, r d
   double yg[FS_NGD_MAX], yd[FS_NGD_MAX], yr[FS_NGD_MAX];
@@ -829,7 +830,7 @@ __global__ void __launch_bounds__(32 * WPB) k_interp64(const double *__restrict_
         t.x += w * m.x;
         t.y += w * m.y;
       };
-#pragma unroll 4
+#pragma unroll (SPLIT > 1 ? 4 : 6)
       for (int i = i0; i < i1; ++i) {
         const double *q = base + s.xoff[i];
         const double2 u0 = __ldg(reinterpret_cast<const double2 *>(q)),

@@ -1254,7 +1254,7 @@ fs_status fcm_init(fs_ctx *c) {
   FS_CUDA(smem((const void *)k_interp_q<16, 1>, 16 * wq));
   c->tune_spread_chunk = 32;
   c->tune_spread_cols = 2;  // 2 x 16 x 8 blocks: fs_autotune's choice at 384^3 and 512^3
-  c->tune_interp_wpb = 4;  // the fastest at 256^3 and 512^3 in both precisions (FP64 833, 873, 911 us for 4, 8, 16)
+  c->tune_interp_wpb = 4;  // the fastest at 256^3 and 512^3 in both precisions (512^3 FP64 before six x steps: 833, 873, 911 us)
   c->tune_fft32 = 0;
   if (lines_supported(c)) {
     FS_TRY(lines_init64(c));

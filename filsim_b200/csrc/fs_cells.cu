@@ -16,6 +16,7 @@
 // round-to-nearest intrinsics (no FMA contraction) to match the reference's
 // x86-64 doubles.
 #include "fs_internal.cuh"
+#include "fs_events.cuh"
 #include "fs_sort.cuh"
 
 fs_status fs_exclusive_scan(const int *in, int *out, int n, int *block_sums, cudaStream_t st);
@@ -250,12 +251,7 @@ __global__ void __launch_bounds__(128) k_barrier(const double *__restrict__ Y, d
     if (l == 0) atomicOr(&flags[FLAG_CAPACITY], 1);
     n = FS_MAX_EVENTS;
   }
-  for (int e = l; e < n; e += G) {
-    const unsigned long long mine = s_key[w][e];
-    int r = 0;
-    for (int o = 0; o < n; ++o) r += s_key[w][o] < mine;
-    s_ord[w][r] = (unsigned char)e;
-  }
+  for (int e = l; e < n; e += G) s_ord[w][event_place(s_key[w], n, e)] = (unsigned char)e;
   __syncwarp();
   // fold in order: adding -f equals subtracting f exactly
   double acc[3] = {0.0, 0.0, 0.0};

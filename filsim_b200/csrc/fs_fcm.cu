@@ -806,14 +806,15 @@ __global__ void __launch_bounds__(32 * WPB) k_interp64(const double *__restrict_
     const int odd = zs & 1, P = (ngd + odd + 1) >> 1, G = 32 / P;
     const int pr = lane % P, g = lane / P;
     double gz[2], dz[2], rz[2];
+    bool in[2];
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
       const int k = 2 * pr + t - odd;
-      const bool in = k >= 0 && k < ngd;
-      const double4 z = rw[2 * ngd + (in ? k : 0)];
-      gz[t] = in ? z.x : 0.0;
-      dz[t] = in ? z.y : 0.0;
-      rz[t] = in ? z.w : 0.0;
+      in[t] = k >= 0 && k < ngd;
+      const double4 z = rw[2 * ngd + (in[t] ? k : 0)];
+      gz[t] = in[t] ? z.x : 0.0;
+      dz[t] = in[t] ? z.y : 0.0;
+      rz[t] = in[t] ? z.w : 0.0;
     }
     int z0 = zs - odd + 2 * pr;
     if (z0 >= Nz) z0 -= Nz;
@@ -846,6 +847,18 @@ __global__ void __launch_bounds__(32 * WPB) k_interp64(const double *__restrict_
         add(Sr[0], wr, u1);
         add(Sr[1], wr, u2);
       }
+      // the pair's point off the run counts for nothing, also where it is no finite number
+      auto drop = [&](double2 &t) {
+        if (!in[0]) t.x = 0.0;
+        if (!in[1]) t.y = 0.0;
+      };
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        drop(Sg[a]);
+        drop(Sd[a]);
+      }
+      drop(Sr[0]);
+      drop(Sr[1]);
       const double yg = s.yg[j], yd = s.yd[j], yr = s.yr[j];
 #pragma unroll
       for (int a = 0; a < 3; ++a) acc[a] += yg * (gz[0] * Sg[a].x + gz[1] * Sg[a].y);

@@ -877,6 +877,8 @@ __global__ void __launch_bounds__(32 * WPB) k_interp64(const double *__restrict_
 // four products summed in FP32 and the sum added in FP64. 0.525 ms at 512^3 / 131,072
 // beads; the FP64 kernel's walk with packed FP32 pairs and FP64 flushes every four x
 // points: 0.62.
+// SINGLE (boxes with Nz < ngd + 6, whose runs can wrap onto a quad twice): the points of the
+// run alone and each product added in FP64, as these boxes were always summed.
 constexpr int IQ_MAX = (FS_NGD_MAX + 6) / 4;  // quads a z run of ngd points can touch
 struct InterpQuad {
   float4 wg[IQ_MAX], wd[IQ_MAX], wr[IQ_MAX];  // g, gd, r of the quad's four points (0 off the run)
@@ -890,7 +892,7 @@ __host__ __device__ constexpr size_t interp_q_warp_bytes(int ngd) {
   return (interp_q_xy_offset() + (size_t)ngd * ngd * (sizeof(XY32) + sizeof(long long)) + 31) / 32 * 32;
 }
 
-template <int WPB, int SPLIT>
+template <int WPB, int SPLIT, bool SINGLE>
 __global__ void __launch_bounds__(32 * WPB) k_interp_q(const float *__restrict__ u, const float4 *__restrict__ rec,
                                                        int np, FcmConsts c, double *__restrict__ V,
                                                        double *__restrict__ W) {
@@ -906,11 +908,12 @@ __global__ void __launch_bounds__(32 * WPB) k_interp_q(const float *__restrict__
   XY32 *xy = reinterpret_cast<XY32 *>(base + interp_q_xy_offset());
   long long *off = reinterpret_cast<long long *>(xy + n2);
   double acc[6] = {0, 0, 0, 0, 0, 0};  // V, W
-  int b = 0, nq = 1;
+  int b = 0, nq = 1, zs = 0;
   if (on) {
     const float4 *rw = rec + (size_t)slot * spread_rec_len(ngd);
     const float4 hd = __ldg(rw);
-    const int sx = __float_as_int(hd.x), sy = __float_as_int(hd.y), zs = __float_as_int(hd.z);
+    const int sx = __float_as_int(hd.x), sy = __float_as_int(hd.y);
+    zs = __float_as_int(hd.z);
     b = __float_as_int(hd.w);
     nq = ((zs & 3) + ngd + 3) >> 2;
     if (lane < nq && ws == 0) {
@@ -962,27 +965,46 @@ __global__ void __launch_bounds__(32 * WPB) k_interp_q(const float *__restrict__
       const float4 a1 = __ldg(reinterpret_cast<const float4 *>(uy + m));
       const float4 a2 = __ldg(reinterpret_cast<const float4 *>(uz + m));
       const float4 g = q.wg[qi], gd = q.wd[qi], r = q.wr[qi];
-      float p0 = 0.f, p1 = 0.f, p2 = 0.f, p3 = 0.f, p4 = 0.f, p5 = 0.f;
-      auto add = [&](float x0, float x1, float x2, float gz, float gdz, float zz) {
-        const float temp = e.gg * gz;  // (gx gy) gz, the reference's order
-        const float tempd = e.dd * gdz;
-        p0 += x0 * temp;
-        p1 += x1 * temp;
-        p2 += x2 * temp;
-        p3 += (x2 * e.ry - x1 * zz) * tempd;
-        p4 += (x0 * zz - x2 * e.rx) * tempd;
-        p5 += (x1 * e.rx - x0 * e.ry) * tempd;
-      };
-      add(a0.x, a1.x, a2.x, g.x, gd.x, r.x);
-      add(a0.y, a1.y, a2.y, g.y, gd.y, r.y);
-      add(a0.z, a1.z, a2.z, g.z, gd.z, r.z);
-      add(a0.w, a1.w, a2.w, g.w, gd.w, r.w);
-      acc[0] += (double)p0;
-      acc[1] += (double)p1;
-      acc[2] += (double)p2;
-      acc[3] += (double)p3;
-      acc[4] += (double)p4;
-      acc[5] += (double)p5;
+      if constexpr (SINGLE) {
+        const int k0 = 4 * qi - (zs & 3);  // stencil index of the quad's first point
+        auto add = [&](int k, float x0, float x1, float x2, float gz, float gdz, float zz) {
+          if (k < 0 || k >= ngd) return;
+          const float temp = e.gg * gz;  // (gx gy) gz, the reference's order
+          const float tempd = e.dd * gdz;
+          acc[0] += (double)(x0 * temp);
+          acc[1] += (double)(x1 * temp);
+          acc[2] += (double)(x2 * temp);
+          acc[3] += (double)((x2 * e.ry - x1 * zz) * tempd);
+          acc[4] += (double)((x0 * zz - x2 * e.rx) * tempd);
+          acc[5] += (double)((x1 * e.rx - x0 * e.ry) * tempd);
+        };
+        add(k0, a0.x, a1.x, a2.x, g.x, gd.x, r.x);
+        add(k0 + 1, a0.y, a1.y, a2.y, g.y, gd.y, r.y);
+        add(k0 + 2, a0.z, a1.z, a2.z, g.z, gd.z, r.z);
+        add(k0 + 3, a0.w, a1.w, a2.w, g.w, gd.w, r.w);
+      } else {
+        float p0 = 0.f, p1 = 0.f, p2 = 0.f, p3 = 0.f, p4 = 0.f, p5 = 0.f;
+        auto add = [&](float x0, float x1, float x2, float gz, float gdz, float zz) {
+          const float temp = e.gg * gz;  // (gx gy) gz, the reference's order
+          const float tempd = e.dd * gdz;
+          p0 += x0 * temp;
+          p1 += x1 * temp;
+          p2 += x2 * temp;
+          p3 += (x2 * e.ry - x1 * zz) * tempd;
+          p4 += (x0 * zz - x2 * e.rx) * tempd;
+          p5 += (x1 * e.rx - x0 * e.ry) * tempd;
+        };
+        add(a0.x, a1.x, a2.x, g.x, gd.x, r.x);
+        add(a0.y, a1.y, a2.y, g.y, gd.y, r.y);
+        add(a0.z, a1.z, a2.z, g.z, gd.z, r.z);
+        add(a0.w, a1.w, a2.w, g.w, gd.w, r.w);
+        acc[0] += (double)p0;
+        acc[1] += (double)p1;
+        acc[2] += (double)p2;
+        acc[3] += (double)p3;
+        acc[4] += (double)p4;
+        acc[5] += (double)p5;
+      }
       qi += dq;
       ij += dij;
       if (qi >= nq) {
@@ -1189,24 +1211,31 @@ fs_status interp_t(fs_ctx *c, const FcmConsts &k, double *V, double *W, int np) 
   const int sms = FS_INTERP_WARPS * c->num_sms;
   const int split = 4 * np <= sms ? 4 : 2 * np <= sms ? 2 : 1;
   const size_t wb = sizeof(R) == 4 ? interp_q_warp_bytes(k.ngd) : 0;  // dynamic shared memory per bead of a CTA
-  const int wpb = split > 1 ? 4 : (c->tune_interp_wpb == 16 && 16 * wb > FS_SMEM_MAX) ? 8 : c->tune_interp_wpb;
-#define FS_INTERP_LAUNCH(WPB, SPLIT)                                                                             \
+  const bool single = sizeof(R) == 4 && k.N[2] < k.ngd + 6;
+  const int wpb = split > 1 || single ? 4 : (c->tune_interp_wpb == 16 && 16 * wb > FS_SMEM_MAX) ? 8 : c->tune_interp_wpb;
+#define FS_INTERP_LAUNCH(WPB, SPLIT, SINGLE)                                                                     \
   if constexpr (sizeof(R) == 4)                                                                                  \
-    fs_launch(k_interp_q<WPB, SPLIT>, fs_blocks(np, WPB / SPLIT), 32 * WPB, WPB / SPLIT * wb, c->stream, \
-              (const float *)c->grid_real, (const float4 *)c->bead_rec, np, k, V, W); \
+    fs_launch(k_interp_q<WPB, SPLIT, SINGLE>, fs_blocks(np, WPB / SPLIT), 32 * WPB, WPB / SPLIT * wb, c->stream, \
+              (const float *)c->grid_real, (const float4 *)c->bead_rec, np, k, V, W);                            \
   else                                                                                                           \
-    fs_launch(k_interp64<WPB, SPLIT>, fs_blocks(np, WPB / SPLIT), 32 * WPB, 0, c->stream, \
+    fs_launch(k_interp64<WPB, SPLIT>, fs_blocks(np, WPB / SPLIT), 32 * WPB, 0, c->stream,                        \
               (const double *)c->grid_real, (const double4 *)c->bead_rec, np, k, V, W)
-  if (split == 4) {
-    FS_INTERP_LAUNCH(4, 4);
+  if (single && split == 4) {
+    FS_INTERP_LAUNCH(4, 4, true);
+  } else if (single && split == 2) {
+    FS_INTERP_LAUNCH(4, 2, true);
+  } else if (single) {
+    FS_INTERP_LAUNCH(4, 1, true);
+  } else if (split == 4) {
+    FS_INTERP_LAUNCH(4, 4, false);
   } else if (split == 2) {
-    FS_INTERP_LAUNCH(4, 2);
+    FS_INTERP_LAUNCH(4, 2, false);
   } else if (wpb == 4) {
-    FS_INTERP_LAUNCH(4, 1);
+    FS_INTERP_LAUNCH(4, 1, false);
   } else if (wpb == 16) {
-    FS_INTERP_LAUNCH(16, 1);
+    FS_INTERP_LAUNCH(16, 1, false);
   } else {
-    FS_INTERP_LAUNCH(8, 1);
+    FS_INTERP_LAUNCH(8, 1, false);
   }
 #undef FS_INTERP_LAUNCH
   FS_LAUNCH_CHECK();
@@ -1262,9 +1291,10 @@ fs_status fcm_init(fs_ctx *c) {
   FS_CUDA(smem((const void *)k_spread64<4>, sizeof(SpreadStage64<4>)));
   FS_CUDA(smem((const void *)k_spread64<8>, sizeof(SpreadStage64<8>)));
   const size_t wq = interp_q_warp_bytes(FS_NGD_MAX);
-  FS_CUDA(smem((const void *)k_interp_q<4, 1>, 4 * wq));
-  FS_CUDA(smem((const void *)k_interp_q<8, 1>, 8 * wq));
-  FS_CUDA(smem((const void *)k_interp_q<16, 1>, 16 * wq));
+  FS_CUDA(smem((const void *)k_interp_q<4, 1, false>, 4 * wq));
+  FS_CUDA(smem((const void *)k_interp_q<4, 1, true>, 4 * wq));
+  FS_CUDA(smem((const void *)k_interp_q<8, 1, false>, 8 * wq));
+  FS_CUDA(smem((const void *)k_interp_q<16, 1, false>, 16 * wq));
   c->tune_spread_chunk = 32;
   c->tune_spread_cols = 2;  // 2 x 16 x 8 blocks: fs_autotune's choice at 384^3 and 512^3
   c->tune_interp_wpb = 4;  // the fastest at 256^3 and 512^3 in both precisions (512^3 FP64 before six x steps: 833, 873, 911 us)

@@ -713,7 +713,16 @@ fs_status y_lines(fs_ctx *c, V16 *A, const V16 *tw, bool inv) {
   const int nv = lines_nv<T>(c->nz), nvp = lines_nvp<T>(c->nz), ncol = 3 * c->nx * nv;
   typedef YShape<N, T> Y;
   const size_t smem = Y::SMEM;
-  if (inv)
+  // The inverse follows the x pass, for whose long lines the SMs give nearly all of their memory
+  // to shared memory (51 to 101 KB a CTA from 256 points on). An SM is split anew only when it is
+  // empty. Placed programmatically, while the last x CTAs run, the y CTAs kept the x pass's split,
+  // and the chain handed it on, L1 short, up to the interpolation's gathers. Whole solves, us,
+  // programmatic and plain: FP64 512^3 10,950 and 9,980, FP32 512 x 512 x 256 4,480 and 4,020, FP64
+  // 512 x 64 x 64 258 and 240, 256 x 512 x 512 6,510 and 6,360, 320^3 3,190 and 3,140, 256^3 1,280
+  // both; on shorter x lines a plain launch is 1 to 3 us more (FP32 64^3 59 and 61).
+  if (inv && c->nx >= 256)
+    k_lines_y<N, T, true><<<fs_blocks(ncol, Y::COLS), Y::THREADS, smem, c->stream>>>(A, ncol, nv, nvp, tw);
+  else if (inv)
     fs_launch(k_lines_y<N, T, true>, fs_blocks(ncol, Y::COLS), Y::THREADS, smem, c->stream, A, ncol, nv, nvp, tw);
   else
     fs_launch(k_lines_y<N, T, false>, fs_blocks(ncol, Y::COLS), Y::THREADS, smem, c->stream, A, ncol, nv, nvp, tw);

@@ -19,6 +19,7 @@ struct F2 {
 __device__ __forceinline__ F2 operator+(F2 a, F2 b) { return {f2_add(a.v, b.v)}; }
 __device__ __forceinline__ F2 operator-(F2 a, F2 b) { return {f2_sub(a.v, b.v)}; }
 __device__ __forceinline__ F2 operator*(F2 a, F2 b) { return {f2_mul(a.v, b.v)}; }
+__device__ __forceinline__ F2 operator-(F2 a) { return {f2_neg(a.v)}; }
 
 template <typename T>
 struct Num;

@@ -35,6 +35,7 @@ __device__ __forceinline__ f2p f2_mul(f2p a, f2p b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
+__device__ __forceinline__ f2p f2_neg(f2p a) { return a ^ 0x8000000080000000ull; }
 // a * b + c, one rounding per half
 __device__ __forceinline__ f2p f2_fma(f2p a, f2p b, f2p c) {
   f2p d;

@@ -52,11 +52,7 @@ template <typename T>
 __device__ __forceinline__ void mul_w(T &re, T &im, const V16 &w) {
   T wr, wi;
   Io<T>::get(w, wr, wi);
-  T a;
-  if constexpr (Num<T>::IS_DOUBLE)
-    a = fma(re, wr, -(im * wi));
-  else
-    a = re * wr - im * wi;
+  const T a = Num<T>::fma(re, wr, -(im * wi));  // one rounding less than a difference of products
   im = Num<T>::fma(re, wi, im * wr);
   re = a;
 }
@@ -288,7 +284,7 @@ struct Wave<F2> {
   }
   static __device__ __forceinline__ F2 inv(F2 s) {
     const float2 f = f2_unpack(s.v);
-    return {f2_pack(__fdividef(1.0f, f.x), __fdividef(1.0f, f.y))};
+    return {f2_pack(__frcp_rn(f.x), __frcp_rn(f.y))};
   }
   static __device__ __forceinline__ void zero(int v, F2 &s) {  // kz = 0 is the first of its pair
     if (v == 0) s.v = f2_pack(0.f, f2_unpack(s.v).y);
@@ -298,7 +294,8 @@ struct Wave<F2> {
 struct XArgs {
   int ncol, ny, nv, nvp;
   size_t rstride, cstride;  // between x planes and between components
-  double ffx, ffy, ffz, inv_total;
+  double ffx, ffy, ffz;
+  double inv_total, inv_total_lo;  // 1 / (Nx Ny Nz) to this precision, and what rounding it left out
 };
 template <int N, typename T>
 __global__ void __launch_bounds__(XShape<N>::THREADS, XShape<N>::CTAS)
@@ -354,17 +351,18 @@ __global__ void __launch_bounds__(XShape<N>::THREADS, XShape<N>::CTAS)
     for (int j = 0; j < L::RL; ++j) {
       const int k = L::last_index(t, j);
       const T q1 = Num<T>::c((double)((k <= N / 2) ? k : k - N) * g.ffx);
-      const T norm = Wave<T>::inv(Num<T>::fma(q2, q2, q1 * q1) + Num<T>::c(1e-18) + q3 * q3);
-      const T kfr = (q1 * zr[0][j] + q2 * zr[1][j] + q3 * zr[2][j]) * norm;
-      const T kfi = (q1 * zi[0][j] + q2 * zi[1][j] + q3 * zi[2][j]) * norm;
-      T sc = norm * Num<T>::c(g.inv_total);
+      const T norm = Wave<T>::inv(Num<T>::fma(q3, q3, Num<T>::fma(q2, q2, q1 * q1) + Num<T>::c(1e-18)));
+      // minus q . f / q^2, so that f - q (q . f) / q^2 is one rounding
+      const T kfr = -(Num<T>::fma(q3, zr[2][j], Num<T>::fma(q2, zr[1][j], q1 * zr[0][j])) * norm);
+      const T kfi = -(Num<T>::fma(q3, zi[2][j], Num<T>::fma(q2, zi[1][j], q1 * zi[0][j])) * norm);
+      T sc = Num<T>::fma(norm, Num<T>::c(g.inv_total), norm * Num<T>::c(g.inv_total_lo));
       if (k == 0 && y == 0) Wave<T>::zero(v, sc);
-      zr[0][j] = sc * (zr[0][j] - q1 * kfr);
-      zi[0][j] = sc * (zi[0][j] - q1 * kfi);
-      zr[1][j] = sc * (zr[1][j] - q2 * kfr);
-      zi[1][j] = sc * (zi[1][j] - q2 * kfi);
-      zr[2][j] = sc * (zr[2][j] - q3 * kfr);
-      zi[2][j] = sc * (zi[2][j] - q3 * kfi);
+      zr[0][j] = sc * Num<T>::fma(q1, kfr, zr[0][j]);
+      zi[0][j] = sc * Num<T>::fma(q1, kfi, zi[0][j]);
+      zr[1][j] = sc * Num<T>::fma(q2, kfr, zr[1][j]);
+      zi[1][j] = sc * Num<T>::fma(q2, kfi, zi[1][j]);
+      zr[2][j] = sc * Num<T>::fma(q3, kfr, zr[2][j]);
+      zi[2][j] = sc * Num<T>::fma(q3, kfi, zi[2][j]);
     }
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
@@ -742,7 +740,9 @@ fs_status x_lines(fs_ctx *c, V16 *A, const V16 *tw) {
   g.ffx = TwoPI / (c->nx * c->p.dx);
   g.ffy = TwoPI / (c->ny * c->p.dx);
   g.ffz = TwoPI / (c->nz * c->p.dx);
-  g.inv_total = 1.0 / ((double)c->nx * (double)c->ny * (double)c->nz);
+  const long double inv = 1.0L / ((long double)c->nx * c->ny * c->nz);
+  g.inv_total = Num<T>::IS_DOUBLE ? (double)inv : (double)(float)inv;
+  g.inv_total_lo = (double)(inv - (long double)g.inv_total);
   typedef XShape<N> X;
   fs_launch(k_lines_x_project<N, T>, fs_blocks(g.ncol, X::COLS), X::THREADS, X::SMEM, c->stream, A, g, tw);
   FS_LAUNCH_CHECK();

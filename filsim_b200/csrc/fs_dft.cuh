@@ -283,4 +283,10 @@ struct Dft<12, T> : DftAB<3, 4, T> {};
 template <typename T>
 struct Dft<14, T> : DftAB<2, 7, T> {};
 template <typename T>
+struct Dft<15, T> : DftAB<3, 5, T> {};
+template <typename T>
 struct Dft<16, T> : DftAB<4, 4, T> {};
+template <typename T>
+struct Dft<18, T> : DftAB<2, 9, T> {};
+template <typename T>
+struct Dft<20, T> : DftAB<4, 5, T> {};

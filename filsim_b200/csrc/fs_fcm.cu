@@ -1308,15 +1308,7 @@ fs_status fcm_init(fs_ctx *c) {
   return fft32_init(c);
 }
 
-bool lines_supported(const fs_ctx *c) {
-  auto len = [](int n) {
-    static const int ok[] = {32, 48, 64, 80, 96, 112, 128, 144, 160, 192, 224, 256, 320, 384, 448, 512};
-    for (int v : ok)
-      if (n == v) return true;
-    return false;
-  };
-  return len(c->nx) && len(c->ny) && len(c->nz);
-}
+bool lines_supported(const fs_ctx *c) { return line_length(c->nx) && line_length(c->ny) && line_length(c->nz); }
 
 void fcm_free(fs_ctx *c) {
   for (int p = 0; p < 2; ++p)

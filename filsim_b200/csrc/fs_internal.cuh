@@ -253,7 +253,23 @@ fs_status fcm_spread_only(fs_ctx *c, const double *Y, const double *F, const dou
 fs_status fcm_interpolate_only(fs_ctx *c, const double *u, const double *Y, int np, double *V, double *W);
 void slab_free(fs_ctx *c);
 
-bool lines_supported(const fs_ctx *c);  // every axis has a length of the line transforms (fs_lines.cuh)
+// Line lengths of the line transforms (fs_lines.cuh): grid lengths (multiples of 16) of the factors
+// 2, 3, 5 and 7, whose small transforms fs_dft.cuh has, from 32, two steps of at least four points
+// on a z line's half, to 512, beyond which two CTAs' x lines do not fit an SM's shared memory.
+// cuFFT takes about twice as long on all of them (flow solves, FP64: 240^3 1.83 and 1.00 ms, 432^3
+// 11.7 and 6.9, 480 x 64 x 64 0.27 and 0.16; FP32 with its conversions 240^3 1.11 and 0.64).
+constexpr bool line_length(int n) {
+  if (n < 32 || n > 512 || n % FS_TILE) return false;
+  for (int f : {2, 3, 5, 7})
+    while (n % f == 0) n /= f;
+  return n == 1;
+}
+constexpr int line_lengths() {
+  int count = 0;
+  for (int n = 0; n <= 512; ++n) count += line_length(n);
+  return count;
+}
+bool lines_supported(const fs_ctx *c);  // every axis has such a length
 fs_status lines_init64(fs_ctx *c);
 fs_status lines_init32(fs_ctx *c);
 fs_status lines_prepare64(fs_ctx *c);

@@ -1,5 +1,5 @@
-// fs_lines.cuh -- the line transforms of the periodic Stokes solve (fs_lines.cu) for
-// double and for packed FP32 pairs.
+// fs_lines.cuh -- the line transforms of the periodic Stokes solve, for double (fs_lines64.cu)
+// and for packed FP32 pairs (fs_lines32.cu).
 //
 // A line of N = R1 R2 (R3) points is transformed by a few threads, each holding one
 // radix-R group in registers at a time, with one exchange through shared memory
@@ -12,6 +12,7 @@
 // f32x2 instructions and both precisions share the code and the access patterns.
 #pragma once
 #include "fs_internal.cuh"
+#include <type_traits>
 #include "fs_dft.cuh"
 
 typedef ulonglong2 V16;  // one transform value in memory: (re, im) of T
@@ -61,9 +62,10 @@ __device__ __forceinline__ void mul_tw(T &re, T &im, const V16 *__restrict__ w) 
   mul_w<T>(re, im, __ldg(w));
 }
 
-// radices of a line. Y and z lines: at most 16 points in registers, the fewest
-// exchanges, and as even a split as the factors allow (threads per line = N / smallest
-// radix). X lines hold three components per thread: at most 8 points each.
+// Radices of a line. Y and z lines: at most 16 points in registers (18 and 20 for z lines of 432
+// and 400 points, which like all z lines take two steps), the fewest exchanges, and as even a
+// split as the factors allow (threads per line = N / smallest radix). X lines end with three
+// components per thread: at most 8 points each there.
 template <int N>
 struct Radices;
 template <int N>
@@ -84,15 +86,25 @@ FS_RADICES(Radices, 72, 8, 9, 1)
 FS_RADICES(Radices, 80, 8, 10, 1)
 FS_RADICES(Radices, 96, 8, 12, 1)
 FS_RADICES(Radices, 112, 8, 14, 1)
+FS_RADICES(Radices, 120, 10, 12, 1)
 FS_RADICES(Radices, 128, 8, 16, 1)
 FS_RADICES(Radices, 144, 12, 12, 1)
 FS_RADICES(Radices, 160, 10, 16, 1)
+FS_RADICES(Radices, 168, 12, 14, 1)
 FS_RADICES(Radices, 192, 12, 16, 1)
+FS_RADICES(Radices, 200, 10, 20, 1)
+FS_RADICES(Radices, 216, 12, 18, 1)
 FS_RADICES(Radices, 224, 14, 16, 1)
+FS_RADICES(Radices, 240, 15, 16, 1)
 FS_RADICES(Radices, 256, 16, 16, 1)
+FS_RADICES(Radices, 288, 8, 6, 6)
 FS_RADICES(Radices, 320, 8, 8, 5)
+FS_RADICES(Radices, 336, 8, 6, 7)
 FS_RADICES(Radices, 384, 8, 8, 6)
+FS_RADICES(Radices, 400, 8, 10, 5)
+FS_RADICES(Radices, 432, 8, 9, 6)
 FS_RADICES(Radices, 448, 8, 8, 7)
+FS_RADICES(Radices, 480, 8, 10, 6)
 FS_RADICES(Radices, 512, 8, 8, 8)
 FS_RADICES(RadicesX, 32, 4, 8, 1)
 FS_RADICES(RadicesX, 48, 6, 8, 1)
@@ -105,10 +117,16 @@ FS_RADICES(RadicesX, 144, 4, 6, 6)
 FS_RADICES(RadicesX, 160, 8, 4, 5)
 FS_RADICES(RadicesX, 192, 8, 4, 6)
 FS_RADICES(RadicesX, 224, 8, 4, 7)
+FS_RADICES(RadicesX, 240, 8, 6, 5)
 FS_RADICES(RadicesX, 256, 8, 8, 4)
+FS_RADICES(RadicesX, 288, 8, 6, 6)
 FS_RADICES(RadicesX, 320, 8, 8, 5)
+FS_RADICES(RadicesX, 336, 8, 6, 7)
 FS_RADICES(RadicesX, 384, 8, 8, 6)
+FS_RADICES(RadicesX, 400, 8, 10, 5)
+FS_RADICES(RadicesX, 432, 8, 9, 6)
 FS_RADICES(RadicesX, 448, 8, 8, 7)
+FS_RADICES(RadicesX, 480, 8, 10, 6)
 FS_RADICES(RadicesX, 512, 8, 8, 8)
 #undef FS_RADICES
 
@@ -203,7 +221,8 @@ struct YShape {
   static constexpr int THREADS = COLS * Line<N>::TH;
   static constexpr int MS = COLS < 8 ? Line<N>::M | 1 : Line<N>::M;
   static constexpr size_t SMEM = sizeof(V16) * (size_t)COLS * Line<N>::R1 * MS;
-  static constexpr int CTAS = THREADS >= 512 ? 2 : THREADS >= 256 ? 4 : 512 / THREADS;  // at 64 and 128 registers
+  // at 64 registers from 256 threads on, at 128 below
+  static constexpr int CTAS = THREADS > 512 ? 1 : THREADS >= 256 ? 1024 / THREADS : 512 / THREADS;
 };
 template <int N, typename T, bool INV>
 __global__ void __launch_bounds__(YShape<N, T>::THREADS, YShape<N, T>::CTAS)
@@ -265,7 +284,7 @@ struct XShape {
   static constexpr int MS = COLS < 8 ? LineX<N>::M | 1 : LineX<N>::M;
   static constexpr int NS = COLS * LineX<N>::R1 * MS;  // one component's exchange buffer
   static constexpr size_t SMEM = sizeof(V16) * 3 * NS;
-  static constexpr int CTAS = 512 / THREADS > 1 ? 512 / THREADS : 1;  // at most 128 registers
+  static constexpr int CTAS = THREADS > 256 ? 2 : 512 / THREADS;  // at most 128 registers, 96 above 256 threads
 };
 template <typename T>
 struct Wave;  // kz of one value and the reciprocal of the squared wavenumber
@@ -612,26 +631,24 @@ int lines_nv(int nz) { return Num<T>::IS_DOUBLE ? nz / 2 + 1 : nz / 4 + 1; }
 template <typename T>
 int lines_nvp(int nz) { return (lines_nv<T>(nz) + 1) & ~1; }
 
-#define FS_LINES_SWITCH(n, fn, ...)                \
-  switch (n) {                                     \
-    case 32: FS_TRY((fn<32, T>(__VA_ARGS__))); break;     \
-    case 48: FS_TRY((fn<48, T>(__VA_ARGS__))); break;     \
-    case 64: FS_TRY((fn<64, T>(__VA_ARGS__))); break;     \
-    case 80: FS_TRY((fn<80, T>(__VA_ARGS__))); break;     \
-    case 96: FS_TRY((fn<96, T>(__VA_ARGS__))); break;     \
-    case 112: FS_TRY((fn<112, T>(__VA_ARGS__))); break;   \
-    case 128: FS_TRY((fn<128, T>(__VA_ARGS__))); break;   \
-    case 144: FS_TRY((fn<144, T>(__VA_ARGS__))); break;   \
-    case 160: FS_TRY((fn<160, T>(__VA_ARGS__))); break;   \
-    case 192: FS_TRY((fn<192, T>(__VA_ARGS__))); break;   \
-    case 224: FS_TRY((fn<224, T>(__VA_ARGS__))); break;   \
-    case 256: FS_TRY((fn<256, T>(__VA_ARGS__))); break;   \
-    case 320: FS_TRY((fn<320, T>(__VA_ARGS__))); break;   \
-    case 384: FS_TRY((fn<384, T>(__VA_ARGS__))); break;   \
-    case 448: FS_TRY((fn<448, T>(__VA_ARGS__))); break;   \
-    case 512: FS_TRY((fn<512, T>(__VA_ARGS__))); break;   \
-    default: return FS_ERR_INVALID_ARG;            \
-  }
+#define FS_LINE_LENGTHS(X)                                                                                   \
+  X(32) X(48) X(64) X(80) X(96) X(112) X(128) X(144) X(160) X(192) X(224) X(240) X(256) X(288) X(320) X(336) \
+  X(384) X(400) X(432) X(448) X(480) X(512)
+// the list is line_length's rule: each length that it takes, and no other
+#define FS_LINE_COUNT(N) +(line_length(N) ? 1 : 100)
+static_assert(FS_LINE_LENGTHS(FS_LINE_COUNT) == line_lengths(), "lengths of the line transforms");
+#undef FS_LINE_COUNT
+#define FS_LINE_CASE(N) \
+  case N: return f(std::integral_constant<int, N>());
+// f with the length n as a constant
+template <typename F>
+fs_status with_length(int n, F f) {
+  switch (n) { FS_LINE_LENGTHS(FS_LINE_CASE) }
+  return FS_ERR_INVALID_ARG;
+}
+#undef FS_LINE_CASE
+#define FS_LINES_SWITCH(n, fn, ...) \
+  FS_TRY(with_length(n, [&](auto len) { return fn<decltype(len)::value, T>(__VA_ARGS__); }))
 
 // table values of one line: first- and second-step twiddles, then (z lines) w^k, k <= N
 struct TwRoot {

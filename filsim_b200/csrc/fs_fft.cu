@@ -1,5 +1,5 @@
-// fs_fft.cu -- FP32 periodic Stokes solve on the largest grids (fft32_preferred) for sm_100a:
-// the forward real 3-D transform, the projection of flow_solve
+// fs_fft.cu -- FP32 periodic Stokes solve on the largest grids (fft32_preferred: 512 points along
+// x, 384 or 512 along y and z) for sm_100a: the forward real 3-D transform, the projection of flow_solve
 // (FCMfunctions.cpp:648-736) and the inverse real transform in five passes
 // over HBM, replacing cuFFT R2C + projection + C2R in the mixed-precision path.
 //
@@ -12,7 +12,8 @@
 //                         --y_inv-->    A[c][kz][x][y]
 //                         --z_c2r-->    u[c][x][y][z] (real)
 // Each pass reads and writes the grid once with 128-byte rows. Every line is
-// transformed by one warp in registers: N = 32*M points, M per lane, an
+// transformed by one warp in registers: N = 32*M points, M per lane (512 points, or three times
+// 128 after a radix-3 step), an
 // M-point radix-2 DFT per lane, a transpose through a padded per-warp shared
 // buffer, a second M-point DFT and log2(32/M) radix-2 stages across lanes with
 // shuffles. Transforms are unnormalised; the projection divides by Nx*Ny*Nz as
@@ -21,6 +22,7 @@
 // along x and y, the semantics of the reference's multi-dimensional real
 // inverse transform. Along z a warp transforms its two real lines a, b as one
 // complex line a + i b and separates (or assembles) their half spectra.
+#include <vector>
 #include "fs_internal.cuh"
 #include "fs_f32x2.cuh"
 
@@ -38,7 +40,7 @@ constexpr int TW_FULL = 1024;            // tw[j] = exp(-2 pi i j / 1024)
 // spreads the lanes of each half-warp over distinct banks.
 template <int N>
 __host__ __device__ constexpr int prow(int k) {
-  return N == 32 ? k + (k >> 4) : k + (k / ((N / 32) * (N / 32))) * (16 / (32 / (N / 32)));
+  return k + (k / ((N / 32) * (N / 32))) * (16 / (32 / (N / 32)));
 }
 
 template <int N>
@@ -48,7 +50,8 @@ struct Fft {
   static constexpr int RS = 32 + (G < 16 ? G : 0);       // padded transpose row
   static constexpr int PEXT = prow<N>(N - 1) + 1;        // rows of a swizzled N-point buffer
   static constexpr int SW = (PEXT > M * RS ? PEXT : M * RS);  // per-warp scratch (float2)
-  static constexpr int LANE_TAB = TW_FULL + N - 32;      // offset of the per-lane twiddle table
+  static constexpr int LANE_TAB = TW_FULL + (N == 512 ? 0 : 512);  // offset of the per-lane twiddle table
+  static_assert(N == 512 || N == 128, "lines of 512 points and thirds of 384");
 };
 
 __host__ __device__ constexpr int bitrev_c(int i, int n) {
@@ -218,14 +221,12 @@ __device__ __forceinline__ void fft_n2p(float2 (&v)[Fft<N>::M], float2 *S, const
 #pragma unroll
   for (int i = 1; i < M; ++i) v[i] = cmul(v[i], twd<D>(tw + Fft<N>::LANE_TAB, bitrev_c(i, M) * 32 + lane));
   const int c = lane / G, h = lane & (G - 1);
-  if (M > 1) {
 #pragma unroll
-    for (int i = 0; i < M; ++i) S[bitrev_c(i, M) * RS + lane] = v[i];
-    __syncwarp();
+  for (int i = 0; i < M; ++i) S[bitrev_c(i, M) * RS + lane] = v[i];
+  __syncwarp();
 #pragma unroll
-    for (int j = 0; j < M; ++j) v[j] = S[c * RS + h + G * j];
-    __syncwarp();
-  }
+  for (int j = 0; j < M; ++j) v[j] = S[c * RS + h + G * j];
+  __syncwarp();
   dif_reg<M, D>(v);
   stage2_twiddle<N, D>(v, tw, h);
   // radix-2 stages across lanes: lower lane a + b, upper lane (a - b) w
@@ -265,43 +266,34 @@ __device__ __forceinline__ void fft_p2n(float2 (&v)[Fft<N>::M], float2 *S, const
   }
   stage2_twiddle<N, D>(v, tw, h);
   dit_reg<M, D>(v);
-  if (M > 1) {
 #pragma unroll
-    for (int j = 0; j < M; ++j) S[c * RS + h + G * j] = v[j];
-    __syncwarp();
+  for (int j = 0; j < M; ++j) S[c * RS + h + G * j] = v[j];
+  __syncwarp();
 #pragma unroll
-    for (int i = 0; i < M; ++i) v[i] = S[bitrev_c(i, M) * RS + lane];
-    __syncwarp();
-  }
+  for (int i = 0; i < M; ++i) v[i] = S[bitrev_c(i, M) * RS + lane];
+  __syncwarp();
 #pragma unroll
   for (int i = 1; i < M; ++i) v[i] = cmul(v[i], twd<D>(tw + Fft<N>::LANE_TAB, bitrev_c(i, M) * 32 + lane));
   dit_reg<M, D>(v);
 }
 
-// ---- lines of any supported length --------------------------------------------
-// N = 2^p (32..512) runs the pipelines above. N = 3P, P = 2^p (96, 192, 384) adds a
+// ---- lines of 512 and 384 points -------------------------------------------------
+// N = 512 runs the pipelines above. N = 3P = 384 adds a
 // radix-3 step: a lane's registers m, m + P/32, m + 2P/32 hold the points n, n + P,
 // n + 2P (n = lane + 32 m); one 3-point DFT across them, the twiddles
 // exp(-D 2 pi i n k3 / N) (k3 = 1, 2), then the three P-point warp transforms, so
-// that register k3 P/32 + i holds X[3 index_P(i) + k3] (decimation in frequency;
-// the adjoint runs the steps backwards). The twiddles come from a per-N table of
-// exp(-2 pi i j / N), j < 2P, after the power-of-two tables.
-constexpr int TW3_BASE = TW_FULL + 512 - 32 + 512;
-constexpr int TW3_LEN = 64 + 128 + 256;  // 2P for N = 96, 192, 384
-template <int N>
-__host__ __device__ constexpr int tw3_off() {
-  return TW3_BASE + (N == 96 ? 0 : N == 192 ? 64 : 192);
-}
-// Row of spectrum index k in a natural-order buffer. For N = 3P a warp writes
-// register i to X = 3 index_P(lane, i) + k3, i.e. 3c + 48h + K (P = 128 and 32:
-// c < 4 or c = 0, h the lane's bit-reversed column, K < 48 the same for all lanes)
-// or 3c + 12h + K (P = 64, c < 2, K < 12); k + 4 floor(k / 48), resp. k + floor(k / 12),
+// that register k3 P/32 + i holds X[3 index_P(i) + k3] (decimation in frequency).
+// The twiddles come from a table of exp(-2 pi i j / N), j < 2P, after the power-of-two tables.
+constexpr int TW3 = TW_FULL + 512 + 128;  // its offset
+constexpr int TW3_LEN = 256;
+// Row of spectrum index k in a natural-order buffer. For N = 384 a warp writes
+// register i to X = 3 index_P(lane, i) + k3, i.e. 3c + 48h + K (c < 4,
+// h the lane's bit-reversed column, K < 48 the same for all lanes); k + 4 floor(k / 48)
 // puts the 32 lanes on 16 distinct 8-byte bank pairs, two each (the minimum), and
 // keeps consecutive k on consecutive rows apart from one skip per block.
 template <int N>
 __host__ __device__ constexpr int xf_row(int k) {
-  if constexpr (N == 192) return k + k / 12;
-  else if constexpr (N % 3 == 0) return k + 4 * (k / 48);
+  if constexpr (N % 3 == 0) return k + 4 * (k / 48);
   else return prow<N>(k);
 }
 template <int N>
@@ -343,7 +335,7 @@ template <int N, int D>
 __device__ __forceinline__ void xf_fwd(float2 (&v)[N / 32], float2 *S, const float2 *__restrict__ tw, int lane) {
   if constexpr (N % 3 == 0) {
     constexpr int P = N / 3, MP = P / 32;
-    const float2 *t3 = tw + tw3_off<N>();
+    const float2 *t3 = tw + TW3;
 #pragma unroll
     for (int m = 0; m < MP; ++m) {
       radix3<D>(v[m], v[m + MP], v[m + 2 * MP]);
@@ -362,34 +354,6 @@ __device__ __forceinline__ void xf_fwd(float2 (&v)[N / 32], float2 *S, const flo
     }
   } else {
     fft_n2p<N, D>(v, S, tw, lane);
-  }
-}
-
-// the adjoint of xf_fwd: register-order input, natural output; xf_inv<N, -1>
-// inverts xf_fwd<N, +1> up to the factor N
-template <int N, int D>
-__device__ __forceinline__ void xf_inv(float2 (&v)[N / 32], float2 *S, const float2 *__restrict__ tw, int lane) {
-  if constexpr (N % 3 == 0) {
-    constexpr int P = N / 3, MP = P / 32;
-    const float2 *t3 = tw + tw3_off<N>();
-#pragma unroll
-    for (int k3 = 0; k3 < 3; ++k3) {
-      float2 u[MP];
-#pragma unroll
-      for (int i = 0; i < MP; ++i) u[i] = v[k3 * MP + i];
-      fft_p2n<P, D>(u, S, tw, lane);
-#pragma unroll
-      for (int i = 0; i < MP; ++i) v[k3 * MP + i] = u[i];
-    }
-#pragma unroll
-    for (int m = 0; m < MP; ++m) {
-      const int n = lane + 32 * m;
-      v[m + MP] = cmul(v[m + MP], twd<D>(t3, n));
-      v[m + 2 * MP] = cmul(v[m + 2 * MP], twd<D>(t3, 2 * n));
-      radix3<D>(v[m], v[m + MP], v[m + 2 * MP]);
-    }
-  } else {
-    fft_p2n<N, D>(v, S, tw, lane);
   }
 }
 
@@ -437,11 +401,10 @@ __device__ __forceinline__ float wavenumber_f(int i, int n, float ff) { return (
 // reciprocal is the fast one (2 ulp), well inside the FP32 chain's error.
 constexpr int XP_PAIRS = 1;                    // (kz, ky) lines per CTA (1: 5% faster than 2 at 512^3)
 constexpr int XP_THREADS = 3 * 32 * XP_PAIRS;  // one warp per component and line
-template <int NX>
 __global__ void __launch_bounds__(XP_THREADS) k_fft_x_project(float2 *__restrict__ B, int ny, int nzh,
                                                               size_t cstride, float ffx, float ffy, float ffz,
                                                               float inv_total, const float2 *__restrict__ tw) {
-  constexpr int M = (NX / 32), SW = xf_sw<NX>();
+  constexpr int NX = 512, M = NX / 32, SW = Fft<NX>::SW;
   __shared__ float2 Sall[3 * XP_PAIRS * SW];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int comp = warp % 3, pl = warp / 3;
@@ -454,7 +417,7 @@ __global__ void __launch_bounds__(XP_THREADS) k_fft_x_project(float2 *__restrict
   if (active) {
 #pragma unroll
     for (int m = 0; m < M; ++m) v[m] = line[lane + 32 * m];
-    xf_fwd<NX, 1>(v, S, tw, lane);
+    fft_n2p<NX, 1>(v, S, tw, lane);
 #pragma unroll
     for (int i = 0; i < M; ++i) S[lane + 32 * i] = v[i];
   }
@@ -464,7 +427,7 @@ __global__ void __launch_bounds__(XP_THREADS) k_fft_x_project(float2 *__restrict
     const float q2 = wavenumber_f(ky, ny, ffy), q3 = (float)kz * ffz;
 #pragma unroll
     for (int i = 0; i < M; ++i) {
-      const int kx = xf_index<NX>(lane, i);
+      const int kx = out_index<NX>(lane, i);
       const float q1 = wavenumber_f(kx, NX, ffx);
       const float qq = q2 * q2 + q1 * q1 + 1e-18f;
       const float norm = __fdividef(1.0f, qq + q3 * q3);
@@ -478,7 +441,7 @@ __global__ void __launch_bounds__(XP_THREADS) k_fft_x_project(float2 *__restrict
   }
   __syncthreads();
   if (active) {
-    xf_inv<NX, -1>(v, S, tw, lane);
+    fft_p2n<NX, -1>(v, S, tw, lane);
 #pragma unroll
     for (int m = 0; m < M; ++m) line[lane + 32 * m] = v[m];
   }
@@ -532,10 +495,14 @@ __global__ void __launch_bounds__(FFT_THREADS) k_fft_y_inv(const float2 *__restr
 // (k <= NZ/2, the imaginary parts of A_0, A_{NZ/2}, B_0, B_{NZ/2} dropped) and
 // Z_{NZ-k} = conj A_k + i conj B_k, then a = Re z, b = Im z. One full-length
 // transform per line pair instead of two half-length ones.
-// ZT y tiles per CTA, consecutive in y: a warp issues the loads of its next line
+// Z_TILES y tiles per CTA, consecutive in y (24 or 32 in all): a warp issues the loads of its next line
 // pair before the CTA writes the current tile out, so each warp keeps one pair
-// of lines in flight through the store phase.
-template <int NZ, int ZT>
+// of lines in flight through the store phase. (The same
+// overlap in z_c2r and y_inv, with the next tile's asynchronous copy under the
+// current tile's transforms, was slower at 512^3: 0.732 vs 0.724 ms and 0.689 vs
+// 0.667 ms.)
+constexpr int Z_TILES = 2;
+template <int NZ>
 __global__ void __launch_bounds__(FFT_THREADS) k_fft_z_r2c(const float *__restrict__ f, float2 *__restrict__ A,
                                                             int nx, int ny, const float2 *__restrict__ tw) {
   static_assert(FFT_TILE == 2 * FFT_WARPS, "two lines per warp");
@@ -544,7 +511,7 @@ __global__ void __launch_bounds__(FFT_THREADS) k_fft_z_r2c(const float *__restri
   float2 *T = fft_smem;  // (H + 1) x FFT_TS
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float2 *S = fft_smem + (H + 1) * FFT_TS + warp * SW;
-  const int nyg = ny / (FFT_TILE * ZT);  // groups of ZT tiles along y
+  const int nyg = ny / (FFT_TILE * Z_TILES);  // groups of tiles along y
   const int yg = blockIdx.x % nyg;
   const int x = (blockIdx.x / nyg) % nx;
   const int c = blockIdx.x / (nyg * nx);
@@ -557,14 +524,14 @@ __global__ void __launch_bounds__(FFT_THREADS) k_fft_z_r2c(const float *__restri
 #pragma unroll
     for (int m = 0; m < M; ++m) v[m] = make_float2(__ldg(la + lane + 32 * m), __ldg(lb + lane + 32 * m));
   };
-  load(yg * ZT);
+  load(yg * Z_TILES);
 #pragma unroll 1
-  for (int t = 0; t < ZT; ++t) {
-    const int yt = yg * ZT + t;
+  for (int t = 0; t < Z_TILES; ++t) {
+    const int yt = yg * Z_TILES + t;
     xf_fwd<NZ, 1>(v, S, tw, lane);
 #pragma unroll
     for (int i = 0; i < M; ++i) S[xf_row<NZ>(xf_index<NZ>(lane, i))] = v[i];
-    if (t + 1 < ZT) load(yt + 1);
+    if (t + 1 < Z_TILES) load(yt + 1);
     __syncwarp();
 #pragma unroll
     for (int m = 0; m < (H + 32) / 32; ++m) {
@@ -581,7 +548,7 @@ __global__ void __launch_bounds__(FFT_THREADS) k_fft_z_r2c(const float *__restri
       const int k = idx / FFT_TILE, j = idx % FFT_TILE;
       out[(size_t)k * plane + j] = T[k * FFT_TS + j];
     }
-    if (t + 1 < ZT) __syncthreads();  // T and S are rewritten by the next tile
+    if (t + 1 < Z_TILES) __syncthreads();  // T and S are rewritten by the next tile
   }
 }
 
@@ -650,19 +617,9 @@ constexpr size_t smem_z() { return sizeof(float2) * ((NZ / 2 + 1) * FFT_TS + FFT
 template <int NY>
 constexpr size_t smem_y() { return sizeof(float2) * (xf_rows<NY>() * FFT_TS + FFT_WARPS * xf_sw<NY>()); }
 
-bool pow2_in(int n, int lo, int hi) { return n >= lo && n <= hi && (n & (n - 1)) == 0; }
-
-// y tiles per z_r2c CTA where the grid has an even number of y tiles (the same
-// overlap in z_c2r and y_inv, with the next tile's asynchronous copy under the
-// current tile's transforms, was slower at 512^3: 0.732 vs 0.724 ms and 0.689 vs
-// 0.667 ms)
-constexpr int Z_TILES = 2;
-
 template <int NZ>
 fs_status z_attr() {
-  FS_CUDA(cudaFuncSetAttribute(k_fft_z_r2c<NZ, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_z<NZ>()));
-  FS_CUDA(cudaFuncSetAttribute(k_fft_z_r2c<NZ, Z_TILES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)smem_z<NZ>()));
+  FS_CUDA(cudaFuncSetAttribute(k_fft_z_r2c<NZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_z<NZ>()));
   FS_CUDA(cudaFuncSetAttribute(k_fft_z_c2r<NZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_z<NZ>()));
   return FS_OK;
 }
@@ -675,12 +632,8 @@ fs_status y_attr() {
 
 template <int NZ>
 fs_status z_fwd(fs_ctx *c, const float *f, float2 *A, const float2 *tw) {
-  const int nyt = c->ny / FFT_TILE;
-  if (nyt % Z_TILES == 0)
-    k_fft_z_r2c<NZ, Z_TILES><<<3 * c->nx * (nyt / Z_TILES), FFT_THREADS, smem_z<NZ>(), c->stream>>>(f, A, c->nx,
-                                                                                                    c->ny, tw);
-  else
-    k_fft_z_r2c<NZ, 1><<<3 * c->nx * nyt, FFT_THREADS, smem_z<NZ>(), c->stream>>>(f, A, c->nx, c->ny, tw);
+  k_fft_z_r2c<NZ><<<3 * c->nx * (c->ny / (FFT_TILE * Z_TILES)), FFT_THREADS, smem_z<NZ>(), c->stream>>>(f, A, c->nx,
+                                                                                                      c->ny, tw);
   FS_LAUNCH_CHECK();
   return FS_OK;
 }
@@ -702,83 +655,58 @@ fs_status y_inv(fs_ctx *c, const float2 *B, float2 *A, const float2 *tw) {
   FS_LAUNCH_CHECK();
   return FS_OK;
 }
-template <int NX>
 fs_status x_project(fs_ctx *c, float2 *B, const float2 *tw) {
   const double TwoPI = 2. * FS_PI;
   const float ffx = (float)(TwoPI / (c->nx * c->p.dx)), ffy = (float)(TwoPI / (c->ny * c->p.dx)),
               ffz = (float)(TwoPI / (c->nz * c->p.dx));
-  // 1 / (Nx Ny Nz) is a power of two here, so the product equals the reference's quotient
+  // a power of two at 512^3, where the product equals the reference's quotient
   const float inv_total = (float)(1.0 / ((double)c->nx * (double)c->ny * (double)c->nz));
   const int pairs = c->nzh * c->ny;
   const size_t cstride = (size_t)c->nzh * c->ny * c->nx;
-  k_fft_x_project<NX><<<fs_blocks(pairs, XP_PAIRS), XP_THREADS, 0, c->stream>>>(B, c->ny, c->nzh, cstride, ffx, ffy,
+  k_fft_x_project<<<fs_blocks(pairs, XP_PAIRS), XP_THREADS, 0, c->stream>>>(B, c->ny, c->nzh, cstride, ffx, ffy,
                                                                                 ffz, inv_total, tw);
   FS_LAUNCH_CHECK();
   return FS_OK;
 }
 
-#define FS_FFT_SWITCH_Z(n, fn, ...)                  \
-  switch (n) {                                       \
-    case 64: FS_TRY(fn<64>(__VA_ARGS__)); break;     \
-    case 96: FS_TRY(fn<96>(__VA_ARGS__)); break;     \
-    case 128: FS_TRY(fn<128>(__VA_ARGS__)); break;   \
-    case 192: FS_TRY(fn<192>(__VA_ARGS__)); break;   \
-    case 256: FS_TRY(fn<256>(__VA_ARGS__)); break;   \
-    case 384: FS_TRY(fn<384>(__VA_ARGS__)); break;   \
-    case 512: FS_TRY(fn<512>(__VA_ARGS__)); break;   \
-    default: return FS_ERR_INVALID_ARG;              \
-  }
-#define FS_FFT_SWITCH(n, fn, ...)                    \
-  if (n == 32) {                                     \
-    FS_TRY(fn<32>(__VA_ARGS__));                     \
-  } else {                                           \
-    FS_FFT_SWITCH_Z(n, fn, __VA_ARGS__)              \
-  }
+#define FS_FFT_SWITCH(n, fn, ...) FS_TRY((n) == 512 ? fn<512>(__VA_ARGS__) : fn<384>(__VA_ARGS__))
 
 }  // namespace
 
-// line lengths of the warp transforms: 2^p in [lo, 512], or 96, 192, 384
-static bool fft_len(int n, int lo) { return n >= lo && (pow2_in(n, lo, 512) || n == 96 || n == 192 || n == 384); }
-
-// Where the warp transform is the faster one: 512-point x lines of the largest boxes,
-// whose contiguous x pass it does in 0.73 ms at 512^3 against 1.05 ms for the strided
-// one of the line transforms, more than its z passes lose (3.50 against 3.77 ms in all).
-// At 512 x 512 x 256 and 512 x 256 x 512 the two are equal (1.87, 1.89 and 1.82, 1.82 ms),
-// below them the line transforms lead (512 x 512 x 128: 0.99 against 1.08 ms, 384^3: 1.69
-// against 1.97 ms, 256^3: 0.50 against 0.57 ms, 384 x 96 x 96: 0.15 against 0.24 ms).
+// Where the warp transform is the faster one: 512-point x lines of the largest boxes, whose
+// contiguous x pass it does in 0.75 ms at 512^3 against 1.05 ms for the strided one of the line
+// transforms, more than its z and y passes lose there (solves of 131,072 beads 4.90 and 5.15 ms).
+// With 384 points along y or z the two are within 4 % (512 x 384 x 512 3.82 and 3.86 ms, 512 x 512 x
+// 384 3.77 and 3.79, 512 x 384 x 384 3.04 and 2.92); below, the line transforms lead (512 x 512 x
+// 256 4.3 against 4.0 ms with 209,000 beads).
 bool fft32_preferred(const fs_ctx *c) {
-  return c->fft_tw && c->nx == 512 && (size_t)c->ny * c->nz > 512 * 256;
+  auto len = [](int n) { return n == 384 || n == 512; };
+  return c->nx == 512 && len(c->ny) && len(c->nz);
 }
-
-bool fft32_supported(const fs_ctx *c) { return fft_len(c->nx, 32) && fft_len(c->ny, 32) && fft_len(c->nz, 64); }
 
 fs_status fft32_init(fs_ctx *c) {
   c->fft_tw = nullptr;
-  if (!fft32_supported(c)) return FS_OK;
-  // [0, 1024): exp(-2 pi i j / 1024); then per N in {32, ..., 512}, at 1024 + N - 32,
-  // the lane table [k2 * 32 + lane] = exp(-2 pi i lane k2 / N), k2 < N / 32; then per
-  // N in {96, 192, 384}, at tw3_off<N>, exp(-2 pi i j / N), j < 2N/3.
-  const int ntw = TW3_BASE + TW3_LEN;
-  float2 *h = (float2 *)malloc(sizeof(float2) * ntw);
-  if (!h) return FS_ERR_OOM;
-  const double TwoPI = 2. * FS_PI;
-  for (int j = 0; j < TW_FULL; ++j) h[j] = make_float2((float)cos(TwoPI * j / TW_FULL), (float)-sin(TwoPI * j / TW_FULL));
-  for (int n = 32; n <= 512; n <<= 1)
+  if (!fft32_preferred(c)) return FS_OK;
+  // [0, 1024): exp(-2 pi i j / 1024); then per N = 512 and 128, at Fft<N>::LANE_TAB, the lane
+  // table [k2 * 32 + lane] = exp(-2 pi i lane k2 / N), k2 < N / 32; then, at TW3,
+  // exp(-2 pi i j / 384), j < 256
+  std::vector<float2> h(TW3 + TW3_LEN);
+  auto root = [](int j, int n) {
+    const double a = 2. * FS_PI * j / n;
+    return make_float2((float)cos(a), (float)-sin(a));
+  };
+  for (int j = 0; j < TW_FULL; ++j) h[j] = root(j, TW_FULL);
+  for (int n : {512, 128}) {
+    const int at = n == 512 ? Fft<512>::LANE_TAB : Fft<128>::LANE_TAB;
     for (int k2 = 0; k2 < n / 32; ++k2)
-      for (int l = 0; l < 32; ++l) {
-        const long long j = (long long)l * k2;
-        h[TW_FULL + n - 32 + k2 * 32 + l] = make_float2((float)cos(TwoPI * j / n), (float)-sin(TwoPI * j / n));
-      }
-  const int n3[3] = {96, 192, 384}, off3[3] = {tw3_off<96>(), tw3_off<192>(), tw3_off<384>()};
-  for (int q = 0; q < 3; ++q)
-    for (int j = 0; j < 2 * n3[q] / 3; ++j)
-      h[off3[q] + j] = make_float2((float)cos(TwoPI * j / n3[q]), (float)-sin(TwoPI * j / n3[q]));
-  cudaError_t e = cudaMalloc(&c->fft_tw, sizeof(float2) * ntw);
-  if (e == cudaSuccess) e = cudaMemcpy(c->fft_tw, h, sizeof(float2) * ntw, cudaMemcpyHostToDevice);
-  free(h);
-  if (e != cudaSuccess) return e == cudaErrorMemoryAllocation ? FS_ERR_OOM : FS_ERR_CUDA;
-  c->bytes += sizeof(float2) * ntw;
-  FS_FFT_SWITCH_Z(c->nz, z_attr);
+      for (int l = 0; l < 32; ++l) h[at + k2 * 32 + l] = root(l * k2, n);
+  }
+  for (int j = 0; j < TW3_LEN; ++j) h[TW3 + j] = root(j, 384);
+  const size_t bytes = sizeof(float2) * h.size();
+  FS_CUDA(cudaMalloc(&c->fft_tw, bytes));
+  c->bytes += bytes;
+  FS_CUDA(cudaMemcpy(c->fft_tw, h.data(), bytes, cudaMemcpyHostToDevice));
+  FS_FFT_SWITCH(c->nz, z_attr);
   FS_FFT_SWITCH(c->ny, y_attr);
   return FS_OK;
 }
@@ -799,14 +727,14 @@ fs_status fft32_flow_solve(fs_ctx *c) {
     ProfScope ps(c, FS_STAGE_FFT_FWD);
     {
       ProfScope pk(c, FS_STAGE_K_FFT_Z_FWD);
-      FS_FFT_SWITCH_Z(c->nz, z_fwd, c, g, A, tw);
+      FS_FFT_SWITCH(c->nz, z_fwd, c, g, A, tw);
     }
     ProfScope pk(c, FS_STAGE_K_FFT_Y_FWD);
     FS_FFT_SWITCH(c->ny, y_fwd, c, A, B, tw);
   }
   {
     ProfScope ps(c, FS_STAGE_PROJECT);
-    FS_FFT_SWITCH(c->nx, x_project, c, B, tw);
+    FS_TRY(x_project(c, B, tw));
   }
   {
     ProfScope ps(c, FS_STAGE_FFT_INV);
@@ -815,7 +743,7 @@ fs_status fft32_flow_solve(fs_ctx *c) {
       FS_FFT_SWITCH(c->ny, y_inv, c, B, A, tw);
     }
     ProfScope pk(c, FS_STAGE_K_FFT_Z_INV);
-    FS_FFT_SWITCH_Z(c->nz, z_inv, c, A, g, tw);
+    FS_FFT_SWITCH(c->nz, z_inv, c, A, g, tw);
   }
   return FS_OK;
 }

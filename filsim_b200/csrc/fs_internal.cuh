@@ -277,7 +277,6 @@ fs_status lines_prepare32(fs_ctx *c);
 fs_status lines_flow_solve64(fs_ctx *c);
 fs_status lines_flow_solve32(fs_ctx *c);
 
-bool fft32_supported(const fs_ctx *c);
 bool fft32_preferred(const fs_ctx *c);  // FP32: the warp transform rather than the line transforms
 fs_status fft32_init(fs_ctx *c);
 void fft32_free(fs_ctx *c);

@@ -814,8 +814,12 @@ fs_status lines_prepare_t(fs_ctx *c) {
 // holds the half spectrum
 template <typename T>
 fs_status lines_flow_solve_t(fs_ctx *c) {
-  // the single-kernel stages stand for FP32 grids of 2^p and 3 2^p lengths (filsim_gpu.h)
-  const bool kernel_stages = !Num<T>::IS_DOUBLE && fft32_supported(c);
+  // the single-kernel stages are recorded in FP32 on these grids only (filsim_gpu.h)
+  auto timed = [](int n, int from) {
+    const int odd = n / (n & -n);
+    return odd == 1 ? n >= from : odd == 3 && n >= 96;
+  };
+  const bool kernel_stages = !Num<T>::IS_DOUBLE && timed(c->nx, 32) && timed(c->ny, 32) && timed(c->nz, 64);
   const int prec = Num<T>::IS_DOUBLE ? FS_PREC_FP64 : FS_PREC_FP32;
   const V16 *twx = (const V16 *)c->line_tw[prec][0], *twy = (const V16 *)c->line_tw[prec][1],
             *twz = (const V16 *)c->line_tw[prec][2];

@@ -406,6 +406,7 @@ enum {
   FS_STAGE_LEARN = 13,      /* warm-start features + MLP inference, and MLP training steps */
   /* single kernels inside the stages above (their time also counts there) */
   FS_STAGE_K_SPREAD = 14,   /* the force-distribution kernel alone (no binning or records) */
+  /* FP32 transforms of either kind, on grids of 2^p (z from 64) or 3 2^p >= 96 points per axis */
   FS_STAGE_K_FFT_Z_FWD = 15, /* FP32 transform: the forward pass over z lines */
   FS_STAGE_K_FFT_Y_FWD = 16, /* FP32 transform: the forward pass over y lines */
   FS_STAGE_K_FFT_Y_INV = 17, /* FP32 transform: the inverse pass over y lines */

@@ -26,7 +26,7 @@ NEW = [n for n in RULE if n not in TESTED]  # the others are solved in test_gpu_
 
 
 def kernels(call):
-    with profile(activities=[ProfilerActivity.CUDA]) as p:
+    with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as p:
         call()
         torch.cuda.synchronize()
     names = [e.key for e in p.key_averages()]

@@ -1203,6 +1203,12 @@ fs_status spread_t(fs_ctx *c, const FcmConsts &k, const double *Y, const double 
 // warps an SM is given before beads stop being split over several
 #define FS_INTERP_WARPS 20
 
+int interp_split(const fs_ctx *c, int np) {
+  const int warps = FS_INTERP_WARPS * c->num_sms;
+  return 4 * np <= warps ? 4 : 2 * np <= warps ? 2 : 1;
+}
+bool interp_single(const fs_ctx *c) { return c->nz < c->p.ngd + 6; }  // FP32: k_interp_q's SINGLE
+
 // interpolation of U, Omega from the velocity grid in c->grid_real (R precision); the
 // beads must have been binned (bin_t) at this precision
 template <typename R>
@@ -1210,10 +1216,9 @@ fs_status interp_t(fs_ctx *c, const FcmConsts &k, double *V, double *W, int np) 
   if (np <= 0) return FS_OK;
   ProfScope ps(c, FS_STAGE_INTERP);
   ProfScope pk(c, FS_STAGE_K_INTERP);
-  const int sms = FS_INTERP_WARPS * c->num_sms;
-  const int split = 4 * np <= sms ? 4 : 2 * np <= sms ? 2 : 1;
+  const int split = interp_split(c, np);
   const size_t wb = sizeof(R) == 4 ? interp_q_warp_bytes(k.ngd) : 0;  // dynamic shared memory per bead of a CTA
-  const bool single = sizeof(R) == 4 && k.N[2] < k.ngd + 6;
+  const bool single = sizeof(R) == 4 && interp_single(c);
   const int wpb = split > 1 || single ? 4 : (c->tune_interp_wpb == 16 && 16 * wb > FS_SMEM_MAX) ? 8 : c->tune_interp_wpb;
 #define FS_INTERP_LAUNCH(WPB, SPLIT, SINGLE)                                                                     \
   if constexpr (sizeof(R) == 4)                                                                                  \
@@ -1330,6 +1335,10 @@ void fcm_free(fs_ctx *c) {
   c->bead_sw = nullptr;
   cudaFree(c->bead_rec);
   c->bead_rec = nullptr;
+}
+
+bool fcm_interp_wpb_used(const fs_ctx *c, int np) {
+  return interp_split(c, np) == 1 && !(c->precision == FS_PREC_FP32 && interp_single(c));
 }
 
 fs_status fcm_set_stream(fs_ctx *c, cudaStream_t st) {

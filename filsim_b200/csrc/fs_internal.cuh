@@ -70,13 +70,13 @@ struct fs_ctx {
   int *bead_sw;        // per bead, wrapped Gaussian stencil start per axis
   void *bead_rec;      // per sorted bead: stencil starts, F, T/2 and Gaussian weights (FP64 or FP32 record)
   int last_grid_prec;  // precision of the grids from the last solve (-1: none)
-  int tune_spread_chunk;  // beads staged per spread pass: 32 or 64 (fs_autotune)
+  int tune_spread_chunk;  // FP32 spread: beads staged per pass, 32 or 64 (fs_autotune)
   int tune_spread_cols;   // FP32 spread: x width of a warp's column block (2, 4 or 8)
   int tune_interp_wpb;    // beads (warps) per interpolation CTA: 4, 8 or 16
   int tune_fft32;         // FP32 grids: 0 own transform where there is one (fs_lines.cuh, fs_fft.cu), 1 cuFFT
   bool line_ready[2];   // [precision]: the line kernels' attributes are set
   void *line_tw[2][3];  // [precision][axis]: tables of the line transforms (fs_lines.cuh; null: not a supported grid)
-  void *fft_tw;        // twiddle tables of the FP32 warp transform (null: grid not handled by fs_fft.cu)
+  void *fft_tw;        // twiddle tables of the FP32 warp transform (null: not a grid of fft32_preferred)
 
   // collision cells
   int M[3], ncell;
@@ -249,6 +249,7 @@ void fcm_free(fs_ctx *c);
 fs_status fcm_mobility(fs_ctx *c, const double *Y, const double *F, const double *T, double *V, double *W, int np);
 fs_status fcm_friction(fs_ctx *c, const double *F, const double *T, double *V, double *W, int np);
 fs_status fcm_flow_solve_only(fs_ctx *c, const double *f, double *u);
+bool fcm_interp_wpb_used(const fs_ctx *c, int np);  // the solves of np beads read tune_interp_wpb
 fs_status fcm_spread_only(fs_ctx *c, const double *Y, const double *F, const double *T, int np, double *f);
 fs_status fcm_interpolate_only(fs_ctx *c, const double *u, const double *Y, int np, double *V, double *W);
 void slab_free(fs_ctx *c);

@@ -2,12 +2,13 @@
 // the fastest combination of the FCM launch variants, timed on the device with
 // the context's own beads. No reference counterpart.
 //
-// Knobs: beads staged per spread pass (32 or 64; the 16^3 tile is fixed by the
-// binning), beads per interpolation CTA (4, 8 or 16 warps), on FP32
-// power-of-two grids the transform (the five-pass warp FFT of fs_fft.cu or
-// cuFFT), and the shape of a warp's column block in the FP32 spread tile
-// (x width 2, 4 or 8: 2 x 16 x 8, 4 x 16 x 4 or 8 x 16 x 2 points). A captured
-// step graph bakes the launch shapes, so tuning invalidates it.
+// Knobs: beads staged per pass of the FP32 spread (32 or 64; the 16^3 tile is fixed by the
+// binning), beads per interpolation CTA (4, 8 or 16 warps), on FP32 grids that have a transform
+// of this library (fs_lines.cuh, fs_fft.cu) that one or cuFFT, and the shape of a warp's column
+// block in the FP32 spread tile (x width 2, 4 or 8: 2 x 16 x 8, 4 x 16 x 4 or 8 x 16 x 2 points). A
+// knob that this suspension's solves do not read keeps its value: the spread's two in FP64, the
+// interpolation's where beads are split over warps. A captured step graph bakes the launch
+// shapes, so tuning invalidates it.
 #include "fs_internal.cuh"
 
 extern "C" {
@@ -33,16 +34,17 @@ fs_status fs_autotune(fs_ctx *c, int reps, int *choice_h, float *best_ms_h) {
   cudaEvent_t e0, e1;
   FS_CUDA(cudaEventCreate(&e0));
   FS_CUDA(cudaEventCreate(&e1));
-  const int ffts = (c->precision == FS_PREC_FP32 && c->fft_tw) ? 2 : 1;
+  const bool f32 = c->precision == FS_PREC_FP32, wpb_used = fcm_interp_wpb_used(c, c->np);
   float best = 1e30f;
-  // the column shape only changes the FP32 spread (FP64 keeps the current one)
-  const bool f32 = c->precision == FS_PREC_FP32;
-  const int cx_lo = f32 ? 2 : c->tune_spread_cols, cx_hi = f32 ? 8 : c->tune_spread_cols;
-  int bch = 64, bwpb = 8, bfft = 0, bcx = c->tune_spread_cols;
+  int bch = c->tune_spread_chunk, bwpb = c->tune_interp_wpb, bfft = c->tune_fft32, bcx = c->tune_spread_cols;
+  const int ch_lo = f32 ? 32 : bch, ch_hi = f32 ? 64 : bch, wpb_lo = wpb_used ? 4 : bwpb, wpb_hi = wpb_used ? 16 : bwpb;
+  const int cx_lo = f32 ? 2 : bcx, cx_hi = f32 ? 8 : bcx;
+  const bool two = f32 && c->line_tw[FS_PREC_FP32][0];
+  const int fft_lo = two ? 0 : bfft, fft_hi = two ? 1 : bfft;
   fs_status st = FS_OK;
-  for (int ch = 32; ch <= 64 && st == FS_OK; ch *= 2)
-    for (int wpb = 4; wpb <= 16 && st == FS_OK; wpb *= 2)
-      for (int fft = 0; fft < ffts && st == FS_OK; ++fft)
+  for (int ch = ch_lo; ch <= ch_hi && st == FS_OK; ch *= 2)
+    for (int wpb = wpb_lo; wpb <= wpb_hi && st == FS_OK; wpb *= 2)
+      for (int fft = fft_lo; fft <= fft_hi && st == FS_OK; ++fft)
         for (int cx = cx_lo; cx <= cx_hi && st == FS_OK; cx *= 2) {
         c->tune_spread_chunk = ch;
         c->tune_spread_cols = cx;

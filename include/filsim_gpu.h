@@ -360,8 +360,8 @@ fs_status fs_get_diag(fs_ctx *ctx, fs_diag *d_h);
 fs_status fs_set_graph_mode(fs_ctx *ctx, int on);
 
 /* ---- autotuner (no reference counterpart) -----------------------------------
- * choice = {beads staged per spread pass (32 | 64), beads per interpolation CTA
- * (4 | 8 | 16), FP32 grids of 2^p or 3 2^p points: 0 own transform | 1 cuFFT, FP32 spread: x
+ * choice = {FP32 spread: beads staged per pass (32 | 64), beads per interpolation CTA
+ * (4 | 8 | 16), FP32 grids: 0 this library's transform where it has one | 1 cuFFT, FP32 spread: x
  * width of a warp's column block in the 16^3 tile (2 | 4 | 8; the block is
  * w x 16 x 16/w points)}: four ints. fs_autotune times every combination on the
  * uploaded suspension (reps mobility solves each, after one warm-up) and keeps

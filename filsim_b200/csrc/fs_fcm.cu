@@ -773,7 +773,11 @@ struct InterpWarp64 {
   double yg[FS_NGD_MAX], yd[FS_NGD_MAX], yr[FS_NGD_MAX];
   long long xoff[FS_NGD_MAX];
 };
-template <int WPB, int SPLIT>
+// MASK (velocities that a caller gives): the pair's point off the run is dropped from the sums and
+// not only given a weight of zero, which would not do where it is no finite number. After a
+// solve, whose velocities are finite all or none, it would only cost (a bead's warps at 20
+// points 76 -> 132 us for 1,480 beads).
+template <int WPB, int SPLIT, bool MASK>
 __global__ void __launch_bounds__(32 * WPB) k_interp64(const double *__restrict__ u, const double4 *__restrict__ rec,
                                                        int np, FcmConsts c, double *__restrict__ V,
                                                        double *__restrict__ W) {
@@ -847,18 +851,18 @@ __global__ void __launch_bounds__(32 * WPB) k_interp64(const double *__restrict_
         add(Sr[0], wr, u1);
         add(Sr[1], wr, u2);
       }
-      // the pair's point off the run counts for nothing, also where it is no finite number
-      auto drop = [&](double2 &t) {
-        if (!in[0]) t.x = 0.0;
-        if (!in[1]) t.y = 0.0;
-      };
+      if constexpr (MASK) {
+        auto drop = [&](double2 &t) {
+          if (!in[0]) t.x = 0.0;
+          if (!in[1]) t.y = 0.0;
+        };
 #pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        drop(Sg[a]);
-        drop(Sd[a]);
+        for (int a = 0; a < 3; ++a) {
+          drop(Sg[a]);
+          drop(Sd[a]);
+          if (a < 2) drop(Sr[a]);
+        }
       }
-      drop(Sr[0]);
-      drop(Sr[1]);
       const double yg = s.yg[j], yd = s.yd[j], yr = s.yr[j];
 #pragma unroll
       for (int a = 0; a < 3; ++a) acc[a] += yg * (gz[0] * Sg[a].x + gz[1] * Sg[a].y);
@@ -1210,28 +1214,29 @@ int interp_split(const fs_ctx *c, int np) {
 bool interp_single(const fs_ctx *c) { return c->nz < c->p.ngd + 6; }  // FP32: k_interp_q's SINGLE
 
 // interpolation of U, Omega from the velocity grid in c->grid_real (R precision); the
-// beads must have been binned (bin_t) at this precision
+// beads must have been binned (bin_t) at this precision. given: the grid is a caller's
 template <typename R>
-fs_status interp_t(fs_ctx *c, const FcmConsts &k, double *V, double *W, int np) {
+fs_status interp_t(fs_ctx *c, const FcmConsts &k, double *V, double *W, int np, bool given) {
   if (np <= 0) return FS_OK;
   ProfScope ps(c, FS_STAGE_INTERP);
   ProfScope pk(c, FS_STAGE_K_INTERP);
   const int split = interp_split(c, np);
   const size_t wb = sizeof(R) == 4 ? interp_q_warp_bytes(k.ngd) : 0;  // dynamic shared memory per bead of a CTA
-  const bool single = sizeof(R) == 4 && interp_single(c);
-  const int wpb = split > 1 || single ? 4 : (c->tune_interp_wpb == 16 && 16 * wb > FS_SMEM_MAX) ? 8 : c->tune_interp_wpb;
-#define FS_INTERP_LAUNCH(WPB, SPLIT, SINGLE)                                                                     \
-  if constexpr (sizeof(R) == 4)                                                                                  \
-    fs_launch(k_interp_q<WPB, SPLIT, SINGLE>, fs_blocks(np, WPB / SPLIT), 32 * WPB, WPB / SPLIT * wb, c->stream, \
-              (const float *)c->grid_real, (const float4 *)c->bead_rec, np, k, V, W);                            \
-  else                                                                                                           \
-    fs_launch(k_interp64<WPB, SPLIT>, fs_blocks(np, WPB / SPLIT), 32 * WPB, 0, c->stream,                        \
+  // the forms for single points (FP32) and with MASK (FP64) exist with four warps
+  const bool other = sizeof(R) == 4 ? interp_single(c) : given;
+  const int wpb = split > 1 || other ? 4 : (c->tune_interp_wpb == 16 && 16 * wb > FS_SMEM_MAX) ? 8 : c->tune_interp_wpb;
+#define FS_INTERP_LAUNCH(WPB, SPLIT, OTHER)                                                                     \
+  if constexpr (sizeof(R) == 4)                                                                                 \
+    fs_launch(k_interp_q<WPB, SPLIT, OTHER>, fs_blocks(np, WPB / SPLIT), 32 * WPB, WPB / SPLIT * wb, c->stream, \
+              (const float *)c->grid_real, (const float4 *)c->bead_rec, np, k, V, W);                           \
+  else                                                                                                          \
+    fs_launch(k_interp64<WPB, SPLIT, OTHER>, fs_blocks(np, WPB / SPLIT), 32 * WPB, 0, c->stream,                \
               (const double *)c->grid_real, (const double4 *)c->bead_rec, np, k, V, W)
-  if (single && split == 4) {
+  if (other && split == 4) {
     FS_INTERP_LAUNCH(4, 4, true);
-  } else if (single && split == 2) {
+  } else if (other && split == 2) {
     FS_INTERP_LAUNCH(4, 2, true);
-  } else if (single) {
+  } else if (other) {
     FS_INTERP_LAUNCH(4, 1, true);
   } else if (split == 4) {
     FS_INTERP_LAUNCH(4, 4, false);
@@ -1257,7 +1262,7 @@ fs_status mobility_t(fs_ctx *c, const double *Y, const double *F, const double *
     FS_TRY(spread_t<R>(c, k, Y, F, T, np));
   }
   FS_TRY(flow_solve_t<R>(c));
-  FS_TRY(interp_t<R>(c, k, V, W, np));
+  FS_TRY(interp_t<R>(c, k, V, W, np, false));
   c->last_grid_prec = sizeof(R) == 8 ? FS_PREC_FP64 : FS_PREC_FP32;
   return FS_OK;
 }
@@ -1375,10 +1380,10 @@ fs_status fcm_interpolate_only(fs_ctx *c, const double *u, const double *Y, int 
   if (c->precision == FS_PREC_FP32) {
     k_convert<double, float><<<fs_blocks((long long)n, 256), 256, 0, c->stream>>>(u, (float *)c->grid_real, n);
     FS_LAUNCH_CHECK();
-    FS_TRY(interp_t<float>(c, k, V, W, np));
+    FS_TRY(interp_t<float>(c, k, V, W, np, true));
   } else {
     FS_CUDA(cudaMemcpyAsync(c->grid_real, u, sizeof(double) * n, cudaMemcpyDeviceToDevice, c->stream));
-    FS_TRY(interp_t<double>(c, k, V, W, np));
+    FS_TRY(interp_t<double>(c, k, V, W, np, true));
   }
   c->last_grid_prec = -1;
   return FS_OK;

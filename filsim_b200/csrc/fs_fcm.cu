@@ -421,8 +421,12 @@ struct SpreadStage32 {
 //   8 warps, 2 passes   27    35    27    36        86            226      992
 //   4 warps, 4 passes   53    68    47    57       121            254      909
 // so quarter tiles below one tile per SM, then half tiles; the list is made once for a whole
-// tile where there are many CTAs and few beads in each, and by four warps only if it also
-// fits one stage (4,096 tiles with twice the beads: half 306, whole 313).
+// tile where the CTAs are enough without a split and a tile's beads few (half / whole: 384 tiles
+// reached by 10, 27 and 40 beads 22 / 18, 30 / 30, 35 / 42; 1,000 tiles 41 / 32, 54 / 51, 68 / 72; 1,584
+// 56 / 40, 78 / 69, 97 / 99; 4,096 by 40 and 60 236 / 236, 333 / 339), and by four warps, which fit
+// an SM more often, where the beads fit one stage and the CTAs many waves (whole / by four
+// warps: 1,584 tiles reached by 4 and 10 beads 34 / 30, 40 / 40; 4,096 by 10 and 20 95 / 83, 130 /
+// 134; 8,000 by 20 and 27 237 / 223, 296 / 295; 21,952 by 27 and 40 780 / 752, 1,200 / 1,292).
 template <int CH, int CX, int NW, int PASSES>
 __global__ void __launch_bounds__(32 * NW, NW == 4 && PASSES == 4 ? 6 : 3)
     k_spread32(const int *__restrict__ bin_start, const float4 *__restrict__ rec, FcmConsts c,
@@ -1161,8 +1165,9 @@ fs_status spread_t(fs_ctx *c, const FcmConsts &k, const double *Y, const double 
     const float4 *rec = (const float4 *)c->bead_rec;
     // beads whose stencil reaches a tile, if they lie evenly
     const double e = (k.ngd + FS_TILE - 1) / (double)FS_TILE, reach = (double)np / c->nbins * (e * e * e);
-    const bool quarter = c->nbins < c->num_sms, sparse = c->nbins >= 8192 && reach <= 28,
-               whole = c->nbins >= 10 * c->num_sms && reach <= 48;
+    const int per_sm = c->nbins / c->num_sms;
+    const bool quarter = per_sm < 1, sparse = (reach <= 12 && per_sm >= 10) || (reach <= 28 && per_sm >= 40),
+               whole = reach <= (per_sm >= 10 ? 48 : 24) && per_sm >= 2;
 #define FS_SPREAD32_LAUNCH1(CHV, CXV, NWV, PV)                                                                    \
   {                                                                                                               \
     constexpr size_t bytes = sizeof(SpreadStage32<CHV>);                                                          \

@@ -1209,11 +1209,16 @@ fs_status spread_t(fs_ctx *c, const FcmConsts &k, const double *Y, const double 
   return FS_OK;
 }
 
-// warps an SM is given before beads stop being split over several
-#define FS_INTERP_WARPS 20
-
-int interp_split(const fs_ctx *c, int np) {
-  const int warps = FS_INTERP_WARPS * c->num_sms;
+// Warps a bead is split over. FP64 (16 warps an SM): four up to 4 beads per SM, two up to 8
+// (four / two / one warp, 256^3, 12 points: 592 beads 21 / 23 / 23 us, 740 29 / 25 / 25, 1,000 34 / 27 /
+// 28, 1,480 44 / 40 / 34). FP32, short stencils (27 warps an SM): four up to 6.75, two up to 13.5 (740
+// beads 17 / 21 / 27, 1,000 20 / 23 / 29, 1,480 27 / 25 / 32, 2,000 29 / 29 / 34, 2,960 37 / 39 / 38). From 15
+// points on a bead's FP32 tables, which its warps share, leave an SM less than 40 warps of whole
+// beads, so beads are always split (256^3, 20 points: 1,480 beads 55 / 60 / 101, 6,000 104 / 117 / 216,
+// 12,000 179 / 184 / 277, 100,000 1,305 / 1,272 / 1,512).
+int interp_split(const fs_ctx *c, int prec, int np) {
+  if (prec == FS_PREC_FP32 && c->p.ngd >= 15) return np <= 40 * c->num_sms ? 4 : 2;
+  const int warps = (prec == FS_PREC_FP32 ? 27 : 16) * c->num_sms;
   return 4 * np <= warps ? 4 : 2 * np <= warps ? 2 : 1;
 }
 bool interp_single(const fs_ctx *c) { return c->nz < c->p.ngd + 6; }  // FP32: k_interp_q's SINGLE
@@ -1225,7 +1230,7 @@ fs_status interp_t(fs_ctx *c, const FcmConsts &k, double *V, double *W, int np, 
   if (np <= 0) return FS_OK;
   ProfScope ps(c, FS_STAGE_INTERP);
   ProfScope pk(c, FS_STAGE_K_INTERP);
-  const int split = interp_split(c, np);
+  const int split = interp_split(c, sizeof(R) == 4 ? FS_PREC_FP32 : FS_PREC_FP64, np);
   const size_t wb = sizeof(R) == 4 ? interp_q_warp_bytes(k.ngd) : 0;  // dynamic shared memory per bead of a CTA
   // the forms for single points (FP32) and with MASK (FP64) exist with four warps
   const bool other = sizeof(R) == 4 ? interp_single(c) : given;
@@ -1348,7 +1353,7 @@ void fcm_free(fs_ctx *c) {
 }
 
 bool fcm_interp_wpb_used(const fs_ctx *c, int np) {
-  return interp_split(c, np) == 1 && !(c->precision == FS_PREC_FP32 && interp_single(c));
+  return interp_split(c, c->precision, np) == 1 && !(c->precision == FS_PREC_FP32 && interp_single(c));
 }
 
 fs_status fcm_set_stream(fs_ctx *c, cudaStream_t st) {

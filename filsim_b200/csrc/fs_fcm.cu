@@ -421,12 +421,13 @@ struct SpreadStage32 {
 //   8 warps, 2 passes   27    35    27    36        86            226      992
 //   4 warps, 4 passes   53    68    47    57       121            254      909
 // so quarter tiles below one tile per SM, then half tiles; the list is made once for a whole
-// tile where the CTAs are enough without a split and a tile's beads few (half / whole: 384 tiles
-// reached by 10, 27 and 40 beads 22 / 18, 30 / 30, 35 / 42; 1,000 tiles 41 / 32, 54 / 51, 68 / 72; 1,584
-// 56 / 40, 78 / 69, 97 / 99; 4,096 by 40 and 60 236 / 236, 333 / 339), and by four warps, which fit
-// an SM more often, where the beads fit one stage and the CTAs many waves (whole / by four
-// warps: 1,584 tiles reached by 4 and 10 beads 34 / 30, 40 / 40; 4,096 by 10 and 20 95 / 83, 130 /
-// 134; 8,000 by 20 and 27 237 / 223, 296 / 295; 21,952 by 27 and 40 780 / 752, 1,200 / 1,292).
+// tile where the CTAs are enough without a split and a tile's beads few (half / whole: 343 tiles
+// reached by 22 beads 25 / 28; 384 by 10, 20 and 27 22 / 18, 26 / 24, 30 / 30; 1,000 by 10, 27 and 40
+// 41 / 32, 54 / 51, 68 / 72; 1,584 by 10, 27 and 40 56 / 40, 78 / 69, 97 / 99; 4,096 by 40 and 60
+// 236 / 236, 333 / 339), and by four warps, which fit an SM more often, where the beads fit one
+// stage and the CTAs are many waves (whole / by four warps: 1,584 tiles reached by 4 and 10 beads
+// 34 / 30, 40 / 40; 4,096 by 10 and 20 95 / 83, 130 / 134; 8,000 by 20 and 27 237 / 223, 296 / 295;
+// 21,952 by 27 and 40 780 / 752, 1,200 / 1,292).
 template <int CH, int CX, int NW, int PASSES>
 __global__ void __launch_bounds__(32 * NW, NW == 4 && PASSES == 4 ? 6 : 3)
     k_spread32(const int *__restrict__ bin_start, const float4 *__restrict__ rec, FcmConsts c,
@@ -1167,7 +1168,7 @@ fs_status spread_t(fs_ctx *c, const FcmConsts &k, const double *Y, const double 
     const double e = (k.ngd + FS_TILE - 1) / (double)FS_TILE, reach = (double)np / c->nbins * (e * e * e);
     const int per_sm = c->nbins / c->num_sms;
     const bool quarter = per_sm < 1, sparse = (reach <= 12 && per_sm >= 10) || (reach <= 28 && per_sm >= 40),
-               whole = reach <= (per_sm >= 10 ? 48 : 24) && per_sm >= 2;
+               whole = reach <= (per_sm >= 10 ? 48 : 20) && per_sm >= 2;
 #define FS_SPREAD32_LAUNCH1(CHV, CXV, NWV, PV)                                                                    \
   {                                                                                                               \
     constexpr size_t bytes = sizeof(SpreadStage32<CHV>);                                                          \

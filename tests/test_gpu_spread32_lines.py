@@ -1,5 +1,5 @@
 """The FP32 spread on both sides of the lines between its splits of a tile over CTAs: 2, 10 and 40
-tiles per SM, and 12, 24, 28 and 48 beads reaching a tile, also with clusters that fill several lists.
+tiles per SM, and 12, 20, 28 and 48 beads reaching a tile, also with clusters that fill several lists.
 Against the FP64 spread, with the bar of test_gpu_spread32.py."""
 import numpy as np
 import pytest
@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 
 
 # grids of n x 4 x 4 tiles; 12-point stencils reach (27 / 16)^3 = 4.8 tiles
-@pytest.mark.parametrize("per_sm,reach", [(2, 24), (10, 12), (10, 48), (40, 28)])
+@pytest.mark.parametrize("per_sm,reach", [(2, 20), (10, 12), (10, 48), (40, 28)])
 @pytest.mark.parametrize("more_tiles", [False, True])
 @pytest.mark.parametrize("more_beads", [False, True])
 @pytest.mark.parametrize("clump", [1.0, 0.08])

@@ -194,11 +194,14 @@ extern unsigned long long g_fs_kernel_launches;
 // Launches with programmatic stream serialization: the kernel may be placed on the SMs while
 // the one before it in the stream still runs, and does nothing until FS_AFTER_PREVIOUS, its
 // first statement, has waited for that kernel's end and its memory. In a chain of short
-// kernels this takes the launch latency out of the chain: a solve at 64^3 90 -> 81 us on the
-// host's clock, 384 x 96 x 96 408 -> 389, three steps at 64^3 2,786 -> 2,276, an MLP
-// gradient and forward pass 461 -> 399. Plain launches stay where a kernel's CTAs would crowd
-// the SMs that the one before leaves free (k_jacobian_factor) and for the warp transform of the
-// largest grids (fs_fft.cu: a 512^3 solve 4.99 ms so, 5.5 with it).
+// kernels this takes the launch latency out of the chain (host's clock, plain and so): a solve at
+// 64^3 74 and 66 us in FP64, 69 and 60 in FP32, at 48^3 in FP32 65 and 49; when it came in, three
+// steps at 64^3 2,786 and 2,276, an MLP gradient and forward pass 461 and 399. Plain launches stay
+// where a kernel's CTAs would crowd the SMs that the one before leaves free (k_jacobian_factor),
+// where they would inherit an SM's split of L1 and shared memory from large ones (the y inverse
+// after long x lines, fs_lines.cuh, and through it the rest of a solve), where the wait outweighs a
+// CTA's work (k_convert) and for the warp transform of the largest grids (fs_fft.cu: a 512^3 solve
+// 4.99 ms so, 5.5 with it).
 template <typename... P, typename... A>
 inline void fs_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... a) {
   cudaLaunchConfig_t cfg = {};

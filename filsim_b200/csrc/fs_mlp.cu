@@ -1091,7 +1091,8 @@ fs_status fs_mlp_gradients(fs_ctx *c, const float *features_d, const float *targ
   FS_TRY(forward(c, n, nullptr));
   FS_TRY(backward(c, targets_d, n));
   // through pinned memory, the copy to the caller's array overlapping the next chunk's
-  // transfer: 459,000 gradients, 550 us a call with pageable copies of each result, 409 so
+  // transfer: 459,000 gradients, 550 us a call with pageable copies of each result, 409 so (368
+  // into an array that the caller has not zeroed first, as the Python binding's)
   const size_t np = param_count(m);
   float *hg = (float *)m->host;
   struct Tail {

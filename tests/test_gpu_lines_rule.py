@@ -2,6 +2,8 @@
 and 7 (line_length, fs_internal.cuh). Every such length on every axis runs the line transforms and
 none runs cuFFT, shown by the kernels that ran, and solves as a PyTorch FP64 flow solve does, with the
 bars of test_gpu_lines.py; a length off the rule on one axis leaves the grid to cuFFT."""
+import time
+
 import pytest
 import torch
 from torch.profiler import ProfilerActivity, profile
@@ -26,13 +28,25 @@ NEW = [n for n in RULE if n not in TESTED]  # the others are solved in test_gpu_
 
 
 def kernels(call):
+    """Names of the kernels that call() launches, run twice with pauses around it: the tracer may drop
+    what runs close to the ends of its window."""
     with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as p:
-        call()
-        torch.cuda.synchronize()
+        for _ in range(2):
+            time.sleep(0.02)
+            call()
+            torch.cuda.synchronize()
+        time.sleep(0.02)
     names = [e.key for e in p.key_averages()]
     if not any("k_" in k or "fft" in k for k in names):
         pytest.skip("no kernel is traced on this machine")
     return names
+
+
+def route(names):
+    """The transform that ran."""
+    found = {r for r, mark in (("lines", "k_lines_"), ("warp", "k_fft_"), ("cufft", "k_project")) if any(mark in k for k in names)}
+    assert len(found) == 1, names
+    return found.pop()
 
 
 @pytest.mark.parametrize("n", RULE)
@@ -45,16 +59,15 @@ def test_every_length_runs_the_lines(gpu_lib, n, axis):
     f = torch.zeros([3] + dims, dtype=torch.float64, device="cuda")
     for prec in (abi.FS_PREC_FP64, abi.FS_PREC_FP32):
         ctx.set_precision(prec)
-        names = kernels(lambda: fcm.flow_solve(f))
-        assert sum("k_lines_" in k for k in names) == 5, names
+        assert route(kernels(lambda: fcm.flow_solve(f))) == "lines"
     ctx.close()
 
 
 @pytest.mark.parametrize("dims", [(16, 32, 32), (32, 176, 32), (32, 32, 272)])
 def test_other_lengths_do_not(gpu_lib, dims):
     ctx = Context(params_for(dims), max_beads=1)
-    names = kernels(lambda: Fcm(ctx, 1).flow_solve(torch.zeros((3,) + dims, dtype=torch.float64, device="cuda")))
-    assert not any("k_lines_" in k for k in names) and any("k_project" in k for k in names), names
+    f = torch.zeros((3,) + dims, dtype=torch.float64, device="cuda")
+    assert route(kernels(lambda: Fcm(ctx, 1).flow_solve(f))) == "cufft"
     ctx.close()
 
 

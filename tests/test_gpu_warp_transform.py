@@ -11,7 +11,7 @@ from filsim_b200 import abi
 from filsim_b200.configs import params_for
 from filsim_b200.fcm import Context, Fcm
 from test_gpu_lines import flow_solve
-from test_gpu_lines_rule import kernels
+from test_gpu_lines_rule import kernels, route
 
 pytestmark = pytest.mark.gpu
 
@@ -34,12 +34,11 @@ def test_matches_fp64(gpu_lib, dims):
             assert float((ref - exact).abs().max() / exact.abs().max()) < 1e-12
             del exact
         ctx.set_precision(abi.FS_PREC_FP32)
-        out = []
-        names = kernels(lambda: out.append(fcm.flow_solve(f))) if kind == "noise" else None
-        assert names is None or sum("k_fft_" in k for k in names) == 5 and not any("k_lines_" in k for k in names)
-        u = out[0] if out else fcm.flow_solve(f)
+        if kind == "noise":
+            assert route(kernels(lambda: fcm.flow_solve(f))) == "warp"
+        u = fcm.flow_solve(f)
         assert float((u - ref).abs().max() / ref.abs().max()) < 1e-5, kind
-        del f, u, ref, out
+        del f, u, ref
     ones = torch.full_like(noise, 3.0)
     # the zero mode is dropped; what the transforms leave of it is rounding of the force over the
     # smallest q^2

@@ -1197,8 +1197,8 @@ fs_status spread_t(fs_ctx *c, const FcmConsts &k, const double *Y, const double 
     const double4 *rec = (const double4 *)c->bead_rec;
     double *f = (double *)c->grid_real;
     // half tiles, or quarter tiles where the half tiles would not fill the SMs three times
-    // (before the FMA chains 64^3 21 us against 28; half tiles 256^3 301 against 308, 512^3 1.63
-    // against 1.77 ms)
+    // (quarter / half, us, tiles reached by 10 and 27 beads: 64 tiles 12 / 15, 14 / 17; 216 19 / 16, 23 /
+    // 25; 343 23 / 23, 30 / 32; 512 30 / 28, 39 / 39; 4,096 181 / 161, 247 / 229)
     if (2 * c->nbins < 3 * c->num_sms)
       fs_launch(k_spread64<4>, 4 * c->nbins, FS_SPREAD64_THREADS, sizeof(SpreadStage64<4>), c->stream, c->bins.start,
                 rec, k, f);
